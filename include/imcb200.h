@@ -126,7 +126,10 @@ typedef struct imc_step_params {
   int32_t chunk;                /* histories claimed per warp ticket (guided: at most this) */
   int32_t reserved;             /* bit 0: shared-memory cell table (default: up to 4096 (group, cell)
                                    entries); bit 1: per-block tallies in shared memory with that
-                                   table, bit 2: never (default: up to 2048 entries); bit 3:
+                                   table (default: up to 2048 entries), bit 2: none, the wide
+                                   blocks' below included; larger meshes run one wide block per SM
+                                   (as many threads as block_size x blocks_per_sm, at most 1024)
+                                   with its tally in shared memory while that fits; bit 3:
                                    event-by-event tracking (workspace of imc_workspace_bytes_event);
                                    bit 4: prefetched refills (each lane copies its next history's
                                    bank record into shared memory while it tracks the current one;

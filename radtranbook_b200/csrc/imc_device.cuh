@@ -113,15 +113,33 @@ __device__ __forceinline__ float scatter_distance(float ss, float L, uint32_t x,
   return BIGF;
 }
 
+// Whether a scatter at -log(u)/sigma, u = u01(x), can come before s_other.  With p = 1 - u
+// (exact in FP32, at least 2^-24) the scatter is at least p/sigma away, so p >= sigma s_other
+// (1 + 1e-6) rules it out whatever the rounding of the logarithm and the quotient; that
+// settles nearly every flight of a thin cell.  What is left is tested in FP64 with a short
+// series of exp(-sigma s_other) when sigma s_other is small, so that the logarithm is
+// evaluated only when it can win.
+__device__ __forceinline__ bool scatter_may_win(uint32_t x, float sig, float s_other) {
+  if (1.0f - u01f(x) >= sig * s_other * 1.000001f) return false;
+  const double t = (double)sig * (double)s_other;
+  if (!(t < 0.01)) return true;
+  const double thr = 1.0 - t * (1.0 - t * (0.5 - t * (1.0 / 6.0)));
+  return u01d(x) > thr;
+}
+
 struct Ev {
   float d;       // path length of this event
   int evt;       // EV_*
   int cross;     // X_*
 };
 
+// The tracking's approximate quotient and reciprocal square root.
+__device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
+__device__ __forceinline__ float frsqrt(float x) { return rsqrtf(x); }
+
 // ---- 1-D slab: distance to the exit face in the direction of mu ----
 __device__ __forceinline__ float slab_face(float x, float mu, float xl, float xr) {
-  const float db = __fdividef(mu > 0.f ? (xr - x) : (xl - x), mu);
+  const float db = fdiv(mu > 0.f ? (xr - x) : (xl - x), mu);
   return fmaxf(db, 0.f);
 }
 
@@ -129,18 +147,18 @@ __device__ __forceinline__ float slab_face(float x, float mu, float xl, float xr
 // sqrt(x) = x * x^(-1/2): one hardware reciprocal square root and a multiply (a few ulp,
 // against the ~10-instruction correctly rounded sqrtf); 0 for x <= 0.  Tracking is FP32
 // with statistical tolerances, and every kernel that replays a history uses the same form.
-__device__ __forceinline__ float sqrt_nn(float x) { return x > 0.f ? x * rsqrtf(x) : 0.f; }
+__device__ __forceinline__ float sqrt_nn(float x) { return x > 0.f ? x * frsqrt(x) : 0.f; }
 
 __device__ __forceinline__ float outer_root(float r, float mu, float R, float b2) {
   const float q = sqrt_nn(fmaf(R, R, -b2));
-  float l = (mu >= 0.f) ? __fdividef((R - r) * (R + r), fmaxf(fmaf(r, mu, q), 1e-30f)) : q - r * mu;
+  float l = (mu >= 0.f) ? fdiv((R - r) * (R + r), fmaxf(fmaf(r, mu, q), 1e-30f)) : q - r * mu;
   return fmaxf(l, 0.f);
 }
 __device__ __forceinline__ float inner_root(float r, float mu, float R, float b2) {
   if (!(R > 0.f) || !(mu < 0.f)) return BIGF;
   const float disc = fmaf(R, R, -b2);
   if (!(disc > 0.f)) return BIGF;
-  const float l = __fdividef((r - R) * (r + R), disc * rsqrtf(disc) - r * mu);
+  const float l = fdiv((r - R) * (r + R), disc * frsqrt(disc) - r * mu);
   return fmaxf(l, 0.f);
 }
 

@@ -56,9 +56,7 @@ struct EvOut {
   bool flush;      // a cell visit to flush: deposition f_lost, path length f_wd, into flush_cell
   int flush_cell;
   double f_lost, f_wd;
-  bool cen;        // the history ended alive: its weight goes to the comb's census sums
-  int cen_bin;
-  bool finished;
+  bool finished;   // the history ended: history_retire stores its final state
 };
 
 template <int GEOM, bool SMEM_CELLS, bool MG, bool CF>
@@ -81,8 +79,6 @@ __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut
   bool& flush = o.flush;
   int& flush_cell = o.flush_cell;
   double &f_lost = o.f_lost, &f_wd = o.f_wd;
-  bool& cen = o.cen;
-  int& cen_bin = o.cen_bin;
   const int c = ci + a.nx * cj;
   const int cq = MG ? c + a.nc * grp : c;  // (group, cell) table / tally index
   const float sa = tab.x, ss = tab.y;
@@ -114,8 +110,8 @@ __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut
     } else if (GEOM == G_XY) {
       const float xl = E1[ci], xr = E1[ci + 1], yl = E2[cj], yr = E2[cj + 1];
       L = fminf(xr - xl, yr - yl);
-      if (u > 0.f) sx = __fdividef(xr - x, u); else if (u < 0.f) sx = __fdividef(xl - x, u);
-      if (v > 0.f) sy = __fdividef(yr - y, v); else if (v < 0.f) sy = __fdividef(yl - y, v);
+      if (u > 0.f) sx = fdiv(xr - x, u); else if (u < 0.f) sx = fdiv(xl - x, u);
+      if (v > 0.f) sy = fdiv(yr - y, v); else if (v < 0.f) sy = fdiv(yl - y, v);
       sx = fmaxf(sx, 0.f); sy = fmaxf(sy, 0.f);
       sb = fminf(sx, sy);
     } else {
@@ -123,34 +119,28 @@ __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut
       L = fminf(rout - rin, zhi - zlo);
       const float sin2 = (1.f - v) * (1.f + v);
       if (sin2 >= 1e-15f) {
-        const float ist = rsqrtf(sin2);
+        const float ist = frsqrt(sin2);
         st_ = sin2 * ist;
         const float b2 = x * x * ((1.f - u) * (1.f + u));
         s_rout = outer_root(x, u, rout, b2) * ist;
         const float li = inner_root(x, u, rin, b2);
         if (li < BIGF) s_rin = li * ist;
       }
-      if (v > 1e-15f) s_zhi = fmaxf(__fdividef(zhi - y, v), 0.f);
-      else if (v < -1e-15f) s_zlo = fmaxf(__fdividef(zlo - y, v), 0.f);
+      if (v > 1e-15f) s_zhi = fmaxf(fdiv(zhi - y, v), 0.f);
+      else if (v < -1e-15f) s_zlo = fmaxf(fdiv(zlo - y, v), 0.f);
       sb = fminf(fminf(s_rin, s_rout), fminf(s_zlo, s_zhi));
     }
     // ---- effective-scatter distance (reference cap: sigma_s*L > 1e4 -> 1e4/L) ----
-    // -log(u)/sigma competes with s_other = min(boundary, census); when sigma*s_other
-    // is small the scatter loses unless u > exp(-sigma*s_other), tested in FP64 with a
-    // short series, so the logarithm is evaluated only when it can win.
+    // -log(u)/sigma competes with s_other = min(boundary, census); the logarithm is
+    // evaluated only when it can win (scatter_may_win).
     float ds = BIGF;
     {
       const bool capped = !MG2 && ss * L > 10000.0f;
       const float sig = capped ? 10000.0f / L : (ss > ss_thr ? ss : 0.f);
       if (sig > 0.f) {
         const float s_other = fminf(sb, dcen);
-        const double t = (double)sig * (double)s_other;
-        bool may = true;
-        if (t < 0.01) {
-          const double thr = 1.0 - t * (1.0 - t * (0.5 - t * (1.0 / 6.0)));
-          may = u01d(r.x) > thr;
-        }
-        if (may) ds = capped ? neglog_u(r.x) * (L * 1e-4f) : __fdividef(neglog_u(r.x), ss);
+        if (scatter_may_win(r.x, sig, s_other))
+          ds = capped ? neglog_u(r.x) * (L * 1e-4f) : fdiv(neglog_u(r.x), ss);
       }
     }
     d = sb; evt = EV_BOUNDARY;
@@ -197,7 +187,7 @@ __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut
       const float ax = fmaf(u, l, x);
       float rn = sqrt_nn(fmaf(ax, ax, l * l * ((1.f - u) * (1.f + u))));
       yn = fmaf(d, v, y);
-      if (rn > 1e-15f && l > 0.f) un = fminf(1.f, fmaxf(-1.f, __fdividef(fmaf(x, u, l), rn)));
+      if (rn > 1e-15f && l > 0.f) un = fminf(1.f, fmaxf(-1.f, fdiv(fmaf(x, u, l), rn)));
       if (evt == EV_BOUNDARY) {
         if (sb == s_rin) { rn = rin; cross = X_IM; }
         else if (sb == s_rout) { rn = rout; cross = X_IP; }
@@ -229,7 +219,7 @@ __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut
       } else if (a.cf_fastpath > 0.f && tr > 1e-14f && rate * tr > a.cf_fastpath) {
         captured = u01f(ub) < __expf(-rate * tr);
       } else {
-        const float delay = __fdividef(neglog_u(ub), rate);
+        const float delay = fdiv(neglog_u(ub), rate);
         if (ONED ? (tr > 1e-14f && delay < tr) : (delay < tr - 1e-15f)) dcen = fmaxf(0.f, (tr - delay) * c_light);
         else captured = true;
       }
@@ -315,17 +305,248 @@ __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut
       if (lost != 0.0 || acc_wd != 0.0) { flush = true; flush_cell = cq; f_lost = lost; f_wd = acc_wd; }
     }
     acc_wd = 0.0;
-    a.w[pid] = w;
-    // census, cap and frozen histories keep their (pre-event, when frozen) state
-    if (w > 0.f) {
-      a.p1[pid] = x; a.d1[pid] = u;
-      if (GEOM == G_XY || GEOM == G_RZ) { a.p2[pid] = y; a.d2[pid] = v; }
-      a.cell[pid] = ci + a.nx * cj;
-      cen = true;
-      cen_bin = ci + a.nx * cj + (a.ecen_by_group ? a.nc * grp : 0);
-    }
   }
   o.finished = finished;
+}
+
+// Stores the final state of an ended history.  True when it ended alive, its weight then
+// belonging to the comb's census sums in bin `cen_bin`.
+template <int GEOM>
+__device__ __forceinline__ bool history_retire(const TrackArgs& a, const Hist& h, int& cen_bin) {
+  a.w[h.pid] = h.w;
+  if (!(h.w > 0.f)) return false;
+  // census, cap and frozen histories keep their (pre-event, when frozen) state
+  const int c = h.ci + a.nx * h.cj;
+  a.p1[h.pid] = h.x; a.d1[h.pid] = h.u;
+  if (GEOM == G_XY || GEOM == G_RZ) { a.p2[h.pid] = h.y; a.d2[h.pid] = h.v; }
+  a.cell[h.pid] = c;
+  cen_bin = c + (a.ecen_by_group ? a.nc * h.grp : 0);
+  return true;
+}
+
+// The block's claim of bank entries for one warp (guided: a share of what is left, at most
+// `chunk`, at least 32, so early claims are long contiguous (coherent) runs and the drain is
+// finely balanced).  Every lane calls it; false when the queue is past n.
+__device__ __forceinline__ bool claim_run(const TrackArgs& a, uint32_t n, uint32_t& next, uint32_t& end) {
+  unsigned long long base = 0, claim = 0;
+  if ((threadIdx.x & 31) == 0) {
+    const unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(a.queue);
+    const unsigned long long left = cur < (unsigned long long)n ? (unsigned long long)n - cur : 0ull;
+    const unsigned long long nw = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+    claim = min((unsigned long long)a.chunk, max(32ull, left / (2ull * nw)));
+    base = atomicAdd(a.queue, claim);
+  }
+  base = __shfl_sync(FULL, base, 0);
+  claim = __shfl_sync(FULL, claim, 0);
+  if (base >= (unsigned long long)n) return false;
+  next = (uint32_t)base;
+  end = (uint32_t)min(base + claim, (unsigned long long)n);
+  return true;
+}
+
+// 64-bit add to a shared-memory tally as two 32-bit adds, the low word's carry going into the
+// high word: the sum is exact modulo 2^64 in any order, and both adds are native shared-memory
+// atomics, where the 64-bit one is a compare-and-swap loop (crooked pipe, 68 M segments a launch:
+// 1.53 ms with the 64-bit atomic, 1.37 ms so).
+__device__ __forceinline__ void smem_add_u64(unsigned long long* t, unsigned long long v) {
+  unsigned* q = reinterpret_cast<unsigned*>(t);
+  const unsigned lo = (unsigned)v;
+  const unsigned old = atomicAdd(q, lo);
+  const unsigned hi = (unsigned)(v >> 32) + (old + lo < lo ? 1u : 0u);
+  if (hi) atomicAdd(q + 1, hi);
+}
+
+// Where a cell visit's deposition (fixed point) and path-length intensity (FP64) are summed:
+//   T_GLOBAL  global memory, the warp's lanes grouped by cell first (one reduction per cell)
+//   T_SMALL   both per block in shared memory, added to the global ones at the block's end
+//   T_WIDE    one block per SM (kWideThreads at most) with the step's main tally per (group, cell)
+//             in shared memory: the deposition, or with Carter-Forest the intensity (nothing is
+//             deposited in flight there); the other tally, rare, goes to global memory
+// Grouping lanes by cell costs a warp-wide match and a serial sum over each group's lanes at nearly
+// every event; a shared-memory atomic per flushing lane does not.  T_SMALL serves meshes whose
+// tallies fit beside each of several blocks an SM; T_WIDE every mesh whose one tally fits in an
+// SM's shared memory once (26 thousand entries).  Crooked pipe 60 x 210, 8.7 M histories, 68 M
+// segments a launch: 2.47 ms with T_GLOBAL at the default launch shape, 1.37 ms with T_WIDE.
+//
+// Ended histories wait until kRefillMin lanes of the warp are idle; then their final states and
+// census sums are stored and the lanes refilled in one go, so this part runs once per kRefillMin
+// endings instead of whenever any lane ends (at about 8 segments per history, nearly every
+// event): the same launch 1.57 ms at 1, 1.43 at 4, 1.37 at 8, 1.37 at 12.
+constexpr int kRefillMin = 8;
+constexpr int kWideThreads = 1024;
+enum : int { T_GLOBAL = 0, T_SMALL, T_WIDE };
+
+template <int GEOM, bool SMEM_CELLS, bool MG, bool CF, int TALLY>
+__global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY == T_WIDE ? 1 : 4) k_track(TrackArgs a) {
+  pdl_wait();     // the previous kernel of the stream has completed
+  pdl_trigger();  // the next one may be scheduled
+  const float dtk = a.dt_dev ? (float)*a.dt_dev : a.dt;  // graph replay: step length and Philox
+  const uint32_t stepk = a.step_dev ? *a.step_dev : a.step;  // step counter from device memory
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ unsigned blk_cnt[B_N];
+  __shared__ unsigned long long blk_esc[4];
+  constexpr bool ONED = GEOM == G_SLAB || GEOM == G_SPHERE;
+  constexpr bool MG2 = MG && !ONED;  // MG_IMC2D history rules
+  constexpr bool TD_S = TALLY == T_SMALL || (TALLY == T_WIDE && !CF);  // deposition in shared memory
+  constexpr bool TS_S = TALLY == T_SMALL || (TALLY == T_WIDE && CF);   // intensity in shared memory
+  WarpStage* stages = reinterpret_cast<WarpStage*>(smem);
+  const int nwarps = blockDim.x >> 5;
+  float* E1 = reinterpret_cast<float*>(stages + nwarps);
+  float* E2 = E1 + (a.nx + 1);
+  float2* CS = reinterpret_cast<float2*>(E2 + (a.ny + 1) + ((a.nx + a.ny) & 1));
+  const int ncg = a.nc * a.ng;
+  unsigned long long* TD = reinterpret_cast<unsigned long long*>(CS + (SMEM_CELLS ? ncg : 0));
+  double* TS = reinterpret_cast<double*>(TD + (TD_S ? ncg : 0));
+  unsigned long long* const dep_t = TD_S ? TD : a.dep_fx;
+  for (int q = threadIdx.x; q <= a.nx; q += blockDim.x) E1[q] = a.e1[q];
+  for (int q = threadIdx.x; q <= a.ny; q += blockDim.x) E2[q] = a.e2[q];
+  if (SMEM_CELLS)
+    for (int q = threadIdx.x; q < ncg; q += blockDim.x) CS[q] = a.sass[q];
+  if (TD_S) for (int q = threadIdx.x; q < ncg; q += blockDim.x) TD[q] = 0ull;
+  if (TS_S) for (int q = threadIdx.x; q < ncg; q += blockDim.x) TS[q] = 0.0;
+  if (threadIdx.x < B_N) blk_cnt[threadIdx.x] = 0u;
+  if (threadIdx.x < 4) blk_esc[threadIdx.x] = 0ull;
+  __syncthreads();
+
+  const int lane = threadIdx.x & 31;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  WarpStage* st = stages + (threadIdx.x >> 5);
+  const uint32_t n = (uint32_t)*a.n_dev;
+
+  uint32_t chunk_next = 0, chunk_end = 0;  // warp-uniform run of claimed entries
+  bool drained = false;
+  bool has = false, pend = false;  // pend: an ended history whose final state is not stored yet
+  Hist h;
+  h.pid = 0; h.ev = 0; h.x = h.y = h.u = h.v = h.w = h.dcen = h.w_in = 0.f;
+  h.ci = h.cj = h.grp = 0; h.tab = make_float2(0.f, 0.f); h.acc_wd = 0.0;
+  auto table = [&](int cq) { return SMEM_CELLS ? CS[cq] : __ldg(a.sass + cq); };
+  unsigned s_bd = 0, s_sc = 0;
+  unsigned n_alive = 0;                 // entries alive at the end (census sums for the comb)
+  const float c_light = (float)C_LIGHT;
+  // weight floor, IMC/IMC1D.py:1007 / IMC/IMC2D.py:1771 (1e-10); MG_IMC/MG_IMC1D.py:1127 (1e-14)
+  const float weight_floor = (float)(a.floor_coef * (*a.wsum) / (double)(n > 0 ? n : 1));
+  const double inv_q = fx_inv_quantum(*a.wsum);  // fixed-point energy tallies
+  const float inv_nx = 1.0f / (float)a.nx;  // cell -> (i, j) at refill without an integer divide
+
+  for (;;) {
+    unsigned need = __ballot_sync(FULL, !has);
+    if (need == FULL || (!drained && __popc(need) >= kRefillMin)) {
+      // ---------------- store the ended histories, refill from the warp's run ----------------
+      bool cen = false;
+      int cen_bin = 0;
+      if (pend) cen = history_retire<GEOM>(a, h, cen_bin);
+      if (a.ecen) {
+        warp_tally1(cen, cen_bin, (double)h.w, a.ecen, st);
+        n_alive += cen ? 1u : 0u;
+      }
+      pend = false;
+      while (need && !drained) {
+        if (chunk_next >= chunk_end && !claim_run(a, n, chunk_next, chunk_end)) { drained = true; break; }
+        const uint32_t avail = chunk_end - chunk_next;
+        const uint32_t rank = __popc(need & lt_mask);
+        if (!has && rank < avail) {
+          h.pid = chunk_next + rank;
+          h.w = a.w[h.pid];
+          h.dcen = (dtk - a.t[h.pid]) * c_light;
+          const bool moves = (MG2 || CF ? h.w > weight_floor : h.w > 0.f) && h.dcen > 0.f;
+          if (!moves && h.w > 0.f && a.ecen) {
+            // not tracked but alive: part of the census the comb sees
+            const int b = a.cell[h.pid] + (a.ecen_by_group ? a.nc * a.group[h.pid] : 0);
+#ifdef IMC_CHECKED
+            if (b >= 0 && b < a.nc * (a.ecen_by_group ? a.ng : 1))
+#endif
+            { atomicAdd(a.ecen + b, (double)h.w); ++n_alive; }
+          }
+          if (moves) {
+            h.x = a.p1[h.pid]; h.u = a.d1[h.pid];
+            if (MG) h.grp = a.group[h.pid];
+            if (GEOM == G_XY || GEOM == G_RZ) { h.y = a.p2[h.pid]; h.v = a.d2[h.pid]; }
+            const int c = a.cell[h.pid];
+#ifdef IMC_CHECKED
+            // bounds-checked build: an entry outside the mesh (or group range), or with a
+            // non-finite weight, is reported and left untouched
+            if (c < 0 || c >= a.nc || (MG && (h.grp < 0 || h.grp >= a.ng)) || !isfinite(h.w)) {
+              atomicOr(a.flags, (int)IMC_FLAG_BOUNDS);
+            } else
+#endif
+            {
+              // j from a float estimate, corrected to the exact quotient (the estimate is off
+              // by at most one for any int c)
+              h.cj = __float2int_rd(((float)c + 0.5f) * inv_nx);
+              h.ci = c - h.cj * a.nx;
+              if (h.ci < 0) { --h.cj; h.ci += a.nx; } else if (h.ci >= a.nx) { ++h.cj; h.ci -= a.nx; }
+              h.tab = table(MG ? c + a.nc * h.grp : c);
+              h.ev = 0;
+              h.w_in = h.w;
+              h.acc_wd = 0.0;
+              has = true;
+            }
+          }
+        }
+        chunk_next += min((uint32_t)__popc(need), avail);
+        need = __ballot_sync(FULL, !has);
+      }
+      if (need == FULL) break;
+    }
+#ifdef IMC_CHECKED
+    if (has && (h.ci < 0 || h.ci >= a.nx || h.cj < 0 || h.cj >= a.ny || !isfinite(h.w) || !isfinite(h.x) ||
+                !isfinite(h.dcen))) {
+      atomicOr(a.flags, (int)IMC_FLAG_BOUNDS);
+      h.w_in = h.w; h.acc_wd = 0.0;  // nothing is tallied at an invalid index
+      has = false;
+    }
+#endif
+    EvOut o{false, 0, 0.0, 0.0, false};
+    if (has) {
+      history_event<GEOM, SMEM_CELLS, MG, CF>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t, stepk, weight_floor,
+                                              inv_q, s_bd, s_sc);
+      if (o.finished) { has = false; pend = true; }
+    }
+    // ---------------- tally flush ----------------
+    // deposited energy in fixed point; w*s (raw, only from cells without absorption) in FP64
+    if (TALLY == T_GLOBAL) {
+      unsigned long long ud = 0ull;
+      double vs = 0.0;
+      if (o.flush) { ud = fx_units(o.f_lost, inv_q); vs = o.f_wd; }
+      warp_tally_fx(o.flush, o.flush_cell, ud, vs, dep_t, a.si, st);
+    } else {
+      unsigned long long ud = 0ull;
+      if (o.flush) {
+        ud = fx_units(o.f_lost, inv_q);
+        if (TD_S && ud) smem_add_u64(TD + o.flush_cell, ud);
+        if (TS_S && o.f_wd != 0.0) atomicAdd(TS + o.flush_cell, o.f_wd);
+      }
+      if (!TS_S) warp_tally1(o.flush && o.f_wd != 0.0, o.flush_cell, o.f_wd, a.si, st);
+      if (!TD_S) warp_tally_fx(o.flush && ud != 0ull, o.flush_cell, ud, 0.0, a.dep_fx, a.si, st);
+    }
+  }
+
+  // ---------------- statistics ----------------
+  const unsigned long long t_bd = warp_sum_u(s_bd), t_sc = warp_sum_u(s_sc);
+  if (a.ecen) {
+    const unsigned long long t_alive = warp_sum_u(n_alive);
+    if (lane == 0 && t_alive) atomicAdd(a.n_live, t_alive);
+  }
+  if (lane == 0) {
+    if (t_bd) atomicAdd(a.stats + S_BOUNDARY, t_bd);
+    if (t_sc) atomicAdd(a.stats + S_SCATTER, t_sc);
+    if (t_bd + t_sc) atomicAdd(a.stats + S_EVENTS, t_bd + t_sc);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned long long cen = blk_cnt[B_CENSUS], cap = blk_cnt[B_CAP], capt = blk_cnt[B_CAPTURE];
+    if (cen) atomicAdd(a.stats + S_CENSUS, cen);
+    if (capt) atomicAdd(a.stats + S_CAPTURE, capt);
+    if (cen + cap + capt) atomicAdd(a.stats + S_EVENTS, cen + cap + capt);
+    if (blk_cnt[B_FLOOR]) atomicAdd(a.stats + S_FLOOR, (unsigned long long)blk_cnt[B_FLOOR]);
+    if (blk_cnt[B_REFLECT]) atomicAdd(a.stats + S_REFLECT, (unsigned long long)blk_cnt[B_REFLECT]);
+    if (cap) atomicAdd(a.stats + S_CAP, cap);
+    if (blk_cnt[B_ESCAPE]) atomicAdd(a.stats + S_ESCAPE, (unsigned long long)blk_cnt[B_ESCAPE]);
+  }
+  if (threadIdx.x < 4 && blk_esc[threadIdx.x] != 0ull) atomicAdd(a.esc_fx + threadIdx.x, blk_esc[threadIdx.x]);
+  // the block's tallies (every warp's last flush is behind the __syncthreads above)
+  if (TD_S) for (int q = threadIdx.x; q < ncg; q += blockDim.x) if (TD[q]) atomicAdd(a.dep_fx + q, TD[q]);
+  if (TS_S) for (int q = threadIdx.x; q < ncg; q += blockDim.x) if (TS[q] != 0.0) atomicAdd(a.si + q, TS[q]);
 }
 
 // SMEM_TALLY (small meshes): the block sums its deposition (fixed point) and intensity per
@@ -341,8 +562,8 @@ __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut
 enum : int { PF_W = 0, PF_T, PF_P1, PF_D1, PF_CELL, PF_P2, PF_D2, PF_GROUP, PF_PID, PF_NF };
 inline size_t pf_smem(int block) { return sizeof(float) * PF_NF * (size_t)block; }
 
-template <int GEOM, bool SMEM_CELLS, bool MG, bool CF, bool SMEM_TALLY, bool PF>
-__global__ void __launch_bounds__(256, PF ? 4 : 1) k_track(TrackArgs a) {  // PF: at most 64 registers
+template <int GEOM, bool SMEM_CELLS, bool MG, bool CF, bool SMEM_TALLY>
+__global__ void __launch_bounds__(256, 4) k_track_pf(TrackArgs a) {  // at most 64 registers
   pdl_wait();     // the previous kernel of the stream has completed
   pdl_trigger();  // the next one may be scheduled
   const float dtk = a.dt_dev ? (float)*a.dt_dev : a.dt;  // graph replay: step length and Philox
@@ -412,7 +633,7 @@ __global__ void __launch_bounds__(256, PF ? 4 : 1) k_track(TrackArgs a) {  // PF
 
   for (;;) {
     // ---------------- refill idle lanes from the warp's chunk ----------------
-    if (PF) {
+    {
       // An idle lane takes the record in its slot; every lane without a claim takes the next
       // entry of the warp's chunk (a new guided ticket when it runs out) and starts its copies,
       // which land while the lane tracks.  Leaves with every lane tracking or holding no claim;
@@ -501,68 +722,6 @@ __global__ void __launch_bounds__(256, PF ? 4 : 1) k_track(TrackArgs a) {  // PF
         if (!__any_sync(FULL, !has && pv)) break;
       }
     }
-    unsigned need = PF ? 0u : __ballot_sync(FULL, !has);
-    while (need && !drained) {
-      if (chunk_next >= chunk_end) {
-        // guided claim: a share of what is left, at most `chunk`, at least 32, so early
-        // claims are long contiguous (coherent) runs and the drain is finely balanced
-        unsigned long long base = 0, claim = 0;
-        if (lane == 0) {
-          const unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(a.queue);
-          const unsigned long long left = cur < (unsigned long long)n ? (unsigned long long)n - cur : 0ull;
-          const unsigned long long nw = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-          claim = min((unsigned long long)a.chunk, max(32ull, left / (2ull * nw)));
-          base = atomicAdd(a.queue, claim);
-        }
-        base = __shfl_sync(FULL, base, 0);
-        claim = __shfl_sync(FULL, claim, 0);
-        if (base >= (unsigned long long)n) { drained = true; break; }
-        chunk_next = (uint32_t)base;
-        chunk_end = (uint32_t)min(base + claim, (unsigned long long)n);
-      }
-      const uint32_t avail = chunk_end - chunk_next;
-      const uint32_t rank = __popc(need & lt_mask);
-      if (!has && rank < avail) {
-        pid = chunk_next + rank;
-        w = a.w[pid];
-        dcen = (dtk - a.t[pid]) * c_light;
-        const bool moves = (MG2 || CF ? w > weight_floor : w > 0.f) && dcen > 0.f;
-        if (!moves && w > 0.f && a.ecen) {
-          // not tracked but alive: part of the census the comb sees
-          const int b = a.cell[pid] + (a.ecen_by_group ? a.nc * a.group[pid] : 0);
-#ifdef IMC_CHECKED
-          if (b >= 0 && b < a.nc * (a.ecen_by_group ? a.ng : 1))
-#endif
-          { atomicAdd(a.ecen + b, (double)w); ++n_alive; }
-        }
-        if (moves) {
-          x = a.p1[pid]; u = a.d1[pid];
-          if (MG) grp = a.group[pid];
-          if (GEOM == G_XY || GEOM == G_RZ) { y = a.p2[pid]; v = a.d2[pid]; }
-          const int c = a.cell[pid];
-#ifdef IMC_CHECKED
-          // bounds-checked build: an entry outside the mesh (or group range), or with a
-          // non-finite weight, is reported and left untouched
-          if (c < 0 || c >= a.nc || (MG && (grp < 0 || grp >= a.ng)) || !isfinite(w)) {
-            atomicOr(a.flags, (int)IMC_FLAG_BOUNDS);
-          } else
-#endif
-          {
-            // j from a float estimate, corrected to the exact quotient (the estimate is off
-            // by at most one for any int c)
-            cj = __float2int_rd(((float)c + 0.5f) * inv_nx);
-            ci = c - cj * a.nx;
-            if (ci < 0) { --cj; ci += a.nx; } else if (ci >= a.nx) { ++cj; ci -= a.nx; }
-            tab = table(MG ? c + a.nc * grp : c);
-            ev = 0;
-            w_in = w;
-            has = true;
-          }
-        }
-      }
-      chunk_next += min((uint32_t)__popc(need), avail);
-      need = __ballot_sync(FULL, !has);
-    }
     if (!__any_sync(FULL, has)) break;
 #ifdef IMC_CHECKED
     if (has && (ci < 0 || ci >= a.nx || cj < 0 || cj >= a.ny || !isfinite(w) || !isfinite(x) || !isfinite(dcen))) {
@@ -572,17 +731,19 @@ __global__ void __launch_bounds__(256, PF ? 4 : 1) k_track(TrackArgs a) {  // PF
     }
 #endif
 
-    EvOut o{false, 0, 0.0, 0.0, false, 0, false};
+    EvOut o{false, 0, 0.0, 0.0, false};
+    bool cen = false;
+    int cen_bin = 0;
     if (has) {
       Hist h{pid, ev, x, y, u, v, w, dcen, w_in, ci, cj, grp, tab, acc_wd};
       history_event<GEOM, SMEM_CELLS, MG, CF>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t, stepk, weight_floor,
                                               inv_q, s_bd, s_sc);
       pid = h.pid; ev = h.ev; x = h.x; y = h.y; u = h.u; v = h.v; w = h.w; dcen = h.dcen; w_in = h.w_in;
       ci = h.ci; cj = h.cj; grp = h.grp; tab = h.tab; acc_wd = h.acc_wd;
-      if (o.finished) has = false;
+      if (o.finished) { has = false; cen = history_retire<GEOM>(a, h, cen_bin); }
     }
-    const bool flush = o.flush, cen = o.cen;
-    const int flush_cell = o.flush_cell, cen_bin = o.cen_bin;
+    const bool flush = o.flush;
+    const int flush_cell = o.flush_cell;
     const double f_lost = o.f_lost, f_wd = o.f_wd;
     // ---------------- converged tally flush ----------------
     // deposited energy in fixed point; w*s (raw, only from cells without absorption) in FP64
@@ -637,34 +798,49 @@ __global__ void __launch_bounds__(256, PF ? 4 : 1) k_track(TrackArgs a) {  // PF
   }
 }
 
-template <int GEOM, bool SM, bool MG, bool CF, bool ST, bool PF>
-cudaError_t launch_one(const TrackArgs& a, int block, int grid, cudaStream_t s) {
-  const int nwarps = block / 32;
-  size_t sh = nwarps * sizeof(WarpStage) + sizeof(float) * (a.nx + a.ny + 4);
-  if (SM) sh += sizeof(float2) * a.nc * a.ng;
-  if (ST) sh += (sizeof(unsigned long long) + sizeof(double)) * a.nc * a.ng;
-  if (PF) sh += pf_smem(block);
+// dynamic shared memory of the tracking kernels: per-warp staging, edges, the cell table and
+// `tallies` 8-byte block tallies per (group, cell)
+inline size_t track_smem(const TrackArgs& a, int block, bool cells, int tallies) {
+  size_t sh = (block / 32) * sizeof(WarpStage) + sizeof(float) * (a.nx + a.ny + 4);
+  if (cells) sh += sizeof(float2) * a.nc * a.ng;
+  return sh + 8ull * tallies * a.nc * a.ng;
+}
+
+template <typename K>
+cudaError_t launch_sized(K kernel, const TrackArgs& a, int block, int grid, size_t sh, cudaStream_t s) {
   if (sh > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_track<GEOM, SM, MG, CF, ST, PF>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
     if (e != cudaSuccess) return e;
   }
-  IMC_LAUNCH_PDL((k_track<GEOM, SM, MG, CF, ST, PF>), grid, block, sh, s, a);
+  IMC_LAUNCH_PDL(kernel, grid, block, sh, s, a);
   return cudaGetLastError();
 }
 
-// the block tallies are built only with the shared-memory cell table (small meshes)
-template <int GEOM, bool MG, bool CF, bool PF>
-cudaError_t launch_pf(const TrackArgs& a, int block, int grid, bool sm, bool st, cudaStream_t s) {
-  if (sm && st) return launch_one<GEOM, true, MG, CF, true, PF>(a, block, grid, s);
-  return sm ? launch_one<GEOM, true, MG, CF, false, PF>(a, block, grid, s)
-            : launch_one<GEOM, false, MG, CF, false, PF>(a, block, grid, s);
-}
+constexpr size_t kSmemPerBlock = 226 * 1024;  // dynamic, beside the kernel's own few hundred bytes
 
+// T_SMALL is built only with the shared-memory cell table (small meshes)
 template <int GEOM, bool MG, bool CF = false>
-cudaError_t launch_geom(const TrackArgs& a, int block, int grid, bool sm, bool st, bool pf, cudaStream_t s) {
-  return pf ? launch_pf<GEOM, MG, CF, true>(a, block, grid, sm, st, s)
-            : launch_pf<GEOM, MG, CF, false>(a, block, grid, sm, st, s);
+cudaError_t launch_geom(const TrackArgs& a, const TrackLaunch& l, cudaStream_t s) {
+  const int block = l.block, grid = l.sms * l.blocks_per_sm;
+  const bool sm = l.smem_cells, st = l.smem_tally, pf = l.prefetch;
+  if (pf) {
+    const size_t sh = track_smem(a, block, sm, sm && st ? 2 : 0) + pf_smem(block);
+    if (sm && st) return launch_sized(k_track_pf<GEOM, true, MG, CF, true>, a, block, grid, sh, s);
+    return sm ? launch_sized(k_track_pf<GEOM, true, MG, CF, false>, a, block, grid, sh, s)
+              : launch_sized(k_track_pf<GEOM, false, MG, CF, false>, a, block, grid, sh, s);
+  }
+  // One wide block per SM holding as many threads as the requested shape keeps resident there,
+  // when its tally fits; the cell table beside it if that fits too (else it is read through L1,
+  // which measured the same on the crooked pipe).
+  const int wide = std::max(128, std::min(kWideThreads, block * l.blocks_per_sm)) & ~31;
+  if (!st && l.wide_ok && block <= 256 && track_smem(a, wide, false, 1) <= kSmemPerBlock) {
+    if (sm && track_smem(a, wide, true, 1) <= kSmemPerBlock)
+      return launch_sized(k_track<GEOM, true, MG, CF, T_WIDE>, a, wide, l.sms, track_smem(a, wide, true, 1), s);
+    return launch_sized(k_track<GEOM, false, MG, CF, T_WIDE>, a, wide, l.sms, track_smem(a, wide, false, 1), s);
+  }
+  if (sm && st) return launch_sized(k_track<GEOM, true, MG, CF, T_SMALL>, a, block, grid, track_smem(a, block, true, 2), s);
+  return sm ? launch_sized(k_track<GEOM, true, MG, CF, T_GLOBAL>, a, block, grid, track_smem(a, block, true, 0), s)
+            : launch_sized(k_track<GEOM, false, MG, CF, T_GLOBAL>, a, block, grid, track_smem(a, block, false, 0), s);
 }
 
 // ---------------------------------------------------------------------------------
@@ -736,7 +912,7 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
   for (uint32_t it = 0; it < trips; ++it) {
     const uint32_t i = it * stride + blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = i < n_in;
-    EvOut o{false, 0, 0.0, 0.0, false, 0, false};
+    EvOut o{false, 0, 0.0, 0.0, false};
     bool alive = false;
     uint32_t pid = 0;
     if (active) {
@@ -763,6 +939,8 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
         h.tab = __ldg(a.sass + (MG ? c + a.nc * h.grp : c));
         history_event<GEOM, false, MG, CF>(a, h, o, E1, E2, nullptr, blk_cnt, blk_esc, a.dep_fx, stepk,
                                            weight_floor, inv_q, s_bd, s_sc);
+        int bin;
+        if (o.finished) history_retire<GEOM>(a, h, bin);
       }
       if (!o.finished) {
         alive = true;
@@ -921,31 +1099,30 @@ cudaError_t imc_run_event_tracking(const TrackArgs& a, int geom, void* scratch, 
   return cudaSuccess;
 }
 
-cudaError_t imc_launch_track(const TrackArgs& a, int geom, int block, int grid, bool sm, bool st, bool pf,
-                             cudaStream_t s) {
+cudaError_t imc_launch_track(const TrackArgs& a, int geom, const TrackLaunch& l, cudaStream_t s) {
   ++g_imc_launches;
   if (a.ng > 1) {  // multigroup: 2-D (MG_IMC/MG_IMC2D.py) and the 1-D sphere (MG_IMC/MG_IMC1D.py)
     switch (geom) {
-      case G_SPHERE: return launch_geom<G_SPHERE, true>(a, block, grid, sm, st, pf, s);
-      case G_XY: return launch_geom<G_XY, true>(a, block, grid, sm, st, pf, s);
-      case G_RZ: return launch_geom<G_RZ, true>(a, block, grid, sm, st, pf, s);
+      case G_SPHERE: return launch_geom<G_SPHERE, true>(a, l, s);
+      case G_XY: return launch_geom<G_XY, true>(a, l, s);
+      case G_RZ: return launch_geom<G_RZ, true>(a, l, s);
       default: return cudaErrorInvalidValue;
     }
   }
   if (a.cf_rate) {  // Carter-Forest, gray
     switch (geom) {
-      case G_SLAB: return launch_geom<G_SLAB, false, true>(a, block, grid, sm, st, pf, s);
-      case G_SPHERE: return launch_geom<G_SPHERE, false, true>(a, block, grid, sm, st, pf, s);
-      case G_XY: return launch_geom<G_XY, false, true>(a, block, grid, sm, st, pf, s);
-      case G_RZ: return launch_geom<G_RZ, false, true>(a, block, grid, sm, st, pf, s);
+      case G_SLAB: return launch_geom<G_SLAB, false, true>(a, l, s);
+      case G_SPHERE: return launch_geom<G_SPHERE, false, true>(a, l, s);
+      case G_XY: return launch_geom<G_XY, false, true>(a, l, s);
+      case G_RZ: return launch_geom<G_RZ, false, true>(a, l, s);
       default: return cudaErrorInvalidValue;
     }
   }
   switch (geom) {
-    case G_SLAB: return launch_geom<G_SLAB, false>(a, block, grid, sm, st, pf, s);
-    case G_SPHERE: return launch_geom<G_SPHERE, false>(a, block, grid, sm, st, pf, s);
-    case G_XY: return launch_geom<G_XY, false>(a, block, grid, sm, st, pf, s);
-    case G_RZ: return launch_geom<G_RZ, false>(a, block, grid, sm, st, pf, s);
+    case G_SLAB: return launch_geom<G_SLAB, false>(a, l, s);
+    case G_SPHERE: return launch_geom<G_SPHERE, false>(a, l, s);
+    case G_XY: return launch_geom<G_XY, false>(a, l, s);
+    case G_RZ: return launch_geom<G_RZ, false>(a, l, s);
     default: return cudaErrorInvalidValue;
   }
 }
