@@ -31,7 +31,7 @@ using namespace imcdev;
 namespace {
 
 template <int GEOM>
-__global__ void __launch_bounds__(256) k_adjoint(AdjointArgs A) {
+__global__ void __launch_bounds__(256, 4) k_adjoint(AdjointArgs A) {
   const TrackArgs& a = A.t;
   extern __shared__ __align__(16) unsigned char smem[];
   WarpStage* stages = reinterpret_cast<WarpStage*>(smem);
@@ -48,7 +48,6 @@ __global__ void __launch_bounds__(256) k_adjoint(AdjointArgs A) {
   const uint32_t n = (uint32_t)*a.n_dev;
   const float c_light = (float)C_LIGHT;
   const float weight_floor = (float)(1e-10 * (*a.wsum) / (double)(n > 0 ? n : 1));
-  const float ss_thr = 1e-12f;
 
   uint32_t chunk_next = 0, chunk_end = 0;
   bool drained = false;
@@ -120,8 +119,8 @@ __global__ void __launch_bounds__(256) k_adjoint(AdjointArgs A) {
         if (GEOM == G_XY) {
           const float xl = E1[ci], xr = E1[ci + 1], yl = E2[cj], yr = E2[cj + 1];
           Lc = fminf(xr - xl, yr - yl);
-          if (u > 0.f) sx = __fdividef(xr - x, u); else if (u < 0.f) sx = __fdividef(xl - x, u);
-          if (v > 0.f) sy = __fdividef(yr - y, v); else if (v < 0.f) sy = __fdividef(yl - y, v);
+          if (u > 0.f) sx = fdiv(xr - x, u); else if (u < 0.f) sx = fdiv(xl - x, u);
+          if (v > 0.f) sy = fdiv(yr - y, v); else if (v < 0.f) sy = fdiv(yl - y, v);
           sx = fmaxf(sx, 0.f); sy = fmaxf(sy, 0.f);
           sb = fminf(sx, sy);
         } else {
@@ -129,33 +128,24 @@ __global__ void __launch_bounds__(256) k_adjoint(AdjointArgs A) {
           Lc = fminf(rout - rin, zhi - zlo);
           const float sin2 = (1.f - v) * (1.f + v);
           if (sin2 >= 1e-15f) {
-            const float ist = rsqrtf(sin2);
+            const float ist = frsqrt(sin2);
             st_ = sin2 * ist;
             const float b2 = x * x * ((1.f - u) * (1.f + u));
             s_rout = outer_root(x, u, rout, b2) * ist;
             const float li = inner_root(x, u, rin, b2);
             if (li < BIGF) s_rin = li * ist;
           }
-          if (v > 1e-15f) s_zhi = fmaxf(__fdividef(zhi - y, v), 0.f);
-          else if (v < -1e-15f) s_zlo = fmaxf(__fdividef(zlo - y, v), 0.f);
+          if (v > 1e-15f) s_zhi = fmaxf(fdiv(zhi - y, v), 0.f);
+          else if (v < -1e-15f) s_zlo = fmaxf(fdiv(zlo - y, v), 0.f);
           sb = fminf(fminf(s_rin, s_rout), fminf(s_zlo, s_zhi));
         }
-        // effective scatter, as the forward kernel (cap sigma_s L > 1e4; series test)
+        // effective scatter, as the forward kernel (table entry: > 0 the opacity, < 0 capped)
         float ds = BIGF;
-        const bool capped = ss * Lc > 10000.0f;
-        const bool scores = !capped && ss > ss_thr;  // sampling depends on sigma_s here
-        {
-          const float sig = capped ? 10000.0f / Lc : (ss > ss_thr ? ss : 0.f);
-          if (sig > 0.f) {
-            const float s_other = fminf(sb, dcen);
-            const double t = (double)sig * (double)s_other;
-            bool may = true;
-            if (t < 0.01) {
-              const double thr = 1.0 - t * (1.0 - t * (0.5 - t * (1.0 / 6.0)));
-              may = u01d(r.x) > thr;
-            }
-            if (may) ds = capped ? neglog_u(r.x) * (Lc * 1e-4f) : __fdividef(neglog_u(r.x), ss);
-          }
+        const bool scores = ss > 0.f;  // sampling depends on sigma_s here
+        if (ss != 0.f) {
+          const float s_other = fminf(sb, dcen);
+          if (scatter_may_win(r.x, ss > 0.f ? ss : 10000.0f / Lc, s_other))
+            ds = ss > 0.f ? fdiv(neglog_u(r.x), ss) : neglog_u(r.x) * (Lc * 1e-4f);
         }
         d = sb; evt = EV_BOUNDARY;
         if (ds < d) { d = ds; evt = EV_SCATTER; }
@@ -182,7 +172,7 @@ __global__ void __launch_bounds__(256) k_adjoint(AdjointArgs A) {
           const float ax = fmaf(u, l, x);
           float rn = sqrt_nn(fmaf(ax, ax, l * l * ((1.f - u) * (1.f + u))));
           yn = fmaf(d, v, y);
-          if (rn > 1e-15f && l > 0.f) un = fminf(1.f, fmaxf(-1.f, __fdividef(fmaf(x, u, l), rn)));
+          if (rn > 1e-15f && l > 0.f) un = fminf(1.f, fmaxf(-1.f, fdiv(fmaf(x, u, l), rn)));
           if (evt == EV_BOUNDARY) {
             if (sb == s_rin) { rn = rin; cross = X_IM; }
             else if (sb == s_rout) { rn = rout; cross = X_IP; }

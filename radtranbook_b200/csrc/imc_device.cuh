@@ -77,6 +77,31 @@ __device__ __forceinline__ U4 draw_rk(const uint32_t* rk, uint32_t idx, uint32_t
   return c;
 }
 
+// draw_rk for a run of blocks of one (idx, step, tag): the first two rounds' products of the
+// words that do not change with the block are formed once (draw_key), and each draw starts
+// after round 2 with one of its four products instead of four.  Same numbers as draw_rk.
+struct DrawKey { uint32_t a, b, c; };
+__device__ __forceinline__ DrawKey draw_key(const uint32_t* rk, uint32_t idx, uint32_t step, uint32_t tag) {
+  const uint32_t lo0 = 0xD2511F53u * idx, hi0 = __umulhi(0xD2511F53u, idx);
+  const uint32_t z1 = hi0 ^ tag ^ rk[1];  // word z after round 1
+  return DrawKey{__umulhi(0xCD9E8D57u, z1) ^ (0xCD9E8D57u * step) ^ rk[2], 0xCD9E8D57u * z1, lo0 ^ rk[3]};
+}
+// rkx = high half of 0xCD9E8D57 * step, ^ rk[0] (the step's, the same for every history)
+__device__ __forceinline__ uint32_t draw_step_key(const uint32_t* rk, uint32_t step) {
+  return __umulhi(0xCD9E8D57u, step) ^ rk[0];
+}
+__device__ __forceinline__ U4 draw_next(const uint32_t* rk, const DrawKey& k, uint32_t rkx, uint32_t block) {
+  const uint32_t x1 = rkx ^ block;  // word x after round 1
+  U4 c{k.a, k.b, __umulhi(0xD2511F53u, x1) ^ k.c, 0xD2511F53u * x1};
+#pragma unroll
+  for (int r = 2; r < 10; ++r) {
+    const uint32_t lo0 = 0xD2511F53u * c.x, hi0 = __umulhi(0xD2511F53u, c.x);
+    const uint32_t lo1 = 0xCD9E8D57u * c.z, hi1 = __umulhi(0xCD9E8D57u, c.z);
+    c = U4{hi1 ^ c.y ^ rk[2 * r], lo1, hi0 ^ c.w ^ rk[2 * r + 1], lo0};
+  }
+  return c;
+}
+
 // draw_rk with the round keys read as five 16-byte words (rk4: the 20 keys of
 // philox_round_keys, 16-byte aligned, e.g. staged in shared memory): the same numbers, five
 // vector loads where draw_rk makes twenty scalar ones.
@@ -133,9 +158,20 @@ struct Ev {
   int cross;     // X_*
 };
 
-// The tracking's approximate quotient and reciprocal square root.
-__device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
-__device__ __forceinline__ float frsqrt(float x) { return rsqrtf(x); }
+// The tracking's approximate quotient and reciprocal square root: the hardware approximations
+// without the steps that widen them to subnormal operands, which no distance, direction or
+// opacity here has (histories are bit-identical to __fdividef / rsqrtf; a crossing has up to
+// eight of them: 12.7 -> 11.9 ms for the ten launches of a 2M crooked-pipe run).
+__device__ __forceinline__ float fdiv(float a, float b) {
+  float q;
+  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(q) : "f"(a), "f"(b));
+  return q;
+}
+__device__ __forceinline__ float frsqrt(float x) {
+  float q;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(x));
+  return q;
+}
 
 // ---- 1-D slab: distance to the exit face in the direction of mu ----
 __device__ __forceinline__ float slab_face(float x, float mu, float xl, float xr) {

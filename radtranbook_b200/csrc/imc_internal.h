@@ -18,7 +18,7 @@ struct TrackArgs {
   int nx, ny, nc, ng;
   const float* e1;           // nx+1 edges (FP32 copy)
   const float* e2;           // ny+1
-  const float2* sass;        // [g][c] (Fleck absorption, effective scatter), FP32
+  const float2* sass;        // [g][c] (Fleck absorption, scatter slot: scatter_entry), FP32
   const double2* cellf;      // [g][c] (1/V, 1/(sigma_a V dt) or -1/(V dt))
   double* dep;               // [g][c]
   double* si;                // [g][c]

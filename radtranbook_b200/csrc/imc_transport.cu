@@ -26,7 +26,7 @@ using namespace imcdev;
 namespace {
 
 // Block-level counters for rare events (shared-memory atomics keep them out of registers).
-enum : int { B_CENSUS = 0, B_FLOOR, B_REFLECT, B_CAP, B_ESCAPE, B_CAPTURE, B_N };
+enum : int { B_FLOOR = 0, B_REFLECT, B_CAP, B_ESCAPE, B_CAPTURE, B_N };
 
 // MG: group-indexed tables and tallies, escaped energy also by group.  In 2-D the rules of
 // MG_IMC/MG_IMC2D.py:580-989 (no effective-scatter cap, no absorption for sigma_a <= 1e-12,
@@ -49,170 +49,175 @@ struct Hist {
   uint32_t pid, ev;
   float x, y, u, v, w, dcen, w_in;
   int ci, cj, grp;
-  float2 tab;      // (sigma_a, sigma_s) of the current (group, cell)
-  double acc_wd;   // w*s in the current cell (cells without absorption only)
+  float2 tab;      // cell table entry of the current (group, cell)
+  DrawKey key;     // the history's part of its Philox draws
 };
 struct EvOut {
-  bool flush;      // a cell visit to flush: deposition f_lost, path length f_wd, into flush_cell
-  int flush_cell;
-  double f_lost, f_wd;
+  int cell;        // (group, cell) index of the cell the event took place in
+  bool flush;      // its visit ends: deposition `lost`
+  float wd;        // w*s of the flight in a cell without absorption (else 0)
+  double lost;
   bool finished;   // the history ended: history_retire stores its final state
 };
 
+// What an event costs is its instructions: the kernel issues one in four of every five cycles, so
+// the geometry is written for few and uniform ones.  Against the straightforward form (one branch
+// per face and root, thresholds and caps tested per flight, all ten Philox rounds per draw, FP64
+// path length carried in registers) the ten launches of a 2M crooked-pipe run take 10.4 ms
+// instead of 12.6, the slab Marshak wave's twenty 7.1 instead of 8.5; every history is
+// bit-identical.
+
+// The scatter slot of a table entry (scatter_entry): > 0 the effective scatter opacity, 0 none
+// (at or below the geometry's threshold), < 0 minus the opacity of a cell whose distance is
+// capped (sigma_s L > 1e4 -> 1e4 / L; IMC/IMC1D.py:83-88, IMC/IMC2D.py:758-765).
+template <bool CAPS>
+__device__ __forceinline__ float scatter_flight(float ss, float L, uint32_t x, float s_other) {
+  if (ss > 0.f) {
+    if (scatter_may_win(x, ss, s_other)) return fdiv(neglog_u(x), ss);
+  } else if (CAPS && ss < 0.f) {
+    if (scatter_may_win(x, 10000.0f / L, s_other)) return neglog_u(x) * (L * 1e-4f);
+  }
+  return BIGF;
+}
+
 template <int GEOM, bool SMEM_CELLS, bool MG, bool CF>
-__device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut& o, const float* E1,
-                                              const float* E2, const float2* CS, unsigned* blk_cnt,
+__device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut& o, const float2* E1,
+                                              const float2* E2, const float2* CS, unsigned* blk_cnt,
                                               unsigned long long* blk_esc, unsigned long long* dep_t,
-                                              uint32_t stepk, float weight_floor, double inv_q,
-                                              unsigned& s_bd, unsigned& s_sc) {
+                                              uint32_t rkx, float weight_floor, double inv_q,
+                                              unsigned& s_cen, unsigned& s_sc) {
   constexpr bool ONED = GEOM == G_SLAB || GEOM == G_SPHERE;
   constexpr bool MG2 = MG && !ONED;  // MG_IMC2D history rules
   const float c_light = (float)C_LIGHT;
-  const float ss_thr = ONED ? 1e-10f : 1e-12f;
   auto table = [&](int cq) { return SMEM_CELLS ? CS[cq] : __ldg(a.sass + cq); };
-  uint32_t& pid = h.pid;
-  uint32_t& ev = h.ev;
-  float &x = h.x, &y = h.y, &u = h.u, &v = h.v, &w = h.w, &dcen = h.dcen, &w_in = h.w_in;
-  int &ci = h.ci, &cj = h.cj, &grp = h.grp;
-  float2& tab = h.tab;
-  double& acc_wd = h.acc_wd;
-  bool& flush = o.flush;
-  int& flush_cell = o.flush_cell;
-  double &f_lost = o.f_lost, &f_wd = o.f_wd;
-  const int c = ci + a.nx * cj;
-  const int cq = MG ? c + a.nc * grp : c;  // (group, cell) table / tally index
-  const float sa = tab.x, ss = tab.y;
-  bool finished = false, frozen = false;
-  if (ev >= (uint32_t)a.max_events) {
+  const float x = h.x, y = h.y, u = h.u, v = h.v, w = h.w;
+  const int c = h.ci + a.nx * h.cj;
+  const int cq = MG ? c + a.nc * h.grp : c;  // (group, cell) table / tally index
+  o.cell = cq;
+  const float sa = h.tab.x, ss = h.tab.y;
+  bool finished = false;
+  if (h.ev >= (uint32_t)a.max_events) {
     // events-per-history cap (IMC/IMC2D.py:974-977): stops, weight stays in census
     atomicAdd(&blk_cnt[B_CAP], 1u);
     if (!a.cap_is_reference) atomicOr(a.flags, (int)IMC_FLAG_EVENT_CAP);
     finished = true;
   } else {
-    const U4 r = draw_rk(a.rk, a.id_base + pid, ev, stepk, TAG_TRANSPORT);
-    ++ev;
-    float d, sb, L, xn = x, yn = y, un = u, vn = v;
-    int evt, cross = X_NONE;
+    const U4 r = draw_next(a.rk, h.key, rkx, h.ev);
+    ++h.ev;
+    const float2 e1 = E1[h.ci];  // the cell's edges in each direction
+    float d, sb, xn, yn = y, un = u, vn = v;
+    int evt, di = 0, dj = 0;     // the cell step of a boundary crossing
     // ---- distance to the cell boundary ----
-    float s_rin = BIGF, s_rout = BIGF, s_zlo = BIGF, s_zhi = BIGF, st_ = 0.f, sx = BIGF, sy = BIGF;
-    float din = BIGF, dout = BIGF;
+    float s_rin = BIGF, s_rout = BIGF, st_ = 0.f, sx = BIGF, sy = BIGF;  // sy: z faces in RZ
+    float din = BIGF, dout = BIGF, om = 0.f;
+    float2 e2 = make_float2(0.f, 0.f);
     if (GEOM == G_SLAB) {
-      const float xl = E1[ci], xr = E1[ci + 1];
-      L = xr - xl;
-      sb = slab_face(x, u, xl, xr);
+      sb = slab_face(x, u, e1.x, e1.y);
     } else if (GEOM == G_SPHERE) {
-      const float r0 = E1[ci], r1 = E1[ci + 1];
-      L = r1 - r0;
-      const float b2 = x * x * ((1.f - u) * (1.f + u));
-      dout = outer_root(x, u, r1, b2);
-      din = inner_root(x, u, r0, b2);
+      om = (1.f - u) * (1.f + u);
+      const float b2 = x * x * om;
+      dout = outer_root(x, u, e1.y, b2);
+      din = inner_root(x, u, e1.x, b2);
       sb = fminf(dout, din);
-    } else if (GEOM == G_XY) {
-      const float xl = E1[ci], xr = E1[ci + 1], yl = E2[cj], yr = E2[cj + 1];
-      L = fminf(xr - xl, yr - yl);
-      if (u > 0.f) sx = fdiv(xr - x, u); else if (u < 0.f) sx = fdiv(xl - x, u);
-      if (v > 0.f) sy = fdiv(yr - y, v); else if (v < 0.f) sy = fdiv(yl - y, v);
-      sx = fmaxf(sx, 0.f); sy = fmaxf(sy, 0.f);
-      sb = fminf(sx, sy);
     } else {
-      const float rin = E1[ci], rout = E1[ci + 1], zlo = E2[cj], zhi = E2[cj + 1];
-      L = fminf(rout - rin, zhi - zlo);
-      const float sin2 = (1.f - v) * (1.f + v);
-      if (sin2 >= 1e-15f) {
-        const float ist = frsqrt(sin2);
-        st_ = sin2 * ist;
-        const float b2 = x * x * ((1.f - u) * (1.f + u));
-        s_rout = outer_root(x, u, rout, b2) * ist;
-        const float li = inner_root(x, u, rin, b2);
-        if (li < BIGF) s_rin = li * ist;
+      e2 = E2[h.cj];
+      if (GEOM == G_XY) {
+        if (u != 0.f) sx = fdiv((u > 0.f ? e1.y : e1.x) - x, u);
+        if (v != 0.f) sy = fdiv((v > 0.f ? e2.y : e2.x) - y, v);
+        sx = fmaxf(sx, 0.f); sy = fmaxf(sy, 0.f);
+        sb = fminf(sx, sy);
+      } else {
+        const float sin2 = (1.f - v) * (1.f + v);
+        om = (1.f - u) * (1.f + u);
+        if (sin2 >= 1e-15f) {
+          // outer_root and inner_root with one quotient: moving outwards (u >= 0) only the
+          // outer face is met and its root is a quotient; moving inwards the inner root is the
+          // quotient, the outer one q - r u
+          const float ist = frsqrt(sin2);
+          st_ = sin2 * ist;
+          const float b2 = x * x * om;
+          const float q = sqrt_nn(fmaf(e1.y, e1.y, -b2));
+          const float disc = fmaf(e1.x, e1.x, -b2);
+          const bool out = u >= 0.f;
+          const float R = out ? e1.y : e1.x;
+          const float P = (R - x) * (R + x);
+          const float den = out ? fmaxf(fmaf(x, u, q), 1e-30f) : (disc * frsqrt(disc) - x * u);
+          const float quo = fdiv(out ? P : -P, den);
+          s_rout = fmaxf(out ? quo : q - x * u, 0.f) * ist;
+          if (!out && e1.x > 0.f && disc > 0.f) s_rin = fmaxf(quo, 0.f) * ist;
+        }
+        if (fabsf(v) > 1e-15f) sy = fmaxf(fdiv((v > 0.f ? e2.y : e2.x) - y, v), 0.f);
+        sb = fminf(fminf(s_rin, s_rout), sy);
       }
-      if (v > 1e-15f) s_zhi = fmaxf(fdiv(zhi - y, v), 0.f);
-      else if (v < -1e-15f) s_zlo = fmaxf(fdiv(zlo - y, v), 0.f);
-      sb = fminf(fminf(s_rin, s_rout), fminf(s_zlo, s_zhi));
     }
-    // ---- effective-scatter distance (reference cap: sigma_s*L > 1e4 -> 1e4/L) ----
-    // -log(u)/sigma competes with s_other = min(boundary, census); the logarithm is
-    // evaluated only when it can win (scatter_may_win).
-    float ds = BIGF;
-    {
-      const bool capped = !MG2 && ss * L > 10000.0f;
-      const float sig = capped ? 10000.0f / L : (ss > ss_thr ? ss : 0.f);
-      if (sig > 0.f) {
-        const float s_other = fminf(sb, dcen);
-        if (scatter_may_win(r.x, sig, s_other))
-          ds = capped ? neglog_u(r.x) * (L * 1e-4f) : fdiv(neglog_u(r.x), ss);
-      }
-    }
+    // ---- effective scatter and census ----
+    float L = e1.y - e1.x;  // used by capped cells only
+    if (!ONED) L = fminf(L, e2.y - e2.x);
+    const float ds = scatter_flight<!MG2>(ss, L, r.x, fminf(sb, h.dcen));
     d = sb; evt = EV_BOUNDARY;
     if (ds < d) { d = ds; evt = EV_SCATTER; }
-    if (dcen < d) { d = dcen; evt = EV_CENSUS; }
+    if (h.dcen < d) { d = h.dcen; evt = EV_CENSUS; }
     // ---- move ----
     if (GEOM == G_SLAB) {
-      const float xl = E1[ci], xr = E1[ci + 1];
       xn = fmaf(u, d, x);
-      if (evt == EV_BOUNDARY) { if (u > 0.f) { xn = xr; cross = X_IP; } else { xn = xl; cross = X_IM; } }
-      else { if (evt == EV_SCATTER) un = fmaf(2.f, u01f(r.y), -1.f); xn = fminf(fmaxf(xn, xl), xr); }
+      if (evt == EV_BOUNDARY) { di = u > 0.f ? 1 : -1; xn = u > 0.f ? e1.y : e1.x; }
+      else { if (evt == EV_SCATTER) un = fmaf(2.f, u01f(r.y), -1.f); xn = fminf(fmaxf(xn, e1.x), e1.y); }
     } else if (GEOM == G_SPHERE) {
-      const float r0 = E1[ci], r1 = E1[ci + 1];
       const float ax = fmaf(u, d, x);
-      float rn = sqrt_nn(fmaf(ax, ax, d * d * ((1.f - u) * (1.f + u))));
+      float rn = sqrt_nn(fmaf(ax, ax, d * d * om));
       float mun = rn > 1e-15f ? (x * u + d) / rn : 1.f;
       if (evt == EV_BOUNDARY) {
-        if (dout <= din) { rn = r1; mun = (x * u + d) / r1; cross = X_IP; }
-        else { rn = r0; mun = (x * u + d) / r0; cross = X_IM; }
+        di = dout <= din ? 1 : -1;
+        rn = dout <= din ? e1.y : e1.x;
+        mun = (x * u + d) / rn;
       } else {
         if (evt == EV_SCATTER) mun = fmaf(2.f, u01f(r.y), -1.f);
-        rn = fminf(fmaxf(rn, r0), r1);
+        rn = fminf(fmaxf(rn, e1.x), e1.y);
       }
       xn = rn; un = fminf(1.f, fmaxf(-1.f, mun));
     } else if (GEOM == G_XY) {
-      const float xl = E1[ci], xr = E1[ci + 1], yl = E2[cj], yr = E2[cj + 1];
       xn = fmaf(u, d, x); yn = fmaf(v, d, y);
       if (evt == EV_BOUNDARY) {
-        if (sx <= sy) { if (u > 0.f) { xn = xr; cross = X_IP; } else { xn = xl; cross = X_IM; } yn = fminf(fmaxf(yn, yl), yr); }
-        else { if (v > 0.f) { yn = yr; cross = X_JP; } else { yn = yl; cross = X_JM; } xn = fminf(fmaxf(xn, xl), xr); }
-      } else {
-        if (evt == EV_SCATTER) {
-          const float uz = fmaf(2.f, u01f(r.y), -1.f);
-          const float rxy = sqrt_nn((1.f - uz) * (1.f + uz));
-          float sp, cp;
-          sincospif(2.f * u01f(r.z), &sp, &cp);
-          un = rxy * cp; vn = rxy * sp;
-        }
-        xn = fminf(fmaxf(xn, xl), xr); yn = fminf(fmaxf(yn, yl), yr);
+        if (sx <= sy) di = u > 0.f ? 1 : -1;
+        else dj = v > 0.f ? 1 : -1;
+      } else if (evt == EV_SCATTER) {
+        const float uz = fmaf(2.f, u01f(r.y), -1.f);
+        const float rxy = sqrt_nn((1.f - uz) * (1.f + uz));
+        float sp, cp;
+        sincospif(2.f * u01f(r.z), &sp, &cp);
+        un = rxy * cp; vn = rxy * sp;
       }
+      xn = di > 0 ? e1.y : di < 0 ? e1.x : fminf(fmaxf(xn, e1.x), e1.y);
+      yn = dj > 0 ? e2.y : dj < 0 ? e2.x : fminf(fmaxf(yn, e2.x), e2.y);
     } else {
-      const float rin = E1[ci], rout = E1[ci + 1], zlo = E2[cj], zhi = E2[cj + 1];
       const float l = d * st_;
       const float ax = fmaf(u, l, x);
-      float rn = sqrt_nn(fmaf(ax, ax, l * l * ((1.f - u) * (1.f + u))));
+      const float rn = sqrt_nn(fmaf(ax, ax, l * l * om));
       yn = fmaf(d, v, y);
       if (rn > 1e-15f && l > 0.f) un = fminf(1.f, fmaxf(-1.f, fdiv(fmaf(x, u, l), rn)));
       if (evt == EV_BOUNDARY) {
-        if (sb == s_rin) { rn = rin; cross = X_IM; }
-        else if (sb == s_rout) { rn = rout; cross = X_IP; }
-        else if (sb == s_zlo) { yn = zlo; cross = X_JM; }
-        else { yn = zhi; cross = X_JP; }
+        if (sb == s_rin) di = -1;
+        else if (sb == s_rout) di = 1;
+        else dj = v < 0.f ? -1 : 1;
       } else if (evt == EV_SCATTER) {
         vn = fmaf(2.f, u01f(r.y), -1.f);
         un = cospif(2.f * u01f(r.z));
       }
-      if (cross != X_IM && cross != X_IP) rn = fminf(fmaxf(rn, rin), rout);
-      if (cross != X_JM && cross != X_JP) yn = fminf(fmaxf(yn, zlo), zhi);
-      xn = rn;
+      xn = di > 0 ? e1.y : di < 0 ? e1.x : fminf(fmaxf(rn, e1.x), e1.y);
+      yn = dj > 0 ? e2.y : dj < 0 ? e2.x : fminf(fmaxf(yn, e2.x), e2.y);
     }
     // implicit capture (the energy removed is counted at the flush, w_in - w)
     const float wn = (MG2 && !(sa > 1e-12f)) ? w : w * __expf(-sa * d);
     // path-length intensity: w*s is needed only in cells without absorption (table
     // entry 0: below the estimator's threshold, or Carter-Forest); elsewhere it is
     // lost / (sigma_a V dt), formed from the deposition tally when the step ends
-    if (!(sa > 0.f)) acc_wd += (double)(w * d);
-    dcen -= d;
+    if (!(sa > 0.f)) o.wd = w * d;
+    h.dcen -= d;
     bool captured = false;
     if (CF && evt == EV_SCATTER) {
       // absorption (IMC/IMC1D_CarterForest.py:146-194, IMC/IMC2D_CarterForest.py:189-210)
       const float rate = __ldg(a.cf_rate + c);
-      const float tr = dcen / c_light;  // time left after the flight
+      const float tr = h.dcen / c_light;  // time left after the flight
       const uint32_t ub = ONED ? r.z : r.w;
       if (!(rate > 0.f)) {
         captured = !ONED;  // no re-emission: 1-D redirects, 2-D captures
@@ -220,56 +225,49 @@ __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut
         captured = u01f(ub) < __expf(-rate * tr);
       } else {
         const float delay = fdiv(neglog_u(ub), rate);
-        if (ONED ? (tr > 1e-14f && delay < tr) : (delay < tr - 1e-15f)) dcen = fmaxf(0.f, (tr - delay) * c_light);
+        if (ONED ? (tr > 1e-14f && delay < tr) : (delay < tr - 1e-15f)) h.dcen = fmaxf(0.f, (tr - delay) * c_light);
         else captured = true;
       }
       // a capture deposits the whole weight: w becomes 0 below, so w_in - w includes it
+      if (captured) atomicAdd(&blk_cnt[B_CAPTURE], 1u);
     }
-    if (evt == EV_BOUNDARY) ++s_bd;
-    else if (captured) atomicAdd(&blk_cnt[B_CAPTURE], 1u);
-    else if (evt == EV_SCATTER) ++s_sc;
-    else atomicAdd(&blk_cnt[B_CENSUS], 1u);
+    // crossings are counted as the events that are nothing else
+    s_sc += evt == EV_SCATTER && !captured ? 1u : 0u;
+    s_cen += evt == EV_CENSUS ? 1u : 0u;
 
-    if (!MG && !CF && (GEOM == G_XY || GEOM == G_RZ)) {
-      if (wn <= weight_floor) {
-        // IMC/IMC2D.py:1043-1047: history stops in place keeping its weight
-        atomicAdd(&blk_cnt[B_FLOOR], 1u);
-        w = wn;
-        frozen = true;
-        finished = true;
-      }
-    }
-    if (!frozen) {
-      w = captured ? 0.f : wn; x = xn; y = yn; u = un; v = vn;
+    if (!MG && !CF && !ONED && wn <= weight_floor) {
+      // IMC/IMC2D.py:1043-1047: history stops in place keeping its weight
+      atomicAdd(&blk_cnt[B_FLOOR], 1u);
+      h.w = wn;
+      finished = true;
+    } else {
+      h.w = captured ? 0.f : wn; h.x = xn; h.y = yn; h.u = un; h.v = vn;
       if (CF && captured) finished = true;
-      if (cross != X_NONE) {
+      if ((di | dj) != 0) {
         // leaving the cell: flush the visit (before an escape zeroes w) and start the next
-        flush = true; flush_cell = cq; f_lost = (double)w_in - (double)w; f_wd = acc_wd;
-        w_in = w; acc_wd = 0.0;
-        int ni = ci, nj = cj;
-        if (cross == X_IP) ++ni; else if (cross == X_IM) --ni; else if (cross == X_JP) ++nj; else --nj;
-        int side = -1;
-        if (ni < 0) side = 0; else if (ni >= a.nx) side = 1; else if (nj < 0) side = 2; else if (nj >= a.ny) side = 3;
-        if (side >= 0) {
-          if ((a.reflect_mask >> side) & 1) {
-            if (side < 2) { u = -u; ni = side == 0 ? 0 : a.nx - 1; }
-            else { v = -v; nj = side == 2 ? 0 : a.ny - 1; }
+        o.flush = true; o.lost = (double)h.w_in - (double)h.w;
+        h.w_in = h.w;
+        const int ni = h.ci + di, nj = h.cj + dj;
+        if ((unsigned)ni >= (unsigned)a.nx || (unsigned)nj >= (unsigned)a.ny) {
+          const int side = ni < 0 ? 0 : ni >= a.nx ? 1 : nj < 0 ? 2 : 3;
+          if ((a.reflect_mask >> side) & 1) {  // stays in its cell
+            if (side < 2) h.u = -h.u; else h.v = -h.v;
             atomicAdd(&blk_cnt[B_REFLECT], 1u);
           } else {
-            const unsigned long long uw = fx_units((double)w, inv_q);
+            const unsigned long long uw = fx_units((double)h.w, inv_q);
             atomicAdd(&blk_esc[side], uw);
-            if (MG) atomicAdd(a.esc_fx + 4 + grp, uw);
+            if (MG) atomicAdd(a.esc_fx + 4 + h.grp, uw);
             atomicAdd(&blk_cnt[B_ESCAPE], 1u);
-            w = 0.f;
+            h.w = 0.f;
             finished = true;
-            ni = ci; nj = cj;
           }
+        } else {
+          h.ci = ni; h.cj = nj;
+          h.tab = table(cq + di + a.nx * dj);
         }
-        ci = ni; cj = nj;
-        if (!finished) tab = table(MG ? ci + a.nx * cj + a.nc * grp : ci + a.nx * cj);
       }
-      if (GEOM == G_SLAB || GEOM == G_SPHERE) {
-        if (!CF && !finished && w < weight_floor) {
+      if (ONED) {
+        if (!CF && !finished && h.w < weight_floor) {
           // IMC/IMC1D.py:188-195: kill and deposit the remainder in the current cell
           // (every cell, including the two edge cells the reference skips).  Without a
           // crossing in this event the visit's flush at the history end (w_in - 0) carries
@@ -277,35 +275,29 @@ __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut
           // the new cell here.  Its intensity share, lost / (sigma_a V dt), follows from the
           // deposition tally.
           atomicAdd(&blk_cnt[B_FLOOR], 1u);
-          if (flush) {
-            const int c2 = ci + a.nx * cj + (MG ? a.nc * grp : 0);
-            atomicAdd(dep_t + c2, fx_units((double)w, inv_q));
+          if (o.flush) {
+            const int c2 = h.ci + a.nx * h.cj + (MG ? a.nc * h.grp : 0);
+            atomicAdd(dep_t + c2, fx_units((double)h.w, inv_q));
           }
-          w = 0.f;
+          h.w = 0.f;
           finished = true;
         }
-      } else if (MG2 && !finished && dcen > 0.f && w <= weight_floor) {
+      } else if (MG2 && !finished && h.dcen > 0.f && h.w <= weight_floor) {
         // MG_IMC/MG_IMC2D.py:858-860: the next event would stop at the floor (a weight
         // that underflowed to 0 included)
         atomicAdd(&blk_cnt[B_FLOOR], 1u);
         finished = true;
-      } else if (!finished && !(w > 0.f)) {
-        w = 0.f;
+      } else if (!finished && !(h.w > 0.f)) {
+        h.w = 0.f;
         finished = true;
       }
-      if (!finished && !(dcen > 0.f)) finished = true;
+      if (!(h.dcen > 0.f)) finished = true;
     }
   }
-  if (finished) {
-    // A history that ends without leaving its cell flushes that cell's visit now.  (One
-    // that ended by crossing has already queued the old cell and holds nothing new: a
-    // 1-D weight-floor kill after a crossing deposits directly.)
-    if (!flush) {
-      const double lost = (double)w_in - (double)w;
-      if (lost != 0.0 || acc_wd != 0.0) { flush = true; flush_cell = cq; f_lost = lost; f_wd = acc_wd; }
-    }
-    acc_wd = 0.0;
-  }
+  // A history that ends without leaving its cell flushes that cell's visit now.  (One
+  // that ended by crossing has already queued the old cell and holds nothing new: a
+  // 1-D weight-floor kill after a crossing deposits directly.)
+  if (finished && !o.flush) { o.flush = true; o.lost = (double)h.w_in - (double)h.w; }
   o.finished = finished;
 }
 
@@ -344,10 +336,42 @@ __device__ __forceinline__ bool claim_run(const TrackArgs& a, uint32_t n, uint32
   return true;
 }
 
+// The block's event counts and escaped energy to the global ones (every thread calls it; ends
+// with the block synchronised): events, scatters and census events from the threads' own
+// counters, the rare ones from blk_cnt; crossings are the events that are none of those.
+__device__ __forceinline__ void add_event_counts(const TrackArgs& a, const unsigned* blk_cnt,
+                                                 const unsigned long long* blk_esc, unsigned s_ev, unsigned s_cen,
+                                                 unsigned s_sc) {
+  __shared__ unsigned long long tot[3];
+  if (threadIdx.x < 3) tot[threadIdx.x] = 0ull;
+  __syncthreads();
+  const unsigned long long t_ev = warp_sum_u(s_ev), t_cen = warp_sum_u(s_cen), t_sc = warp_sum_u(s_sc);
+  if ((threadIdx.x & 31) == 0) {
+    if (t_ev) atomicAdd(&tot[0], t_ev);
+    if (t_cen) atomicAdd(&tot[1], t_cen);
+    if (t_sc) atomicAdd(&tot[2], t_sc);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned long long cap = blk_cnt[B_CAP], capt = blk_cnt[B_CAPTURE];
+    const unsigned long long bd = tot[0] - tot[1] - tot[2] - capt;
+    if (tot[0] + cap) atomicAdd(a.stats + S_EVENTS, tot[0] + cap);
+    if (bd) atomicAdd(a.stats + S_BOUNDARY, bd);
+    if (tot[2]) atomicAdd(a.stats + S_SCATTER, tot[2]);
+    if (tot[1]) atomicAdd(a.stats + S_CENSUS, tot[1]);
+    if (capt) atomicAdd(a.stats + S_CAPTURE, capt);
+    if (blk_cnt[B_FLOOR]) atomicAdd(a.stats + S_FLOOR, (unsigned long long)blk_cnt[B_FLOOR]);
+    if (blk_cnt[B_REFLECT]) atomicAdd(a.stats + S_REFLECT, (unsigned long long)blk_cnt[B_REFLECT]);
+    if (cap) atomicAdd(a.stats + S_CAP, cap);
+    if (blk_cnt[B_ESCAPE]) atomicAdd(a.stats + S_ESCAPE, (unsigned long long)blk_cnt[B_ESCAPE]);
+  }
+  if (threadIdx.x < 4 && blk_esc[threadIdx.x] != 0ull) atomicAdd(a.esc_fx + threadIdx.x, blk_esc[threadIdx.x]);
+}
+
 // 64-bit add to a shared-memory tally as two 32-bit adds, the low word's carry going into the
 // high word: the sum is exact modulo 2^64 in any order, and both adds are native shared-memory
-// atomics, where the 64-bit one is a compare-and-swap loop (crooked pipe, 68 M segments a launch:
-// 1.53 ms with the 64-bit atomic, 1.37 ms so).
+// atomics, where the 64-bit one is a compare-and-swap loop (the ten launches of a 2M crooked-pipe
+// run: 14.0 ms with the 64-bit atomic, 12.6 ms so).
 __device__ __forceinline__ void smem_add_u64(unsigned long long* t, unsigned long long v) {
   unsigned* q = reinterpret_cast<unsigned*>(t);
   const unsigned lo = (unsigned)v;
@@ -365,13 +389,14 @@ __device__ __forceinline__ void smem_add_u64(unsigned long long* t, unsigned lon
 // Grouping lanes by cell costs a warp-wide match and a serial sum over each group's lanes at nearly
 // every event; a shared-memory atomic per flushing lane does not.  T_SMALL serves meshes whose
 // tallies fit beside each of several blocks an SM; T_WIDE every mesh whose one tally fits in an
-// SM's shared memory once (26 thousand entries).  Crooked pipe 60 x 210, 8.7 M histories, 68 M
-// segments a launch: 2.47 ms with T_GLOBAL at the default launch shape, 1.37 ms with T_WIDE.
+// SM's shared memory once (26 thousand entries).  The ten launches of a crooked-pipe run
+// (60 x 210, up to 8.7 M histories and 68 M segments a launch): 18.6 ms with T_GLOBAL at the
+// default launch shape, 12.6 ms with T_WIDE.
 //
 // Ended histories wait until kRefillMin lanes of the warp are idle; then their final states and
 // census sums are stored and the lanes refilled in one go, so this part runs once per kRefillMin
 // endings instead of whenever any lane ends (at about 8 segments per history, nearly every
-// event): the same launch 1.57 ms at 1, 1.43 at 4, 1.37 at 8, 1.37 at 12.
+// event): the same ten launches 14.5 ms at 1, 13.2 at 4, 12.6 at 8, 12.6 at 12.
 constexpr int kRefillMin = 8;
 constexpr int kWideThreads = 1024;
 enum : int { T_GLOBAL = 0, T_SMALL, T_WIDE };
@@ -391,15 +416,15 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
   constexpr bool TS_S = TALLY == T_SMALL || (TALLY == T_WIDE && CF);   // intensity in shared memory
   WarpStage* stages = reinterpret_cast<WarpStage*>(smem);
   const int nwarps = blockDim.x >> 5;
-  float* E1 = reinterpret_cast<float*>(stages + nwarps);
-  float* E2 = E1 + (a.nx + 1);
-  float2* CS = reinterpret_cast<float2*>(E2 + (a.ny + 1) + ((a.nx + a.ny) & 1));
+  float2* E1 = reinterpret_cast<float2*>(stages + nwarps);  // (lower, upper) edge per index
+  float2* E2 = E1 + a.nx;
+  float2* CS = E2 + a.ny;
   const int ncg = a.nc * a.ng;
   unsigned long long* TD = reinterpret_cast<unsigned long long*>(CS + (SMEM_CELLS ? ncg : 0));
   double* TS = reinterpret_cast<double*>(TD + (TD_S ? ncg : 0));
   unsigned long long* const dep_t = TD_S ? TD : a.dep_fx;
-  for (int q = threadIdx.x; q <= a.nx; q += blockDim.x) E1[q] = a.e1[q];
-  for (int q = threadIdx.x; q <= a.ny; q += blockDim.x) E2[q] = a.e2[q];
+  for (int q = threadIdx.x; q < a.nx; q += blockDim.x) E1[q] = make_float2(a.e1[q], a.e1[q + 1]);
+  for (int q = threadIdx.x; q < a.ny; q += blockDim.x) E2[q] = make_float2(a.e2[q], a.e2[q + 1]);
   if (SMEM_CELLS)
     for (int q = threadIdx.x; q < ncg; q += blockDim.x) CS[q] = a.sass[q];
   if (TD_S) for (int q = threadIdx.x; q < ncg; q += blockDim.x) TD[q] = 0ull;
@@ -418,9 +443,10 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
   bool has = false, pend = false;  // pend: an ended history whose final state is not stored yet
   Hist h;
   h.pid = 0; h.ev = 0; h.x = h.y = h.u = h.v = h.w = h.dcen = h.w_in = 0.f;
-  h.ci = h.cj = h.grp = 0; h.tab = make_float2(0.f, 0.f); h.acc_wd = 0.0;
+  h.ci = h.cj = h.grp = 0; h.tab = make_float2(0.f, 0.f); h.key = DrawKey{0u, 0u, 0u};
+  const uint32_t rkx = draw_step_key(a.rk, stepk);
   auto table = [&](int cq) { return SMEM_CELLS ? CS[cq] : __ldg(a.sass + cq); };
-  unsigned s_bd = 0, s_sc = 0;
+  unsigned s_ev = 0, s_cen = 0, s_sc = 0;  // events of ended histories, census events, scatters
   unsigned n_alive = 0;                 // entries alive at the end (census sums for the comb)
   const float c_light = (float)C_LIGHT;
   // weight floor, IMC/IMC1D.py:1007 / IMC/IMC2D.py:1771 (1e-10); MG_IMC/MG_IMC1D.py:1127 (1e-14)
@@ -434,7 +460,7 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
       // ---------------- store the ended histories, refill from the warp's run ----------------
       bool cen = false;
       int cen_bin = 0;
-      if (pend) cen = history_retire<GEOM>(a, h, cen_bin);
+      if (pend) { cen = history_retire<GEOM>(a, h, cen_bin); s_ev += h.ev; }
       if (a.ecen) {
         warp_tally1(cen, cen_bin, (double)h.w, a.ecen, st);
         n_alive += cen ? 1u : 0u;
@@ -478,7 +504,7 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
               h.tab = table(MG ? c + a.nc * h.grp : c);
               h.ev = 0;
               h.w_in = h.w;
-              h.acc_wd = 0.0;
+              h.key = draw_key(a.rk, a.id_base + h.pid, stepk, TAG_TRANSPORT);
               has = true;
             }
           }
@@ -492,58 +518,33 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
     if (has && (h.ci < 0 || h.ci >= a.nx || h.cj < 0 || h.cj >= a.ny || !isfinite(h.w) || !isfinite(h.x) ||
                 !isfinite(h.dcen))) {
       atomicOr(a.flags, (int)IMC_FLAG_BOUNDS);
-      h.w_in = h.w; h.acc_wd = 0.0;  // nothing is tallied at an invalid index
-      has = false;
+      has = false;  // nothing more is tallied at an invalid index
     }
 #endif
-    EvOut o{false, 0, 0.0, 0.0, false};
+    EvOut o{0, false, 0.f, 0.0, false};
     if (has) {
-      history_event<GEOM, SMEM_CELLS, MG, CF>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t, stepk, weight_floor,
-                                              inv_q, s_bd, s_sc);
+      history_event<GEOM, SMEM_CELLS, MG, CF>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t, rkx, weight_floor,
+                                              inv_q, s_cen, s_sc);
       if (o.finished) { has = false; pend = true; }
     }
-    // ---------------- tally flush ----------------
-    // deposited energy in fixed point; w*s (raw, only from cells without absorption) in FP64
-    if (TALLY == T_GLOBAL) {
-      unsigned long long ud = 0ull;
-      double vs = 0.0;
-      if (o.flush) { ud = fx_units(o.f_lost, inv_q); vs = o.f_wd; }
-      warp_tally_fx(o.flush, o.flush_cell, ud, vs, dep_t, a.si, st);
-    } else {
-      unsigned long long ud = 0ull;
-      if (o.flush) {
-        ud = fx_units(o.f_lost, inv_q);
-        if (TD_S && ud) smem_add_u64(TD + o.flush_cell, ud);
-        if (TS_S && o.f_wd != 0.0) atomicAdd(TS + o.flush_cell, o.f_wd);
-      }
-      if (!TS_S) warp_tally1(o.flush && o.f_wd != 0.0, o.flush_cell, o.f_wd, a.si, st);
-      if (!TD_S) warp_tally_fx(o.flush && ud != 0ull, o.flush_cell, ud, 0.0, a.dep_fx, a.si, st);
-    }
+    // ---------------- tallies ----------------
+    // deposited energy in fixed point when a cell visit ends; w*s (raw, only from cells without
+    // absorption) in FP64 at every flight
+    const unsigned long long ud = o.flush ? fx_units(o.lost, inv_q) : 0ull;
+    const double vs = (double)o.wd;
+    if (TD_S && ud) smem_add_u64(TD + o.cell, ud);
+    if (TS_S && o.wd != 0.f) atomicAdd(TS + o.cell, vs);
+    if (!TD_S && !TS_S) warp_tally_fx(ud != 0ull || o.wd != 0.f, o.cell, ud, vs, a.dep_fx, a.si, st);
+    else if (!TD_S) warp_tally_fx(ud != 0ull, o.cell, ud, 0.0, a.dep_fx, a.si, st);
+    else if (!TS_S) warp_tally1(o.wd != 0.f, o.cell, vs, a.si, st);
   }
 
   // ---------------- statistics ----------------
-  const unsigned long long t_bd = warp_sum_u(s_bd), t_sc = warp_sum_u(s_sc);
   if (a.ecen) {
     const unsigned long long t_alive = warp_sum_u(n_alive);
     if (lane == 0 && t_alive) atomicAdd(a.n_live, t_alive);
   }
-  if (lane == 0) {
-    if (t_bd) atomicAdd(a.stats + S_BOUNDARY, t_bd);
-    if (t_sc) atomicAdd(a.stats + S_SCATTER, t_sc);
-    if (t_bd + t_sc) atomicAdd(a.stats + S_EVENTS, t_bd + t_sc);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned long long cen = blk_cnt[B_CENSUS], cap = blk_cnt[B_CAP], capt = blk_cnt[B_CAPTURE];
-    if (cen) atomicAdd(a.stats + S_CENSUS, cen);
-    if (capt) atomicAdd(a.stats + S_CAPTURE, capt);
-    if (cen + cap + capt) atomicAdd(a.stats + S_EVENTS, cen + cap + capt);
-    if (blk_cnt[B_FLOOR]) atomicAdd(a.stats + S_FLOOR, (unsigned long long)blk_cnt[B_FLOOR]);
-    if (blk_cnt[B_REFLECT]) atomicAdd(a.stats + S_REFLECT, (unsigned long long)blk_cnt[B_REFLECT]);
-    if (cap) atomicAdd(a.stats + S_CAP, cap);
-    if (blk_cnt[B_ESCAPE]) atomicAdd(a.stats + S_ESCAPE, (unsigned long long)blk_cnt[B_ESCAPE]);
-  }
-  if (threadIdx.x < 4 && blk_esc[threadIdx.x] != 0ull) atomicAdd(a.esc_fx + threadIdx.x, blk_esc[threadIdx.x]);
+  add_event_counts(a, blk_cnt, blk_esc, s_ev, s_cen, s_sc);
   // the block's tallies (every warp's last flush is behind the __syncthreads above)
   if (TD_S) for (int q = threadIdx.x; q < ncg; q += blockDim.x) if (TD[q]) atomicAdd(a.dep_fx + q, TD[q]);
   if (TS_S) for (int q = threadIdx.x; q < ncg; q += blockDim.x) if (TS[q] != 0.0) atomicAdd(a.si + q, TS[q]);
@@ -575,17 +576,17 @@ __global__ void __launch_bounds__(256, 4) k_track_pf(TrackArgs a) {  // at most 
   constexpr bool MG2 = MG && !ONED;  // MG_IMC2D history rules
   WarpStage* stages = reinterpret_cast<WarpStage*>(smem);
   const int nwarps = blockDim.x >> 5;
-  float* E1 = reinterpret_cast<float*>(stages + nwarps);
-  float* E2 = E1 + (a.nx + 1);
-  float2* CS = reinterpret_cast<float2*>(E2 + (a.ny + 1) + ((a.nx + a.ny) & 1));
+  float2* E1 = reinterpret_cast<float2*>(stages + nwarps);  // (lower, upper) edge per index
+  float2* E2 = E1 + a.nx;
+  float2* CS = E2 + a.ny;
   const int ncg = a.nc * a.ng;
   // block tallies after the table (8-byte aligned: CS is), deposition then intensity
   unsigned long long* TD = reinterpret_cast<unsigned long long*>(CS + (SMEM_CELLS ? ncg : 0));
   double* TS = reinterpret_cast<double*>(TD + ncg);
   unsigned long long* const dep_t = SMEM_TALLY ? TD : a.dep_fx;
   double* const si_t = SMEM_TALLY ? TS : a.si;
-  for (int q = threadIdx.x; q <= a.nx; q += blockDim.x) E1[q] = a.e1[q];
-  for (int q = threadIdx.x; q <= a.ny; q += blockDim.x) E2[q] = a.e2[q];
+  for (int q = threadIdx.x; q < a.nx; q += blockDim.x) E1[q] = make_float2(a.e1[q], a.e1[q + 1]);
+  for (int q = threadIdx.x; q < a.ny; q += blockDim.x) E2[q] = make_float2(a.e2[q], a.e2[q + 1]);
   if (SMEM_CELLS)
     for (int q = threadIdx.x; q < ncg; q += blockDim.x) CS[q] = a.sass[q];
   if (SMEM_TALLY)
@@ -615,8 +616,9 @@ __global__ void __launch_bounds__(256, 4) k_track_pf(TrackArgs a) {  // at most 
   // energy removed in the current cell visit: the per-flight differences telescope, so it is
   // the weight at the visit's start minus the weight now (one FP64 difference at the flush)
   float w_in = 0.f;
-  double acc_wd = 0.0;  // w*s in the current cell (cells without absorption only)
-  unsigned s_bd = 0, s_sc = 0;          // per-event counters (census/cap counted at finish)
+  DrawKey key{0u, 0u, 0u};
+  const uint32_t rkx = draw_step_key(a.rk, stepk);
+  unsigned s_ev = 0, s_cen = 0, s_sc = 0;  // events of ended histories, census events, scatters
   unsigned n_alive = 0;                 // entries alive at the end (census sums for the comb)
 
   const float c_light = (float)C_LIGHT;
@@ -671,6 +673,7 @@ __global__ void __launch_bounds__(256, 4) k_track_pf(TrackArgs a) {  // at most 
               tab = table(MG ? c + a.nc * grp : c);
               ev = 0;
               w_in = w;
+              key = draw_key(a.rk, a.id_base + pid, stepk, TAG_TRANSPORT);
               has = true;
             }
           }
@@ -726,39 +729,28 @@ __global__ void __launch_bounds__(256, 4) k_track_pf(TrackArgs a) {  // at most 
 #ifdef IMC_CHECKED
     if (has && (ci < 0 || ci >= a.nx || cj < 0 || cj >= a.ny || !isfinite(w) || !isfinite(x) || !isfinite(dcen))) {
       atomicOr(a.flags, (int)IMC_FLAG_BOUNDS);
-      w_in = w; acc_wd = 0.0;  // nothing is tallied at an invalid index
-      has = false;
+      has = false;  // nothing more is tallied at an invalid index
     }
 #endif
 
-    EvOut o{false, 0, 0.0, 0.0, false};
+    EvOut o{0, false, 0.f, 0.0, false};
     bool cen = false;
     int cen_bin = 0;
     if (has) {
-      Hist h{pid, ev, x, y, u, v, w, dcen, w_in, ci, cj, grp, tab, acc_wd};
-      history_event<GEOM, SMEM_CELLS, MG, CF>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t, stepk, weight_floor,
-                                              inv_q, s_bd, s_sc);
+      Hist h{pid, ev, x, y, u, v, w, dcen, w_in, ci, cj, grp, tab, key};
+      history_event<GEOM, SMEM_CELLS, MG, CF>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t, rkx, weight_floor,
+                                              inv_q, s_cen, s_sc);
       pid = h.pid; ev = h.ev; x = h.x; y = h.y; u = h.u; v = h.v; w = h.w; dcen = h.dcen; w_in = h.w_in;
-      ci = h.ci; cj = h.cj; grp = h.grp; tab = h.tab; acc_wd = h.acc_wd;
-      if (o.finished) { has = false; cen = history_retire<GEOM>(a, h, cen_bin); }
+      ci = h.ci; cj = h.cj; grp = h.grp; tab = h.tab;
+      if (o.finished) { has = false; cen = history_retire<GEOM>(a, h, cen_bin); s_ev += h.ev; }
     }
-    const bool flush = o.flush;
-    const int flush_cell = o.flush_cell;
-    const double f_lost = o.f_lost, f_wd = o.f_wd;
-    // ---------------- converged tally flush ----------------
-    // deposited energy in fixed point; w*s (raw, only from cells without absorption) in FP64
-    unsigned long long ud = 0ull;
-    double vs = 0.0;
-    if (flush) {
-      ud = fx_units(f_lost, inv_q);
-      vs = f_wd;
-    }
+    const unsigned long long ud = o.flush ? fx_units(o.lost, inv_q) : 0ull;
+    const double vs = (double)o.wd;
     if (SMEM_TALLY) {
-      // block tallies in shared memory: one shared atomic per flushing lane costs less than
-      // grouping the warp's lanes by cell first (the grouping pays off for global tallies)
-      if (flush) { if (ud) atomicAdd(dep_t + flush_cell, ud); if (vs != 0.0) atomicAdd(si_t + flush_cell, vs); }
+      if (ud) smem_add_u64(dep_t + o.cell, ud);
+      if (o.wd != 0.f) atomicAdd(si_t + o.cell, vs);
     } else {
-      warp_tally_fx(flush, flush_cell, ud, vs, dep_t, si_t, st);
+      warp_tally_fx(ud != 0ull || o.wd != 0.f, o.cell, ud, vs, dep_t, si_t, st);
     }
     if (a.ecen) {
       warp_tally1(cen, cen_bin, (double)w, a.ecen, st);
@@ -767,28 +759,11 @@ __global__ void __launch_bounds__(256, 4) k_track_pf(TrackArgs a) {  // at most 
   }
 
   // ---------------- statistics ----------------
-  const unsigned long long t_bd = warp_sum_u(s_bd), t_sc = warp_sum_u(s_sc);
   if (a.ecen) {
     const unsigned long long t_alive = warp_sum_u(n_alive);
     if (lane == 0 && t_alive) atomicAdd(a.n_live, t_alive);
   }
-  if (lane == 0) {
-    if (t_bd) atomicAdd(a.stats + S_BOUNDARY, t_bd);
-    if (t_sc) atomicAdd(a.stats + S_SCATTER, t_sc);
-    if (t_bd + t_sc) atomicAdd(a.stats + S_EVENTS, t_bd + t_sc);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned long long cen = blk_cnt[B_CENSUS], cap = blk_cnt[B_CAP], capt = blk_cnt[B_CAPTURE];
-    if (cen) atomicAdd(a.stats + S_CENSUS, cen);
-    if (capt) atomicAdd(a.stats + S_CAPTURE, capt);
-    if (cen + cap + capt) atomicAdd(a.stats + S_EVENTS, cen + cap + capt);
-    if (blk_cnt[B_FLOOR]) atomicAdd(a.stats + S_FLOOR, (unsigned long long)blk_cnt[B_FLOOR]);
-    if (blk_cnt[B_REFLECT]) atomicAdd(a.stats + S_REFLECT, (unsigned long long)blk_cnt[B_REFLECT]);
-    if (cap) atomicAdd(a.stats + S_CAP, cap);
-    if (blk_cnt[B_ESCAPE]) atomicAdd(a.stats + S_ESCAPE, (unsigned long long)blk_cnt[B_ESCAPE]);
-  }
-  if (threadIdx.x < 4 && blk_esc[threadIdx.x] != 0ull) atomicAdd(a.esc_fx + threadIdx.x, blk_esc[threadIdx.x]);
+  add_event_counts(a, blk_cnt, blk_esc, s_ev, s_cen, s_sc);
   if (SMEM_TALLY) {
     // the block's tallies (every warp's last flush is behind the __syncthreads above)
     for (int q = threadIdx.x; q < ncg; q += blockDim.x) {
@@ -801,7 +776,7 @@ __global__ void __launch_bounds__(256, 4) k_track_pf(TrackArgs a) {  // at most 
 // dynamic shared memory of the tracking kernels: per-warp staging, edges, the cell table and
 // `tallies` 8-byte block tallies per (group, cell)
 inline size_t track_smem(const TrackArgs& a, int block, bool cells, int tallies) {
-  size_t sh = (block / 32) * sizeof(WarpStage) + sizeof(float) * (a.nx + a.ny + 4);
+  size_t sh = (block / 32) * sizeof(WarpStage) + sizeof(float2) * (a.nx + a.ny);
   if (cells) sh += sizeof(float2) * a.nc * a.ng;
   return sh + 8ull * tallies * a.nc * a.ng;
 }
@@ -853,7 +828,7 @@ cudaError_t launch_geom(const TrackArgs& a, const TrackLaunch& l, cudaStream_t s
 struct EventScratch {
   uint32_t* live[2];        // lists of live bank indices
   unsigned* count;          // [2] their lengths
-  uint32_t* ev; float* dcen; float* w_in; double* acc_wd;  // [capacity]
+  uint32_t* ev; float* dcen; float* w_in; // [capacity]
 };
 
 // The histories that move (as k_track's refill decides) into list 0, with their scratch state.
@@ -872,7 +847,7 @@ __global__ void k_event_init(TrackArgs a, EventScratch e) {
       const float w = a.w[k];
       const float dc = (dtk - a.t[k]) * (float)C_LIGHT;
       moves = (MG2CF ? w > weight_floor : w > 0.f) && dc > 0.f;
-      if (moves) { e.ev[k] = 0u; e.dcen[k] = dc; e.w_in[k] = w; e.acc_wd[k] = 0.0; }
+      if (moves) { e.ev[k] = 0u; e.dcen[k] = dc; e.w_in[k] = w; }
     }
     const unsigned m = __ballot_sync(FULL, moves);
     unsigned base = 0;
@@ -890,10 +865,10 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
   __shared__ unsigned long long blk_esc[4];
   WarpStage* stages = reinterpret_cast<WarpStage*>(smem);
   const int nwarps = blockDim.x >> 5;
-  float* E1 = reinterpret_cast<float*>(stages + nwarps);
-  float* E2 = E1 + (a.nx + 1);
-  for (int q = threadIdx.x; q <= a.nx; q += blockDim.x) E1[q] = a.e1[q];
-  for (int q = threadIdx.x; q <= a.ny; q += blockDim.x) E2[q] = a.e2[q];
+  float2* E1 = reinterpret_cast<float2*>(stages + nwarps);
+  float2* E2 = E1 + a.nx;
+  for (int q = threadIdx.x; q < a.nx; q += blockDim.x) E1[q] = make_float2(a.e1[q], a.e1[q + 1]);
+  for (int q = threadIdx.x; q < a.ny; q += blockDim.x) E2[q] = make_float2(a.e2[q], a.e2[q + 1]);
   if (threadIdx.x < B_N) blk_cnt[threadIdx.x] = 0u;
   if (threadIdx.x < 4) blk_esc[threadIdx.x] = 0ull;
   __syncthreads();
@@ -906,13 +881,14 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
   const uint32_t* live_in = e.live[cur];
   uint32_t* live_out = e.live[cur ^ 1];
   unsigned* n_out = e.count + (cur ^ 1);
-  unsigned s_bd = 0, s_sc = 0;
+  unsigned s_ev = 0, s_cen = 0, s_sc = 0;  // events, census events, scatters
+  const uint32_t rkx = draw_step_key(a.rk, stepk);
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t trips = (n_in + stride - 1) / stride;
   for (uint32_t it = 0; it < trips; ++it) {
     const uint32_t i = it * stride + blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = i < n_in;
-    EvOut o{false, 0, 0.0, 0.0, false};
+    EvOut o{0, false, 0.f, 0.0, false};
     bool alive = false;
     uint32_t pid = 0;
     if (active) {
@@ -924,7 +900,7 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
       if (GEOM == G_XY || GEOM == G_RZ) { h.y = a.p2[pid]; h.v = a.d2[pid]; }
       h.grp = MG ? a.group[pid] : 0;
       const int c = a.cell[pid];
-      h.ev = e.ev[pid]; h.dcen = e.dcen[pid]; h.w_in = e.w_in[pid]; h.acc_wd = e.acc_wd[pid];
+      h.ev = e.ev[pid]; h.dcen = e.dcen[pid]; h.w_in = e.w_in[pid];
 #ifdef IMC_CHECKED
       // bounds-checked build: an entry outside the mesh or group range, or with a non-finite
       // weight or position, is reported and dropped from the loop untouched
@@ -937,8 +913,11 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
       {
         h.cj = c / a.nx; h.ci = c - h.cj * a.nx;
         h.tab = __ldg(a.sass + (MG ? c + a.nc * h.grp : c));
-        history_event<GEOM, false, MG, CF>(a, h, o, E1, E2, nullptr, blk_cnt, blk_esc, a.dep_fx, stepk,
-                                           weight_floor, inv_q, s_bd, s_sc);
+        h.key = draw_key(a.rk, a.id_base + pid, stepk, TAG_TRANSPORT);
+        const uint32_t ev0 = h.ev;
+        history_event<GEOM, false, MG, CF>(a, h, o, E1, E2, nullptr, blk_cnt, blk_esc, a.dep_fx, rkx,
+                                           weight_floor, inv_q, s_cen, s_sc);
+        s_ev += h.ev - ev0;
         int bin;
         if (o.finished) history_retire<GEOM>(a, h, bin);
       }
@@ -947,7 +926,7 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
         a.p1[pid] = h.x; a.d1[pid] = h.u; a.w[pid] = h.w;
         if (GEOM == G_XY || GEOM == G_RZ) { a.p2[pid] = h.y; a.d2[pid] = h.v; }
         a.cell[pid] = h.ci + a.nx * h.cj;
-        e.ev[pid] = h.ev; e.dcen[pid] = h.dcen; e.w_in[pid] = h.w_in; e.acc_wd[pid] = h.acc_wd;
+        e.ev[pid] = h.ev; e.dcen[pid] = h.dcen; e.w_in[pid] = h.w_in;
       }
     }
     // survivors into the next list (warp-aggregated append)
@@ -956,32 +935,15 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
     if (lane == 0 && m) base = atomicAdd(n_out, (unsigned)__popc(m));
     base = __shfl_sync(FULL, base, 0);
     if (alive) live_out[base + __popc(m & ((1u << lane) - 1u))] = pid;
-    const unsigned long long ud = o.flush ? fx_units(o.f_lost, inv_q) : 0ull;
-    warp_tally_fx(o.flush, o.flush_cell, ud, o.flush ? o.f_wd : 0.0, a.dep_fx, a.si, st);
+    const unsigned long long ud = o.flush ? fx_units(o.lost, inv_q) : 0ull;
+    warp_tally_fx(ud != 0ull || o.wd != 0.f, o.cell, ud, (double)o.wd, a.dep_fx, a.si, st);
   }
-  const unsigned long long t_bd = warp_sum_u(s_bd), t_sc = warp_sum_u(s_sc);
-  if (lane == 0) {
-    if (t_bd) atomicAdd(a.stats + S_BOUNDARY, t_bd);
-    if (t_sc) atomicAdd(a.stats + S_SCATTER, t_sc);
-    if (t_bd + t_sc) atomicAdd(a.stats + S_EVENTS, t_bd + t_sc);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned long long cen = blk_cnt[B_CENSUS], cap = blk_cnt[B_CAP], capt = blk_cnt[B_CAPTURE];
-    if (cen) atomicAdd(a.stats + S_CENSUS, cen);
-    if (capt) atomicAdd(a.stats + S_CAPTURE, capt);
-    if (cen + cap + capt) atomicAdd(a.stats + S_EVENTS, cen + cap + capt);
-    if (blk_cnt[B_FLOOR]) atomicAdd(a.stats + S_FLOOR, (unsigned long long)blk_cnt[B_FLOOR]);
-    if (blk_cnt[B_REFLECT]) atomicAdd(a.stats + S_REFLECT, (unsigned long long)blk_cnt[B_REFLECT]);
-    if (cap) atomicAdd(a.stats + S_CAP, cap);
-    if (blk_cnt[B_ESCAPE]) atomicAdd(a.stats + S_ESCAPE, (unsigned long long)blk_cnt[B_ESCAPE]);
-  }
-  if (threadIdx.x < 4 && blk_esc[threadIdx.x] != 0ull) atomicAdd(a.esc_fx + threadIdx.x, blk_esc[threadIdx.x]);
+  add_event_counts(a, blk_cnt, blk_esc, s_ev, s_cen, s_sc);
 }
 
 template <int GEOM, bool MG, bool CF>
 cudaError_t launch_event(const TrackArgs& a, const EventScratch& e, int cur, int block, int grid, cudaStream_t s) {
-  const size_t sh = (block / 32) * sizeof(WarpStage) + sizeof(float) * (a.nx + a.ny + 4);
+  const size_t sh = (block / 32) * sizeof(WarpStage) + sizeof(float2) * (a.nx + a.ny);
   if (sh > 48 * 1024) {
     cudaError_t err = cudaFuncSetAttribute(k_event<GEOM, MG, CF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
     if (err != cudaSuccess) return err;
@@ -1051,7 +1013,7 @@ cudaError_t imc_launch_tally_finalize(const TrackArgs& a, cudaStream_t s) {
 size_t imc_event_scratch_bytes(long long capacity) {
   const size_t cap = (size_t)(capacity > 0 ? capacity : 1);
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  return al(8) + 2 * al(4 * cap) + 3 * al(4 * cap) + al(8 * cap);
+  return al(8) + 2 * al(4 * cap) + 3 * al(4 * cap);
 }
 
 cudaError_t imc_run_event_tracking(const TrackArgs& a, int geom, void* scratch, long long capacity,
@@ -1066,8 +1028,7 @@ cudaError_t imc_run_event_tracking(const TrackArgs& a, int geom, void* scratch, 
   e.live[1] = reinterpret_cast<uint32_t*>(p); p += al(4 * cap);
   e.ev = reinterpret_cast<uint32_t*>(p); p += al(4 * cap);
   e.dcen = reinterpret_cast<float*>(p); p += al(4 * cap);
-  e.w_in = reinterpret_cast<float*>(p); p += al(4 * cap);
-  e.acc_wd = reinterpret_cast<double*>(p);
+  e.w_in = reinterpret_cast<float*>(p);
   *cap_hit = false;
   cudaError_t err = cudaMemsetAsync(e.count, 0, 8, s);
   if (err != cudaSuccess) return err;
