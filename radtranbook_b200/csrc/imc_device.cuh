@@ -187,14 +187,14 @@ __device__ __forceinline__ float sqrt_nn(float x) { return x > 0.f ? x * frsqrt(
 
 __device__ __forceinline__ float outer_root(float r, float mu, float R, float b2) {
   const float q = sqrt_nn(fmaf(R, R, -b2));
-  float l = (mu >= 0.f) ? fdiv((R - r) * (R + r), fmaxf(fmaf(r, mu, q), 1e-30f)) : q - r * mu;
+  float l = (mu >= 0.f) ? fdiv((R - r) * (R + r), fmaxf(fmaf(r, mu, q), 1e-30f)) : fmaf(-r, mu, q);
   return fmaxf(l, 0.f);
 }
 __device__ __forceinline__ float inner_root(float r, float mu, float R, float b2) {
   if (!(R > 0.f) || !(mu < 0.f)) return BIGF;
   const float disc = fmaf(R, R, -b2);
   if (!(disc > 0.f)) return BIGF;
-  const float l = fdiv((r - R) * (r + R), disc * frsqrt(disc) - r * mu);
+  const float l = fdiv((r - R) * (r + R), fmaf(disc, frsqrt(disc), -(r * mu)));
   return fmaxf(l, 0.f);
 }
 

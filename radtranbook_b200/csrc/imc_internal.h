@@ -58,6 +58,7 @@ struct TrackArgs {
 // smem_tally: per-block deposition / intensity tallies in shared memory (with smem_cells only);
 // wide_ok: one block per SM with its tally in shared memory may be used where that fits;
 // prefetch: lanes copy their next history's bank record into shared memory while they track
+constexpr size_t kSmemPerBlock = 226 * 1024;  // dynamic shared memory of a wide block, beside its few hundred static bytes
 struct TrackLaunch {
   int block, blocks_per_sm, sms;
   bool smem_cells, smem_tally, wide_ok, prefetch;
@@ -83,8 +84,11 @@ struct AdjointArgs {
   const double* sa64;     // [c] Fleck absorption opacity (FP64)
   const double* ss64;     // [c] effective scatter opacity (FP64)
   const double* sig64;    // [c] opacity sigma
+  // workspace tables, written before the replay
+  double* score;          // [c] cot / V: score per unit of deposited energy
+  double2* chain;         // [c] (f^2, (1 - f^2) / sigma_s): the chain rule's factors
 };
-cudaError_t imc_launch_adjoint(const AdjointArgs& a, int geom, int block, int grid, cudaStream_t s);
+cudaError_t imc_launch_adjoint(const AdjointArgs& a, int geom, int block, int blocks_per_sm, int sms, cudaStream_t s);
 
 // ---------------------------------------------------------------------------------
 // Workspace layout (byte offsets into the caller's workspace, 256-aligned pieces)

@@ -18,7 +18,7 @@
 // the run seed, counter (id_base + bank index, event number, step, TAG_TRANSPORT).
 #include <algorithm>
 
-#include "imc_device.cuh"
+#include "imc_event.cuh"
 #include "imc_internal.h"
 
 using namespace imcdev;
@@ -60,26 +60,6 @@ struct EvOut {
   bool finished;   // the history ended: history_retire stores its final state
 };
 
-// What an event costs is its instructions: the kernel issues one in four of every five cycles, so
-// the geometry is written for few and uniform ones.  Against the straightforward form (one branch
-// per face and root, thresholds and caps tested per flight, all ten Philox rounds per draw, FP64
-// path length carried in registers) the ten launches of a 2M crooked-pipe run take 10.4 ms
-// instead of 12.6, the slab Marshak wave's twenty 7.1 instead of 8.5; every history is
-// bit-identical.
-
-// The scatter slot of a table entry (scatter_entry): > 0 the effective scatter opacity, 0 none
-// (at or below the geometry's threshold), < 0 minus the opacity of a cell whose distance is
-// capped (sigma_s L > 1e4 -> 1e4 / L; IMC/IMC1D.py:83-88, IMC/IMC2D.py:758-765).
-template <bool CAPS>
-__device__ __forceinline__ float scatter_flight(float ss, float L, uint32_t x, float s_other) {
-  if (ss > 0.f) {
-    if (scatter_may_win(x, ss, s_other)) return fdiv(neglog_u(x), ss);
-  } else if (CAPS && ss < 0.f) {
-    if (scatter_may_win(x, 10000.0f / L, s_other)) return neglog_u(x) * (L * 1e-4f);
-  }
-  return BIGF;
-}
-
 template <int GEOM, bool SMEM_CELLS, bool MG, bool CF>
 __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut& o, const float2* E1,
                                               const float2* E2, const float2* CS, unsigned* blk_cnt,
@@ -104,108 +84,9 @@ __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut
   } else {
     const U4 r = draw_next(a.rk, h.key, rkx, h.ev);
     ++h.ev;
-    const float2 e1 = E1[h.ci];  // the cell's edges in each direction
-    float d, sb, xn, yn = y, un = u, vn = v;
-    int evt, di = 0, dj = 0;     // the cell step of a boundary crossing
-    // ---- distance to the cell boundary ----
-    float s_rin = BIGF, s_rout = BIGF, st_ = 0.f, sx = BIGF, sy = BIGF;  // sy: z faces in RZ
-    float din = BIGF, dout = BIGF, om = 0.f;
-    float2 e2 = make_float2(0.f, 0.f);
-    if (GEOM == G_SLAB) {
-      sb = slab_face(x, u, e1.x, e1.y);
-    } else if (GEOM == G_SPHERE) {
-      om = (1.f - u) * (1.f + u);
-      const float b2 = x * x * om;
-      dout = outer_root(x, u, e1.y, b2);
-      din = inner_root(x, u, e1.x, b2);
-      sb = fminf(dout, din);
-    } else {
-      e2 = E2[h.cj];
-      if (GEOM == G_XY) {
-        if (u != 0.f) sx = fdiv((u > 0.f ? e1.y : e1.x) - x, u);
-        if (v != 0.f) sy = fdiv((v > 0.f ? e2.y : e2.x) - y, v);
-        sx = fmaxf(sx, 0.f); sy = fmaxf(sy, 0.f);
-        sb = fminf(sx, sy);
-      } else {
-        const float sin2 = (1.f - v) * (1.f + v);
-        om = (1.f - u) * (1.f + u);
-        if (sin2 >= 1e-15f) {
-          // outer_root and inner_root with one quotient: moving outwards (u >= 0) only the
-          // outer face is met and its root is a quotient; moving inwards the inner root is the
-          // quotient, the outer one q - r u
-          const float ist = frsqrt(sin2);
-          st_ = sin2 * ist;
-          const float b2 = x * x * om;
-          const float q = sqrt_nn(fmaf(e1.y, e1.y, -b2));
-          const float disc = fmaf(e1.x, e1.x, -b2);
-          const bool out = u >= 0.f;
-          const float R = out ? e1.y : e1.x;
-          const float P = (R - x) * (R + x);
-          const float den = out ? fmaxf(fmaf(x, u, q), 1e-30f) : (disc * frsqrt(disc) - x * u);
-          const float quo = fdiv(out ? P : -P, den);
-          s_rout = fmaxf(out ? quo : q - x * u, 0.f) * ist;
-          if (!out && e1.x > 0.f && disc > 0.f) s_rin = fmaxf(quo, 0.f) * ist;
-        }
-        if (fabsf(v) > 1e-15f) sy = fmaxf(fdiv((v > 0.f ? e2.y : e2.x) - y, v), 0.f);
-        sb = fminf(fminf(s_rin, s_rout), sy);
-      }
-    }
-    // ---- effective scatter and census ----
-    float L = e1.y - e1.x;  // used by capped cells only
-    if (!ONED) L = fminf(L, e2.y - e2.x);
-    const float ds = scatter_flight<!MG2>(ss, L, r.x, fminf(sb, h.dcen));
-    d = sb; evt = EV_BOUNDARY;
-    if (ds < d) { d = ds; evt = EV_SCATTER; }
-    if (h.dcen < d) { d = h.dcen; evt = EV_CENSUS; }
-    // ---- move ----
-    if (GEOM == G_SLAB) {
-      xn = fmaf(u, d, x);
-      if (evt == EV_BOUNDARY) { di = u > 0.f ? 1 : -1; xn = u > 0.f ? e1.y : e1.x; }
-      else { if (evt == EV_SCATTER) un = fmaf(2.f, u01f(r.y), -1.f); xn = fminf(fmaxf(xn, e1.x), e1.y); }
-    } else if (GEOM == G_SPHERE) {
-      const float ax = fmaf(u, d, x);
-      float rn = sqrt_nn(fmaf(ax, ax, d * d * om));
-      float mun = rn > 1e-15f ? (x * u + d) / rn : 1.f;
-      if (evt == EV_BOUNDARY) {
-        di = dout <= din ? 1 : -1;
-        rn = dout <= din ? e1.y : e1.x;
-        mun = (x * u + d) / rn;
-      } else {
-        if (evt == EV_SCATTER) mun = fmaf(2.f, u01f(r.y), -1.f);
-        rn = fminf(fmaxf(rn, e1.x), e1.y);
-      }
-      xn = rn; un = fminf(1.f, fmaxf(-1.f, mun));
-    } else if (GEOM == G_XY) {
-      xn = fmaf(u, d, x); yn = fmaf(v, d, y);
-      if (evt == EV_BOUNDARY) {
-        if (sx <= sy) di = u > 0.f ? 1 : -1;
-        else dj = v > 0.f ? 1 : -1;
-      } else if (evt == EV_SCATTER) {
-        const float uz = fmaf(2.f, u01f(r.y), -1.f);
-        const float rxy = sqrt_nn((1.f - uz) * (1.f + uz));
-        float sp, cp;
-        sincospif(2.f * u01f(r.z), &sp, &cp);
-        un = rxy * cp; vn = rxy * sp;
-      }
-      xn = di > 0 ? e1.y : di < 0 ? e1.x : fminf(fmaxf(xn, e1.x), e1.y);
-      yn = dj > 0 ? e2.y : dj < 0 ? e2.x : fminf(fmaxf(yn, e2.x), e2.y);
-    } else {
-      const float l = d * st_;
-      const float ax = fmaf(u, l, x);
-      const float rn = sqrt_nn(fmaf(ax, ax, l * l * om));
-      yn = fmaf(d, v, y);
-      if (rn > 1e-15f && l > 0.f) un = fminf(1.f, fmaxf(-1.f, fdiv(fmaf(x, u, l), rn)));
-      if (evt == EV_BOUNDARY) {
-        if (sb == s_rin) di = -1;
-        else if (sb == s_rout) di = 1;
-        else dj = v < 0.f ? -1 : 1;
-      } else if (evt == EV_SCATTER) {
-        vn = fmaf(2.f, u01f(r.y), -1.f);
-        un = cospif(2.f * u01f(r.z));
-      }
-      xn = di > 0 ? e1.y : di < 0 ? e1.x : fminf(fmaxf(rn, e1.x), e1.y);
-      yn = dj > 0 ? e2.y : dj < 0 ? e2.x : fminf(fmaxf(yn, e2.x), e2.y);
-    }
+    const Flight f = next_flight<GEOM, !MG2>(E1[h.ci], ONED ? make_float2(0.f, 0.f) : E2[h.cj], ss, x, y, u, v, h.dcen, r);
+    const float d = f.d;
+    const int evt = f.evt, di = f.di, dj = f.dj;
     // implicit capture (the energy removed is counted at the flush, w_in - w)
     const float wn = (MG2 && !(sa > 1e-12f)) ? w : w * __expf(-sa * d);
     // path-length intensity: w*s is needed only in cells without absorption (table
@@ -241,7 +122,7 @@ __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut
       h.w = wn;
       finished = true;
     } else {
-      h.w = captured ? 0.f : wn; h.x = xn; h.y = yn; h.u = un; h.v = vn;
+      h.w = captured ? 0.f : wn; h.x = f.x; h.y = f.y; h.u = f.u; h.v = f.v;
       if (CF && captured) finished = true;
       if ((di | dj) != 0) {
         // leaving the cell: flush the visit (before an escape zeroes w) and start the next
@@ -313,26 +194,6 @@ __device__ __forceinline__ bool history_retire(const TrackArgs& a, const Hist& h
   if (GEOM == G_XY || GEOM == G_RZ) { a.p2[h.pid] = h.y; a.d2[h.pid] = h.v; }
   a.cell[h.pid] = c;
   cen_bin = c + (a.ecen_by_group ? a.nc * h.grp : 0);
-  return true;
-}
-
-// The block's claim of bank entries for one warp (guided: a share of what is left, at most
-// `chunk`, at least 32, so early claims are long contiguous (coherent) runs and the drain is
-// finely balanced).  Every lane calls it; false when the queue is past n.
-__device__ __forceinline__ bool claim_run(const TrackArgs& a, uint32_t n, uint32_t& next, uint32_t& end) {
-  unsigned long long base = 0, claim = 0;
-  if ((threadIdx.x & 31) == 0) {
-    const unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(a.queue);
-    const unsigned long long left = cur < (unsigned long long)n ? (unsigned long long)n - cur : 0ull;
-    const unsigned long long nw = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-    claim = min((unsigned long long)a.chunk, max(32ull, left / (2ull * nw)));
-    base = atomicAdd(a.queue, claim);
-  }
-  base = __shfl_sync(FULL, base, 0);
-  claim = __shfl_sync(FULL, claim, 0);
-  if (base >= (unsigned long long)n) return false;
-  next = (uint32_t)base;
-  end = (uint32_t)min(base + claim, (unsigned long long)n);
   return true;
 }
 
@@ -467,7 +328,7 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
       }
       pend = false;
       while (need && !drained) {
-        if (chunk_next >= chunk_end && !claim_run(a, n, chunk_next, chunk_end)) { drained = true; break; }
+        if (chunk_next >= chunk_end && !claim_run(a.queue, a.chunk, n, chunk_next, chunk_end)) { drained = true; break; }
         const uint32_t avail = chunk_end - chunk_next;
         const uint32_t rank = __popc(need & lt_mask);
         if (!has && rank < avail) {
@@ -790,8 +651,6 @@ cudaError_t launch_sized(K kernel, const TrackArgs& a, int block, int grid, size
   IMC_LAUNCH_PDL(kernel, grid, block, sh, s, a);
   return cudaGetLastError();
 }
-
-constexpr size_t kSmemPerBlock = 226 * 1024;  // dynamic, beside the kernel's own few hundred bytes
 
 // T_SMALL is built only with the shared-memory cell table (small meshes)
 template <int GEOM, bool MG, bool CF = false>
