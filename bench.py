@@ -931,7 +931,7 @@ def main():
     ap.add_argument("--batch-instances", type=int, default=256,
                     help="instances of the batched form (the workload's 256; fewer for a small profiling case)")
     ap.add_argument("--batch-form", type=int, default=0, choices=(0, 1, 2, 3),
-                    help="batched tracking form: 0 the tuner's choice, 1 work units, 2 the entry queue, 3 work units with prefetched refills")
+                    help="batched tracking form: 0 the tuner's choice, 1 work units (3 the same), 2 the entry queue")
     ap.add_argument("--no-fom", action="store_true")
     ap.add_argument("--fom-seeds", type=int, default=32)
     ap.add_argument("--fom-steps", type=int, default=100)

@@ -497,14 +497,13 @@ typedef struct imc_batch_launch {  /* tracking kernel shape; 0 = default */
   int32_t blocks_per_sm;
   int32_t chunk;                /* histories per work-queue ticket (at most) */
   int32_t refill_min;           /* idle lanes a warp waits for before it refills (1..32) */
-  int32_t form;                 /* tracking form: 1 work units (a block takes chunk x warps entries
-                                   and stages each instance's tables and tallies in shared memory;
-                                   needs imc_batch.max_cells), 2 the entry queue (warps take entries
-                                   of any instance, tables and tallies in global memory; for many
-                                   small instances), 3 work units with prefetched refills (each
-                                   lane copies its next history's bank record into shared memory
-                                   while it tracks the current one), 0 the library's choice (work
-                                   units when max_cells allows) */
+  int32_t form;                 /* tracking form: 1 work units (a block takes at most chunk x warps
+                                   entries at a time, less as the queue drains, and stages each
+                                   instance's table and deposition in shared memory; needs
+                                   imc_batch.max_cells), 2 the entry queue (warps take entries of
+                                   any instance, tables and tallies in global memory), 3 as 1
+                                   (once a variant with another refill), 0 the library's choice
+                                   (work units when max_cells allows) */
 } imc_batch_launch;
 
 IMC_API size_t imc_batch_workspace_bytes(const imc_batch* b);

@@ -19,7 +19,7 @@
 #include <cmath>
 #include <cstring>
 #include "imc_batch.h"
-#include "imc_device.cuh"
+#include "imc_event.cuh"
 #include "imc_sample.cuh"
 
 using namespace imcdev;
@@ -27,7 +27,7 @@ using namespace imcsample;
 
 namespace {
 
-enum : int { B_CENSUS = 0, B_FLOOR, B_REFLECT, B_CAP, B_ESCAPE, B_N };
+enum : int { B_FLOOR = 0, B_REFLECT, B_CAP, B_ESCAPE, B_N };
 
 // last k with pref[k] <= q; for q < pref[K] this is the instance that owns entry q
 // (instances without entries share their prefix value with the next one)
@@ -133,12 +133,111 @@ __global__ void __launch_bounds__(256) k_bwsum(BatchArgs a) {
 }
 
 // ---------------------------------------------------------------- tracking
-// The single-problem slab kernel's event loop (k_track<G_SLAB>) over every instance:
-// persistent warps claim runs of the flattened entry index with guided atomic tickets; a
-// lane that takes entry q looks up its instance once and keeps the instance's constants
+// The single-problem slab kernel's histories (k_track<G_SLAB>) over every instance: the same
+// flights, Philox draws and end rules, in two forms of the work distribution.
+struct BHist {
+  uint32_t pid, ev;              // bank slot, events so far
+  float x, u, w, dcen, w_in;     // w_in: the weight the current cell visit began with
+  float2 tab;                    // cell table entry
+  int ci;                        // cell inside the instance
+  DrawKey key;
+};
+struct BOut {
+  bool flush, finished;  // the cell visit / the history ended
+  double lost;           // the visit's deposition (flush)
+  float wd;              // w*s of a flight in a cell without absorption, else 0
+  float kill;            // weight of a history killed after a crossing, to the cell it entered
+  int escaped;           // face an escaping history left through (its weight in esc_w), else -1
+  float esc_w;
+};
+
+// One event; e: the cell's edges.  After a crossing the caller loads the new cell's table entry.
+__device__ __forceinline__ void batch_event(BHist& h, BOut& o, float2 e, const U4& r, int nc, int rmask, float wfloor,
+                                            unsigned* blk_cnt, int* flags, unsigned& s_cen, unsigned& s_sc) {
+  o = BOut{false, false, 0.0, 0.f, 0.f, -1, 0.f};
+  if (h.ev >= (1u << 30)) {
+    atomicAdd(&blk_cnt[B_CAP], 1u);
+    atomicOr(flags, (int)IMC_FLAG_EVENT_CAP);
+    o.finished = true;
+  } else {
+    ++h.ev;
+    const Flight f = next_flight<G_SLAB, true>(e, e, h.tab.y, h.x, 0.f, h.u, 0.f, h.dcen, r);
+    const float wn = h.w * __expf(-h.tab.x * f.d);
+    if (!(h.tab.x > 0.f)) o.wd = h.w * f.d;
+    h.dcen -= f.d;
+    s_sc += f.evt == EV_SCATTER ? 1u : 0u;
+    s_cen += f.evt == EV_CENSUS ? 1u : 0u;
+    h.w = wn; h.x = f.x; h.u = f.u;
+    if (f.di != 0) {
+      o.flush = true; o.lost = (double)h.w_in - (double)h.w;
+      h.w_in = h.w;
+      const int ni = h.ci + f.di;
+      if ((unsigned)ni >= (unsigned)nc) {
+        const int side = ni < 0 ? 0 : 1;
+        if ((rmask >> side) & 1) {  // stays in its cell
+          h.u = -h.u;
+          atomicAdd(&blk_cnt[B_REFLECT], 1u);
+        } else {
+          o.escaped = side; o.esc_w = h.w;
+          atomicAdd(&blk_cnt[B_ESCAPE], 1u);
+          h.w = 0.f;
+          o.finished = true;
+        }
+      } else {
+        h.ci = ni;
+      }
+    }
+    if (!o.finished && h.w < wfloor) {
+      // IMC/IMC1D.py:188-195: kill and deposit the remainder in the current cell.  Without a
+      // crossing in this event the visit's flush at the history end (w_in - 0) carries it; after
+      // one it goes to the new cell (its intensity follows from the deposition)
+      atomicAdd(&blk_cnt[B_FLOOR], 1u);
+      if (o.flush) o.kill = h.w;
+      h.w = 0.f;
+      o.finished = true;
+    }
+    if (!(h.dcen > 0.f)) o.finished = true;
+  }
+  if (o.finished && !o.flush) { o.flush = true; o.lost = (double)h.w_in - (double)h.w; }
+}
+
+// Stores an ended history.
+__device__ __forceinline__ void batch_retire(const BatchBank& B, const BHist& h) {
+  B.w[h.pid] = h.w;
+  if (h.w > 0.f) { B.p1[h.pid] = h.x; B.d1[h.pid] = h.u; B.cell[h.pid] = h.ci; }
+}
+
+// the block's event counts to the global ones (every thread calls it)
+__device__ __forceinline__ void batch_event_counts(const BatchArgs& a, const unsigned* blk_cnt,
+                                                   unsigned long long events, unsigned s_cen, unsigned s_sc) {
+  __shared__ unsigned long long tot[3];
+  if (threadIdx.x < 3) tot[threadIdx.x] = 0ull;
+  __syncthreads();
+  if (events) atomicAdd(&tot[0], events);
+  const unsigned long long t_cen = warp_sum_u(s_cen), t_sc = warp_sum_u(s_sc);
+  if ((threadIdx.x & 31) == 0) {
+    if (t_cen) atomicAdd(&tot[1], t_cen);
+    if (t_sc) atomicAdd(&tot[2], t_sc);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned long long cap = blk_cnt[B_CAP], bd = tot[0] - tot[1] - tot[2];
+    if (tot[0] + cap) atomicAdd(a.stats + S_EVENTS, tot[0] + cap);
+    if (bd) atomicAdd(a.stats + S_BOUNDARY, bd);
+    if (tot[2]) atomicAdd(a.stats + S_SCATTER, tot[2]);
+    if (tot[1]) atomicAdd(a.stats + S_CENSUS, tot[1]);
+    if (blk_cnt[B_FLOOR]) atomicAdd(a.stats + S_FLOOR, (unsigned long long)blk_cnt[B_FLOOR]);
+    if (blk_cnt[B_REFLECT]) atomicAdd(a.stats + S_REFLECT, (unsigned long long)blk_cnt[B_REFLECT]);
+    if (cap) atomicAdd(a.stats + S_CAP, cap);
+    if (blk_cnt[B_ESCAPE]) atomicAdd(a.stats + S_ESCAPE, (unsigned long long)blk_cnt[B_ESCAPE]);
+  }
+}
+
+// Entry-queue form: persistent warps claim runs of the flattened entry index with guided atomic
+// tickets; a lane that takes entry q looks up its instance once and keeps the instance's constants
 // (cell and edge bases, cell count, reflect mask, weight floor, Philox key) in registers.
 // refill_min: a warp refills its idle lanes once at least that many are idle (1 = at
-// every event boundary, as the single-problem kernel), or when all are idle.
+// every event boundary), or when all are idle.
 __global__ void __launch_bounds__(256) k_btrack(BatchArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ unsigned blk_cnt[B_N];
@@ -158,264 +257,146 @@ __global__ void __launch_bounds__(256) k_btrack(BatchArgs a) {
   const float c_light = (float)C_LIGHT;
   const unsigned refill_min = (unsigned)max(1, min(32, a.refill_min));
 
-  unsigned long long chunk_next = 0, chunk_end = 0;
-  bool drained = false;
-
-  bool has = false;
-  long long pid = 0;
-  uint32_t lid = 0, ev = 0;
-  int k = 0, cb = 0, eb = 0, nc = 0, rmask = 0, ci = 0;
+  uint32_t chunk_next = 0, chunk_end = 0;
+  bool drained = false, has = false;
+  BHist h{};
+  uint32_t lid = 0;
+  int k = 0, cb = 0, eb = 0, nc = 0, rmask = 0;
   uint64_t seed = 0;
-  float wfloor = 0.f, x = 0.f, u = 0.f, w = 0.f, dcen = 0.f;
+  float wfloor = 0.f;
   double inv_q = 0.0;  // the instance's fixed-point energy quantum, inverted
-  double acc_lost = 0.0, acc_wd = 0.0;
-  unsigned s_bd = 0, s_sc = 0;
+  unsigned s_cen = 0, s_sc = 0;
   // events of finished histories, summed per lane while they belong to one instance (a
   // warp's claims are contiguous runs of one instance's entries) and added to the
   // instance's ledger when the instance changes: one atomic per run, not per history
-  unsigned long long ev_acc = 0ull;
+  unsigned long long ev_acc = 0ull, ev_all = 0ull;
   int ev_k = 0;
 
   for (;;) {
     unsigned need = __ballot_sync(FULL, !has);
     if ((unsigned)__popc(need) >= refill_min) {
       while (need && !drained) {
-        if (chunk_next >= chunk_end) {
-          unsigned long long base = 0, claim = 0;
-          if (lane == 0) {
-            const unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(a.queue);
-            const unsigned long long left = cur < n ? n - cur : 0ull;
-            const unsigned long long nw = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-            claim = min((unsigned long long)a.chunk, max(32ull, left / (2ull * nw)));
-            base = atomicAdd(a.queue, claim);
-          }
-          base = __shfl_sync(FULL, base, 0);
-          claim = __shfl_sync(FULL, claim, 0);
-          if (base >= n) { drained = true; break; }
-          chunk_next = base;
-          chunk_end = min(base + claim, n);
+        if (chunk_next >= chunk_end && !claim_run(a.queue, a.chunk, (uint32_t)n, chunk_next, chunk_end)) {
+          drained = true;
+          break;
         }
-        const unsigned long long avail = chunk_end - chunk_next;
-        const unsigned rank = __popc(need & lt_mask);
+        const uint32_t avail = chunk_end - chunk_next;
+        const uint32_t rank = __popc(need & lt_mask);
         if (!has && rank < avail) {
           const long long q = (long long)(chunk_next + rank);
           k = find_inst(pref, a.K, q);
           lid = (uint32_t)(q - pref[k]);
-          pid = a.slot_off[k] + lid;
-          w = B.w[pid];
-          dcen = (dt - B.t[pid]) * c_light;
-          if (w > 0.f && dcen > 0.f) {
-            x = B.p1[pid]; u = B.d1[pid]; ci = B.cell[pid];
+          h.pid = (uint32_t)(a.slot_off[k] + lid);
+          h.w = B.w[h.pid];
+          h.dcen = (dt - B.t[h.pid]) * c_light;
+          if (h.w > 0.f && h.dcen > 0.f) {
+            h.x = B.p1[h.pid]; h.u = B.d1[h.pid]; h.ci = B.cell[h.pid];
             cb = a.cell_off[k]; nc = a.cell_off[k + 1] - cb; eb = cb + k;
             rmask = a.reflect[k]; seed = a.seed[k];
             const long long nb = a.n_bank[k];
             const double W = a.wsum[k];
             wfloor = (float)(1e-10 * W / (double)(nb > 0 ? nb : 1));
             inv_q = fx_inv_quantum(W);
-            ev = 0;
+            h.tab = __ldg(a.sass + cb + h.ci);
+            h.ev = 0;
+            h.w_in = h.w;
             has = true;
           }
         }
-        chunk_next += min((unsigned long long)__popc(need), avail);
+        chunk_next += min((uint32_t)__popc(need), avail);
         need = __ballot_sync(FULL, !has);
       }
     }
     if (!__any_sync(FULL, has)) break;
 
-    bool flush = false;
-    int flush_cell = 0;
-    double f_lost = 0.0, f_wd = 0.0;
+    BOut o{};
+    int cg = 0;
     if (has) {
-      const int cg = cb + ci;
-      const float2 sq = __ldg(a.sass + cg);
-      const float sa = sq.x, ss = sq.y;
-      bool finished = false;
-      if (ev >= (1u << 30)) {
-        atomicAdd(&blk_cnt[B_CAP], 1u);
-        atomicOr(a.flags, (int)IMC_FLAG_EVENT_CAP);
-        finished = true;
-      } else {
-        const U4 r = draw(seed, lid, ev, step, TAG_TRANSPORT);
-        ++ev;
-        const float xl = __ldg(a.ef + eb + ci), xr = __ldg(a.ef + eb + ci + 1);
-        const float L = xr - xl;
-        const float sb = slab_face(x, u, xl, xr);
-        float ds = BIGF;
-        {
-          const bool capped = ss * L > 10000.0f;
-          const float sig = capped ? 10000.0f / L : (ss > 1e-10f ? ss : 0.f);
-          if (sig > 0.f) {
-            const float s_other = fminf(sb, dcen);
-            const double t = (double)sig * (double)s_other;
-            bool may = true;
-            if (t < 0.01) {
-              const double thr = 1.0 - t * (1.0 - t * (0.5 - t * (1.0 / 6.0)));
-              may = u01d(r.x) > thr;
-            }
-            if (may) ds = capped ? neglog_u(r.x) * (L * 1e-4f) : __fdividef(neglog_u(r.x), ss);
-          }
-        }
-        float d = sb;
-        int evt = EV_BOUNDARY, cross = X_NONE;
-        if (ds < d) { d = ds; evt = EV_SCATTER; }
-        if (dcen < d) { d = dcen; evt = EV_CENSUS; }
-        float xn = fmaf(u, d, x), un = u;
-        if (evt == EV_BOUNDARY) { if (u > 0.f) { xn = xr; cross = X_IP; } else { xn = xl; cross = X_IM; } }
-        else { if (evt == EV_SCATTER) un = fmaf(2.f, u01f(r.y), -1.f); xn = fminf(fmaxf(xn, xl), xr); }
-        const float wn = w * __expf(-sa * d);
-        acc_lost += (double)w - (double)wn;
-        acc_wd += (double)(w * d);
-        dcen -= d;
-        if (evt == EV_BOUNDARY) ++s_bd; else if (evt == EV_SCATTER) ++s_sc;
-        else atomicAdd(&blk_cnt[B_CENSUS], 1u);
-        w = wn; x = xn; u = un;
-        if (cross != X_NONE) {
-          flush = true; flush_cell = cg; f_lost = acc_lost; f_wd = acc_wd;
-          acc_lost = 0.0; acc_wd = 0.0;
-          int ni = cross == X_IP ? ci + 1 : ci - 1;
-          const int side = ni < 0 ? 0 : (ni >= nc ? 1 : -1);
-          if (side >= 0) {
-            if ((rmask >> side) & 1) {
-              u = -u;
-              ni = side == 0 ? 0 : nc - 1;
-              atomicAdd(&blk_cnt[B_REFLECT], 1u);
-            } else {
-              atomicAdd(a.esc_fx + 2 * k + side, fx_units((double)w, inv_q));
-              atomicAdd(&blk_cnt[B_ESCAPE], 1u);
-              w = 0.f;
-              finished = true;
-              ni = ci;
-            }
-          }
-          ci = ni;
-        }
-        if (!finished && w < wfloor) {
-          // IMC/IMC1D.py:188-195: kill and deposit the remainder in the current cell
-          atomicAdd(&blk_cnt[B_FLOOR], 1u);
-          atomicAdd(a.dep_fx + cb + ci, fx_units((double)w, inv_q));  // its intensity follows from it
-          w = 0.f;
-          finished = true;
-        }
-        if (!finished && !(dcen > 0.f)) finished = true;
-      }
-      if (finished) {
-        if (!flush && (acc_lost != 0.0 || acc_wd != 0.0)) {
-          flush = true; flush_cell = cb + ci; f_lost = acc_lost; f_wd = acc_wd;
-        }
-        acc_lost = 0.0; acc_wd = 0.0;
-        B.w[pid] = w;
-        if (w > 0.f) { B.p1[pid] = x; B.d1[pid] = u; B.cell[pid] = ci; }
+      cg = cb + h.ci;
+      const U4 r = draw(seed, lid, h.ev, step, TAG_TRANSPORT);
+      const float2 e = make_float2(__ldg(a.ef + eb + h.ci), __ldg(a.ef + eb + h.ci + 1));
+      batch_event(h, o, e, r, nc, rmask, wfloor, blk_cnt, a.flags, s_cen, s_sc);
+      if (o.escaped >= 0) atomicAdd(a.esc_fx + 2 * k + o.escaped, fx_units((double)o.esc_w, inv_q));
+      if (o.kill > 0.f) atomicAdd(a.dep_fx + cb + h.ci, fx_units((double)o.kill, inv_q));
+      if (o.finished) {
+        batch_retire(B, h);
         if (k != ev_k) {
           if (ev_acc) atomicAdd(a.ledger + (size_t)ev_k * IMC_BL_N + IMC_BL_EVENTS, (double)ev_acc);
           ev_k = k;
           ev_acc = 0ull;
         }
-        ev_acc += ev;
+        ev_acc += h.ev;
+        ev_all += h.ev;
         has = false;
+      } else if (o.flush) {
+        h.tab = __ldg(a.sass + cb + h.ci);
       }
     }
-    unsigned long long ud = 0ull;
-    double vs = 0.0;
-    if (flush) {
-      const double2 cf = __ldg(a.cellf + flush_cell);
-      ud = fx_units(f_lost, inv_q);  // lanes of one cell share its instance's quantum
-      vs = cf.y > 0.0 ? 0.0 : f_wd;  // raw w*s of a cell without absorption (the rest follows from ud)
-    }
-    warp_tally_fx(flush, flush_cell, ud, vs, a.dep_fx, a.si, st);
+    // lanes of one cell share its instance's quantum
+    const unsigned long long ud = o.flush ? fx_units(o.lost, inv_q) : 0ull;
+    warp_tally_fx(ud != 0ull || o.wd != 0.f, cg, ud, (double)o.wd, a.dep_fx, a.si, st);
   }
-
   if (ev_acc) atomicAdd(a.ledger + (size_t)ev_k * IMC_BL_N + IMC_BL_EVENTS, (double)ev_acc);
-  const unsigned long long t_bd = warp_sum_u(s_bd), t_sc = warp_sum_u(s_sc);
-  if (lane == 0) {
-    if (t_bd) atomicAdd(a.stats + S_BOUNDARY, t_bd);
-    if (t_sc) atomicAdd(a.stats + S_SCATTER, t_sc);
-    if (t_bd + t_sc) atomicAdd(a.stats + S_EVENTS, t_bd + t_sc);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned long long cen = blk_cnt[B_CENSUS], cap = blk_cnt[B_CAP];
-    if (cen) atomicAdd(a.stats + S_CENSUS, cen);
-    if (cen + cap) atomicAdd(a.stats + S_EVENTS, cen + cap);
-    if (blk_cnt[B_FLOOR]) atomicAdd(a.stats + S_FLOOR, (unsigned long long)blk_cnt[B_FLOOR]);
-    if (blk_cnt[B_REFLECT]) atomicAdd(a.stats + S_REFLECT, (unsigned long long)blk_cnt[B_REFLECT]);
-    if (cap) atomicAdd(a.stats + S_CAP, cap);
-    if (blk_cnt[B_ESCAPE]) atomicAdd(a.stats + S_ESCAPE, (unsigned long long)blk_cnt[B_ESCAPE]);
-  }
+  batch_event_counts(a, blk_cnt, ev_all, s_cen, s_sc);
 }
 
-// Work-unit form of the tracking, for batches whose largest instance has at most
-// IMC_BATCH_SMEM_CELLS cells.  A block claims a unit of chunk x (warps per block) consecutive
-// entries of the batch (instance-major: one instance, or the end of one and the start of the
-// next) and tracks it instance by instance with all its warps, each warp refilling idle lanes
-// from a shared-memory cursor.  For the instance at hand the block keeps the cell table
-// (sigma_a, sigma_s), the edges and the intensity factor in shared memory and sums the
-// deposition (fixed point) and intensity tallies there, adding them to the instance's global
-// tallies when it moves to another instance: the single-problem kernel's on-chip tables, which
-// the entry-granular queue of k_btrack cannot keep because its warps draw entries of any
-// instance.  Per history the computation is k_btrack's (same Philox counters and arithmetic).
-// Five resident 256-thread blocks per SM (48 registers, 20 bytes of spills): 55.5 G segments/s on
-// the 256-instance uneven batch against 53.9 G at four blocks (57 registers).
+// Work-unit form, for batches whose largest instance has at most IMC_BATCH_SMEM_CELLS cells.  A
+// block claims a unit of consecutive entries of the batch (instance-major: one instance, or the
+// end of one and the start of the next) and tracks it instance by instance with all its warps,
+// each refilling idle lanes (kUnitRefillMin at a time) from a shared-memory cursor.  For the
+// instance at hand the block keeps the cell table and the edges in shared memory and sums the
+// deposition there (fixed point), adding it to the instance's global tally when it moves to another
+// instance; w*s, only from cells without absorption, goes to global memory.
+//
+// A unit is 1/kUnitShare of what is left per block, at least one entry per thread and at most
+// chunk x warps.  The instances differ in cost per entry by two orders of magnitude (a few events
+// per history in a thin one, several hundred at a thick wave front), so whole chunks (32 entries a
+// thread at the default) leave the last blocks running long after the others; units much smaller
+// than these wait too often for their longest history.  Three steps of 256 instances with 5.8 M
+// source particles: 28.9 ms with whole chunks, 12.9 at a share of 16, 11.8 at 32; 0.58 M: 6.8, 3.4,
+// 3.4; 58 M: 115 (before this form's other changes), 96, 97.
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) v += __shfl_down_sync(FULL, v, o);
   return v;
 }
 
-__host__ __device__ inline size_t units_smem(int K, int M) {
-  return sizeof(long long) * (size_t)(K + 1) + (size_t)M * (8 + 8 + 8 + 8) + sizeof(float) * (size_t)(M + 1);
-}
+constexpr int kUnitThreads = 256;
+constexpr int kUnitShare = 32;
+constexpr int kUnitRefillMin = 8;
 
-// Prefetched refills (form 3): every lane holds the bank record of its next history in a
-// shared-memory slot, copied there by cp.async while it tracks the current one, so a lane whose
-// history ends takes its next one from shared memory instead of stalling the warp on two
-// dependent HBM reads (weight and birth time, then position, direction and cell).
-constexpr int PF_FIELDS = 6;  // w, t, x, u, cell, entry index inside the instance
-__host__ __device__ inline size_t units_pf_smem(int block) { return sizeof(float) * PF_FIELDS * (size_t)block; }
+inline size_t units_smem(int M) { return (size_t)M * (8 + 8 + 8) + sizeof(WarpStage) * (kUnitThreads / 32); }
 
-template <bool PF>
-__global__ void __launch_bounds__(256, 5) k_btrack_units(BatchArgs a) {
+__global__ void __launch_bounds__(kUnitThreads, 1024 / kUnitThreads) k_btrack_units(BatchArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ unsigned blk_cnt[B_N];
   __shared__ unsigned long long s_base, s_cur, s_unit;
   __shared__ __align__(16) uint32_t s_rk[20];  // Philox round keys of the staged instance's seed
   const int M = a.max_cells;
-  long long* pref = reinterpret_cast<long long*>(smem);                                 // [K+1]
-  unsigned long long* TD = reinterpret_cast<unsigned long long*>(pref + (a.K + 1));    // [M] deposition
-  double* TS = reinterpret_cast<double*>(TD + M);                                       // [M] intensity
-  double* CF = TS + M;                                                                  // [M] cellf.y
-  float2* SS = reinterpret_cast<float2*>(CF + M);                                       // [M] (sa, ss)
-  float* EF = reinterpret_cast<float*>(SS + M);                                         // [M+1] edges
-  // PF: the lane's next bank record, field f of thread i at PQ[f * blockDim.x + i]
-  float* PQ = reinterpret_cast<float*>(smem + units_smem(a.K, M));
-  float* const my_pf = PQ + threadIdx.x;
-  const int pf_stride = blockDim.x;
+  unsigned long long* TD = reinterpret_cast<unsigned long long*>(smem);                 // [M] deposition
+  float2* SS = reinterpret_cast<float2*>(TD + M);                                       // [M] cell table
+  float2* EF = SS + M;                                                                  // [M] edges
+  WarpStage* st = reinterpret_cast<WarpStage*>(EF + M) + (threadIdx.x >> 5);
   if (threadIdx.x < B_N) blk_cnt[threadIdx.x] = 0u;
-  load_pref(pref, a.live_pref, a.K);
 
   const int lane = threadIdx.x & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
-  const unsigned long long n = (unsigned long long)pref[a.K];
+  const unsigned long long n = (unsigned long long)a.live_pref[a.K];
   const BatchBank B = a.bank[*a.sel];
   const uint32_t step = *a.step;
   const float dt = (float)a.dt;
   const float c_light = (float)C_LIGHT;
   const unsigned long long unit = (unsigned long long)max(a.chunk, 32) * (blockDim.x >> 5);
-  unsigned s_bd = 0, s_sc = 0;
+  unsigned s_cen = 0, s_sc = 0;
+  unsigned long long ev_all = 0ull;
   int cur_k = -1, cur_nc = 0, cur_cb = 0;  // block-uniform: the instance whose tallies are staged
 
   for (;;) {
     if (threadIdx.x == 0) {
-      // full units while at least one per block is left; after that the rest shared over the
-      // blocks (a multiple of 32, at least one row per warp), so the blocks finish together
-      // instead of the last full units running on a few SMs
-      unsigned long long u = unit;
       const unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(a.queue);
       const unsigned long long left = cur < n ? n - cur : 0ull;
-      const unsigned long long nb = gridDim.x;
-      if (left < nb * unit) {
-        const unsigned long long floor_u = 32ull * (blockDim.x >> 5);
-        u = min(unit, max(floor_u, (left / nb + 31ull) & ~31ull));
-      }
+      const unsigned long long row = blockDim.x;
+      const unsigned long long u = min(unit, max(1ull, left / (kUnitShare * (unsigned long long)gridDim.x * row)) * row);
       s_unit = u;
       s_base = atomicAdd(a.queue, u);
     }
@@ -424,22 +405,23 @@ __global__ void __launch_bounds__(256, 5) k_btrack_units(BatchArgs a) {
     if (base >= n) break;  // uniform: every thread read the same claim
     const unsigned long long end = min(base + s_unit, n);
     for (unsigned long long q0 = base; q0 < end;) {
-      const int k = find_inst(pref, a.K, (long long)q0);
-      const unsigned long long q1 = min(end, (unsigned long long)pref[k + 1]);
+      // the instance of entry q0: the last whose prefix is not past it
+      int k = -1;
+      for (int q = 0; q < a.K; q += blockDim.x)
+        k += __syncthreads_count(q + (int)threadIdx.x < a.K &&
+                                 (unsigned long long)a.live_pref[q + threadIdx.x] <= q0);
+      const unsigned long long q1 = min(end, (unsigned long long)a.live_pref[k + 1]);
       if (k != cur_k) {
         // the staged tallies to the previous instance, then this instance's tables
-        for (int c = threadIdx.x; c < cur_nc; c += blockDim.x) {
+        for (int c = threadIdx.x; c < cur_nc; c += blockDim.x)
           if (TD[c]) atomicAdd(a.dep_fx + cur_cb + c, TD[c]);
-          if (TS[c] != 0.0) atomicAdd(a.si + cur_cb + c, TS[c]);
-        }
         __syncthreads();
         cur_k = k; cur_cb = a.cell_off[k]; cur_nc = a.cell_off[k + 1] - cur_cb;
         for (int c = threadIdx.x; c < cur_nc; c += blockDim.x) {
-          TD[c] = 0ull; TS[c] = 0.0;
-          CF[c] = a.cellf[cur_cb + c].y;
+          TD[c] = 0ull;
           SS[c] = a.sass[cur_cb + c];
+          EF[c] = make_float2(a.ef[cur_cb + k + c], a.ef[cur_cb + k + c + 1]);
         }
-        for (int c = threadIdx.x; c <= cur_nc; c += blockDim.x) EF[c] = a.ef[cur_cb + k + c];
         if (threadIdx.x == 0) philox_round_keys(a.seed[k], s_rk);
       }
       if (threadIdx.x == 0) s_cur = q0;
@@ -451,215 +433,68 @@ __global__ void __launch_bounds__(256, 5) k_btrack_units(BatchArgs a) {
       const double W = a.wsum[k];
       const float wfloor = (float)(1e-10 * W / (double)(nbk > 0 ? nbk : 1));
       const double inv_q = fx_inv_quantum(W);
-      const long long pk = pref[k], so = a.slot_off[k];
+      const uint32_t so = (uint32_t)a.slot_off[k];
+      const long long pk = a.live_pref[k];
+      const uint32_t rkx = draw_step_key(s_rk, step);
       unsigned long long ev_acc = 0ull;
-      bool has = false, drained = false;
-      bool pv = false;  // PF: the lane's slot holds a claimed record (copy issued)
-      long long pid = 0;
-      uint32_t lid = 0, ev = 0;
-      int ci = 0;
-      float x = 0.f, u = 0.f, w = 0.f, dcen = 0.f;
-      float w_in = 0.f;     // weight at the start of the current cell visit
-      double acc_wd = 0.0;  // w*s in the current cell (cells without absorption only)
+      bool has = false, pend = false, drained = false;
+      BHist h{};
       for (;;) {
-        // ---- refill idle lanes from the block's cursor over [q0, q1) ----
-        if (PF) {
-          // An idle lane takes the record in its slot; every lane without a claimed record
-          // claims the next entry of the unit (one shared atomic per warp) and starts its copy.
-          // Leaves with every lane either tracking or holding no claim; at the unit's end the
-          // cursor is past q1 and no claim is left untaken.
-          for (;;) {
-            if (!has && pv) {
-              cp_async_wait_all();
-              pv = false;
-              lid = __float_as_uint(my_pf[5 * pf_stride]);
-              pid = so + lid;
-              w = my_pf[0];
-              dcen = (dt - my_pf[pf_stride]) * c_light;
-              if (w > 0.f && dcen > 0.f) {
-                x = my_pf[2 * pf_stride]; u = my_pf[3 * pf_stride]; ci = __float_as_int(my_pf[4 * pf_stride]);
-                ev = 0;
-                w_in = w;
+        unsigned need = __ballot_sync(FULL, !has);
+        if (need == FULL || (!drained && __popc(need) >= kUnitRefillMin)) {
+          if (pend) { batch_retire(B, h); ev_acc += h.ev; pend = false; }
+          while (need && !drained) {
+            unsigned long long b0 = 0;
+            if (lane == 0) b0 = atomicAdd(&s_cur, (unsigned long long)__popc(need));
+            b0 = __shfl_sync(FULL, b0, 0);
+            if (b0 >= q1) { drained = true; break; }
+            const unsigned rank = __popc(need & lt_mask);
+            if (!has && b0 + rank < q1) {
+              const uint32_t lid = (uint32_t)((long long)(b0 + rank) - pk);
+              h.pid = so + lid;
+              h.w = B.w[h.pid];
+              h.dcen = (dt - B.t[h.pid]) * c_light;
+              if (h.w > 0.f && h.dcen > 0.f) {
+                h.x = B.p1[h.pid]; h.u = B.d1[h.pid]; h.ci = B.cell[h.pid];
+                h.tab = SS[h.ci];
+                h.key = draw_key(s_rk, lid, step, TAG_TRANSPORT);
+                h.ev = 0;
+                h.w_in = h.w;
                 has = true;
               }
             }
-            if (!drained) {
-              const unsigned pneed = __ballot_sync(FULL, !pv);
-              if (pneed) {
-                unsigned long long b0 = 0;
-                if (lane == 0) b0 = atomicAdd(&s_cur, (unsigned long long)__popc(pneed));
-                b0 = __shfl_sync(FULL, b0, 0);
-                if (b0 >= q1) {
-                  drained = true;
-                } else {
-                  const unsigned rank = __popc(pneed & lt_mask);
-                  if (!pv && b0 + rank < q1) {
-                    const uint32_t nl = (uint32_t)((long long)(b0 + rank) - pk);
-                    const long long np = so + nl;
-                    my_pf[5 * pf_stride] = __uint_as_float(nl);
-                    cp_async4(my_pf, B.w + np);
-                    cp_async4(my_pf + pf_stride, B.t + np);
-                    cp_async4(my_pf + 2 * pf_stride, B.p1 + np);
-                    cp_async4(my_pf + 3 * pf_stride, B.d1 + np);
-                    cp_async4(my_pf + 4 * pf_stride, B.cell + np);
-                    cp_async_commit();
-                    pv = true;
-                  }
-                }
-              }
-            }
-            if (!__any_sync(FULL, !has && pv)) break;
+            need = __ballot_sync(FULL, !has);
           }
-          if (!__any_sync(FULL, has)) break;
+          if (need == FULL) break;
         }
-        unsigned need = PF ? 0u : __ballot_sync(FULL, !has);
-        while (need && !drained) {
-          unsigned long long b0 = 0;
-          if (lane == 0) b0 = atomicAdd(&s_cur, (unsigned long long)__popc(need));
-          b0 = __shfl_sync(FULL, b0, 0);
-          if (b0 >= q1) { drained = true; break; }
-          const unsigned rank = __popc(need & lt_mask);
-          if (!has && b0 + rank < q1) {
-            lid = (uint32_t)((long long)(b0 + rank) - pk);
-            pid = so + lid;
-            w = B.w[pid];
-            dcen = (dt - B.t[pid]) * c_light;
-            if (w > 0.f && dcen > 0.f) {
-              x = B.p1[pid]; u = B.d1[pid]; ci = B.cell[pid];
-              ev = 0;
-              w_in = w;
-              has = true;
-            }
-          }
-          need = __ballot_sync(FULL, !has);
-        }
-        if (!__any_sync(FULL, has)) break;
-        bool flush = false;
-        int flush_cell = 0;
-        double f_lost = 0.0, f_wd = 0.0;
+        BOut o{};
+        int c0 = 0;
         if (has) {
-          const float2 sq = SS[ci];
-          const float sa = sq.x, ss = sq.y;
-          bool finished = false;
-          if (ev >= (1u << 30)) {
-            atomicAdd(&blk_cnt[B_CAP], 1u);
-            atomicOr(a.flags, (int)IMC_FLAG_EVENT_CAP);
-            finished = true;
-          } else {
-            const U4 r = draw_rk4(reinterpret_cast<const uint4*>(s_rk), lid, ev, step, TAG_TRANSPORT);
-            ++ev;
-            const float xl = EF[ci], xr = EF[ci + 1];
-            const float L = xr - xl;
-            const float sb = slab_face(x, u, xl, xr);
-            float ds = BIGF;
-            {
-              const bool capped = ss * L > 10000.0f;
-              const float sig = capped ? 10000.0f / L : (ss > 1e-10f ? ss : 0.f);
-              if (sig > 0.f) {
-                const float s_other = fminf(sb, dcen);
-                const double t = (double)sig * (double)s_other;
-                bool may = true;
-                if (t < 0.01) {
-                  const double thr = 1.0 - t * (1.0 - t * (0.5 - t * (1.0 / 6.0)));
-                  may = u01d(r.x) > thr;
-                }
-                if (may) ds = capped ? neglog_u(r.x) * (L * 1e-4f) : __fdividef(neglog_u(r.x), ss);
-              }
-            }
-            float d = sb;
-            int evt = EV_BOUNDARY, cross = X_NONE;
-            if (ds < d) { d = ds; evt = EV_SCATTER; }
-            if (dcen < d) { d = dcen; evt = EV_CENSUS; }
-            float xn = fmaf(u, d, x), un = u;
-            if (evt == EV_BOUNDARY) { if (u > 0.f) { xn = xr; cross = X_IP; } else { xn = xl; cross = X_IM; } }
-            else { if (evt == EV_SCATTER) un = fmaf(2.f, u01f(r.y), -1.f); xn = fminf(fmaxf(xn, xl), xr); }
-            // implicit capture: the energy removed in a visit is counted at its flush, w_in - w
-            const float wn = w * __expf(-sa * d);
-            if (CF[ci] <= 0.0) acc_wd += (double)(w * d);
-            dcen -= d;
-            if (evt == EV_BOUNDARY) ++s_bd; else if (evt == EV_SCATTER) ++s_sc;
-            else atomicAdd(&blk_cnt[B_CENSUS], 1u);
-            w = wn; x = xn; u = un;
-            if (cross != X_NONE) {
-              flush = true; flush_cell = ci; f_lost = (double)w_in - (double)w; f_wd = acc_wd;
-              w_in = w; acc_wd = 0.0;
-              int ni = cross == X_IP ? ci + 1 : ci - 1;
-              const int side = ni < 0 ? 0 : (ni >= nc ? 1 : -1);
-              if (side >= 0) {
-                if ((rmask >> side) & 1) {
-                  u = -u;
-                  ni = side == 0 ? 0 : nc - 1;
-                  atomicAdd(&blk_cnt[B_REFLECT], 1u);
-                } else {
-                  atomicAdd(a.esc_fx + 2 * k + side, fx_units((double)w, inv_q));
-                  atomicAdd(&blk_cnt[B_ESCAPE], 1u);
-                  w = 0.f;
-                  finished = true;
-                  ni = ci;
-                }
-              }
-              ci = ni;
-            }
-            if (!finished && w < wfloor) {
-              // IMC/IMC1D.py:188-195: kill and deposit the remainder in the current cell.
-              // Without a crossing in this event the visit's flush at the history end (w_in - 0)
-              // carries it; after one, the old cell holds the flush slot and the remainder goes
-              // to the new cell here (its intensity follows from the deposition)
-              atomicAdd(&blk_cnt[B_FLOOR], 1u);
-              if (flush) atomicAdd(TD + ci, fx_units((double)w, inv_q));
-              w = 0.f;
-              finished = true;
-            }
-            if (!finished && !(dcen > 0.f)) finished = true;
+          c0 = h.ci;
+          const U4 r = draw_next4(reinterpret_cast<const uint4*>(s_rk) + 1, h.key, rkx, h.ev);
+          batch_event(h, o, EF[c0], r, nc, rmask, wfloor, blk_cnt, a.flags, s_cen, s_sc);
+          if (o.flush) {
+            const unsigned long long ud = fx_units(o.lost, inv_q);
+            if (ud) smem_add_u64(TD + c0, ud);
+            if (o.escaped >= 0) atomicAdd(a.esc_fx + 2 * k + o.escaped, fx_units((double)o.esc_w, inv_q));
+            if (o.kill > 0.f) smem_add_u64(TD + h.ci, fx_units((double)o.kill, inv_q));
           }
-          if (finished) {
-            if (!flush) {  // the visit the history ends in
-              const double lost = (double)w_in - (double)w;
-              if (lost != 0.0 || acc_wd != 0.0) { flush = true; flush_cell = ci; f_lost = lost; f_wd = acc_wd; }
-            }
-            acc_wd = 0.0;
-            B.w[pid] = w;
-            if (w > 0.f) { B.p1[pid] = x; B.d1[pid] = u; B.cell[pid] = ci; }
-            ev_acc += ev;
-            has = false;
-          }
+          if (o.finished) { has = false; pend = true; }
+          else if (o.flush) h.tab = SS[h.ci];
         }
-        if (flush) {
-          // the cell visit's tallies into the block's staged ones (one shared atomic per lane):
-          // deposition in fixed point, raw w*s only from a cell without absorption (an
-          // absorbing cell's intensity follows from its deposition in the material update)
-          const unsigned long long ud = fx_units(f_lost, inv_q);
-          if (ud) atomicAdd(TD + flush_cell, ud);
-          if (f_wd != 0.0) atomicAdd(TS + flush_cell, f_wd);
-        }
+        warp_tally1(o.wd != 0.f, cur_cb + c0, (double)o.wd, a.si, st);
       }
       // the unit's events of this instance to its ledger, one atomic per warp
+      ev_all += ev_acc;
       const unsigned long long t_ev = warp_sum_u64(ev_acc);
       if (lane == 0 && t_ev) atomicAdd(a.ledger + (size_t)k * IMC_BL_N + IMC_BL_EVENTS, (double)t_ev);
       __syncthreads();  // every warp is done with s_cur and the tables of this range
       q0 = q1;
     }
   }
-  for (int c = threadIdx.x; c < cur_nc; c += blockDim.x) {
+  for (int c = threadIdx.x; c < cur_nc; c += blockDim.x)
     if (TD[c]) atomicAdd(a.dep_fx + cur_cb + c, TD[c]);
-    if (TS[c] != 0.0) atomicAdd(a.si + cur_cb + c, TS[c]);
-  }
-  const unsigned long long t_bd = warp_sum_u(s_bd), t_sc = warp_sum_u(s_sc);
-  if (lane == 0) {
-    if (t_bd) atomicAdd(a.stats + S_BOUNDARY, t_bd);
-    if (t_sc) atomicAdd(a.stats + S_SCATTER, t_sc);
-    if (t_bd + t_sc) atomicAdd(a.stats + S_EVENTS, t_bd + t_sc);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned long long cen = blk_cnt[B_CENSUS], cap = blk_cnt[B_CAP];
-    if (cen) atomicAdd(a.stats + S_CENSUS, cen);
-    if (cen + cap) atomicAdd(a.stats + S_EVENTS, cen + cap);
-    if (blk_cnt[B_FLOOR]) atomicAdd(a.stats + S_FLOOR, (unsigned long long)blk_cnt[B_FLOOR]);
-    if (blk_cnt[B_REFLECT]) atomicAdd(a.stats + S_REFLECT, (unsigned long long)blk_cnt[B_REFLECT]);
-    if (cap) atomicAdd(a.stats + S_CAP, cap);
-    if (blk_cnt[B_ESCAPE]) atomicAdd(a.stats + S_ESCAPE, (unsigned long long)blk_cnt[B_ESCAPE]);
-  }
+  batch_event_counts(a, blk_cnt, ev_all, s_cen, s_sc);
 }
 
 // ---------------------------------------------------------------- comb
@@ -868,16 +703,16 @@ cudaError_t imc_batch_launch_wsum(const BatchArgs& a, cudaStream_t s) {
 }
 
 cudaError_t imc_batch_launch_track(const BatchArgs& a, int block, int grid, cudaStream_t s) {
+  if (block > 256) return cudaErrorInvalidConfiguration;
   ++g_imc_launches;
   if (a.form != 2 && a.max_cells > 0 && a.max_cells <= IMC_BATCH_SMEM_CELLS) {
-    const bool pf = a.form == 3;
-    const size_t sh = units_smem(a.K, a.max_cells) + (pf ? units_pf_smem(block) : 0);
-    auto kern = pf ? k_btrack_units<true> : k_btrack_units<false>;
+    const size_t sh = units_smem(a.max_cells);
     if (sh > 48 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+      const cudaError_t e = cudaFuncSetAttribute(k_btrack_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
       if (e != cudaSuccess) return e;
     }
-    kern<<<grid, block, sh, s>>>(a);
+    const long long blocks = std::max(1LL, (long long)grid * block / kUnitThreads);
+    k_btrack_units<<<(unsigned)blocks, kUnitThreads, sh, s>>>(a);
     return cudaGetLastError();
   }
   const size_t sh = (size_t)(block / 32) * sizeof(WarpStage) + pref_bytes(a);

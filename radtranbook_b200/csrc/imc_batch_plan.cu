@@ -85,7 +85,9 @@ __global__ void k_bmaterial_fleck(BatchArgs a, int update) {
   f = fmin(1.0, fmax(0.0, f));
   const double ss = sig * (1.0 - f);
   const double sa = sig * f;
-  a.sass[c] = make_float2((float)sa, (float)ss);
+  // as the single-problem table: absorption 0 marks a cell whose intensity is its w*s tally
+  const float L = a.ef[c + k + 1] - a.ef[c + k];
+  a.sass[c] = make_float2(sa > 1e-10 ? (float)sa : 0.f, scatter_entry(ss, 1e-10f, L));
   const double iv = 1.0 / V;
   a.cellf[c] = make_double2(iv, sa > 1e-10 ? 1.0 / (sa * V * a.dt) : -1.0 / (V * a.dt));
   a.emit_E[c] = A_RAD * C_LIGHT * pow4(fmax(T, 0.0)) * sa * a.dt * V;

@@ -69,6 +69,15 @@ __device__ inline long long block_scan_counts(const long long* n, long long* off
   return total;
 }
 
+// The tracking table's scatter slot: the effective scatter opacity, 0 at or below the geometry's
+// threshold, negative where the distance is capped (sigma_s L > 1e4 in FP32, L the cell's smaller
+// width; L = 0: no cap), so that a flight neither compares with the threshold nor forms L.
+__device__ __forceinline__ float scatter_entry(double ss64, float threshold, float L) {
+  const float ss = (float)ss64;
+  if (!(ss > threshold)) return 0.f;
+  return ss * L > 10000.0f ? -ss : ss;
+}
+
 // order position o = i*ny + j (the reference's i-outer, j-inner source loops)
 __device__ __forceinline__ int order_to_cell(int o, int nx, int ny) {
   const int i = o / ny, j = o - (o / ny) * ny;

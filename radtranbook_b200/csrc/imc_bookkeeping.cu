@@ -27,19 +27,11 @@ constexpr double PI = 3.14159265358979323846;
 using imcblk::NT;
 using namespace imcblk;
 
-// The tracking table's scatter slot: the effective scatter opacity, 0 at or below the geometry's
-// threshold (1e-10 in 1-D, 1e-12 in 2-D), negative where the distance is capped (sigma_s L > 1e4
-// with L the cell's smaller width, in FP32 as the tracking moves), so that a flight neither
-// compares with the threshold nor forms L.
-__device__ __forceinline__ float scatter_entry(double ss64, bool oned, bool caps, const double* e1, const double* e2,
-                                               int nx, int c) {
-  const float ss = (float)ss64;
-  if (!(ss > (oned ? 1e-10f : 1e-12f))) return 0.f;
-  if (!caps) return ss;
+// The width the scatter cap compares with: the cell's smaller one, in FP32 as the tracking moves.
+__device__ __forceinline__ float cell_width(bool oned, const double* e1, const double* e2, int nx, int c) {
   const int j = c / nx, i = c - j * nx;
-  float L = (float)e1[i + 1] - (float)e1[i];
-  if (!oned) L = fminf(L, (float)e2[j + 1] - (float)e2[j]);
-  return ss * L > 10000.0f ? -ss : ss;
+  const float L = (float)e1[i + 1] - (float)e1[i];
+  return oned ? L : fminf(L, (float)e2[j + 1] - (float)e2[j]);
 }
 
 // Per-cell part of the plan, one thread per cell: Fleck factor, absorption / effective
@@ -68,7 +60,7 @@ __global__ void k_plan_cells(PlanArgs a) {
     // tracking table: sigma_a below the estimator's threshold is entered as 0 (no capture; in
     // FP32 exp(-sigma_a s) is 1 there anyway), which also marks the cell's intensity as the
     // path-length sum w*s; elsewhere the intensity follows from the deposition
-    a.sass[c] = make_float2(sa > sa_thr ? (float)sa : 0.f, scatter_entry(ss, oned, true, a.e1, a.e2, a.nx, c));
+    a.sass[c] = make_float2(sa > sa_thr ? (float)sa : 0.f, scatter_entry(ss, oned ? 1e-10f : 1e-12f, cell_width(oned, a.e1, a.e2, a.nx, c)));
     const double iv = 1.0 / a.vol[c];
     a.cellf[c] = make_double2(iv, sa > sa_thr ? 1.0 / (sa * a.vol[c] * dt) : -1.0 / (a.vol[c] * dt));
     double E = A_RAD * C_LIGHT * pow4(fmax(T, 0.0)) * sa * dt * a.vol[c];
@@ -82,7 +74,7 @@ __global__ void k_plan_cells(PlanArgs a) {
       const double beta = 4.0 * A_RAD * pow3(Tm) / a.cv[c];
       const double rate = C_LIGHT * sig * beta;
       a.sa[c] = sig; a.ss[c] = 0.0;
-      a.sass[c] = make_float2(0.f, scatter_entry(sig, oned, true, a.e1, a.e2, a.nx, c));
+      a.sass[c] = make_float2(0.f, scatter_entry(sig, oned ? 1e-10f : 1e-12f, cell_width(oned, a.e1, a.e2, a.nx, c)));
       a.cellf[c] = make_double2(iv, -1.0 / (a.vol[c] * dt));
       a.cf_rate[c] = (beta > 1e-15 && sig > 1e-15) ? (float)rate : 0.f;
       const double T4 = pow4(fmax(T, 0.0));
@@ -655,7 +647,7 @@ __global__ void __launch_bounds__(256) k_plan_mg_cells(PlanMgArgs a, int cb) {
       const double sa = a.sigma[q] * f;
       a.sa[q] = sa; a.ss[q] = ss;
       // absorption 0: no capture, w*s intensity
-      a.sass[q] = make_float2(sa > 1e-12 ? (float)sa : 0.f, scatter_entry(ss, false, false, a.e1, a.e2, a.nx, c));
+      a.sass[q] = make_float2(sa > 1e-12 ? (float)sa : 0.f, scatter_entry(ss, 1e-12f, 0.f));
       a.cellf[q] = make_double2(1.0 / a.vol[c], sa > 1e-12 ? 1.0 / (sa * a.vol[c] * dt) : -1.0 / (a.vol[c] * dt));
       const double bg = a.emission_fractions ? a.emission_fractions[g] : gc[g];
       run += sa * bg * aT4;
@@ -793,7 +785,7 @@ __global__ void __launch_bounds__(256) k_plan_mg1d_cells(PlanMgArgs a, int cb) {
       const double ss = a.sigma[q] * (1.0 - f);
       a.sa[q] = sa; a.ss[q] = ss;
       // absorption 0: no capture, w*s intensity
-      a.sass[q] = make_float2(sa > 1e-10 ? (float)sa : 0.f, scatter_entry(ss, true, true, a.e1, a.e2, a.nx, c));
+      a.sass[q] = make_float2(sa > 1e-10 ? (float)sa : 0.f, scatter_entry(ss, 1e-10f, cell_width(true, a.e1, a.e2, a.nx, c)));
       // MG_IMC/MG_IMC1D.py:346-350: path-length estimator below sigma_a = 1e-10
       a.cellf[q] = make_double2(1.0 / a.vol[c], sa > 1e-10 ? 1.0 / (sa * a.vol[c] * dt) : -1.0 / (a.vol[c] * dt));
       a.emit_E[q] = cold ? 0.0 : A_RAD * C_LIGHT * pow4(T) * sa * b[g] * dt * a.vol[c] * a.share;

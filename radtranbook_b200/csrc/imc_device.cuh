@@ -102,14 +102,14 @@ __device__ __forceinline__ U4 draw_next(const uint32_t* rk, const DrawKey& k, ui
   return c;
 }
 
-// draw_rk with the round keys read as five 16-byte words (rk4: the 20 keys of
-// philox_round_keys, 16-byte aligned, e.g. staged in shared memory): the same numbers, five
-// vector loads where draw_rk makes twenty scalar ones.
-__device__ __forceinline__ U4 draw_rk4(const uint4* rk4, uint32_t idx, uint32_t block, uint32_t step,
-                                       uint32_t tag) {
-  U4 c{idx, block, step, tag};
+// draw_next with the round keys of rounds 3..10 read as four 16-byte words (rk4: keys 4..19 of
+// philox_round_keys, 16-byte aligned, e.g. staged in shared memory): four vector loads where
+// draw_next makes sixteen scalar ones.
+__device__ __forceinline__ U4 draw_next4(const uint4* rk4, const DrawKey& key, uint32_t rkx, uint32_t block) {
+  const uint32_t x1 = rkx ^ block;
+  U4 c{key.a, key.b, __umulhi(0xD2511F53u, x1) ^ key.c, 0xD2511F53u * x1};
 #pragma unroll
-  for (int q = 0; q < 5; ++q) {
+  for (int q = 0; q < 4; ++q) {
     const uint4 k = rk4[q];
     const uint32_t a0 = 0xD2511F53u * c.x, b0 = __umulhi(0xD2511F53u, c.x);
     const uint32_t a1 = 0xCD9E8D57u * c.z, b1 = __umulhi(0xCD9E8D57u, c.z);
@@ -374,6 +374,18 @@ constexpr double FX_ONE = 1152921504606846976.0;  // 2^60
 __device__ __forceinline__ double fx_inv_quantum(double wsum) { return wsum > 0.0 ? FX_ONE / wsum : 0.0; }
 __device__ __forceinline__ unsigned long long fx_units(double e, double inv_q) { return __double2ull_rn(e * inv_q); }
 __device__ __forceinline__ double fx_energy(unsigned long long u, double wsum) { return (double)u * (wsum / FX_ONE); }
+
+// 64-bit add to a shared-memory tally as two 32-bit adds, the low word's carry going into the
+// high word: the sum is exact modulo 2^64 in any order, and both adds are native shared-memory
+// atomics, where the 64-bit one is a compare-and-swap loop (the ten launches of a 2M crooked-pipe
+// run: 14.0 ms with the 64-bit atomic, 12.6 ms so).
+__device__ __forceinline__ void smem_add_u64(unsigned long long* t, unsigned long long v) {
+  unsigned* q = reinterpret_cast<unsigned*>(t);
+  const unsigned lo = (unsigned)v;
+  const unsigned old = atomicAdd(q, lo);
+  const unsigned hi = (unsigned)(v >> 32) + (old + lo < lo ? 1u : 0u);
+  if (hi) atomicAdd(q + 1, hi);
+}
 
 // warp_tally2 with the first tally in fixed point (a zero value issues no reduction)
 __device__ __forceinline__ void warp_tally_fx(bool flush, int key, unsigned long long ua, double vb,

@@ -229,18 +229,6 @@ __device__ __forceinline__ void add_event_counts(const TrackArgs& a, const unsig
   if (threadIdx.x < 4 && blk_esc[threadIdx.x] != 0ull) atomicAdd(a.esc_fx + threadIdx.x, blk_esc[threadIdx.x]);
 }
 
-// 64-bit add to a shared-memory tally as two 32-bit adds, the low word's carry going into the
-// high word: the sum is exact modulo 2^64 in any order, and both adds are native shared-memory
-// atomics, where the 64-bit one is a compare-and-swap loop (the ten launches of a 2M crooked-pipe
-// run: 14.0 ms with the 64-bit atomic, 12.6 ms so).
-__device__ __forceinline__ void smem_add_u64(unsigned long long* t, unsigned long long v) {
-  unsigned* q = reinterpret_cast<unsigned*>(t);
-  const unsigned lo = (unsigned)v;
-  const unsigned old = atomicAdd(q, lo);
-  const unsigned hi = (unsigned)(v >> 32) + (old + lo < lo ? 1u : 0u);
-  if (hi) atomicAdd(q + 1, hi);
-}
-
 // Where a cell visit's deposition (fixed point) and path-length intensity (FP64) are summed:
 //   T_GLOBAL  global memory, the warp's lanes grouped by cell first (one reduction per cell)
 //   T_SMALL   both per block in shared memory, added to the global ones at the block's end
