@@ -131,9 +131,8 @@ typedef struct imc_step_params {
                                    (as many threads as block_size x blocks_per_sm, at most 1024)
                                    with its tally in shared memory while that fits; bit 3:
                                    event-by-event tracking (workspace of imc_workspace_bytes_event);
-                                   bit 4: prefetched refills (each lane copies its next history's
-                                   bank record into shared memory while it tracks the current one;
-                                   the same histories and tallies); others ignored */
+                                   others ignored (bit 4 once chose another way of refilling, with
+                                   the same histories and tallies) */
   const double* emission_fractions; /* MG: [g] fixed emission spectrum, or NULL = Planck */
   int64_t n_boundary_side[4];   /* > 0: boundary particles on that side instead of n_boundary
                                    (per-side budgets, MG_IMC/MG_IMC1D.py:1000-1040) */

@@ -433,8 +433,6 @@ imc_status transport_async(const imc_mesh* mesh, const imc_material* mat, const 
   const bool smem_tally = smem_cells && !(par->reserved & 4) && ((par->reserved & 2) || (long long)nc * ng <= 2048);
   // bit 2 (no block tallies) also rules out the wide block's
   const bool wide_ok = !(par->reserved & 4);
-  // bit 4: prefetched refills (each lane's next bank record copied to shared memory ahead)
-  const bool prefetch = (par->reserved & 16) != 0;
   if (adj) {
     AdjointArgs A = *adj;
     A.t = ta; A.sa64 = tal->sigma_a; A.ss64 = tal->sigma_s; A.sig64 = mat->sigma;
@@ -451,7 +449,7 @@ imc_status transport_async(const imc_mesh* mesh, const imc_material* mat, const 
     if (cap_hit) return IMC_ERR_EVENT_CAP;
   } else {
     IMC_CUDA(imc_launch_track(ta, mesh->geometry,
-                              TrackLaunch{block, bps, sm_count(), smem_cells, smem_tally, wide_ok, prefetch}, s));
+                              TrackLaunch{block, bps, sm_count(), smem_cells, smem_tally, wide_ok}, s));
   }
   if (pe.ok) { IMC_CUDA(cudaEventRecord(pe.e[2], s)); pe.recorded = true; }
   IMC_CUDA(imc_launch_tally_finalize(ta, s));

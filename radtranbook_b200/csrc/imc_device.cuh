@@ -20,7 +20,6 @@ constexpr unsigned FULL = 0xffffffffu;
 
 enum : int { G_SLAB = 0, G_SPHERE = 1, G_XY = 2, G_RZ = 3 };
 enum : int { EV_CENSUS = 0, EV_BOUNDARY = 1, EV_SCATTER = 2 };
-enum : int { X_NONE = 0, X_IP = 1, X_IM = 2, X_JP = 3, X_JM = 4 };
 enum : int { S_EVENTS = 0, S_BOUNDARY, S_SCATTER, S_CENSUS, S_CAPTURE, S_FLOOR, S_REFLECT, S_CAP, S_ESCAPE, S_N };
 
 enum : uint32_t {
@@ -130,14 +129,6 @@ __device__ __forceinline__ uint32_t u4_word(const U4& r, int q) {
 // -log(u) for u = u01: distance in mean free paths.
 __device__ __forceinline__ float neglog_u(uint32_t x) { return -logf(u01f(x)); }
 
-// Effective-scatter distance with the optically-thick cap of the reference
-// (IMC/IMC1D.py:83-88; IMC/IMC2D.py:758-765): sigma_s*L > 1e4 uses sigma = 1e4/L.
-__device__ __forceinline__ float scatter_distance(float ss, float L, uint32_t x, float thresh, bool cap) {
-  if (cap && ss * L > 10000.0f) return neglog_u(x) * (L * 1e-4f);
-  if (ss > thresh) return neglog_u(x) / ss;
-  return BIGF;
-}
-
 // Whether a scatter at -log(u)/sigma, u = u01(x), can come before s_other.  With p = 1 - u
 // (exact in FP32, at least 2^-24) the scatter is at least p/sigma away, so p >= sigma s_other
 // (1 + 1e-6) rules it out whatever the rounding of the logarithm and the quotient; that
@@ -151,12 +142,6 @@ __device__ __forceinline__ bool scatter_may_win(uint32_t x, float sig, float s_o
   const double thr = 1.0 - t * (1.0 - t * (0.5 - t * (1.0 / 6.0)));
   return u01d(x) > thr;
 }
-
-struct Ev {
-  float d;       // path length of this event
-  int evt;       // EV_*
-  int cross;     // X_*
-};
 
 // The tracking's approximate quotient and reciprocal square root: the hardware approximations
 // without the steps that widen them to subnormal operands, which no distance, direction or
@@ -204,43 +189,6 @@ __device__ __forceinline__ float inner_root(float r, float mu, float R, float b2
 // of each group sums the group's values (staged in per-warp shared memory) and issues
 // one FP64 red per tally.
 struct WarpStage { double a[32]; double b[32]; };
-
-// Asynchronous 4-byte global -> shared copies (cp.async): a thread starts the copies of a bank
-// record it will need later and waits for its own copies only when it reads them.
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-__device__ __forceinline__ void warp_tally2(bool flush, int key, double va, double vb,
-                                            double* __restrict__ ta, double* __restrict__ tb,
-                                            WarpStage* st) {
-  const unsigned fm = __ballot_sync(FULL, flush);
-  if (fm == 0u) return;
-  const int lane = threadIdx.x & 31;
-  const int k = flush ? key : -1 - lane;  // keys >= 0 for flushing lanes are cells
-  const unsigned peers = __match_any_sync(FULL, k);
-  if (__all_sync(FULL, !flush || __popc(peers) == 1)) {
-    if (flush) { atomicAdd(ta + key, va); atomicAdd(tb + key, vb); }
-    return;
-  }
-  st->a[lane] = va; st->b[lane] = vb;
-  __syncwarp();
-  if (flush && (__ffs(peers) - 1) == lane) {
-    double sa = 0.0, sb = 0.0;
-    unsigned m = peers;
-    while (m) {
-      const int l = __ffs(m) - 1;
-      m &= m - 1;
-      sa += st->a[l]; sb += st->b[l];
-    }
-    atomicAdd(ta + key, sa);
-    atomicAdd(tb + key, sb);
-  }
-  __syncwarp();
-}
 
 __device__ __forceinline__ void warp_tally1(bool flush, int key, double va, double* __restrict__ ta,
                                             WarpStage* st) {
@@ -387,7 +335,7 @@ __device__ __forceinline__ void smem_add_u64(unsigned long long* t, unsigned lon
   if (hi) atomicAdd(q + 1, hi);
 }
 
-// warp_tally2 with the first tally in fixed point (a zero value issues no reduction)
+// Two tallies at once, the first in fixed point (a zero value issues no reduction)
 __device__ __forceinline__ void warp_tally_fx(bool flush, int key, unsigned long long ua, double vb,
                                               unsigned long long* __restrict__ ta, double* __restrict__ tb,
                                               WarpStage* st) {

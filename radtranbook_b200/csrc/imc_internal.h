@@ -56,12 +56,11 @@ struct TrackArgs {
 };
 
 // smem_tally: per-block deposition / intensity tallies in shared memory (with smem_cells only);
-// wide_ok: one block per SM with its tally in shared memory may be used where that fits;
-// prefetch: lanes copy their next history's bank record into shared memory while they track
+// wide_ok: one block per SM with its tally in shared memory may be used where that fits
 constexpr size_t kSmemPerBlock = 226 * 1024;  // dynamic shared memory of a wide block, beside its few hundred static bytes
 struct TrackLaunch {
   int block, blocks_per_sm, sms;
-  bool smem_cells, smem_tally, wide_ok, prefetch;
+  bool smem_cells, smem_tally, wide_ok;
 };
 cudaError_t imc_launch_track(const TrackArgs& a, int geom, const TrackLaunch& l, cudaStream_t s);
 // Event-by-event tracking (reserved bit 3 of imc_step_params): scratch bytes for a bank of

@@ -399,229 +399,6 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
   if (TS_S) for (int q = threadIdx.x; q < ncg; q += blockDim.x) if (TS[q] != 0.0) atomicAdd(a.si + q, TS[q]);
 }
 
-// SMEM_TALLY (small meshes): the block sums its deposition (fixed point) and intensity per
-// (group, cell) in shared memory and adds them to the global tallies once, at its end.  On a
-// mesh of a few hundred cells every crossing would otherwise send its reductions to the few
-// dozen cells the wave occupies, which serialise in the L2.
-//
-// PF (prefetched refills): every lane keeps the bank record of its next history in a
-// shared-memory slot, copied there by cp.async while it tracks the current one, so a lane
-// whose history ends starts the next one from shared memory instead of holding its warp on two
-// dependent HBM reads (weight and birth time, then the rest of the record).  The histories,
-// their Philox counters and the tallies are the same; only which lane tracks which differs.
-enum : int { PF_W = 0, PF_T, PF_P1, PF_D1, PF_CELL, PF_P2, PF_D2, PF_GROUP, PF_PID, PF_NF };
-inline size_t pf_smem(int block) { return sizeof(float) * PF_NF * (size_t)block; }
-
-template <int GEOM, bool SMEM_CELLS, bool MG, bool CF, bool SMEM_TALLY>
-__global__ void __launch_bounds__(256, 4) k_track_pf(TrackArgs a) {  // at most 64 registers
-  pdl_wait();     // the previous kernel of the stream has completed
-  pdl_trigger();  // the next one may be scheduled
-  const float dtk = a.dt_dev ? (float)*a.dt_dev : a.dt;  // graph replay: step length and Philox
-  const uint32_t stepk = a.step_dev ? *a.step_dev : a.step;  // step counter from device memory
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ unsigned blk_cnt[B_N];
-  __shared__ unsigned long long blk_esc[4];
-  constexpr bool ONED = GEOM == G_SLAB || GEOM == G_SPHERE;
-  constexpr bool MG2 = MG && !ONED;  // MG_IMC2D history rules
-  WarpStage* stages = reinterpret_cast<WarpStage*>(smem);
-  const int nwarps = blockDim.x >> 5;
-  float2* E1 = reinterpret_cast<float2*>(stages + nwarps);  // (lower, upper) edge per index
-  float2* E2 = E1 + a.nx;
-  float2* CS = E2 + a.ny;
-  const int ncg = a.nc * a.ng;
-  // block tallies after the table (8-byte aligned: CS is), deposition then intensity
-  unsigned long long* TD = reinterpret_cast<unsigned long long*>(CS + (SMEM_CELLS ? ncg : 0));
-  double* TS = reinterpret_cast<double*>(TD + ncg);
-  unsigned long long* const dep_t = SMEM_TALLY ? TD : a.dep_fx;
-  double* const si_t = SMEM_TALLY ? TS : a.si;
-  for (int q = threadIdx.x; q < a.nx; q += blockDim.x) E1[q] = make_float2(a.e1[q], a.e1[q + 1]);
-  for (int q = threadIdx.x; q < a.ny; q += blockDim.x) E2[q] = make_float2(a.e2[q], a.e2[q + 1]);
-  if (SMEM_CELLS)
-    for (int q = threadIdx.x; q < ncg; q += blockDim.x) CS[q] = a.sass[q];
-  if (SMEM_TALLY)
-    for (int q = threadIdx.x; q < ncg; q += blockDim.x) { TD[q] = 0ull; TS[q] = 0.0; }
-  if (threadIdx.x < B_N) blk_cnt[threadIdx.x] = 0u;
-  if (threadIdx.x < 4) blk_esc[threadIdx.x] = 0ull;
-  __syncthreads();
-
-  const int lane = threadIdx.x & 31;
-  const unsigned lt_mask = (1u << lane) - 1u;
-  WarpStage* st = stages + (threadIdx.x >> 5);
-  const uint32_t n = (uint32_t)*a.n_dev;
-
-  // warp-uniform chunk cursor
-  uint32_t chunk_next = 0, chunk_end = 0;
-  bool drained = false;
-
-  // lane state
-  bool has = false;
-  uint32_t pid = 0, ev = 0;
-  float x = 0, y = 0, u = 0, v = 0, w = 0, dcen = 0;
-  int ci = 0, cj = 0, grp = 0;
-  // (sigma_a, sigma_s) of the current (group, cell), loaded as soon as the cell is known (at
-  // refill, after a crossing) so the load overlaps the tally flush and refill of the loop end
-  float2 tab = make_float2(0.f, 0.f);
-  auto table = [&](int cq) { return SMEM_CELLS ? CS[cq] : __ldg(a.sass + cq); };
-  // energy removed in the current cell visit: the per-flight differences telescope, so it is
-  // the weight at the visit's start minus the weight now (one FP64 difference at the flush)
-  float w_in = 0.f;
-  DrawKey key{0u, 0u, 0u};
-  const uint32_t rkx = draw_step_key(a.rk, stepk);
-  unsigned s_ev = 0, s_cen = 0, s_sc = 0;  // events of ended histories, census events, scatters
-  unsigned n_alive = 0;                 // entries alive at the end (census sums for the comb)
-
-  const float c_light = (float)C_LIGHT;
-  // weight floor, IMC/IMC1D.py:1007 / IMC/IMC2D.py:1771 (1e-10); MG_IMC/MG_IMC1D.py:1127 (1e-14)
-  const float weight_floor = (float)(a.floor_coef * (*a.wsum) / (double)(n > 0 ? n : 1));
-  const double inv_q = fx_inv_quantum(*a.wsum);  // fixed-point energy tallies
-  const float inv_nx = 1.0f / (float)a.nx;  // cell -> (i, j) at refill without an integer divide
-
-  // PF: the lane's next bank record, field f of thread i at PQ[f * blockDim.x + i] (after the
-  // block tallies, or after the cell table without them)
-  float* const my_pf = (SMEM_TALLY ? reinterpret_cast<float*>(TS + ncg) : reinterpret_cast<float*>(TD)) + threadIdx.x;
-  const int pfs = blockDim.x;
-  bool pv = false;  // PF: the slot holds a claimed record (copies issued)
-
-  for (;;) {
-    // ---------------- refill idle lanes from the warp's chunk ----------------
-    {
-      // An idle lane takes the record in its slot; every lane without a claim takes the next
-      // entry of the warp's chunk (a new guided ticket when it runs out) and starts its copies,
-      // which land while the lane tracks.  Leaves with every lane tracking or holding no claim;
-      // when the warp stops, the queue is past n and no claim is left untaken.
-      for (;;) {
-        if (!has && pv) {
-          cp_async_wait_all();
-          pv = false;
-          pid = __float_as_uint(my_pf[PF_PID * pfs]);
-          w = my_pf[0];
-          dcen = (dtk - my_pf[pfs]) * c_light;
-          const int c = __float_as_int(my_pf[PF_CELL * pfs]);
-          const int g = MG ? __float_as_int(my_pf[PF_GROUP * pfs]) : 0;
-          const bool moves = (MG2 || CF ? w > weight_floor : w > 0.f) && dcen > 0.f;
-          if (!moves && w > 0.f && a.ecen) {
-            const int b = c + (a.ecen_by_group ? a.nc * g : 0);
-#ifdef IMC_CHECKED
-            if (b >= 0 && b < a.nc * (a.ecen_by_group ? a.ng : 1))
-#endif
-            { atomicAdd(a.ecen + b, (double)w); ++n_alive; }
-          }
-          if (moves) {
-            x = my_pf[2 * pfs]; u = my_pf[3 * pfs];
-            if (MG) grp = g;
-            if (GEOM == G_XY || GEOM == G_RZ) { y = my_pf[PF_P2 * pfs]; v = my_pf[PF_D2 * pfs]; }
-#ifdef IMC_CHECKED
-            if (c < 0 || c >= a.nc || (MG && (grp < 0 || grp >= a.ng)) || !isfinite(w)) {
-              atomicOr(a.flags, (int)IMC_FLAG_BOUNDS);
-            } else
-#endif
-            {
-              cj = __float2int_rd(((float)c + 0.5f) * inv_nx);
-              ci = c - cj * a.nx;
-              if (ci < 0) { --cj; ci += a.nx; } else if (ci >= a.nx) { ++cj; ci -= a.nx; }
-              tab = table(MG ? c + a.nc * grp : c);
-              ev = 0;
-              w_in = w;
-              key = draw_key(a.rk, a.id_base + pid, stepk, TAG_TRANSPORT);
-              has = true;
-            }
-          }
-        }
-        if (!drained) {
-          const unsigned pneed = __ballot_sync(FULL, !pv);
-          if (pneed) {
-            if (chunk_next >= chunk_end) {
-              unsigned long long base = 0, claim = 0;
-              if (lane == 0) {
-                const unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(a.queue);
-                const unsigned long long left = cur < (unsigned long long)n ? (unsigned long long)n - cur : 0ull;
-                const unsigned long long nw = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-                claim = min((unsigned long long)a.chunk, max(32ull, left / (2ull * nw)));
-                base = atomicAdd(a.queue, claim);
-              }
-              base = __shfl_sync(FULL, base, 0);
-              claim = __shfl_sync(FULL, claim, 0);
-              if (base >= (unsigned long long)n) {
-                drained = true;
-              } else {
-                chunk_next = (uint32_t)base;
-                chunk_end = (uint32_t)min(base + claim, (unsigned long long)n);
-              }
-            }
-            if (!drained) {
-              const uint32_t avail = chunk_end - chunk_next;
-              const uint32_t rank = __popc(pneed & lt_mask);
-              if (!pv && rank < avail) {
-                const uint32_t np = chunk_next + rank;
-                my_pf[PF_PID * pfs] = __uint_as_float(np);
-                cp_async4(my_pf, a.w + np);
-                cp_async4(my_pf + pfs, a.t + np);
-                cp_async4(my_pf + 2 * pfs, a.p1 + np);
-                cp_async4(my_pf + 3 * pfs, a.d1 + np);
-                cp_async4(my_pf + PF_CELL * pfs, a.cell + np);
-                if (GEOM == G_XY || GEOM == G_RZ) {
-                  cp_async4(my_pf + PF_P2 * pfs, a.p2 + np);
-                  cp_async4(my_pf + PF_D2 * pfs, a.d2 + np);
-                }
-                if (MG) cp_async4(my_pf + PF_GROUP * pfs, a.group + np);
-                cp_async_commit();
-                pv = true;
-              }
-              chunk_next += min((uint32_t)__popc(pneed), avail);
-            }
-          }
-        }
-        if (!__any_sync(FULL, !has && pv)) break;
-      }
-    }
-    if (!__any_sync(FULL, has)) break;
-#ifdef IMC_CHECKED
-    if (has && (ci < 0 || ci >= a.nx || cj < 0 || cj >= a.ny || !isfinite(w) || !isfinite(x) || !isfinite(dcen))) {
-      atomicOr(a.flags, (int)IMC_FLAG_BOUNDS);
-      has = false;  // nothing more is tallied at an invalid index
-    }
-#endif
-
-    EvOut o{0, false, 0.f, 0.0, false};
-    bool cen = false;
-    int cen_bin = 0;
-    if (has) {
-      Hist h{pid, ev, x, y, u, v, w, dcen, w_in, ci, cj, grp, tab, key};
-      history_event<GEOM, SMEM_CELLS, MG, CF>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t, rkx, weight_floor,
-                                              inv_q, s_cen, s_sc);
-      pid = h.pid; ev = h.ev; x = h.x; y = h.y; u = h.u; v = h.v; w = h.w; dcen = h.dcen; w_in = h.w_in;
-      ci = h.ci; cj = h.cj; grp = h.grp; tab = h.tab;
-      if (o.finished) { has = false; cen = history_retire<GEOM>(a, h, cen_bin); s_ev += h.ev; }
-    }
-    const unsigned long long ud = o.flush ? fx_units(o.lost, inv_q) : 0ull;
-    const double vs = (double)o.wd;
-    if (SMEM_TALLY) {
-      if (ud) smem_add_u64(dep_t + o.cell, ud);
-      if (o.wd != 0.f) atomicAdd(si_t + o.cell, vs);
-    } else {
-      warp_tally_fx(ud != 0ull || o.wd != 0.f, o.cell, ud, vs, dep_t, si_t, st);
-    }
-    if (a.ecen) {
-      warp_tally1(cen, cen_bin, (double)w, a.ecen, st);
-      n_alive += cen ? 1u : 0u;
-    }
-  }
-
-  // ---------------- statistics ----------------
-  if (a.ecen) {
-    const unsigned long long t_alive = warp_sum_u(n_alive);
-    if (lane == 0 && t_alive) atomicAdd(a.n_live, t_alive);
-  }
-  add_event_counts(a, blk_cnt, blk_esc, s_ev, s_cen, s_sc);
-  if (SMEM_TALLY) {
-    // the block's tallies (every warp's last flush is behind the __syncthreads above)
-    for (int q = threadIdx.x; q < ncg; q += blockDim.x) {
-      if (TD[q]) atomicAdd(a.dep_fx + q, TD[q]);
-      if (TS[q] != 0.0) atomicAdd(a.si + q, TS[q]);
-    }
-  }
-}
-
 // dynamic shared memory of the tracking kernels: per-warp staging, edges, the cell table and
 // `tallies` 8-byte block tallies per (group, cell)
 inline size_t track_smem(const TrackArgs& a, int block, bool cells, int tallies) {
@@ -644,13 +421,7 @@ cudaError_t launch_sized(K kernel, const TrackArgs& a, int block, int grid, size
 template <int GEOM, bool MG, bool CF = false>
 cudaError_t launch_geom(const TrackArgs& a, const TrackLaunch& l, cudaStream_t s) {
   const int block = l.block, grid = l.sms * l.blocks_per_sm;
-  const bool sm = l.smem_cells, st = l.smem_tally, pf = l.prefetch;
-  if (pf) {
-    const size_t sh = track_smem(a, block, sm, sm && st ? 2 : 0) + pf_smem(block);
-    if (sm && st) return launch_sized(k_track_pf<GEOM, true, MG, CF, true>, a, block, grid, sh, s);
-    return sm ? launch_sized(k_track_pf<GEOM, true, MG, CF, false>, a, block, grid, sh, s)
-              : launch_sized(k_track_pf<GEOM, false, MG, CF, false>, a, block, grid, sh, s);
-  }
+  const bool sm = l.smem_cells, st = l.smem_tally;
   // One wide block per SM holding as many threads as the requested shape keeps resident there,
   // when its tally fits; the cell table beside it if that fits too (else it is read through L1,
   // which measured the same on the crooked pipe).
