@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(WIDE ? kAdjWide : 256, WIDE ? 1 : 4) k_adjoint
   const float weight_floor = (float)(1e-10 * (*a.wsum) / (double)(n > 0 ? n : 1));
   const uint32_t rkx = draw_step_key(a.rk, a.step);
 
-  uint32_t chunk_next = 0, chunk_end = 0;
+  Runs run = first_run(n, a.sms);
   bool drained = false;
   bool has = false, again = false;  // again: the lane's history is to be followed a second time
   int phase = 0;
@@ -92,13 +92,13 @@ __global__ void __launch_bounds__(WIDE ? kAdjWide : 256, WIDE ? 1 : 4) k_adjoint
       if (again) { phase = 1; again = false; }
       unsigned need = __ballot_sync(FULL, !has && !load);
       for (;;) {
-        if (need && !drained && chunk_next >= chunk_end && !claim_run(a.queue, a.chunk, n, chunk_next, chunk_end))
+        if (need && !drained && run.next >= run.end && !next_run(a.queue, a.chunk, n, a.sms, run))
           drained = true;
         if (need && !drained) {
-          const uint32_t avail = chunk_end - chunk_next;
+          const uint32_t avail = run.end - run.next;
           const uint32_t rank = __popc(need & lt_mask);
-          if (!has && !load && rank < avail) { pid = chunk_next + rank; phase = 0; L = 0.0; load = true; }
-          chunk_next += min((uint32_t)__popc(need), avail);
+          if (!has && !load && rank < avail) { pid = run.next + rank; phase = 0; L = 0.0; load = true; }
+          run.next += min((uint32_t)__popc(need), avail);
         }
         if (load) {
           load = false;

@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(256) k_btrack(BatchArgs a) {
   const float c_light = (float)C_LIGHT;
   const unsigned refill_min = (unsigned)max(1, min(32, a.refill_min));
 
-  uint32_t chunk_next = 0, chunk_end = 0;
+  Runs run{0u, 0u};  // every run a ticket
   bool drained = false, has = false;
   BHist h{};
   uint32_t lid = 0;
@@ -276,14 +276,14 @@ __global__ void __launch_bounds__(256) k_btrack(BatchArgs a) {
     unsigned need = __ballot_sync(FULL, !has);
     if ((unsigned)__popc(need) >= refill_min) {
       while (need && !drained) {
-        if (chunk_next >= chunk_end && !claim_run(a.queue, a.chunk, (uint32_t)n, chunk_next, chunk_end)) {
+        if (run.next >= run.end && !next_run(a.queue, a.chunk, (uint32_t)n, 0, run)) {
           drained = true;
           break;
         }
-        const uint32_t avail = chunk_end - chunk_next;
+        const uint32_t avail = run.end - run.next;
         const uint32_t rank = __popc(need & lt_mask);
         if (!has && rank < avail) {
-          const long long q = (long long)(chunk_next + rank);
+          const long long q = (long long)(run.next + rank);
           k = find_inst(pref, a.K, q);
           lid = (uint32_t)(q - pref[k]);
           h.pid = (uint32_t)(a.slot_off[k] + lid);
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(256) k_btrack(BatchArgs a) {
             has = true;
           }
         }
-        chunk_next += min((uint32_t)__popc(need), avail);
+        run.next += min((uint32_t)__popc(need), avail);
         need = __ballot_sync(FULL, !has);
       }
     }

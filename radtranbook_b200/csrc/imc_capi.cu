@@ -422,6 +422,7 @@ imc_status transport_async(const imc_mesh* mesh, const imc_material* mat, const 
   ta.seed = par->seed; ta.step = par->step;
   imcdev::philox_round_keys(ta.seed, ta.rk);
   ta.chunk = par->chunk > 0 ? par->chunk : 64;
+  ta.sms = sm_count();
   ta.group_edges = mesh->group_edges;
   ta.escaped_group = tal->escaped_group;
   ta.dep_fx = dep_fx; ta.esc_fx = esc_fx;

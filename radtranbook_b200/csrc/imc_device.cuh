@@ -33,6 +33,11 @@ enum : uint32_t {
 
 struct U4 { uint32_t x, y, z, w; };
 
+// The 64-bit product of two 32-bit words as its low and high halves: one wide multiply.
+__device__ __forceinline__ void mul_wide(uint32_t a, uint32_t b, uint32_t& lo, uint32_t& hi) {
+  asm("{\n.reg .u64 p;\nmul.wide.u32 p, %2, %3;\nmov.b64 {%0, %1}, p;\n}" : "=r"(lo), "=r"(hi) : "r"(a), "r"(b));
+}
+
 __device__ __forceinline__ U4 philox4x32_10(U4 c, uint32_t k0, uint32_t k1) {
 #pragma unroll
   for (int r = 0; r < 10; ++r) {
@@ -91,11 +96,14 @@ __device__ __forceinline__ uint32_t draw_step_key(const uint32_t* rk, uint32_t s
 }
 __device__ __forceinline__ U4 draw_next(const uint32_t* rk, const DrawKey& k, uint32_t rkx, uint32_t block) {
   const uint32_t x1 = rkx ^ block;  // word x after round 1
-  U4 c{k.a, k.b, __umulhi(0xD2511F53u, x1) ^ k.c, 0xD2511F53u * x1};
+  uint32_t l, h;
+  mul_wide(0xD2511F53u, x1, l, h);
+  U4 c{k.a, k.b, h ^ k.c, l};
 #pragma unroll
   for (int r = 2; r < 10; ++r) {
-    const uint32_t lo0 = 0xD2511F53u * c.x, hi0 = __umulhi(0xD2511F53u, c.x);
-    const uint32_t lo1 = 0xCD9E8D57u * c.z, hi1 = __umulhi(0xCD9E8D57u, c.z);
+    uint32_t lo0, hi0, lo1, hi1;
+    mul_wide(0xD2511F53u, c.x, lo0, hi0);
+    mul_wide(0xCD9E8D57u, c.z, lo1, hi1);
     c = U4{hi1 ^ c.y ^ rk[2 * r], lo1, hi0 ^ c.w ^ rk[2 * r + 1], lo0};
   }
   return c;
@@ -106,16 +114,18 @@ __device__ __forceinline__ U4 draw_next(const uint32_t* rk, const DrawKey& k, ui
 // draw_next makes sixteen scalar ones.
 __device__ __forceinline__ U4 draw_next4(const uint4* rk4, const DrawKey& key, uint32_t rkx, uint32_t block) {
   const uint32_t x1 = rkx ^ block;
-  U4 c{key.a, key.b, __umulhi(0xD2511F53u, x1) ^ key.c, 0xD2511F53u * x1};
+  uint32_t a0, b0, a1, b1;
+  mul_wide(0xD2511F53u, x1, a0, b0);
+  U4 c{key.a, key.b, b0 ^ key.c, a0};
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const uint4 k = rk4[q];
-    const uint32_t a0 = 0xD2511F53u * c.x, b0 = __umulhi(0xD2511F53u, c.x);
-    const uint32_t a1 = 0xCD9E8D57u * c.z, b1 = __umulhi(0xCD9E8D57u, c.z);
+    mul_wide(0xD2511F53u, c.x, a0, b0);
+    mul_wide(0xCD9E8D57u, c.z, a1, b1);
     c = U4{b1 ^ c.y ^ k.x, a1, b0 ^ c.w ^ k.y, a0};
-    const uint32_t e0 = 0xD2511F53u * c.x, f0 = __umulhi(0xD2511F53u, c.x);
-    const uint32_t e1 = 0xCD9E8D57u * c.z, f1 = __umulhi(0xCD9E8D57u, c.z);
-    c = U4{f1 ^ c.y ^ k.z, e1, f0 ^ c.w ^ k.w, e0};
+    mul_wide(0xD2511F53u, c.x, a0, b0);
+    mul_wide(0xCD9E8D57u, c.z, a1, b1);
+    c = U4{b1 ^ c.y ^ k.z, a1, b0 ^ c.w ^ k.w, a0};
   }
   return c;
 }
@@ -129,6 +139,7 @@ __device__ __forceinline__ uint32_t u4_word(const U4& r, int q) {
 // -log(u) for u = u01: distance in mean free paths.
 __device__ __forceinline__ float neglog_u(uint32_t x) { return -logf(u01f(x)); }
 
+
 // Whether a scatter at -log(u)/sigma, u = u01(x), can come before s_other.  With p = 1 - u
 // (exact in FP32, at least 2^-24) the scatter is at least p/sigma away, so p >= sigma s_other
 // (1 + 1e-6) rules it out whatever the rounding of the logarithm and the quotient; that
@@ -136,7 +147,9 @@ __device__ __forceinline__ float neglog_u(uint32_t x) { return -logf(u01f(x)); }
 // series of exp(-sigma s_other) when sigma s_other is small, so that the logarithm is
 // evaluated only when it can win.
 __device__ __forceinline__ bool scatter_may_win(uint32_t x, float sig, float s_other) {
-  if (1.0f - u01f(x) >= sig * s_other * 1.000001f) return false;
+  const float tf = sig * s_other;
+  if (1.0f - u01f(x) >= tf * 1.000001f) return false;
+  if (tf > 0.010001f) return true;  // not small, whatever the product's rounding
   const double t = (double)sig * (double)s_other;
   if (!(t < 0.01)) return true;
   const double thr = 1.0 - t * (1.0 - t * (0.5 - t * (1.0 / 6.0)));

@@ -143,24 +143,46 @@ __device__ __forceinline__ Flight next_flight(float2 e1, float2 e2, float ss, fl
   return Flight{d, evt, di, dj, xn, yn, un, vn};
 }
 
-// A warp's claim of a run of bank entries (guided: a share of what is left, at most `chunk`, at
-// least 32, so early claims are long contiguous (coherent) runs and the drain is finely
-// balanced).  Every lane calls it; false when the queue is past n.
-__device__ __forceinline__ bool claim_run(unsigned long long* queue, int chunk, uint32_t n, uint32_t& next,
-                                          uint32_t& end) {
+// A warp's runs of bank entries.  The first is its own, without a ticket: `first` consecutive
+// entries, dealt so that neighbouring runs go to different SMs and, within an SM, to different
+// schedulers (warp slots go round the four schedulers, so the blocks of one SM start at different
+// warps); a bank too small to give every warp a full row is spread over about four warps a
+// scheduler.  (With every run a ticket, the warps that came first held the work of a small bank
+// while other schedulers had none: one of 592 executed 6.5 times the average of a 4k slab step's
+// instructions.  The twenty launches of a 20k crooked-pipe run 0.67 -> 0.52 ms, of a 4k slab run
+// 5.5 -> 4.0.)  Later runs are guided tickets: a share of what is left, at most `chunk`, at least 32, so
+// early ones are long contiguous (coherent) runs and the drain is finely balanced.
+struct Runs { uint32_t next, end; };  // the warp's current run
+
+__device__ __forceinline__ uint32_t first_length(uint32_t n, int sms) {
+  const uint32_t slots = (uint32_t)sms * 16u;
+  return min(32u, max(4u, (n + slots - 1) / slots));
+}
+__device__ __forceinline__ Runs first_run(uint32_t n, int sms) {
+  const uint32_t warps = blockDim.x >> 5, first = first_length(n, sms);
+  const uint32_t w = ((threadIdx.x >> 5) + blockIdx.x / (uint32_t)sms) % warps;
+  const uint32_t base = min(n, (w * gridDim.x + blockIdx.x) * first);
+  return Runs{base, min(n, base + first)};
+}
+
+// The next run of a warp whose current one is used up (sms = 0: no first runs were dealt).  Every lane calls it; false when no entry is left.
+__device__ __forceinline__ bool next_run(unsigned long long* queue, int chunk, uint32_t n, int sms, Runs& r) {
   unsigned long long base = 0, claim = 0;
+  const unsigned long long nw = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+  const uint32_t dealt = sms ? (uint32_t)min((unsigned long long)n, nw * first_length(n, sms)) : 0u;
+  const unsigned long long rest = n - dealt;
+  if (rest == 0) return false;
   if ((threadIdx.x & 31) == 0) {
     const unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(queue);
-    const unsigned long long left = cur < (unsigned long long)n ? (unsigned long long)n - cur : 0ull;
-    const unsigned long long nw = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+    const unsigned long long left = cur < rest ? rest - cur : 0ull;
     claim = min((unsigned long long)chunk, max(32ull, left / (2ull * nw)));
     base = atomicAdd(queue, claim);
   }
   base = __shfl_sync(FULL, base, 0);
   claim = __shfl_sync(FULL, claim, 0);
-  if (base >= (unsigned long long)n) return false;
-  next = (uint32_t)base;
-  end = (uint32_t)min(base + claim, (unsigned long long)n);
+  if (base >= rest) return false;
+  r.next = dealt + (uint32_t)base;
+  r.end = dealt + (uint32_t)min(base + claim, rest);
   return true;
 }
 

@@ -53,6 +53,7 @@ struct TrackArgs {
   double* ecen;
   unsigned long long* n_live;
   int ecen_by_group;
+  int sms;                   // multiprocessors of the device
 };
 
 // smem_tally: per-block deposition / intensity tallies in shared memory (with smem_cells only);

@@ -64,8 +64,8 @@ template <int GEOM, bool SMEM_CELLS, bool MG, bool CF>
 __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut& o, const float2* E1,
                                               const float2* E2, const float2* CS, unsigned* blk_cnt,
                                               unsigned long long* blk_esc, unsigned long long* dep_t,
-                                              uint32_t rkx, float weight_floor, double inv_q,
-                                              unsigned& s_cen, unsigned& s_sc) {
+                                              const U4& r, float weight_floor,
+                                              double inv_q, unsigned& s_cen, unsigned& s_sc) {
   constexpr bool ONED = GEOM == G_SLAB || GEOM == G_SPHERE;
   constexpr bool MG2 = MG && !ONED;  // MG_IMC2D history rules
   const float c_light = (float)C_LIGHT;
@@ -82,9 +82,9 @@ __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut
     if (!a.cap_is_reference) atomicOr(a.flags, (int)IMC_FLAG_EVENT_CAP);
     finished = true;
   } else {
-    const U4 r = draw_next(a.rk, h.key, rkx, h.ev);
     ++h.ev;
-    const Flight f = next_flight<GEOM, !MG2>(E1[h.ci], ONED ? make_float2(0.f, 0.f) : E2[h.cj], ss, x, y, u, v, h.dcen, r);
+    const Flight f = next_flight<GEOM, !MG2>(E1[h.ci], ONED ? make_float2(0.f, 0.f) : E2[h.cj], ss, x, y, u, v, h.dcen,
+                                             r);
     const float d = f.d;
     const int evt = f.evt, di = f.di, dj = f.dj;
     // implicit capture (the energy removed is counted at the flush, w_in - w)
@@ -287,7 +287,14 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
   WarpStage* st = stages + (threadIdx.x >> 5);
   const uint32_t n = (uint32_t)*a.n_dev;
 
-  uint32_t chunk_next = 0, chunk_end = 0;  // warp-uniform run of claimed entries
+  // T_SMALL: events between two looks at the idle lanes (long histories; 1 in the checked build,
+  // which looks at every history before every event)
+#ifdef IMC_CHECKED
+  constexpr int kEvents = 1;
+#else
+  constexpr int kEvents = ONED ? 4 : 2;
+#endif
+  Runs run = first_run(n, a.sms);  // warp-uniform
   bool drained = false;
   bool has = false, pend = false;  // pend: an ended history whose final state is not stored yet
   Hist h;
@@ -316,11 +323,11 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
       }
       pend = false;
       while (need && !drained) {
-        if (chunk_next >= chunk_end && !claim_run(a.queue, a.chunk, n, chunk_next, chunk_end)) { drained = true; break; }
-        const uint32_t avail = chunk_end - chunk_next;
+        if (run.next >= run.end && !next_run(a.queue, a.chunk, n, a.sms, run)) { drained = true; break; }
+        const uint32_t avail = run.end - run.next;
         const uint32_t rank = __popc(need & lt_mask);
         if (!has && rank < avail) {
-          h.pid = chunk_next + rank;
+          h.pid = run.next + rank;
           h.w = a.w[h.pid];
           h.dcen = (dtk - a.t[h.pid]) * c_light;
           const bool moves = (MG2 || CF ? h.w > weight_floor : h.w > 0.f) && h.dcen > 0.f;
@@ -358,7 +365,7 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
             }
           }
         }
-        chunk_next += min((uint32_t)__popc(need), avail);
+        run.next += min((uint32_t)__popc(need), avail);
         need = __ballot_sync(FULL, !has);
       }
       if (need == FULL) break;
@@ -370,10 +377,27 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
       has = false;  // nothing more is tallied at an invalid index
     }
 #endif
+    if (TALLY == T_SMALL) {
+#pragma unroll 1
+      for (int rep = 0; rep < kEvents; ++rep) {
+        EvOut o{0, false, 0.f, 0.0, false};
+        if (has) {
+          history_event<GEOM, SMEM_CELLS, MG, CF>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t,
+                                                  draw_next(a.rk, h.key, rkx, h.ev), weight_floor, inv_q, s_cen, s_sc);
+          if (o.finished) { has = false; pend = true; }
+        }
+        __syncwarp();  // the warp together again: lanes left apart run the next event one by one
+        const unsigned long long ud = o.flush ? fx_units(o.lost, inv_q) : 0ull;
+        if (ud) smem_add_u64(TD + o.cell, ud);
+        if (o.wd != 0.f) atomicAdd(TS + o.cell, (double)o.wd);
+        __syncwarp();
+      }
+      continue;
+    }
     EvOut o{0, false, 0.f, 0.0, false};
     if (has) {
-      history_event<GEOM, SMEM_CELLS, MG, CF>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t, rkx, weight_floor,
-                                              inv_q, s_cen, s_sc);
+      history_event<GEOM, SMEM_CELLS, MG, CF>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t,
+                                              draw_next(a.rk, h.key, rkx, h.ev), weight_floor, inv_q, s_cen, s_sc);
       if (o.finished) { has = false; pend = true; }
     }
     // ---------------- tallies ----------------
@@ -383,7 +407,7 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
     const double vs = (double)o.wd;
     if (TD_S && ud) smem_add_u64(TD + o.cell, ud);
     if (TS_S && o.wd != 0.f) atomicAdd(TS + o.cell, vs);
-    if (!TD_S && !TS_S) warp_tally_fx(ud != 0ull || o.wd != 0.f, o.cell, ud, vs, a.dep_fx, a.si, st);
+    if (TALLY == T_GLOBAL) warp_tally_fx(ud != 0ull || o.wd != 0.f, o.cell, ud, vs, a.dep_fx, a.si, st);
     else if (!TD_S) warp_tally_fx(ud != 0ull, o.cell, ud, 0.0, a.dep_fx, a.si, st);
     else if (!TS_S) warp_tally1(o.wd != 0.f, o.cell, vs, a.si, st);
   }
@@ -533,8 +557,8 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
         h.tab = __ldg(a.sass + (MG ? c + a.nc * h.grp : c));
         h.key = draw_key(a.rk, a.id_base + pid, stepk, TAG_TRANSPORT);
         const uint32_t ev0 = h.ev;
-        history_event<GEOM, false, MG, CF>(a, h, o, E1, E2, nullptr, blk_cnt, blk_esc, a.dep_fx, rkx,
-                                           weight_floor, inv_q, s_cen, s_sc);
+        history_event<GEOM, false, MG, CF>(a, h, o, E1, E2, nullptr, blk_cnt, blk_esc, a.dep_fx,
+                                           draw_next(a.rk, h.key, rkx, h.ev), weight_floor, inv_q, s_cen, s_sc);
         s_ev += h.ev - ev0;
         int bin;
         if (o.finished) history_retire<GEOM>(a, h, bin);
