@@ -329,12 +329,65 @@ __global__ void k_material_law(MatArgs a, imc_material_law law, double* T, doubl
   }
 }
 
-// Single block: the canonical total of the census energy and the comb mode.
-__global__ void __launch_bounds__(NT) k_comb_plan(CombPlanArgs a) {
+// The canonical tree over 1024 partial sums, by any number of threads.
+__device__ __forceinline__ double tree_1024(double* red) {
+  for (int h = NT / 2; h >= 1; h >>= 1) {
+    for (int t = threadIdx.x; t < h; t += blockDim.x) red[t] += red[t + h];
+    __syncthreads();
+  }
+  return red[0];
+}
+
+// The canonical total of the census energy and the comb mode; with a.e, the last block sums the
+// internal energy instead.  The 1024 strided partial sums are spread over kPlanBlocks blocks when
+// the bins are many (a single SM reads 126 thousand bins in 22 us, eight in @CP@); the last of
+// them to finish (a ticket; none waits) runs the tree.  The partials stand in ew until the weights
+// kernel, which follows, writes it.
+constexpr int kPlanBlocks = 8;
+constexpr int kPlanManyBins = 16384;
+
+__global__ void __launch_bounds__(NT) k_comb_plan(CombPlanArgs a, int blocks) {
   pdl_wait();     // the previous kernel of the stream has completed
   pdl_trigger();  // the next one may be scheduled
   __shared__ double red[NT];
-  const double E = block_canon_sum<16>(a.ecen, a.nb, red);
+  __shared__ bool last;
+  if ((int)blockIdx.x == blocks) {
+    for (int t = threadIdx.x; t < NT; t += blockDim.x) {
+      double s = 0.0;
+      for (int c = t; c < a.nc; c += NT) s += a.e[c] * a.vol[c];
+      red[t] = s;
+    }
+    __syncthreads();
+    const double E = tree_1024(red);
+    if (threadIdx.x == 0) a.sum->internal_energy = E;
+    return;
+  }
+  constexpr int B = 8;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  double s = 0.0;
+  for (long long i0 = t; i0 < a.nb; i0 += (long long)B * NT) {
+    double v[B];
+#pragma unroll
+    for (int j = 0; j < B; ++j) { const long long i = i0 + (long long)j * NT; v[j] = i < a.nb ? a.ecen[i] : 0.0; }
+#pragma unroll
+    for (int j = 0; j < B; ++j) if (i0 + (long long)j * NT < a.nb) s += v[j];
+  }
+  if (blocks == 1) {
+    red[t] = s;
+    __syncthreads();
+  } else {
+    a.ew[t] = s;  // nb > NT here
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(a.ticket, 1ull) == (unsigned long long)blocks - 1ull;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int q = threadIdx.x; q < NT; q += blockDim.x) red[q] = __ldcg(a.ew + q);
+    if (threadIdx.x == 0) *a.ticket = 0ull;
+    __syncthreads();
+  }
+  const double E = tree_1024(red);
   // MG_IMC/MG_IMC1D.py:1194-1200: Nmax = 0 never combs; Nmax < 0 combs once |Nmax| entries live
   const bool compact = a.force_compact || (a.threshold > 0 && (long long)*a.n_live < a.threshold);
   if (threadIdx.x == 0) { *a.mode = compact ? 1 : 0; a.sum->comb_before = E; a.sum->comb_after = 0.0; }
@@ -415,7 +468,8 @@ cudaError_t imc_launch_zero(const ZeroList& z, cudaStream_t s) {
 }
 cudaError_t imc_launch_comb_plan(const CombPlanArgs& a, cudaStream_t s) {
   g_imc_launches += 2;
-  IMC_LAUNCH_PDL(k_comb_plan, 1, NT, 0, s, a);
+  const int blocks = a.nb >= kPlanManyBins ? kPlanBlocks : 1;
+  IMC_LAUNCH_PDL(k_comb_plan, blocks + (a.e ? 1 : 0), NT / blocks, 0, s, a, blocks);
   if (a.nb > 0) IMC_LAUNCH_PDL(k_comb_weights, (a.nb + 255) / 256, 256, 0, s, a);
   return cudaGetLastError();
 }

@@ -185,7 +185,7 @@ imc_status transport_async(const imc_mesh* mesh, const imc_material* mat, const 
     if (par->census_bins && !adj) {
       const int nb = par->census_bins == IMC_CENSUS_BY_GROUP_CELL ? nc * ng : nc;
       zl.add(ws_ptr<double>(workspace, L.ecen), sizeof(double) * nb);
-      zl.add(ws_ptr<unsigned long long>(workspace, L.comb_mode + 8), sizeof(unsigned long long));
+      zl.add(ws_ptr<unsigned long long>(workspace, L.comb_mode + 8), 3 * sizeof(unsigned long long));  // live count, tickets
     }
     IMC_CUDA(imc_launch_zero(zl, s));
   }
@@ -479,6 +479,7 @@ imc_status comb_async(const imc_mesh* mesh, const imc_bank* in, imc_bank* out, i
   ca.conserve_rad = (per_group & IMC_COMB_CONSERVE_RADIATION) ? 1 : 0;
   ca.mode = ws_ptr<int>(workspace, L.comb_mode);
   ca.n_live = ws_ptr<unsigned long long>(workspace, L.comb_mode + 8);
+  ca.ticket = ws_ptr<unsigned long long>(workspace, L.comb_mode + 16);
   ca.d_n_in = &sum->n_bank; ca.n_bound = in->size; ca.out_capacity = out->capacity;
   ca.w = in->weight; ca.cell = in->cell; ca.group = in->group;
   ca.p1 = in->pos1; ca.p2 = two_d ? in->pos2 : nullptr; ca.d1 = in->dir1; ca.d2 = two_d ? in->dir2 : nullptr;
@@ -498,7 +499,7 @@ imc_status comb_async(const imc_mesh* mesh, const imc_bank* in, imc_bank* out, i
   // ncopy is zeroed by the comb plan's weights kernel, comb_after and the mode by the plan
   if (!census_ready) {  // else the census sums and the live count are the tracking's
     IMC_CUDA(cudaMemsetAsync(ca.ecen, 0, sizeof(double) * nb, s));
-    IMC_CUDA(cudaMemsetAsync(ca.mode, 0, 16, s));
+    IMC_CUDA(cudaMemsetAsync(ca.mode, 0, 32, s));
     IMC_CUDA(imc_launch_comb_ecen(ca, s));
   }
   CombPlanArgs cp{};
@@ -510,10 +511,11 @@ imc_status comb_async(const imc_mesh* mesh, const imc_bank* in, imc_bank* out, i
   cp.threshold = n_max < 0 ? -n_max : 0;
   cp.force_compact = n_max == 0 ? 1 : 0;
   cp.n_live = ca.n_live; cp.mode = ca.mode;
+  cp.ticket = ws_ptr<unsigned long long>(workspace, L.comb_mode + 24);
+  cp.e = e; cp.vol = mesh->volume; cp.nc = nc;
   IMC_CUDA(imc_launch_comb_plan(cp, s));
   IMC_CUDA(imc_launch_comb_count(ca, s));
   IMC_CUDA(imc_launch_comb_scatter(ca, s));
-  if (e) IMC_CUDA(imc_launch_canon_sum_eV(e, mesh->volume, nc, &sum->internal_energy, s));
   return IMC_OK;
 }
 
@@ -548,7 +550,7 @@ WsLayout imc_ws_layout(const imc_mesh* m, int64_t capacity) {
   }
   L.mixcdf = take(8 * 200);
   L.ecen = take(8 * ncg); L.ew = take(8 * ncg); L.ncopy = take(8 * ncg);
-  L.comb_mode = take(16);
+  L.comb_mode = take(32);
   L.dep_fx = take(8 * ncg); L.esc_fx = take(8 * (4 + ng));
   L.cf_rate = take(4 * nc);
   // The regions sized by the capacity come last, so every other offset is the same for any

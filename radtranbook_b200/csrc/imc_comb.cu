@@ -4,16 +4,18 @@
 //   1. ecen[b]  = sum of live weights per bin (cell, or cell + nc*group)      k_comb_ecen
 //   2. ew[b]    = ecen / max(1, rint(Nmax ecen / E))                          k_comb_plan
 //   3. n_k      = floor(w_k / ew[b] + xi_k), xi word k % 4 of Philox block
-//      (k / 4, 1, step, TAG_COMB); per-block totals                          k_comb_count
-//   4. exclusive scan of block totals                                         k_comb_scan
-//   5. copies written in bank order (block-local scan + block offset; entries
-//      staged in shared memory, one thread per output copy)                  k_comb_scatter
-//   6. disc[b] = ecen - (copies in b) * FP32(ew), and optionally that energy
-//      after the comb per bin (exact: equal FP32 weights summed in FP64)         k_comb_disc
+//      (k / 4, 1, step, TAG_COMB); tile totals and, by the last block to finish,
+//      their exclusive scan                                                   k_comb_count
+//   4. copies written in bank order (tile-local scan + tile offset; entries
+//      staged in shared memory, one thread per output copy), and by blocks of
+//      their own disc[b] = ecen - (copies in b) * FP32(ew) and optionally that
+//      energy after the comb per bin (exact: equal FP32 weights summed in FP64) k_comb_scatter
 // Order of the output bank = order of the input bank, so the result is deterministic.
 // Modes (MG_IMC/MG_IMC1D.py:1187-1200, 808-820): when the comb plan decides not to comb
 // (Nmax = 0, or fewer live entries than a threshold) every live entry is copied once with its
 // weight (disc = 0); with conserve_rad each bin's copies share its pre-comb energy equally.
+#include <algorithm>
+
 #include "imc_device.cuh"
 #include "imc_internal.h"
 
@@ -21,9 +23,8 @@ using namespace imcdev;
 
 namespace {
 
-constexpr int TILE = 4096;      // entries per count / scatter block (one block total each for the scan)
-constexpr int CNT_T = 256;      // count threads per block (TILE / CNT_T entries each)
-constexpr int CNT_SLOTS = 512;  // count: shared-memory bins per block
+constexpr int TILE = 1024;      // entries per tile: one count total, one scatter block
+constexpr int WARP_ENTRIES = 128;  // entries a warp counts at a time (four per lane)
 
 __device__ __forceinline__ int bin_of(const CombArgs& a, long long k) {
   return a.per_group ? a.cell[k] + a.nc * a.group[k] : a.cell[k];
@@ -83,15 +84,9 @@ __global__ void __launch_bounds__(256) k_comb_ecen(CombArgs a) {
   bins_flush(t, a.ecen);
 }
 
-// Each block combs a tile of TILE consecutive entries; each of its CNT_T threads takes CNT_PER
-// consecutive entries (16-byte vector loads and stores when the bank arrays allow them):
-// copies per entry, the tile's total for the scan, and copies per bin, summed in registers
-// over runs of equal bins (the bank is largely grouped by cell) and added to the block's
-// table when the bin changes, so the loop has no warp-wide step.
-constexpr int CNT_PER = TILE / CNT_T;
-
 // copies of one entry: floor(w / ew + xi), xi its comb uniform (word k % 4 of Philox block
-// (k / 4, 1, step, TAG_COMB), k the pre-comb index)
+// (k / 4, 1, step, TAG_COMB), k the pre-comb index).  The quotient is formed in FP32 first, off
+// by at most 1e-6 of itself; only where that leaves the floor open is it divided in FP64.
 __device__ __forceinline__ int comb_copies(const CombArgs& a, float wf, int bk, bool compact, uint32_t xw, int& b) {
   b = 0;
   if (!(wf > 0.f) || !bin_ok(a, bk)) return 0;
@@ -99,25 +94,44 @@ __device__ __forceinline__ int comb_copies(const CombArgs& a, float wf, int bk, 
   if (compact) return 1;
   const double ew = a.ew[b];
   if (!(ew > 0.0)) return 0;
+  const float s = __fdividef(wf, (float)ew) + u01f(xw);
+  const float fl = floorf(s), fr = s - fl, open = 1e-6f * (s + 1.f);
+  if (s < 4e6f && fr > open && fr < 1.f - open) return (int)fl;  // false for an infinite or NaN quotient
   return (int)floor((double)wf / ew + u01d(xw));
 }
 
-__global__ void __launch_bounds__(CNT_T) k_comb_count(CombArgs a) {
+// Copies per entry, per tile and per bin.  A block takes `per` consecutive tiles, its warps
+// WARP_ENTRIES entries at a time with 16-byte vector loads (where the bank arrays allow them).
+// Copies per bin are summed in shared memory, runs of equal bins in a lane first, and added to the
+// global ones once per block: in a counter per bin (DENSE: many entries, bins that fit), else in a
+// hash table over the block's one tile.  The last block to finish scans the
+// tile totals (a ticket; no block waits).  With a hash table of bins per 4096 entries instead, which
+// a mixed bank overflows, and an FP64 division per entry this took 94 us for 8.7 M entries in 12600
+// bins and 45 us for 91 thousand in 3150 (23 blocks); now @CNT2M@ and @CNT20K@ us.
+constexpr int kCountMaxTiles = 64;  // tiles a block takes at most
+constexpr int kCountSlots = TILE / 2;  // hash table of a block (a tile rarely has more bins; adds past it go to global memory)
+
+template <bool DENSE>
+__global__ void __launch_bounds__(512, 2) k_comb_count(CombArgs a, long long ntiles, int per) {
   pdl_wait();     // the previous kernel of the stream has completed
   pdl_trigger();  // the next one may be scheduled
+  extern __shared__ unsigned bin_cnt[];  // DENSE: [nb]
+  __shared__ unsigned long long tile_sum[kCountMaxTiles];
+  __shared__ long long sh[32];
+  __shared__ bool last;
   const uint32_t step = a.step_dev ? *a.step_dev : a.step;  // graph replay
-  __shared__ unsigned sh[CNT_T / 32];
-  __shared__ BlockCounts<CNT_SLOTS> t;
-  counts_init(t);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int q = threadIdx.x; q < per; q += blockDim.x) tile_sum[q] = 0ull;
+  BlockCounts<kCountSlots>& hash = *reinterpret_cast<BlockCounts<kCountSlots>*>(bin_cnt);  // else
+  if (DENSE) for (int q = threadIdx.x; q < a.nb; q += blockDim.x) bin_cnt[q] = 0u;
+  else counts_init(hash);
   __syncthreads();
-  const long long n_in = min((long long)*a.d_n_in, (long long)a.n_bound);  // the grid covers n_bound entries
+  const long long n_in = min((long long)*a.d_n_in, (long long)a.n_bound);  // the tiles cover n_bound entries
   const bool compact = *a.mode != 0;
-  const long long k0 = (long long)blockIdx.x * TILE + (long long)threadIdx.x * CNT_PER;
-  unsigned tsum = 0, run_n = 0;
-  int run_b = -1;
-#pragma unroll 1
-  for (int j = 0; j < CNT_PER; j += 4) {
-    const long long kj = k0 + j;
+  const long long tile0 = (long long)blockIdx.x * per;
+  const int units = (int)max(0LL, min((long long)per, ntiles - tile0)) * (TILE / WARP_ENTRIES);
+  for (int u = wid; u < units; u += nw) {
+    const long long kj = tile0 * TILE + (long long)u * WARP_ENTRIES + 4 * lane;
     float wv[4] = {0.f, 0.f, 0.f, 0.f};
     int bv[4] = {0, 0, 0, 0};
     if (a.vec16 && kj + 3 < n_in) {  // kj % 4 == 0: the 16-byte loads are aligned
@@ -139,96 +153,116 @@ __global__ void __launch_bounds__(CNT_T) k_comb_count(CombArgs a) {
       r = draw_rk(a.rk, (uint32_t)(kj >> 2), 1, step, TAG_COMB);
     int nv[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      int b;
-      const int n = kj + q < n_in ? comb_copies(a, wv[q], bv[q], compact, u4_word(r, q), b) : 0;
-      nv[q] = n;
-      tsum += (unsigned)n;
-      if (n > 0) {
-        if (b != run_b) {
-          if (run_n) counts_add(t, run_b, run_n, a.ncopy);
-          run_b = b;
-          run_n = 0;
-        }
-        run_n += (unsigned)n;
-      }
-    }
+    for (int q = 0; q < 4; ++q) nv[q] = comb_copies(a, wv[q], bv[q], compact, u4_word(r, q), bv[q]);
     if (kj + 3 < n_in) {
       *reinterpret_cast<int4*>(a.cnt + kj) = make_int4(nv[0], nv[1], nv[2], nv[3]);  // workspace: aligned
     } else {
       for (int q = 0; q < 4; ++q) if (kj + q < n_in) a.cnt[kj + q] = nv[q];
     }
+    // copies per bin: equal neighbours are one add
+    unsigned run = 0, tsum = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      run += (unsigned)nv[q];
+      tsum += (unsigned)nv[q];
+      const bool ends = run != 0u && (q == 3 || bv[q + 1] != bv[q]);
+      if (ends) { if (DENSE) atomicAdd(bin_cnt + bv[q], run); else counts_add(hash, bv[q], run, a.ncopy); }
+      if (q < 3 && bv[q + 1] != bv[q]) run = 0u;
+    }
+    const unsigned ws = __reduce_add_sync(FULL, tsum);
+    if (lane == 0 && ws) atomicAdd(&tile_sum[u / (TILE / WARP_ENTRIES)], (unsigned long long)ws);
   }
-  if (run_n) counts_add(t, run_b, run_n, a.ncopy);
-  const unsigned ws = __reduce_add_sync(FULL, tsum);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = ws;
   __syncthreads();
-  counts_flush(t, a.ncopy);
-  if (threadIdx.x == 0) {
-    unsigned long long v = 0;
-    for (int q = 0; q < CNT_T / 32; ++q) v += sh[q];
-    a.blk[blockIdx.x] = (long long)v;
+  if (DENSE) {
+    for (int q = threadIdx.x; q < a.nb; q += blockDim.x)
+      if (bin_cnt[q]) atomicAdd(a.ncopy + q, (unsigned long long)bin_cnt[q]);
+  } else {
+    counts_flush(hash, a.ncopy);
+  }
+  for (int q = threadIdx.x; q < per && tile0 + q < ntiles; q += blockDim.x) a.blk[tile0 + q] = (long long)tile_sum[q];
+  // ---- the last block: exclusive scan of the tile totals in place (blk[ntiles] = total) ----
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(a.ticket, 1ull) == (unsigned long long)gridDim.x - 1ull;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x == 0) *a.ticket = 0ull;  // for a comb launched again on this workspace
+  const int t = threadIdx.x, nt = blockDim.x;
+  const long long share = (ntiles + nt - 1) / nt;
+  const long long lo = min((long long)t * share, ntiles), hi = min(lo + share, ntiles);
+  long long sum = 0;
+  for (long long q = lo; q < hi; ++q) sum += __ldcg(a.blk + q);
+  long long x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const long long y = __shfl_up_sync(FULL, x, o); if (lane >= o) x += y; }
+  if (lane == 31) sh[wid] = x;
+  __syncthreads();
+  if (wid == 0) {
+    long long v = lane < nw ? sh[lane] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const long long y = __shfl_up_sync(FULL, v, o); if (lane >= o) v += y; }
+    sh[lane] = v;
+  }
+  __syncthreads();
+  long long run = x - sum + (wid ? sh[wid - 1] : 0);
+  for (long long q = lo; q < hi; ++q) { const long long v = __ldcg(a.blk + q); a.blk[q] = run; run += v; }
+  if (t == 0) {
+    const long long total = sh[31];
+    a.blk[ntiles] = total;
+    a.sum->n_out = total;
+    if (total > a.out_capacity) { atomicOr(&a.sum->flags, (int)IMC_FLAG_COMB_OVERFLOW); a.sum->n_census = 0; }
+    else a.sum->n_census = total;  // the combed bank is the next step's census
   }
 }
 
-// exclusive scan of nblk block totals in place (blk[nblk] = total), single block
-__global__ void __launch_bounds__(1024) k_comb_scan(long long* blk, long long nblk, long long out_capacity,
-                                                    imc_step_summary* sum) {
-  pdl_wait();     // the previous kernel of the stream has completed
-  pdl_trigger();  // the next one may be scheduled
-  __shared__ long long sh[1024];
-  const int t = threadIdx.x;
-  const long long per = (nblk + 1023) / 1024;
-  const long long lo = min((long long)t * per, nblk), hi = min(lo + per, nblk);
-  long long s = 0;
-  for (long long q = lo; q < hi; ++q) s += blk[q];
-  sh[t] = s;
-  __syncthreads();
-  for (int d = 1; d < 1024; d <<= 1) {
-    const long long v = t >= d ? sh[t - d] : 0;
-    __syncthreads();
-    sh[t] += v;
-    __syncthreads();
-  }
-  long long run = sh[t] - s;
-  for (long long q = lo; q < hi; ++q) { const long long x = blk[q]; blk[q] = run; run += x; }
-  if (t == 1023) {
-    const long long total = sh[1023];
-    blk[nblk] = total;
-    sum->n_out = total;
-    if (total > out_capacity) { atomicOr(&sum->flags, (int)IMC_FLAG_COMB_OVERFLOW); sum->n_census = 0; }
-    else sum->n_census = total;  // the combed bank is the next step's census
-  }
-}
-
-// One thread per output copy: the tile's copy counts are scanned in shared memory (each
-// thread owns 4 consecutive entries), each thread finds the entry of its copy by a binary
-// search there and gathers the entry's fields (cached: a tile's entries are few), so the
-// output stores are contiguous across the warp.
-// Shared memory of k_comb_scatter: the tile's inclusive copy counts, then its entries'
-// fields (pos1, dir1, cell; pos2, dir2 in 2-D; group when the bank has one), TILE each.
-__host__ __device__ inline int scatter_fields(bool two_d, bool grp) { return 3 + (two_d ? 2 : 0) + (grp ? 1 : 0); }
+// Shared memory of k_comb_scatter: the tile's inclusive copy counts, then its entries' fields
+// (pos1, dir1, copy weight, cell; pos2, dir2 in 2-D; group when the bank has one), TILE each, and
+// the entry of each of the first SCAT_MAP output copies.
+constexpr int SCAT_T = TILE / 4;
+constexpr int SCAT_MAP = 2 * TILE;
+__host__ __device__ inline int scatter_fields(bool two_d, bool grp) { return 4 + (two_d ? 2 : 0) + (grp ? 1 : 0); }
 __host__ __device__ inline size_t scatter_smem(bool two_d, bool grp) {
-  return sizeof(int) * (size_t)TILE * (1 + scatter_fields(two_d, grp));
+  return sizeof(int) * (size_t)TILE * (1 + scatter_fields(two_d, grp)) + sizeof(unsigned short) * SCAT_MAP;
 }
 
-// The tile's entries are staged in shared memory with 16-byte loads (one thread per four
-// entries, as the count kernel tiled them), then one thread per output copy finds its entry
-// by a binary search of the scanned counts and copies its fields from shared memory, so the
-// global loads and the stores of a warp are both contiguous.
-__global__ void __launch_bounds__(1024) k_comb_scatter(CombArgs a) {
+// One block per tile (the first ntiles blocks): its entries are staged in shared memory with
+// 16-byte loads (one thread per four entries), each thread notes its entries' output positions, and
+// one thread per output copy then copies its entry's fields from shared memory, so the global loads
+// and the stores of a warp are both contiguous.  A tile with more than SCAT_MAP copies finds the
+// entries of the others by a binary search of the scanned counts.  The remaining blocks take 256
+// bins each: disc and the energy after the comb.  Against tiles of 4096 entries, a search for
+// every copy and the copy weight gathered per copy: 87 -> @SC2M@ us for 8.7 M entries, 26 -> @SC20K@ us
+// for 91 thousand.
+__global__ void __launch_bounds__(SCAT_T) k_comb_scatter(CombArgs a, long long ntiles) {
   pdl_wait();     // the previous kernel of the stream has completed
   pdl_trigger();  // the next one may be scheduled
   extern __shared__ __align__(16) int sm_tile[];
-  __shared__ int sh[32];
+  __shared__ int sh[SCAT_T / 32];
+  const bool compact = *a.mode != 0;
+  if ((long long)blockIdx.x >= ntiles) {
+    const long long b = ((long long)blockIdx.x - ntiles) * blockDim.x + threadIdx.x;
+    double after = 0.0;
+    if (b < a.nb) {
+      // compact only: every live entry kept with its weight, nothing is lost
+      after = compact ? a.ecen[b] : (double)a.ncopy[b] * (double)copy_weight(a, (int)b);
+      a.disc[b] = a.ecen[b] - after;
+      if (a.after) a.after[b] = after;
+    }
+    after = warp_sum_d(after);
+    if ((threadIdx.x & 31) == 0 && after != 0.0) atomicAdd(&a.sum->comb_after, after);
+    return;
+  }
   const bool two_d = a.p2 != nullptr, grp = a.group != nullptr;
   int* incl = sm_tile;
   float* sP1 = reinterpret_cast<float*>(incl + TILE);
   float* sD1 = sP1 + TILE;
-  int* sC = reinterpret_cast<int*>(sD1 + TILE);
+  float* sW = sD1 + TILE;
+  int* sC = reinterpret_cast<int*>(sW + TILE);
   float* sP2 = reinterpret_cast<float*>(sC + TILE);   // 2-D only
   float* sD2 = sP2 + TILE;                            // 2-D only
   int* sG = reinterpret_cast<int*>(two_d ? sD2 + TILE : sP2);  // with a group array only
+  unsigned short* entry = reinterpret_cast<unsigned short*>(sm_tile + TILE * (1 + scatter_fields(two_d, grp)));
   const long long tile0 = (long long)blockIdx.x * TILE;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const long long n_in = min((long long)*a.d_n_in, (long long)a.n_bound);
@@ -245,25 +279,38 @@ __global__ void __launch_bounds__(1024) k_comb_scatter(CombArgs a) {
   const int s4 = c[0] + c[1] + c[2] + c[3];
   // stage the fields of the four entries (only where they have copies)
   const uintptr_t al = reinterpret_cast<uintptr_t>(a.p1) | reinterpret_cast<uintptr_t>(a.d1) |
-                       reinterpret_cast<uintptr_t>(a.p2) | reinterpret_cast<uintptr_t>(a.d2);
+                       reinterpret_cast<uintptr_t>(a.p2) | reinterpret_cast<uintptr_t>(a.d2) |
+                       (grp ? reinterpret_cast<uintptr_t>(a.group) : 0);
   if (s4 > 0) {
+    int cl[4] = {0, 0, 0, 0}, gr[4] = {0, 0, 0, 0};
     if (full && a.vec16 && (al & 15u) == 0) {
       *reinterpret_cast<float4*>(sP1 + q0) = *reinterpret_cast<const float4*>(a.p1 + k0);
       *reinterpret_cast<float4*>(sD1 + q0) = *reinterpret_cast<const float4*>(a.d1 + k0);
-      *reinterpret_cast<int4*>(sC + q0) = *reinterpret_cast<const int4*>(a.cell + k0);
+      const int4 C = *reinterpret_cast<const int4*>(a.cell + k0);
+      cl[0] = C.x; cl[1] = C.y; cl[2] = C.z; cl[3] = C.w;
       if (two_d) {
         *reinterpret_cast<float4*>(sP2 + q0) = *reinterpret_cast<const float4*>(a.p2 + k0);
         *reinterpret_cast<float4*>(sD2 + q0) = *reinterpret_cast<const float4*>(a.d2 + k0);
       }
-      if (grp) *reinterpret_cast<int4*>(sG + q0) = *reinterpret_cast<const int4*>(a.group + k0);
+      if (grp) {
+        const int4 G = *reinterpret_cast<const int4*>(a.group + k0);
+        gr[0] = G.x; gr[1] = G.y; gr[2] = G.z; gr[3] = G.w;
+      }
     } else {
       for (int j = 0; j < 4; ++j) {
         if (c[j] == 0) continue;
         const long long k = k0 + j;
-        sP1[q0 + j] = a.p1[k]; sD1[q0 + j] = a.d1[k]; sC[q0 + j] = a.cell[k];
+        sP1[q0 + j] = a.p1[k]; sD1[q0 + j] = a.d1[k]; cl[j] = a.cell[k];
         if (two_d) { sP2[q0 + j] = a.p2[k]; sD2[q0 + j] = a.d2[k]; }
-        if (grp) sG[q0 + j] = a.group[k];
+        if (grp) gr[j] = a.group[k];
       }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (c[j] == 0) continue;
+      sC[q0 + j] = cl[j];
+      if (grp) sG[q0 + j] = gr[j];
+      sW[q0 + j] = compact ? a.w[k0 + j] : copy_weight(a, a.per_group ? cl[j] + a.nc * gr[j] : cl[j]);
     }
   }
   // block-exclusive scan of the threads' sums, then the entries' inclusive sums
@@ -272,48 +319,34 @@ __global__ void __launch_bounds__(1024) k_comb_scatter(CombArgs a) {
   for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(FULL, x, o); if (lane >= o) x += y; }
   if (lane == 31) sh[wid] = x;
   __syncthreads();
-  if (wid == 0) {
-    int v = sh[lane];
+  int run = x - s4;
+  for (int q = 0; q < wid; ++q) run += sh[q];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(FULL, v, o); if (lane >= o) v += y; }
-    sh[lane] = v;
+  for (int j = 0; j < 4; ++j) {
+    for (int o = run; o < run + c[j] && o < SCAT_MAP; ++o) entry[o] = (unsigned short)(q0 + j);
+    run += c[j];
+    incl[q0 + j] = run;
   }
-  __syncthreads();
-  int run = x - s4 + (wid ? sh[wid - 1] : 0);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) { run += c[j]; incl[q0 + j] = run; }
   __syncthreads();
   const int total = incl[TILE - 1];
   const long long out0 = a.blk[blockIdx.x];
-  const bool compact = *a.mode != 0;
   for (int o = threadIdx.x; o < total; o += blockDim.x) {
     const long long dst = out0 + o;
     if (dst >= a.out_capacity) break;  // overflow: flagged by the scan, caller regrows
-    int lo = 0, hi = TILE - 1;  // the entry j with incl[j-1] <= o < incl[j]
-    while (lo < hi) { const int mid = (lo + hi) >> 1; if (incl[mid] > o) hi = mid; else lo = mid + 1; }
-    const int cl = sC[lo];
-    const int gr = grp ? sG[lo] : 0;
-    a.op1[dst] = sP1[lo]; a.od1[dst] = sD1[lo];
-    if (two_d) { a.op2[dst] = sP2[lo]; a.od2[dst] = sD2[lo]; }
-    a.ow[dst] = compact ? a.w[tile0 + lo] : copy_weight(a, a.per_group ? cl + a.nc * gr : cl);
-    a.ot[dst] = 0.f; a.ocell[dst] = cl;
-    if (a.ogroup) a.ogroup[dst] = gr;
+    int e;
+    if (o < SCAT_MAP) {
+      e = entry[o];
+    } else {
+      int lo = 0, hi = TILE - 1;  // the entry j with incl[j-1] <= o < incl[j]
+      while (lo < hi) { const int mid = (lo + hi) >> 1; if (incl[mid] > o) hi = mid; else lo = mid + 1; }
+      e = lo;
+    }
+    a.op1[dst] = sP1[e]; a.od1[dst] = sD1[e];
+    if (two_d) { a.op2[dst] = sP2[e]; a.od2[dst] = sD2[e]; }
+    a.ow[dst] = sW[e];
+    a.ot[dst] = 0.f; a.ocell[dst] = sC[e];
+    if (a.ogroup) a.ogroup[dst] = grp ? sG[e] : 0;
   }
-}
-
-__global__ void k_comb_disc(CombArgs a) {
-  pdl_wait();     // the previous kernel of the stream has completed
-  pdl_trigger();  // the next one may be scheduled
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  double after = 0.0;
-  if (b < a.nb) {
-    // compact only: every live entry kept with its weight, nothing is lost
-    after = *a.mode != 0 ? a.ecen[b] : (double)a.ncopy[b] * (double)copy_weight(a, b);
-    a.disc[b] = a.ecen[b] - after;
-    if (a.after) a.after[b] = after;
-  }
-  after = warp_sum_d(after);
-  if ((threadIdx.x & 31) == 0 && after != 0.0) atomicAdd(&a.sum->comb_after, after);
 }
 
 }  // namespace
@@ -326,36 +359,31 @@ cudaError_t imc_launch_comb_ecen(const CombArgs& a, cudaStream_t s) {
 }
 
 cudaError_t imc_launch_comb_count(const CombArgs& a, cudaStream_t s) {
-  const long long nblk = (a.n_bound + TILE - 1) / TILE;
-  if (nblk > 0) {
-    ++g_imc_launches;
-    IMC_LAUNCH_PDL(k_comb_count, (unsigned)nblk, CNT_T, 0, s, a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
   ++g_imc_launches;
-  IMC_LAUNCH_PDL(k_comb_scan, 1, 1024, 0, s, a.blk, nblk, a.out_capacity, a.sum);
+  const long long ntiles = (a.n_bound + TILE - 1) / TILE;
+  // a counter per bin pays from about half a million entries (below, zeroing and flushing it costs
+  // more than the hash table's probes), two blocks per SM while it fits
+  const size_t dense = sizeof(unsigned) * (size_t)a.nb;
+  if (a.n_bound >= (1LL << 19) && dense <= 100 * 1024) {
+    int per = (int)std::min<long long>(kCountMaxTiles, std::max<long long>(4, (ntiles + 295) / 296));
+    if (dense > 48 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(k_comb_count<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dense);
+      if (e != cudaSuccess) return e;
+    }
+    IMC_LAUNCH_PDL(k_comb_count<true>, (unsigned)((ntiles + per - 1) / per), 512, dense, s, a, ntiles, per);
+  } else {
+    const int per = 1, threads = 32 * (TILE / WARP_ENTRIES);
+    IMC_LAUNCH_PDL(k_comb_count<false>, (unsigned)std::max<long long>(1, ntiles), threads,
+                   sizeof(BlockCounts<kCountSlots>), s, a, ntiles, per);
+  }
   return cudaGetLastError();
 }
 
 cudaError_t imc_launch_comb_scatter(const CombArgs& a, cudaStream_t s) {
-  const long long nblk = (a.n_bound + TILE - 1) / TILE;
-  if (nblk > 0) {
-    ++g_imc_launches;
-    // the attribute allows the largest layout (2-D with groups), set once per device
-    static bool attr_set[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-      e = cudaFuncSetAttribute(k_comb_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)scatter_smem(true, true));
-      if (e != cudaSuccess) return e;
-      if (dev >= 0 && dev < 64) attr_set[dev] = true;
-    }
-    IMC_LAUNCH_PDL(k_comb_scatter, (unsigned)nblk, 1024, scatter_smem(a.p2 != nullptr, a.group != nullptr), s, a);
-  }
+  const long long ntiles = (a.n_bound + TILE - 1) / TILE;
   ++g_imc_launches;
-  IMC_LAUNCH_PDL(k_comb_disc, (a.nb + 255) / 256, 256, 0, s, a);
+  const size_t smem = scatter_smem(a.p2 != nullptr, a.group != nullptr);
+  static_assert(sizeof(int) * TILE * 8 + 2 * SCAT_MAP <= 48 * 1024, "no opt-in for the largest layout");
+  IMC_LAUNCH_PDL(k_comb_scatter, (unsigned)(ntiles + (a.nb + SCAT_T - 1) / SCAT_T), SCAT_T, smem, s, a, ntiles);
   return cudaGetLastError();
 }

@@ -305,19 +305,6 @@ __device__ __forceinline__ void counts_add(BlockCounts<S>& t, int bin, unsigned 
   atomicAdd(global + bin, (unsigned long long)v);
 }
 
-// every lane calls it (converged): per-warp groups by bin (lanes' counts summed with the
-// group's leader), then one shared-memory add per group
-template <int S>
-__device__ __forceinline__ void warp_counts_add(bool add, int key, unsigned v, BlockCounts<S>& t,
-                                                unsigned long long* __restrict__ global) {
-  const unsigned fm = __ballot_sync(FULL, add);
-  if (fm == 0u) return;
-  const int lane = threadIdx.x & 31;
-  const unsigned peers = __match_any_sync(FULL, add ? key : -1 - lane);
-  const unsigned s = __reduce_add_sync(peers, add ? v : 0u);  // the group's sum, on every member
-  if (add && (__ffs(peers) - 1) == lane) counts_add(t, key, s, global);
-}
-
 template <int S>
 __device__ __forceinline__ void counts_flush(BlockCounts<S>& t, unsigned long long* __restrict__ global) {
   for (int i = threadIdx.x; i < S; i += blockDim.x)

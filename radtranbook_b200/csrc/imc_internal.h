@@ -111,7 +111,7 @@ struct WsLayout {
   size_t ecen, ew, ncopy;     // comb: double [nb], double [nb], uint64 [nb]
   size_t cnt;                 // int32 [cap]    comb copies per entry
   size_t blk;                 // int64 [nblk+1] comb block totals / offsets
-  size_t comb_mode;           // int32 mode + uint64 live-entry count (comb)
+  size_t comb_mode;           // int32 mode, uint64 live-entry count, two uint64 block tickets (comb)
   size_t dep_fx, esc_fx;      // uint64 [ncg], [4 + ng] fixed-point energy tallies
   size_t cf_rate;             // float [nc] Carter-Forest re-emission rate
   size_t total;
@@ -189,6 +189,8 @@ struct CombPlanArgs {
   double* ew;
   unsigned long long* ncopy;       // zeroed with the weights (the count accumulates into it)
   imc_step_summary* sum;
+  unsigned long long* ticket;      // zero before and after the launch
+  const double* e; const double* vol; int nc;  // e set: sum->internal_energy = canonical sum e vol
 };
 cudaError_t imc_launch_comb_plan(const CombPlanArgs& a, cudaStream_t s);
 
@@ -275,6 +277,7 @@ struct CombArgs {
   int* mode;                   // set by the comb plan: 0 comb, 1 compact only (copy live entries)
   const uint32_t* step_dev;    // non-NULL: the Philox step counter is read from device memory
   unsigned long long* n_live;  // live entries (counted by k_comb_ecen; zeroed before)
+  unsigned long long* ticket;  // of the count's blocks: zero before and after
   const int64_t* d_n_in;       // entries to comb (device)
   long long n_bound;           // host upper bound of *d_n_in (grid sizing)
   long long out_capacity;
