@@ -178,55 +178,18 @@ __device__ double face_cdf_serial(const double* Ef, double* cdf, int nf) {
   return Et;
 }
 
-__global__ void __launch_bounds__(NT) k_plan(PlanArgs a) {
-  pdl_wait();     // the previous kernel of the stream has completed
-  pdl_trigger();  // the next one may be scheduled
-  const double dt = a.dt_dev ? *a.dt_dev : a.dt;  // device-resident step length (graph replay)
-  __shared__ double red[NT];
-  __shared__ long long sh[NT];
-  const int t = threadIdx.x;
-  const int nc = a.nc;
-  const bool oned = (a.geom == G_SLAB || a.geom == G_SPHERE);
-
-  // ---- emission counts / weights / offsets ----
-  // Carter-Forest 1-D emission counts are max(1, round) in every cell
-  // (IMC/IMC1D_CarterForest.py:499, :932); otherwise ceil
-  const bool cf1 = a.method == IMC_METHOD_CARTER_FOREST && oned;
-  const long long n_emit = plan_volume(a.emit_E, a.n_target, a.nx, a.ny, nc, a.emit_n, a.emit_off,
-                                       a.emit_w, a.emitted, red, sh, cf1);
-  const double e_emit = block_canon_sum(a.emitted, nc, red);
-
-  // ---- fixed source (reference: only when max(source) > 0) ----
-  long long n_src = 0;
-  double e_src = 0.0;
-  if (a.source && a.n_source > 0) {
-    double smax = 0.0;
-    for (int c = t; c < nc; c += NT) {
-      smax = fmax(smax, a.source[c]);
-      a.src_QV[c] = a.source[c] * dt * a.vol[c] * a.share;
-    }
-    red[t] = smax;
-    __syncthreads();
-    for (int h = NT / 2; h >= 1; h >>= 1) { if (t < h) red[t] = fmax(red[t], red[t + h]); __syncthreads(); }
-    const bool any = red[0] > 0.0;
-    __syncthreads();
-    if (any) {
-      n_src = plan_volume(a.src_QV, a.n_source, a.nx, a.ny, nc, a.src_n, a.src_off, a.src_w,
-                          a.src_issued, red, sh);
-      e_src = block_canon_sum(a.src_issued, nc, red);
-    }
-  }
-
-  // ---- boundary faces: energies in parallel, then one thread per side forms the side's
-  // cumulative sums in face order ----
+// The boundary sides of a step: face energies in parallel, then one thread per side forms the
+// side's cumulative sums in face order, its count and the energy issued.
+template <class A>
+__device__ __forceinline__ void plan_faces(const A& a, bool oned, double dt) {
   for (int side = 0; side < 4; ++side) {
     if (a.face_T[side] && a.n_side[side] > 0 && !(oned && side >= 2))
       block_face_energy(a.geom, oned, side, oned ? 1 : (side < 2 ? a.ny : a.nx), a.face_T[side], a.e1, a.e2, a.nx,
                         dt, a.share, a.face + (size_t)(side * 2 + 0) * a.nf);
   }
   __syncthreads();
-  if (t < 4) {
-    const int side = t;
+  if (threadIdx.x < 4) {
+    const int side = threadIdx.x;
     a.sum->n_side[side] = 0;
     a.sum->e_side[side] = 0.0;
     const double* Tf = a.face_T[side];
@@ -242,17 +205,80 @@ __global__ void __launch_bounds__(NT) k_plan(PlanArgs a) {
       }
     }
   }
+}
+
+// Bank layout of the step, census | boundary sides 0..3 | fixed source | emission, by whichever of
+// the two plan blocks (volume sources, faces) finishes last; every thread calls it.
+__device__ __forceinline__ void plan_layout(imc_step_summary* sum, unsigned* ticket) {
+  __threadfence();
   __syncthreads();
+  if (threadIdx.x != 0 || atomicAdd(ticket, 1u) == 0u) return;
+  __threadfence();
+  const volatile imc_step_summary* v = sum;
+  long long base = v->n_census;
+  long long ns[4];
+  for (int q = 0; q < 4; ++q) ns[q] = v->n_side[q];
+  const long long n_src = v->n_source, n_emit = v->n_emission;
+  for (int q = 0; q < 4; ++q) { sum->base_side[q] = base; base += ns[q]; }
+  sum->base_source = base; base += n_src;
+  sum->base_emission = base; base += n_emit;
+  sum->n_bank = base;
+}
+
+// Two blocks: the volume sources' canonical totals, counts and offsets; the boundary faces.  The
+// counts are scanned in shared memory where they fit (smem_cnt).  With the faces after the volume
+// sources, the issued energy summed in a pass of its own and the scan in global memory this took
+// 30 us at 12600 cells and 14 us at 3150; now 17 and 10.
+__global__ void __launch_bounds__(NT) k_plan(PlanArgs a, int smem_cnt) {
+  pdl_wait();     // the previous kernel of the stream has completed
+  pdl_trigger();  // the next one may be scheduled
+  extern __shared__ int cnt_sh[];
+  const double dt = a.dt_dev ? *a.dt_dev : a.dt;  // device-resident step length (graph replay)
+  __shared__ double red[NT];
+  __shared__ long long sh[32];
+  const int t = threadIdx.x;
+  const int nc = a.nc;
+  const bool oned = (a.geom == G_SLAB || a.geom == G_SPHERE);
+  if (blockIdx.x == 1) {
+    plan_faces(a, oned, dt);
+    plan_layout(a.sum, a.ticket);
+    return;
+  }
+  int* s_cnt = smem_cnt ? cnt_sh : nullptr;
+
+  // ---- emission counts / weights / offsets ----
+  // Carter-Forest 1-D emission counts are max(1, round) in every cell
+  // (IMC/IMC1D_CarterForest.py:499, :932); otherwise ceil
+  const bool cf1 = a.method == IMC_METHOD_CARTER_FOREST && oned;
+  double e_emit;
+  const long long n_emit = plan_volume(a.emit_E, a.n_target, a.nx, a.ny, nc, s_cnt, a.emit_n, a.emit_off,
+                                       a.emit_w, a.emitted, red, sh, &e_emit, cf1);
+
+  // ---- fixed source (reference: only when max(source) > 0) ----
+  long long n_src = 0;
+  double e_src = 0.0;
+  if (a.source && a.n_source > 0) {
+    double smax = 0.0;
+    for (int c = t; c < nc; c += NT) {
+      smax = fmax(smax, a.source[c]);
+      a.src_QV[c] = a.source[c] * dt * a.vol[c] * a.share;
+    }
+    red[t] = smax;
+    __syncthreads();
+    for (int h = NT / 2; h >= 1; h >>= 1) { if (t < h) red[t] = fmax(red[t], red[t + h]); __syncthreads(); }
+    const bool any = red[0] > 0.0;
+    __syncthreads();
+    if (any)
+      n_src = plan_volume(a.src_QV, a.n_source, a.nx, a.ny, nc, s_cnt, a.src_n, a.src_off, a.src_w,
+                          a.src_issued, red, sh, &e_src);
+  }
   if (t == 0) {
-    // bank layout of this step: census | boundary sides 0..3 | fixed source | emission
-    long long base = a.sum->n_census;
-    for (int q = 0; q < 4; ++q) { a.sum->base_side[q] = base; base += a.sum->n_side[q]; }
-    a.sum->n_source = n_src; a.sum->base_source = base; base += n_src;
-    a.sum->n_emission = n_emit; a.sum->base_emission = base; base += n_emit;
-    a.sum->n_bank = base;
+    a.sum->n_source = n_src;
+    a.sum->n_emission = n_emit;
     a.sum->source_emission = e_src;
     a.sum->emission_total = e_emit;
   }
+  plan_layout(a.sum, a.ticket);
 }
 
 __global__ void __launch_bounds__(NT) k_ic_plan(IcArgs a) {
@@ -329,18 +355,9 @@ __global__ void k_material_law(MatArgs a, imc_material_law law, double* T, doubl
   }
 }
 
-// The canonical tree over 1024 partial sums, by any number of threads.
-__device__ __forceinline__ double tree_1024(double* red) {
-  for (int h = NT / 2; h >= 1; h >>= 1) {
-    for (int t = threadIdx.x; t < h; t += blockDim.x) red[t] += red[t + h];
-    __syncthreads();
-  }
-  return red[0];
-}
-
 // The canonical total of the census energy and the comb mode; with a.e, the last block sums the
 // internal energy instead.  The 1024 strided partial sums are spread over kPlanBlocks blocks when
-// the bins are many (a single SM reads 126 thousand bins in 22 us, eight in @CP@); the last of
+// the bins are many (126 thousand bins 14 us on one SM, 11 on eight); the last of
 // them to finish (a ticket; none waits) runs the tree.  The partials stand in ew until the weights
 // kernel, which follows, writes it.
 constexpr int kPlanBlocks = 8;
@@ -438,7 +455,13 @@ __global__ void __launch_bounds__(NT) k_canon_eV(const double* e, const double* 
 cudaError_t imc_launch_plan(const PlanArgs& a, cudaStream_t s) {
   g_imc_launches += 2;
   IMC_LAUNCH_PDL(k_plan_cells, (std::max(a.nc, std::max(a.nx, a.ny) + 1) + 255) / 256, 256, 0, s, a);
-  IMC_LAUNCH_PDL(k_plan, 1, NT, 0, s, a);
+  const size_t cnt = sizeof(int) * (size_t)a.nc;
+  const bool smem_cnt = cnt <= 200 * 1024;
+  if (smem_cnt && cnt > 32 * 1024) {  // beside the kernel's own 8 KB
+    const cudaError_t e = cudaFuncSetAttribute(k_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cnt);
+    if (e != cudaSuccess) return e;
+  }
+  IMC_LAUNCH_PDL(k_plan, 2, NT, smem_cnt ? cnt : 0, s, a, smem_cnt ? 1 : 0);
   return cudaGetLastError();
 }
 cudaError_t imc_launch_ic_plan(const IcArgs& a, cudaStream_t s) {
@@ -594,7 +617,12 @@ __device__ void block_canon_prefix(const double* x, int n, double* out, double* 
   const int per = (n + NT - 1) / NT;
   const int lo = min(t * per, n), hi = min(lo + per, n);
   double s = 0.0;
-  for (int i = lo; i < hi; ++i) s += x[i];
+  double first[B];  // the chunk's first B values, read once for both passes
+#pragma unroll
+  for (int j = 0; j < B; ++j) first[j] = lo + j < hi ? x[lo + j] : 0.0;
+#pragma unroll
+  for (int j = 0; j < B; ++j) if (lo + j < hi) s += first[j];
+  for (int i = lo + B; i < hi; ++i) s += x[i];
   sh[t] = s;
   __syncthreads();
   if (t == 0) {
@@ -609,7 +637,9 @@ __device__ void block_canon_prefix(const double* x, int n, double* out, double* 
   }
   __syncthreads();
   double run = sh[t];
-  for (int i0 = lo; i0 < hi; i0 += B) {
+#pragma unroll
+  for (int j = 0; j < B; ++j) if (lo + j < hi) { run += first[j]; out[lo + j] = run; }
+  for (int i0 = lo + B; i0 < hi; i0 += B) {
     double v[B];
 #pragma unroll
     for (int j = 0; j < B; ++j) v[j] = i0 + j < hi ? x[i0 + j] : 0.0;
@@ -633,82 +663,111 @@ constexpr MixCdf mix_cdf_table() {
 }
 __device__ const MixCdf g_mix_cdf = mix_cdf_table();
 
-// The Planck edge integrals of the block's cells [c0, c0 + ncb) at the G + 1 group edges,
-// one (cell, edge) pair per thread: x and its series or tail value at [(c - c0)(G + 1) + k].
-// The tail costs up to 2 + 40/x exponentials, so this is most of a plan's arithmetic; spread
-// over all the block's threads it is no longer one long chain per cell.
-__device__ void block_planck_edges(const double* T, const double* gedges, int G, int c0, int ncb, double* sx,
-                                   double* ss) {
-  const int E = G + 1;
-  for (int i = threadIdx.x; i < ncb * E; i += blockDim.x) {
-    const int cl = i / E, k = i - cl * E;
-    const double Tc = T[c0 + cl];
-    const PlanckEdge pe = planck_edge(Tc > 0.0 ? gedges[k] / Tc : 0.0);
-    sx[i] = pe.x;
-    ss[i] = pe.s;
-  }
-  __syncthreads();
-}
-
-// Per-cell part of the 2-D multigroup plan.  A block takes cb consecutive cells: its threads
-// evaluate the cells' Planck edges into shared memory, then one thread per cell forms the
-// fractions, Planck-mean opacity, Fleck factor and emission by group (each cell's numbers
-// depend on that cell alone, so the result is the single-block loop's).
+// Per-cell part of the multigroup plans (2-D: MG_IMC/MG_IMC2D.py:1703-1943; SPHERE: MG_IMC/
+// MG_IMC1D.py:941-1000): Planck fractions, Planck-mean opacity, Fleck factor, tables, emission by
+// group.  A block takes cb consecutive cells.  All that one (cell, group) or (cell, edge) needs by
+// itself (the edge integrals, quotients, table entries) is a thread of its own, group-major so that a
+// warp's edge integrals have about the same number of terms (a tail takes 2 + 40/x exponentials);
+// only the sums over a cell's groups, in group order, are one thread's per cell.  With the pairs
+// cell-major and everything after the edge integrals one thread per cell this took 25 us for
+// 12600 cells of 10 groups and 20 us for 200; now 14 and 14.
+template <bool SPHERE>
 __global__ void __launch_bounds__(256) k_plan_mg_cells(PlanMgArgs a, int cb) {
   pdl_wait();     // the previous kernel of the stream has completed
   pdl_trigger();  // the next one may be scheduled
   extern __shared__ double plan_sh[];
   const double dt = a.dt_dev ? *a.dt_dev : a.dt;  // device-resident step length (graph replay)
-  const int nc = a.nc, G = a.ng;
+  const int nc = a.nc, G = a.ng, E = G + 1;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   for (int q = t0; q <= a.nx; q += stride) a.e1f[q] = (float)a.e1[q];
   for (int q = t0; q <= a.ny; q += stride) a.e2f[q] = (float)a.e2[q];
   for (int q = t0; q < 200; q += stride) a.mixcdf[q] = g_mix_cdf.v[q];
   const int c0 = blockIdx.x * cb, ncb = min(cb, nc - c0);
-  double* sx = plan_sh;
-  double* sv = plan_sh + (size_t)cb * (G + 1);
-  block_planck_edges(a.T, a.gedges, G, c0, ncb, sx, sv);
-  // ---- per cell: Planck fractions, Planck-mean opacity, Fleck, emission by group ----
+  double* sx = plan_sh;                    // [cb][E]: an edge's x, then a group's fraction
+  double* sv = sx + (size_t)cb * E;        // [cb][E]: its series or tail, then the group's terms
+  double* s_tot = sv + (size_t)cb * E;     // [cb]: sum of the fractions, then the Fleck factor
+  double* s_aT4 = s_tot + cb;              // [cb]
+  for (int i = threadIdx.x; i < ncb * E; i += blockDim.x) {
+    const int k = i / ncb, cl = i - k * ncb;
+    const double Tc = a.T[c0 + cl];
+    const PlanckEdge pe = planck_edge(Tc > 0.0 ? a.gedges[k] / Tc : 0.0);
+    sx[cl * E + k] = pe.x;
+    sv[cl * E + k] = pe.s;
+  }
+  __syncthreads();
+  // fractions in place of the lower edges: a round reads both edges of its groups before any of
+  // them is overwritten, and the next round's lower edges are past this one's groups
+  for (int r = 0; r < ncb * G; r += blockDim.x) {
+    const int i = r + threadIdx.x;
+    const int g = i / ncb, cl = i - g * ncb;
+    double f = 0.0;
+    if (i < ncb * G && a.T[c0 + cl] > 0.0) {
+      const double* x = sx + cl * E + g;
+      const double* s = sv + cl * E + g;
+      f = planck_frac(PlanckEdge{x[0], s[0]}, PlanckEdge{x[1], s[1]});
+    }
+    __syncthreads();
+    if (i < ncb * G) sx[cl * E + g] = f > 0.0 ? f : 0.0;
+    __syncthreads();
+  }
+  if ((int)threadIdx.x < ncb) {
+    double tot = 0.0;
+    for (int g = 0; g < G; ++g) tot += sx[threadIdx.x * E + g];
+    s_tot[threadIdx.x] = tot;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < ncb * G; i += blockDim.x) {
+    const int g = i / ncb, cl = i - g * ncb;
+    const double tot = s_tot[cl], b = tot > 0.0 ? sx[cl * E + g] / tot : 0.0;
+    sx[cl * E + g] = b;
+    sv[cl * E + g] = a.sigma[(size_t)g * nc + c0 + cl] * b;
+  }
+  __syncthreads();
   if ((int)threadIdx.x < ncb) {
     const int c = c0 + threadIdx.x;
-    const int eb = threadIdx.x * (G + 1);
     const double T = a.T[c];
     if (!isfinite(T) || !(a.cv[c] > 0.0)) atomicOr(&a.sum->flags, (int)IMC_FLAG_NONFINITE);
-    double* gc = a.Egc + (size_t)c * G;  // scratch: fractions, then cumulative emission
-    double tot = 0.0;
-    PlanckEdge lo{sx[eb], sv[eb]};
-    for (int g = 0; g < G; ++g) {
-      const PlanckEdge hi{sx[eb + g + 1], sv[eb + g + 1]};
-      const double f = (T > 0.0) ? planck_frac(lo, hi) : 0.0;
-      lo = hi;
-      gc[g] = f > 0.0 ? f : 0.0;
-      tot += gc[g];
-    }
     double sp = 0.0;
-    for (int g = 0; g < G; ++g) {
-      gc[g] = tot > 0.0 ? gc[g] / tot : 0.0;
-      sp += a.sigma[(size_t)g * nc + c] * gc[g];
-    }
+    for (int g = 0; g < G; ++g) sp += sv[threadIdx.x * E + g];
     const double beta = 4.0 * A_RAD * pow3(T) / a.cv[c];
     double f = 1.0 / (1.0 + a.theta * beta * sp * C_LIGHT * dt);
     f = fmin(1.0, fmax(0.0, f));
-    const double aT4 = (a.t_emit_floor > 0.0 && T < a.t_emit_floor) ? 0.0
+    s_tot[threadIdx.x] = f;
+    s_aT4[threadIdx.x] = (a.t_emit_floor > 0.0 && T < a.t_emit_floor) ? 0.0
                                                                       : A_RAD * C_LIGHT * pow4(T) * dt * a.vol[c] * a.share;
-    double run = 0.0;
-    for (int g = 0; g < G; ++g) {
-      const size_t q = (size_t)g * nc + c;
-      const double ss = a.sigma[q] * (1.0 - f);
-      const double sa = a.sigma[q] * f;
-      a.sa[q] = sa; a.ss[q] = ss;
-      // absorption 0: no capture, w*s intensity
-      a.sass[q] = make_float2(sa > 1e-12 ? (float)sa : 0.f, scatter_entry(ss, 1e-12f, 0.f));
-      a.cellf[q] = make_double2(1.0 / a.vol[c], sa > 1e-12 ? 1.0 / (sa * a.vol[c] * dt) : -1.0 / (a.vol[c] * dt));
-      const double bg = a.emission_fractions ? a.emission_fractions[g] : gc[g];
-      run += sa * bg * aT4;
-      gc[g] = run;  // cumulative over groups
-    }
-    a.Ec[c] = run;
   }
+  __syncthreads();
+  const double thr = SPHERE ? 1e-10 : 1e-12;  // MG_IMC/MG_IMC1D.py:346-350; MG_IMC/MG_IMC2D.py:580-989
+  for (int i = threadIdx.x; i < ncb * G; i += blockDim.x) {
+    const int g = i / ncb, cl = i - g * ncb, c = c0 + cl;
+    const size_t q = (size_t)g * nc + c;
+    const double f = s_tot[cl], b = sx[cl * E + g];
+    const double ss = a.sigma[q] * (1.0 - f);
+    const double sa = a.sigma[q] * f;
+    a.sa[q] = sa; a.ss[q] = ss;
+    // absorption 0: no capture, w*s intensity
+    a.sass[q] = make_float2(sa > thr ? (float)sa : 0.f,
+                            SPHERE ? scatter_entry(ss, 1e-10f, cell_width(true, a.e1, a.e2, a.nx, c))
+                                   : scatter_entry(ss, 1e-12f, 0.f));
+    a.cellf[q] = make_double2(1.0 / a.vol[c], sa > thr ? 1.0 / (sa * a.vol[c] * dt) : -1.0 / (a.vol[c] * dt));
+    if (SPHERE) {
+      const bool cold = a.t_emit_floor > 0.0 && a.T[c] < a.t_emit_floor;
+      a.emit_E[q] = cold ? 0.0 : A_RAD * C_LIGHT * pow4(a.T[c]) * sa * b * dt * a.vol[c] * a.share;
+    } else {
+      const double bg = a.emission_fractions ? a.emission_fractions[g] : b;
+      sv[cl * E + g] = sa * bg * s_aT4[cl];
+    }
+  }
+  if (SPHERE) return;
+  __syncthreads();
+  if ((int)threadIdx.x < ncb) {
+    double run = 0.0;
+    for (int g = 0; g < G; ++g) { run += sv[threadIdx.x * E + g]; sv[threadIdx.x * E + g] = run; }
+    a.Ec[c0 + threadIdx.x] = run;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < ncb * G; i += blockDim.x)  // cumulative over groups, [c][g]
+    a.Egc[(size_t)c0 * G + i] = sv[(i / G) * E + i % G];
   // fixed source [g][c] (MG_IMC/MG_IMC2D.py:1098-1170): per-cell cumulative over groups
   if (a.source && a.n_source > 0) {
     for (int c = t0; c < nc; c += stride) {
@@ -722,7 +781,7 @@ __global__ void __launch_bounds__(256) k_plan_mg_cells(PlanMgArgs a, int cb) {
   }
 }
 
-// Single-block part: canonical prefix sums and totals, counts, boundary faces, bank layout.
+// Canonical prefix sums, totals and counts in one block, the boundary faces in another.
 __global__ void __launch_bounds__(NT) k_plan_mg(PlanMgArgs a) {
   pdl_wait();     // the previous kernel of the stream has completed
   pdl_trigger();  // the next one may be scheduled
@@ -730,6 +789,11 @@ __global__ void __launch_bounds__(NT) k_plan_mg(PlanMgArgs a) {
   __shared__ double sh[NT];
   const int t = threadIdx.x;
   const int nc = a.nc;
+  if (blockIdx.x == 1) {
+    plan_faces(a, false, dt);
+    plan_layout(a.sum, a.ticket);
+    return;
+  }
   block_canon_prefix(a.Ec, nc, a.cdf, sh);
   const double Eemit = a.cdf[nc - 1];
   long long n_emit = 0;
@@ -753,100 +817,18 @@ __global__ void __launch_bounds__(NT) k_plan_mg(PlanMgArgs a) {
       e_src = (double)n_src * (double)(float)(St / (double)n_src);
     }
   }
-
-  // ---- boundary faces (as gray: energies in parallel, cumulative sums per side) ----
-  for (int side = 0; side < 4; ++side) {
-    if (a.face_T[side] && a.n_side[side] > 0)
-      block_face_energy(a.geom, false, side, side < 2 ? a.ny : a.nx, a.face_T[side], a.e1, a.e2, a.nx, dt, a.share,
-                        a.face + (size_t)(side * 2 + 0) * a.nf);
-  }
-  __syncthreads();
-  if (t < 4) {
-    const int side = t;
-    a.sum->n_side[side] = 0;
-    a.sum->e_side[side] = 0.0;
-    const double* Tf = a.face_T[side];
-    const long long nbs = a.n_side[side];
-    if (Tf && nbs > 0) {
-      const int nf = side < 2 ? a.ny : a.nx;
-      const double Et = face_cdf_serial(a.face + (size_t)(side * 2 + 0) * a.nf,
-                                        a.face + (size_t)(side * 2 + 1) * a.nf, nf);
-      if (Et > 0.0) {
-        a.sum->n_side[side] = nbs;
-        a.sum->e_side[side] = (double)nbs * (double)(float)(Et / (double)nbs);
-      }
-    }
-  }
-  __syncthreads();
   if (t == 0) {
-    long long base = a.sum->n_census;
-    for (int q = 0; q < 4; ++q) { a.sum->base_side[q] = base; base += a.sum->n_side[q]; }
-    a.sum->n_source = n_src; a.sum->base_source = base; base += n_src;
-    a.sum->n_emission = n_emit; a.sum->base_emission = base; base += n_emit;
-    a.sum->n_bank = base;
+    a.sum->n_source = n_src;
+    a.sum->n_emission = n_emit;
     a.sum->source_emission = e_src;
     a.sum->emission_total = issued;
   }
+  plan_layout(a.sum, a.ticket);
 }
 
-// Multigroup 1-D sphere planning (MG_IMC/MG_IMC1D.py:941-1120): Planck fractions, Fleck
-// factor with the Planck-mean opacity, emission E_gc = a c T^4 sigma_a,g b*_g dt V per
-// (group, cell) bin b = g*nc + c with stratified counts max(1, round(N E_b / E)) (fixed
-// source: round, no minimum), inner / outer sphere boundary faces.
-// Per-shell part of the sphere plan, one thread per shell over a wide grid (each shell's
-// numbers depend on that shell alone, so the result is the single-block loop's).
-__global__ void __launch_bounds__(256) k_plan_mg1d_cells(PlanMgArgs a, int cb) {
-  pdl_wait();     // the previous kernel of the stream has completed
-  pdl_trigger();  // the next one may be scheduled
-  extern __shared__ double plan_sh[];
-  const double dt = a.dt_dev ? *a.dt_dev : a.dt;  // device-resident step length (graph replay)
-  const int nc = a.nc, G = a.ng;
-  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  for (int q = t0; q <= a.nx; q += stride) a.e1f[q] = (float)a.e1[q];
-  for (int q = t0; q <= a.ny; q += stride) a.e2f[q] = (float)a.e2[q];
-  for (int q = t0; q < 200; q += stride) a.mixcdf[q] = g_mix_cdf.v[q];
-  const int c0 = blockIdx.x * cb, ncb = min(cb, nc - c0);
-  double* sx = plan_sh;
-  double* sv = plan_sh + (size_t)cb * (G + 1);
-  block_planck_edges(a.T, a.gedges, G, c0, ncb, sx, sv);
-  if ((int)threadIdx.x < ncb) {
-    const int c = c0 + threadIdx.x;
-    const int eb = threadIdx.x * (G + 1);
-    const double T = a.T[c];
-    if (!isfinite(T) || !(a.cv[c] > 0.0)) atomicOr(&a.sum->flags, (int)IMC_FLAG_NONFINITE);
-    double* b = a.Egc + (size_t)c * G;  // scratch: Planck fractions of this cell
-    double tot = 0.0;
-    PlanckEdge lo{sx[eb], sv[eb]};
-    for (int g = 0; g < G; ++g) {
-      const PlanckEdge hi{sx[eb + g + 1], sv[eb + g + 1]};
-      const double f = (T > 0.0) ? planck_frac(lo, hi) : 0.0;
-      lo = hi;
-      b[g] = f > 0.0 ? f : 0.0;
-      tot += b[g];
-    }
-    double sp = 0.0;
-    for (int g = 0; g < G; ++g) {
-      b[g] = tot > 0.0 ? b[g] / tot : 0.0;
-      sp += a.sigma[(size_t)g * nc + c] * b[g];
-    }
-    const double beta = 4.0 * A_RAD * pow3(T) / a.cv[c];
-    double f = 1.0 / (1.0 + a.theta * beta * sp * C_LIGHT * dt);
-    f = fmin(1.0, fmax(0.0, f));
-    const bool cold = a.t_emit_floor > 0.0 && T < a.t_emit_floor;
-    for (int g = 0; g < G; ++g) {
-      const size_t q = (size_t)g * nc + c;
-      const double sa = a.sigma[q] * f;
-      const double ss = a.sigma[q] * (1.0 - f);
-      a.sa[q] = sa; a.ss[q] = ss;
-      // absorption 0: no capture, w*s intensity
-      a.sass[q] = make_float2(sa > 1e-10 ? (float)sa : 0.f, scatter_entry(ss, 1e-10f, cell_width(true, a.e1, a.e2, a.nx, c)));
-      // MG_IMC/MG_IMC1D.py:346-350: path-length estimator below sigma_a = 1e-10
-      a.cellf[q] = make_double2(1.0 / a.vol[c], sa > 1e-10 ? 1.0 / (sa * a.vol[c] * dt) : -1.0 / (a.vol[c] * dt));
-      a.emit_E[q] = cold ? 0.0 : A_RAD * C_LIGHT * pow4(T) * sa * b[g] * dt * a.vol[c] * a.share;
-    }
-  }
-}
-
+// Multigroup 1-D sphere planning (MG_IMC/MG_IMC1D.py:941-1120): emission
+// E_gc = a c T^4 sigma_a,g b*_g dt V per (group, cell) bin b = g*nc + c with stratified counts
+// max(1, round(N E_b / E)) (fixed source: round, no minimum), inner / outer sphere boundary faces.
 // Single-block part of the sphere plan: canonical totals, stratified counts and scans,
 // fixed source, boundary faces, bank layout.
 __global__ void __launch_bounds__(NT) k_plan_mg1d(PlanMgArgs a) {
@@ -958,12 +940,12 @@ __global__ void __launch_bounds__(NT) k_ic_plan_mg(IcMgArgs a) {
 
 // Launch shape of the per-cell multigroup plan: as many cells a block as leave one
 // (cell, group edge) pair per thread (the edge integrals are the long part; at most 32 cells),
-// two doubles per pair of shared memory; above 48 KB the kernel is opted in to more.
+// two doubles per pair and cell of shared memory; above 48 KB the kernel is opted in to more.
 template <typename K>
 cudaError_t launch_plan_cells(K kernel, const PlanMgArgs& a, cudaStream_t s) {
   const long long E = (long long)a.ng + 1;
   const int cb = (int)std::max(1LL, std::min(32LL, 256LL / E));
-  const size_t smem = (size_t)2 * cb * E * sizeof(double);
+  const size_t smem = (size_t)2 * cb * (E + 1) * sizeof(double);
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -975,15 +957,15 @@ cudaError_t launch_plan_cells(K kernel, const PlanMgArgs& a, cudaStream_t s) {
 
 cudaError_t imc_launch_plan_mg(const PlanMgArgs& a, cudaStream_t s) {
   g_imc_launches += 2;
-  const cudaError_t e = launch_plan_cells(k_plan_mg_cells, a, s);
+  const cudaError_t e = launch_plan_cells(k_plan_mg_cells<false>, a, s);
   if (e != cudaSuccess) return e;
-  IMC_LAUNCH_PDL(k_plan_mg, 1, NT, 0, s, a);
+  IMC_LAUNCH_PDL(k_plan_mg, 2, NT, 0, s, a);
   return cudaGetLastError();
 }
 
 cudaError_t imc_launch_plan_mg1d(const PlanMgArgs& a, cudaStream_t s) {
   g_imc_launches += 2;
-  const cudaError_t e = launch_plan_cells(k_plan_mg1d_cells, a, s);
+  const cudaError_t e = launch_plan_cells(k_plan_mg_cells<true>, a, s);
   if (e != cudaSuccess) return e;
   IMC_LAUNCH_PDL(k_plan_mg1d, 1, NT, 0, s, a);
   return cudaGetLastError();

@@ -181,7 +181,7 @@ imc_status transport_async(const imc_mesh* mesh, const imc_material* mat, const 
     zl.add(esc_fx, sizeof(unsigned long long) * (4 + ng));
     zl.add(tal->si, sizeof(double) * nc * ng);
     zl.add(tal->stats, sizeof(unsigned long long) * IMC_STAT_N);
-    zl.add(queue, 8);
+    zl.add(queue, 16);  // tracking ticket, plan ticket
     if (par->census_bins && !adj) {
       const int nb = par->census_bins == IMC_CENSUS_BY_GROUP_CELL ? nc * ng : nc;
       zl.add(ws_ptr<double>(workspace, L.ecen), sizeof(double) * nb);
@@ -215,6 +215,7 @@ imc_status transport_async(const imc_mesh* mesh, const imc_material* mat, const 
   pa.emitted = tal->emitted;
   pa.face = ws_ptr<double>(workspace, L.face); pa.nf = std::max(mesh->nx, mesh->ny);
   pa.sum = sum;
+  pa.ticket = reinterpret_cast<unsigned*>(queue + 1);
   PlanMgArgs pm{};
   if (!mg) {
     IMC_CUDA(imc_launch_plan(pa, s));
@@ -238,6 +239,7 @@ imc_status transport_async(const imc_mesh* mesh, const imc_material* mat, const 
     pm.src_QV = pa.src_QV; pm.src_n = pa.src_n; pm.src_off = pa.src_off; pm.src_w = pa.src_w;
     pm.src_issued = pa.src_issued;
     pm.sum = sum;
+    pm.ticket = pa.ticket;
     pm.dt_dev = par->dt_dev;
     pm.share = share;
     IMC_CUDA(imc_launch_plan_mg1d(pm, s));
@@ -260,6 +262,7 @@ imc_status transport_async(const imc_mesh* mesh, const imc_material* mat, const 
     pm.emitted = tal->emitted; pm.face = pa.face; pm.nf = pa.nf;
     pm.mixcdf = ws_ptr<double>(workspace, L.mixcdf);
     pm.sum = sum;
+    pm.ticket = pa.ticket;
     pm.dt_dev = par->dt_dev;
     pm.share = share;
     IMC_CUDA(imc_launch_plan_mg(pm, s));
@@ -535,7 +538,7 @@ WsLayout imc_ws_layout(const imc_mesh* m, int64_t capacity) {
   const size_t nf = std::max(nx, ny);
   const size_t cap = (size_t)std::max<int64_t>(capacity, 1);
   auto take = [&](size_t bytes) { const size_t r = o; o += al256(bytes); return r; };
-  L.summary = take(sizeof(imc_step_summary)); L.queue = take(8);
+  L.summary = take(sizeof(imc_step_summary)); L.queue = take(16);
   L.e1f = take(4 * (nx + 1)); L.e2f = take(4 * (ny + 1));
   L.sass = take(8 * ncg); L.cellf = take(16 * ncg);
   L.emit_E = take(8 * ncg); L.emit_n = take(8 * ncg); L.emit_off = take(8 * (ncg + 1)); L.emit_w = take(4 * ncg);

@@ -107,7 +107,7 @@ __device__ __forceinline__ int comb_copies(const CombArgs& a, float wf, int bk, 
 // hash table over the block's one tile.  The last block to finish scans the
 // tile totals (a ticket; no block waits).  With a hash table of bins per 4096 entries instead, which
 // a mixed bank overflows, and an FP64 division per entry this took 94 us for 8.7 M entries in 12600
-// bins and 45 us for 91 thousand in 3150 (23 blocks); now @CNT2M@ and @CNT20K@ us.
+// bins and 45 us for 91 thousand in 3150 (23 blocks); now 55 and 13 us.
 constexpr int kCountMaxTiles = 64;  // tiles a block takes at most
 constexpr int kCountSlots = TILE / 2;  // hash table of a block (a tile rarely has more bins; adds past it go to global memory)
 
@@ -232,8 +232,9 @@ __host__ __device__ inline size_t scatter_smem(bool two_d, bool grp) {
 // and the stores of a warp are both contiguous.  A tile with more than SCAT_MAP copies finds the
 // entries of the others by a binary search of the scanned counts.  The remaining blocks take 256
 // bins each: disc and the energy after the comb.  Against tiles of 4096 entries, a search for
-// every copy and the copy weight gathered per copy: 87 -> @SC2M@ us for 8.7 M entries, 26 -> @SC20K@ us
-// for 91 thousand.
+// every copy, the copy weight gathered per copy and a launch of its own for the bins: 28 -> 13 us
+// for 91 thousand entries, 29 -> 20 us for 1.7 M; 8.7 M take the same 88 us (0.40 GB moved, at two
+// thirds of the rate of a copy).
 __global__ void __launch_bounds__(SCAT_T) k_comb_scatter(CombArgs a, long long ntiles) {
   pdl_wait();     // the previous kernel of the stream has completed
   pdl_trigger();  // the next one may be scheduled

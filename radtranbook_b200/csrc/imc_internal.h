@@ -107,7 +107,7 @@ struct WsLayout {
   size_t face;                // double [4][2][nf] per-side face energies and CDF
   size_t mg_gcdf, mg_ec, mg_cdf, mg_sgcdf, mg_sc, mg_scdf, mixcdf;  // multigroup tables
   size_t summary;             // imc_step_summary used by the synchronous wrappers
-  size_t queue;               // uint64 ticket counter
+  size_t queue;               // uint64 ticket counter of the tracking, uint32 of the plan's blocks
   size_t ecen, ew, ncopy;     // comb: double [nb], double [nb], uint64 [nb]
   size_t cnt;                 // int32 [cap]    comb copies per entry
   size_t blk;                 // int64 [nblk+1] comb block totals / offsets
@@ -151,6 +151,7 @@ struct PlanArgs {
   double* face;                    // [4][2][nf]
   int nf;
   imc_step_summary* sum;
+  unsigned* ticket;                // of the plan's two blocks, zero before
 };
 cudaError_t imc_launch_plan(const PlanArgs& a, cudaStream_t s);
 
@@ -358,6 +359,7 @@ struct PlanMgArgs {
   double* src_QV; long long* src_n; long long* src_off; float* src_w; double* src_issued;
   const double* dt_dev;            // non-NULL: dt read from device memory (graph replay)
   double share;                    // fraction of the source energy issued (1: all of it)
+  unsigned* ticket;                // of the plan's two blocks, zero before
 };
 cudaError_t imc_launch_plan_mg(const PlanMgArgs& a, cudaStream_t s);
 cudaError_t imc_launch_plan_mg1d(const PlanMgArgs& a, cudaStream_t s);
