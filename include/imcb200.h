@@ -390,6 +390,31 @@ IMC_API imc_status imc_mg_report_fields(const imc_mesh* mesh, const double* si, 
                                         const double* e, const double* T, const double* Tr,
                                         const double* boundary_group, const double* escaped_group,
                                         double* out, void* stream);
+/* imc_mg_report_fields into out_dev and the written sections copied on to out_host (pinned, the
+ * same layout), in one call: on `side` (a stream; with fork and done, events) after the work
+ * `stream` holds, beside what is queued on it next, `done` recorded after the copies; or, with
+ * side NULL, on `stream`. */
+IMC_API imc_status imc_mg_report_to_host(const imc_mesh* mesh, const double* si, const double* after,
+                                         const double* e, const double* T, const double* Tr,
+                                         const double* boundary_group, const double* escaped_group,
+                                         double* out_dev, double* out_host, void* stream, void* side, void* fork,
+                                         void* done);
+/* n cell fields (1 to 4) from the engine's flat order c = i + nx j into out, one after the other, in
+ * the reference's (nx, ny) C order (1-D: as they are), and `done` (an event, or NULL) recorded
+ * after; the reverse takes n fields in that order from src to the flat arrays.  out and src may be
+ * pinned host memory: the kernel writes or reads it in place. */
+IMC_API imc_status imc_fields_to_host(const imc_mesh* mesh, const double* const* fields, int32_t n, double* out,
+                                      void* done, void* stream);
+IMC_API imc_status imc_fields_from_host(const imc_mesh* mesh, const double* src, int32_t n, double* const* fields,
+                                        void* stream);
+/* An asynchronous copy of bytes from src to dst (device or pinned host) and `done` (an event)
+ * recorded after it. */
+IMC_API imc_status imc_copy_record(void* dst, const void* src, size_t bytes, void* done, void* stream);
+/* Per (group, cell) bin of a 1-D bank (multigroup: bin c + nc g), sums over its live entries:
+ * out[0, ncg) the energy, out[ncg, 2 ncg) c sum(w mu) / V (MG_IMC/MG_IMC1D.py:1209-1227).  n_dev: the
+ * number of entries (device). */
+IMC_API imc_status imc_bank_moments(const imc_mesh* mesh, const imc_bank* bank, const int64_t* n_dev, double* out,
+                                    void* stream);
 IMC_API imc_status imc_bank_energy_by_bin(const imc_mesh* mesh, const imc_bank* bank, const int64_t* n_dev,
                                           int32_t per_group, double* out, void* stream);
 /* Device time (ms) of the source fill and of tracking in this host thread's last

@@ -84,31 +84,13 @@ class GrayState:
             object.__setattr__(self, "_host_copy_mode", True)
         return arrays
 
-    def host_copies(self):
-        """(device, pinned host) pair for the end-of-step copy of e, T and Tr: the three fields
-        stacked on the device in the reference's layout ((nx, ny) in 2-D), one copy into the
-        step's host buffer."""
-        src = torch.stack([self.grid(self._e), self.grid(self._T), self.grid(self._Tr)]).reshape(-1)
-        pin = self.host_buffer(src.numel())
-        object.__setattr__(self, "_hpin", pin)
-        return [(src, pin)]
-
-    def host_copies_early(self) -> "torch.cuda.Event":
-        """Queue the copy of host_copies() on a side stream of the engine, after the work the
-        current stream holds so far (the material update), so that it runs beside the work
-        queued next (the comb).  Returns the side stream's event after the copy: the caller
-        synchronises the host on it before reading the buffer and before the step returns
-        (nothing that changes e, T or Tr is queued before then)."""
+    def report(self, done: "torch.cuda.Event | None" = None) -> None:
+        """Queue e, T and Tr into the step's pinned host buffer in the reference's layout ((nx, ny) in
+        2-D), one kernel that writes the buffer in place; `done` is recorded after it."""
         eng = self._engine
-        side = eng.side_stream()
-        main = torch.cuda.current_stream(eng.device)
-        side.wait_stream(main)
-        with torch.cuda.stream(side):
-            for d, h in self.host_copies():
-                h.copy_(d, non_blocking=True)
-        done = torch.cuda.Event()
-        done.record(side)
-        return done
+        pin = self.host_buffer(3 * eng.nc)
+        object.__setattr__(self, "_hpin", pin)
+        eng.fields_to_host((self._e, self._T, self._Tr), pin, done)
 
     def take_host_copies(self, publish: bool = True) -> list:
         """Host mirrors of e, T and Tr from the buffer filled by the last fetch (no device
@@ -175,17 +157,22 @@ def _pinned(state, key: str, n: int) -> torch.Tensor:
     return bufs[key]
 
 
-def _staged(state, key: str, n: int) -> dict:
-    """A pinned host buffer and its device twin (n doubles each) kept on the state: the
-    stage / stage_dev pair of materials.evaluate, so a host callable's result reaches the
-    device without a device allocation per step."""
+def _device_field(state, key: str, n: int) -> torch.Tensor:
+    """A device buffer of n doubles kept on the state (allocated once)."""
     devs = state.__dict__.get("_stage_dev")
     if devs is None:
         devs = {}
         object.__setattr__(state, "_stage_dev", devs)
     if key not in devs or devs[key].numel() != n:
         devs[key] = torch.empty(n, dtype=torch.float64, device=state._engine.device)
-    return {"stage": _pinned(state, key, n), "stage_dev": devs[key]}
+    return devs[key]
+
+
+def _staged(state, key: str, n: int) -> dict:
+    """A pinned host buffer and its device twin (n doubles each) kept on the state: the
+    stage / stage_dev pair of materials.evaluate, so a host callable's result reaches the
+    device without a device allocation per step."""
+    return {"stage": _pinned(state, key, n), "stage_dev": _device_field(state, key, n)}
 
 
 def _same(key, objs: tuple) -> bool:
@@ -355,11 +342,12 @@ def gray_step(state: GrayState, *, Ntarget, Nboundary, Nsource, Nmax, T_boundary
         state.__dict__.pop("_law_next", None)
         eng.material_update(state._e, state._Tr)
     # e and Tr are final now (no comb discrepancy booked into e), and so is T with the device
-    # law: their copy to the host runs on a side stream beside the comb.  A host inv_eos then
-    # evaluates T from that copy of e while the comb runs.
+    # law: they go to the host before the comb.  A host inv_eos then evaluates T from that e
+    # while the comb runs.
     host_inv = law is None and not conserve_comb_energy and not is_device(inv_eos)
-    early = state.host_copies_early() if (law is not None and not conserve_comb_energy) or host_inv else None
-    t_up = None
+    early = law is not None or host_inv
+    if early:
+        state.report(eng.event("fields") if host_inv else None)
     eng.comb_async(Nmax, state.count, state._e)
     if conserve_comb_energy:
         sum_tensors(dist, [eng.disc])
@@ -369,45 +357,44 @@ def gray_step(state: GrayState, *, Ntarget, Nboundary, Nsource, Nmax, T_boundary
     if law is not None:
         pass  # T = e / cv came with the material update
     elif host_inv:
-        # the early copy holds e, (the old) T and Tr in the reference's layout: T = inv_eos(e)
-        # replaces the T slot (the host mirror this step returns) and goes up to the device on
-        # the side stream (nothing queued on the current stream reads T before the step ends)
-        early.synchronize()
+        # the report holds e, (the old) T and Tr in the reference's layout: T = inv_eos(e)
+        # replaces the T slot (the host mirror this step returns), and goes up to the device, with
+        # the next step's opacity and heat capacity at this T when both are host callables (the
+        # next step takes them if it passes the same callables and nothing has set T since): one
+        # launch behind the comb, ahead of the summary that the step waits for
+        eng.event("fields").synchronize()
         n = eng.nc
         shape = (n,) if state._dim == 1 else tuple(state._shape)
         hp = state._hpin.numpy()
         Tn = np.asarray(inv_eos(hp[:n].reshape(shape)), dtype=np.float64)
-        np.copyto(hp[n:2 * n].reshape(shape), np.broadcast_to(Tn, shape))
-        side = eng.side_stream()
-        with torch.cuda.stream(side):
-            _upload_flat(state, Tn, _pinned(state, "T_new", n), state._T)
-            if not is_device(sigma_a_func) and not is_device(cv):
-                # the next step's opacity and heat capacity at this T (the host mirror it
-                # returns), while the comb runs; the next step takes them if it passes the same
-                # callables and nothing has set T since (this step's own inputs are read)
-                T_ref = hp[n:2 * n].reshape(shape)
-                st_s, st_c = _staged(state, "sigma", n), _staged(state, "cv", n)
-                sig_n = _upload_flat(state, sigma_a_func(T_ref), st_s["stage"], st_s["stage_dev"])
-                cv_n = _upload_flat(state, cv(T_ref), st_c["stage"], st_c["stage_dev"])
-                state.__dict__["_host_next"] = ((sigma_a_func, cv), state.count + 1, sig_n, cv_n)
-        t_up = torch.cuda.Event()
-        t_up.record(side)
+        T_ref = hp[n:2 * n].reshape(shape)
+        np.copyto(T_ref, Tn)
+        stage = _pinned(state, "up", 3 * n)
+        up = stage.numpy()
+        np.copyto(up[:n].reshape(shape), Tn)
+        dst = [state._T]
+        if not is_device(sigma_a_func) and not is_device(cv):
+            sig_n, cv_n = _device_field(state, "sigma", n), _device_field(state, "cv", n)
+            np.copyto(up[n:2 * n].reshape(shape), sigma_a_func(T_ref))
+            np.copyto(up[2 * n:].reshape(shape), cv(T_ref))
+            dst += [sig_n, cv_n]
+            state.__dict__["_host_next"] = ((sigma_a_func, cv), state.count + 1, sig_n, cv_n)
+        eng.fields_from_host(stage, dst)
+        _lib.TRANSFER["h2d"] += 8 * n * len(dst)
     else:
         Tn = evaluate(inv_eos, state.grid(state._e), lambda: _host_copy(state.grid(state._e)), like)
         state._T.copy_(state.flat(Tn))
-    copies = state.host_copies() if early is None else ()
+    if not early:
+        state.report()
+    eng.queue_summary()
     # the phase times wait for the tracking only: read while the comb still runs on the device
     ms_src, ms_tr = eng.phase_times()
     try:
-        sm = eng.fetch(copies)
+        sm = eng.fetch()
     except _lib.ImcError as ex:
         if ex.status == 3:
             raise AssertionError("Fleck factor out of bounds / non-positive temperature in material state") from ex
         raise
-    if early is not None:
-        early.synchronize()  # done long before the comb
-    if t_up is not None:
-        t_up.synchronize()
     t_post = _time.perf_counter()
     pre_comb = eng.spare  # the tracked (pre-comb) bank after the swap
     if not use_scalar_intensity_Tr:

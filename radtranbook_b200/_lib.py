@@ -178,6 +178,11 @@ SIGNATURES = {
                                    c_uint64, c_void_p, c_int32, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "imc_mg_report_fields": (c_int, [POINTER(ImcMesh), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                      c_void_p, c_void_p, c_void_p]),
+    "imc_mg_report_to_host": (c_int, [POINTER(ImcMesh)] + [c_void_p] * 13),
+    "imc_fields_to_host": (c_int, [POINTER(ImcMesh), c_void_p, c_int32, c_void_p, c_void_p, c_void_p]),
+    "imc_fields_from_host": (c_int, [POINTER(ImcMesh), c_void_p, c_int32, c_void_p, c_void_p]),
+    "imc_copy_record": (c_int, [c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
+    "imc_bank_moments": (c_int, [POINTER(ImcMesh), POINTER(ImcBank), c_void_p, c_void_p, c_void_p]),
     "imc_bank_energy_by_bin": (c_int, [POINTER(ImcMesh), POINTER(ImcBank), c_void_p, c_int32, c_void_p,
                                        c_void_p]),
     "imc_phase_times": (c_int, [POINTER(ctypes.c_float), POINTER(ctypes.c_float)]),

@@ -534,6 +534,79 @@ cudaError_t imc_launch_mg_report(const ReportArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// Cell fields to or from the reference's order, the grid side contiguous across a warp (it may be
+// pinned host memory).  A step's e, T and Tr reach the host in one launch, where stacking,
+// transposing and copying them took eight calls and 86 us of the host.
+template <bool TO_GRID>
+__global__ void k_fields(FieldsArgs a) {
+  pdl_wait();     // the previous kernel of the stream has completed
+  pdl_trigger();  // the next one may be scheduled
+  const int nc = a.nx * a.ny;
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= nc) return;
+  const int i = r / a.ny, j = r - i * a.ny;
+  const int c = i + a.nx * j;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (k >= a.n) break;
+    if (TO_GRID) a.grid[(size_t)k * nc + r] = a.flat[k][c];
+    else a.flat[k][c] = a.grid[(size_t)k * nc + r];
+  }
+}
+
+cudaError_t imc_launch_fields(const FieldsArgs& a, bool to_grid, cudaStream_t s) {
+  ++g_imc_launches;
+  const unsigned blocks = (unsigned)((a.nx * a.ny + 255) / 256);
+  if (to_grid) IMC_LAUNCH_PDL(k_fields<true>, blocks, 256, 0, s, a);
+  else IMC_LAUNCH_PDL(k_fields<false>, blocks, 256, 0, s, a);
+  return cudaGetLastError();
+}
+
+// Energy and w mu per bin over a bank's live entries, the warp's lanes grouped by bin (a census is
+// largely ordered by bin); k_moments_scale then turns the second into c sum(w mu) / V.
+__global__ void __launch_bounds__(256) k_moments(const float* w, const float* mu, const int* cell, const int* group,
+                                                 const int64_t* d_n, long long n_bound, int nc, int nb, double* out) {
+  pdl_wait();     // the previous kernel of the stream has completed
+  pdl_trigger();  // the next one may be scheduled
+  __shared__ WarpStage stages[8];
+  WarpStage* st = stages + (threadIdx.x >> 5);
+  const long long n = min((long long)*d_n, n_bound);
+  const long long base = (long long)blockIdx.x * 1024;
+  for (int q = 0; q < 1024; q += 256) {
+    const long long k = base + q + threadIdx.x;
+    const float wf = k < n ? w[k] : 0.f;
+    // (an overflowed comb leaves entries unwritten: whatever they hold stays out of the sums)
+    const int cl = wf > 0.f ? cell[k] : -1, g = wf > 0.f ? group[k] : -1;
+    const bool live = (unsigned)cl < (unsigned)nc && (unsigned)g < (unsigned)(nb / nc);
+    const int b = live ? cl + nc * g : 0;
+    warp_tally1(live, b, (double)wf, out, st);
+    warp_tally1(live, b, live ? (double)wf * (double)mu[k] : 0.0, out + nb, st);
+  }
+}
+__global__ void k_moments_scale(const double* vol, int nc, int nb, double* out) {
+  pdl_wait();     // the previous kernel of the stream has completed
+  pdl_trigger();  // the next one may be scheduled
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < nb) out[nb + b] = C_LIGHT * out[nb + b] / vol[b % nc];
+}
+
+cudaError_t imc_launch_moments(const float* w, const float* mu, const int* cell, const int* group, const int64_t* d_n,
+                               long long n_bound, int nc, int ng, const double* vol, double* out, cudaStream_t s) {
+  const int nb = nc * ng;
+  ZeroList z{};
+  z.add(out, sizeof(double) * 2 * (size_t)nb);
+  cudaError_t e = imc_launch_zero(z, s);
+  if (e != cudaSuccess) return e;
+  if (n_bound > 0) {
+    ++g_imc_launches;
+    IMC_LAUNCH_PDL(k_moments, (unsigned)((n_bound + 1023) / 1024), 256, 0, s, w, mu, cell, group, d_n, n_bound, nc, nb,
+                   out);
+  }
+  ++g_imc_launches;
+  IMC_LAUNCH_PDL(k_moments_scale, (unsigned)((nb + 255) / 256), 256, 0, s, vol, nc, nb, out);
+  return cudaGetLastError();
+}
+
 cudaError_t imc_launch_canon_sum_eV(const double* e, const double* vol, int nc, double* out, cudaStream_t s) {
   ++g_imc_launches;
   IMC_LAUNCH_PDL(k_canon_eV, 1, NT, 0, s, e, vol, nc, out);

@@ -853,6 +853,86 @@ imc_status imc_mg_report_fields(const imc_mesh* mesh, const double* si, const do
   return IMC_OK;
 }
 
+imc_status imc_mg_report_to_host(const imc_mesh* mesh, const double* si, const double* after, const double* e,
+                                 const double* T, const double* Tr, const double* boundary_group,
+                                 const double* escaped_group, double* out_dev, double* out_host, void* stream,
+                                 void* side, void* fork, void* done) {
+  if (!mesh || !out_dev || !out_host || (side && (!fork || !done))) return IMC_ERR_INVALID_ARG;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (side) {
+    IMC_CUDA(cudaEventRecord((cudaEvent_t)fork, s));
+    s = (cudaStream_t)side;
+    IMC_CUDA(cudaStreamWaitEvent(s, (cudaEvent_t)fork, 0));
+  }
+  const imc_status st = imc_mg_report_fields(mesh, si, after, e, T, Tr, boundary_group, escaped_group, out_dev, s);
+  if (st != IMC_OK) return st;
+  // the written stretches: [0, G nc) si, [G nc, 2G nc) after, the rest
+  const size_t gnc = (size_t)mesh->nx * mesh->ny * mesh->n_groups;
+  const size_t total = 2 * gnc + 3 * (size_t)mesh->nx * mesh->ny + 2 * (size_t)mesh->n_groups;
+  const bool rest = e || T || Tr || boundary_group || escaped_group;
+  size_t q = 0;
+  while (q < total) {
+    const bool part[3] = {si != nullptr, after != nullptr, rest};
+    const size_t ends[3] = {gnc, 2 * gnc, total};
+    int k = q < gnc ? 0 : q < 2 * gnc ? 1 : 2;
+    if (!part[k]) { q = ends[k]; continue; }
+    size_t stop = ends[k];
+    while (k < 2 && part[k + 1]) stop = ends[++k];
+    IMC_CUDA(cudaMemcpyAsync(out_host + q, out_dev + q, sizeof(double) * (stop - q), cudaMemcpyDeviceToHost, s));
+    q = stop;
+  }
+  if (done) IMC_CUDA(cudaEventRecord((cudaEvent_t)done, s));
+  return IMC_OK;
+}
+
+imc_status imc_fields_to_host(const imc_mesh* mesh, const double* const* fields, int32_t n, double* out, void* done,
+                              void* stream) {
+  imc_status st = check_mesh(mesh);
+  if (st != IMC_OK) return st;
+  if (!fields || n < 1 || n > 4 || !out) return IMC_ERR_INVALID_ARG;
+  FieldsArgs fa{mesh->nx, mesh->ny, n, {}, out};
+  for (int k = 0; k < n; ++k) {
+    if (!fields[k]) return IMC_ERR_INVALID_ARG;
+    fa.flat[k] = const_cast<double*>(fields[k]);
+  }
+  IMC_CUDA(imc_launch_fields(fa, true, (cudaStream_t)stream));
+  if (done) IMC_CUDA(cudaEventRecord((cudaEvent_t)done, (cudaStream_t)stream));
+  return IMC_OK;
+}
+
+imc_status imc_fields_from_host(const imc_mesh* mesh, const double* src, int32_t n, double* const* fields,
+                                void* stream) {
+  imc_status st = check_mesh(mesh);
+  if (st != IMC_OK) return st;
+  if (!fields || n < 1 || n > 4 || !src) return IMC_ERR_INVALID_ARG;
+  FieldsArgs fa{mesh->nx, mesh->ny, n, {}, const_cast<double*>(src)};
+  for (int k = 0; k < n; ++k) {
+    if (!fields[k]) return IMC_ERR_INVALID_ARG;
+    fa.flat[k] = fields[k];
+  }
+  IMC_CUDA(imc_launch_fields(fa, false, (cudaStream_t)stream));
+  return IMC_OK;
+}
+
+imc_status imc_copy_record(void* dst, const void* src, size_t bytes, void* done, void* stream) {
+  if (!dst || !src || !done) return IMC_ERR_INVALID_ARG;
+  IMC_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, (cudaStream_t)stream));
+  IMC_CUDA(cudaEventRecord((cudaEvent_t)done, (cudaStream_t)stream));
+  return IMC_OK;
+}
+
+imc_status imc_bank_moments(const imc_mesh* mesh, const imc_bank* bank, const int64_t* n_dev, double* out,
+                            void* stream) {
+  imc_status st = check_mesh(mesh);
+  if (st != IMC_OK) return st;
+  if (mesh->ny != 1 || !bank || !bank->weight || !bank->dir1 || !bank->cell || !bank->group || !n_dev || !out ||
+      bank->capacity < 0)
+    return IMC_ERR_INVALID_ARG;
+  IMC_CUDA(imc_launch_moments(bank->weight, bank->dir1, bank->cell, bank->group, n_dev, bank->capacity, mesh->nx,
+                              std::max(1, mesh->n_groups), mesh->volume, out, (cudaStream_t)stream));
+  return IMC_OK;
+}
+
 imc_status imc_bank_energy_by_bin(const imc_mesh* mesh, const imc_bank* bank, const int64_t* n_dev,
                                   int32_t per_group, double* out, void* stream) {
   imc_status st = check_mesh(mesh);

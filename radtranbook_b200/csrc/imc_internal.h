@@ -214,6 +214,11 @@ struct ReportArgs {
   long long q0, q1;  // the entries of out written: [q0, q1), sections whose input is NULL skipped
 };
 cudaError_t imc_launch_mg_report(const ReportArgs& a, cudaStream_t s);
+// up to four cell fields between the flat order i + nx j and (nx, ny) C order
+struct FieldsArgs { int nx, ny, n; double* flat[4]; double* grid; };
+cudaError_t imc_launch_fields(const FieldsArgs& a, bool to_grid, cudaStream_t s);
+cudaError_t imc_launch_moments(const float* w, const float* mu, const int* cell, const int* group, const int64_t* d_n,
+                               long long n_bound, int nc, int ng, const double* vol, double* out, cudaStream_t s);
 
 // ---------------------------------------------------------------------------------
 // Source fill kernels (element count and first bank index read from device memory)

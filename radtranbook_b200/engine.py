@@ -64,14 +64,18 @@ class Bank:
             for k in self.FIELDS_F + ("cell",) + (("group",) if self.multigroup else ()):
                 getattr(self, k)[: self.size].copy_(old[k][: self.size])
         self.capacity = cap
+        self._c = ImcBank(_ptr(self.pos1), _ptr(self.pos2), _ptr(self.dir1), _ptr(self.dir2), _ptr(self.weight),
+                          _ptr(self.time), _ptr(self.cell), _ptr(self.group), 0, cap)
 
     def ensure(self, cap: int) -> None:
         if cap > self.capacity:
             self._alloc(int(cap * 1.25) + 1024)
 
     def c(self) -> ImcBank:
-        return ImcBank(_ptr(self.pos1), _ptr(self.pos2), _ptr(self.dir1), _ptr(self.dir2), _ptr(self.weight),
-                       _ptr(self.time), _ptr(self.cell), _ptr(self.group), self.size, self.capacity)
+        """The C view of the bank: one struct per bank (the pointers change only in _alloc), its
+        size and capacity as they are now."""
+        self._c.size, self._c.capacity = self.size, self.capacity
+        return self._c
 
     def view(self, name: str) -> torch.Tensor:
         return getattr(self, name)[: self.size]
@@ -159,6 +163,8 @@ class Engine:
                                      _ptr(self.boundary_group))
         self._census_dev_valid = False
         self._upper = 0
+        self._par_key = None
+        self._summary_queued = False
         mg = n_groups > 1
         self.bank = Bank(capacity, dev, mg)
         self.spare = Bank(capacity, dev, mg)
@@ -392,14 +398,28 @@ class Engine:
                                                 t_emit_floor=t_emit_floor, n_boundary_side=n_boundary_side,
                                                 method=method, cf_fastpath=cf_fastpath))
         self._mat = ImcMaterial(_ptr(T), _ptr(sigma), _ptr(cv), _ptr(source))
-        self._par = self._params(step, dt, theta, n_target, n_boundary, n_source, face_T, reflect, max_events,
-                                 rz_linear_source, t_emit_floor, n_boundary_side, method, cf_fastpath,
-                                 step_dev, dt_dev)
-        self._census_bins = 0
-        if self.fuse_census and not self.launch.get("event_based"):
-            self._census_bins = _lib.CENSUS_BY_GROUP_CELL if self.ng > 1 else _lib.CENSUS_BY_CELL
-        self._par.census_bins = self._census_bins
-        bound = int(self.lib.imc_source_bound(ctypes.byref(self.cmesh), ctypes.byref(self._par)))
+        # the parameter block of the last step again when only the step and dt differ (a time loop's
+        # steps: all that enters it besides is compared by value)
+        if n_boundary_side is not None:
+            n_boundary_side = tuple(n_boundary_side)
+        key = (theta, n_target, n_boundary, n_source, [_ptr(f) for f in face_T], tuple(reflect), max_events,
+               rz_linear_source, t_emit_floor, n_boundary_side, method,
+               cf_fastpath, _ptr(step_dev), _ptr(dt_dev), dict(self.launch), self._seed, self.id_base,
+               self.energy_share, _ptr(self.emission_fractions), self.fuse_census)
+        if key == self._par_key:
+            self._par.step, self._par.dt = int(step) & 0xFFFFFFFF, float(dt)
+        else:
+            self._par = self._params(step, dt, theta, n_target, n_boundary, n_source, face_T, reflect, max_events,
+                                     rz_linear_source, t_emit_floor, n_boundary_side, method, cf_fastpath,
+                                     step_dev, dt_dev)
+            self._par_bins = 0
+            if self.fuse_census and not self.launch.get("event_based"):
+                self._par_bins = _lib.CENSUS_BY_GROUP_CELL if self.ng > 1 else _lib.CENSUS_BY_CELL
+            self._par.census_bins = self._par_bins
+            self._par_bound = int(self.lib.imc_source_bound(ctypes.byref(self.cmesh), ctypes.byref(self._par)))
+            self._par_key = key
+        self._census_bins = self._par_bins
+        bound = self._par_bound
         self.bank.ensure(self.bank.size + bound)
         wsp, wsn = self._ws(self.bank.capacity)
         cb = self.bank.c()
@@ -420,6 +440,7 @@ class Engine:
         (with step_dev; n_max > 0 then sizes the spare bank); out_capacity: cap the combed census
         below the spare bank's capacity (a larger one is flagged as an overflow and the census
         is emptied); write_after: the energy after the comb per bin goes to comb_after."""
+        self._summary_queued = False
         self.spare.size = 0
         want = int(1.15 * n_max) if n_max > 0 else self._upper
         self.spare.ensure(want + 2 * self.nc * self.ng + 4096)
@@ -465,6 +486,17 @@ class Engine:
                                             self._stream())
         _lib.check("imc_bank_energy_by_bin", st)
 
+    def moments(self, bank: Bank, n_ptr: int) -> torch.Tensor:
+        """Queue imc_bank_moments of a 1-D bank whose entry count lies at n_ptr (device): a
+        (2, G, nc) tensor of the engine, energy and flux per (group, cell), rewritten by each call."""
+        m = self.__dict__.get("_moments")
+        if m is None:
+            m = self.__dict__["_moments"] = torch.empty((2, self.ng, self.nc), dtype=torch.float64, device=self.device)
+        cb = bank.c()
+        _lib.check("imc_bank_moments", self.lib.imc_bank_moments(
+            ctypes.byref(self.cmesh), ctypes.byref(cb), n_ptr, _ptr(m), self._stream()))
+        return m
+
     def side_stream(self) -> torch.cuda.Stream:
         """A second stream of the engine's device (created once): device-to-host copies of
         fields that are final before the comb run on it beside the comb."""
@@ -496,15 +528,62 @@ class Engine:
             _ptr(self.report_dev), self._stream()))
         return n
 
+    def mg_report_to_host(self, e, T, Tr, out: torch.Tensor, sections: str = "all", beside: bool = False) -> None:
+        """mg_report_fields, its sections copied on to the pinned `out` (the same layout), in one
+        call; beside: on the side stream after the work the current stream holds, with the
+        engine's "report" event recorded after the copies."""
+        self.report_buffer()
+        early, post = sections in ("all", "early"), sections in ("all", "post")
+        side = self.side_stream().cuda_stream if beside else None
+        _lib.check("imc_mg_report_to_host", self.lib.imc_mg_report_to_host(
+            ctypes.byref(self.cmesh), _ptr(self.si) if early else None, _ptr(self.comb_after) if post else None,
+            _ptr(e) if early else None, _ptr(T) if early else None, _ptr(Tr) if early else None,
+            _ptr(self.boundary_group) if early else None, _ptr(self.escaped_group) if early else None,
+            _ptr(self.report_dev), out.data_ptr(), self._stream(), side,
+            self.event("fork").cuda_event if beside else None, self.event("report").cuda_event if beside else None))
+
+    def event(self, name: str) -> "torch.cuda.Event":
+        """A persistent event of this engine by name, with its handle created."""
+        ev = self.__dict__.setdefault("_events", {}).get(name)
+        if ev is None:
+            ev = self._events[name] = torch.cuda.Event()
+            ev.record(torch.cuda.current_stream(self.device))
+        return ev
+
+    def fields_to_host(self, fields, out: torch.Tensor, done: "torch.cuda.Event | None" = None) -> None:
+        """Queue up to four cell fields (flat, device) into the pinned `out` in the reference's
+        order, and record `done`."""
+        p = (ctypes.c_void_p * len(fields))(*[f.data_ptr() for f in fields])
+        _lib.check("imc_fields_to_host", self.lib.imc_fields_to_host(
+            ctypes.byref(self.cmesh), p, len(fields), out.data_ptr(), None if done is None else done.cuda_event,
+            self._stream()))
+
+    def fields_from_host(self, src: torch.Tensor, fields) -> None:
+        """Queue up to four cell fields, one after the other in the pinned `src` in the reference's
+        order, into flat device fields.  src must not be refilled before the stream is past it."""
+        p = (ctypes.c_void_p * len(fields))(*[f.data_ptr() for f in fields])
+        _lib.check("imc_fields_from_host", self.lib.imc_fields_from_host(
+            ctypes.byref(self.cmesh), src.data_ptr(), len(fields), p, self._stream()))
+
+    def queue_summary(self) -> None:
+        """Queue the copy of the step summary to the host behind all that the step has queued: fetch()
+        then waits for it, so whatever the host does in between runs beside the device."""
+        _lib.check("imc_copy_record", self.lib.imc_copy_record(
+            self.summary_host.data_ptr(), self.summary_dev.data_ptr(), self.summary_host.numel(),
+            self.event("summary").cuda_event, self._stream()))
+        self._summary_queued = True
+
     def fetch(self, host_copies=()) -> ImcStepSummary:
-        """Copy the summary (and any (device, pinned host) pairs) to the host and synchronise.
-        A comb overflow is handled by growing the output bank and combing again (the input
-        bank is untouched by the comb)."""
+        """Copy the summary (and any (device, pinned host) pairs) to the host and wait for the
+        copies (queue_summary, or here).  A comb overflow is handled by growing the output bank and
+        combing again (the input bank is untouched by the comb)."""
         stream = torch.cuda.current_stream(self.device)
         for d, h in host_copies:
             h.copy_(d, non_blocking=True)
-        self.summary_host.copy_(self.summary_dev, non_blocking=True)
-        stream.synchronize()
+        if not self._summary_queued or host_copies:
+            self.queue_summary()
+        self._summary_queued = False
+        self.event("summary").synchronize()
         _lib.TRANSFER["d2h"] += self.summary_host.numel()
         sm = self.summary
         self.comb_repeated = False

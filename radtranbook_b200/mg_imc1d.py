@@ -26,7 +26,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._gray import GrayState, _host_copy, _staged, check_partition, face_temperatures
+from ._gray import GrayState, _host_copy, _pinned, _staged, check_partition, face_temperatures
 from .engine import A_RAD, C_LIGHT, Engine
 from .materials import evaluate, evaluate_groups
 from .mg_imc2d import planck_fractions
@@ -52,17 +52,11 @@ class SimulationState1DMG(GrayState):
 
 def _census_moments(eng: Engine) -> tuple[torch.Tensor, torch.Tensor]:
     """Per (group, cell) sums over the live census: energy (GJ) and radial flux
-    c * sum(w mu) / V (MG_IMC/MG_IMC1D.py:1209-1227), each (G, I)."""
-    G, nc = eng.ng, eng.nc
-    E = torch.zeros(G * nc, dtype=torch.float64, device=eng.device)
-    F = torch.zeros(G * nc, dtype=torch.float64, device=eng.device)
-    if eng.bank.size:
-        w = eng.bank.view("weight").double()
-        live = w > 0
-        idx = (eng.bank.view("cell").long() + nc * eng.bank.view("group").long())[live]
-        E.index_add_(0, idx, w[live])
-        F.index_add_(0, idx, (w * eng.bank.view("dir1").double())[live])
-    return E.view(G, nc), C_LIGHT * F.view(G, nc) / eng.vol.view(1, nc)
+    c * sum(w mu) / V (MG_IMC/MG_IMC1D.py:1209-1227), each (G, I): views of one buffer."""
+    n = torch.tensor([eng.bank.size], dtype=torch.int64, device=eng.device)
+    m = eng.moments(eng.bank, n.data_ptr())
+    torch.cuda.current_stream(eng.device).synchronize()  # n is read on the device
+    return m[0], m[1]
 
 
 def _comb_mode(conserve_comb_energy) -> str:
@@ -195,10 +189,17 @@ def step(state, Ntarget, Nboundary, Nsource, Nmax, T_boundary, dt, mesh, energy_
         state._e.add_(eng.disc.view(G, I).sum(0) / eng.vol)
     Tn = evaluate(inv_eos, state._e, lambda: _host_copy(state._e), like, **_staged(state, "T_new", I))
     state._T.copy_(Tn.reshape(-1))
-    copies = state.host_copies()
+    # the combed census' moments (its size is still on the device), the escaped energy by group,
+    # e, T and Tr reach the host with the step's one wait
+    moments = eng.moments(eng.spare, eng.summary_dev.data_ptr() + _lib.ImcStepSummary.n_out.offset)
+    hm = _pinned(state, "moments", (2 * I + 1) * G)
+    hm[:2 * G * I].copy_(moments.reshape(-1), non_blocking=True)
+    hm[2 * G * I:].copy_(eng.escaped_group, non_blocking=True)
+    state.report()
+    eng.queue_summary()
     ms_src, ms_tr = eng.phase_times()  # waits for the tracking only (the comb still runs)
     try:
-        sm = eng.fetch(copies)
+        sm = eng.fetch()
     except _lib.ImcError as ex:
         if ex.status == 3:
             raise AssertionError("non-finite or non-positive material state") from ex
@@ -214,8 +215,16 @@ def step(state, Ntarget, Nboundary, Nsource, Nmax, T_boundary, dt, mesh, energy_
         state.refresh_host()
     else:
         state.take_host_copies()
-    rad_g, flux_g = _census_moments(eng)
-    sum_tensors(dist, [rad_g, flux_g])
+    hm = hm.numpy()
+    if eng.comb_repeated:  # the comb ran again after an overflow: the moments of its census
+        hm[:2 * G * I] = torch.stack(_census_moments(eng)).reshape(-1).cpu().numpy()
+    by_group = np.array(hm[:2 * G * I]).reshape(2, G, I)
+    loss_by_group = np.array(hm[2 * G * I:])
+    if dist is not None:
+        t = torch.as_tensor(by_group, device=eng.device)
+        sum_tensors(dist, [t])
+        by_group = t.cpu().numpy()
+    rad_g, flux_g = by_group[0], by_group[1]
     internal = float(sm.internal_energy)  # the same material state on every rank
     tot = summary_totals(dist, sm, eng.bank.size, eng.device)  # summed over the ranks of a partition
     rad = tot["rad"]
@@ -232,8 +241,8 @@ def step(state, Ntarget, Nboundary, Nsource, Nmax, T_boundary, dt, mesh, energy_
     dE = total - state.previous_total_energy
     residual = dE - boundary_emission + boundary_loss - source_emission
     closure = residual + (0.0 if mode == "material" else comb_disc)
-    state.__dict__["radiation_energy_by_group"] = rad_g.cpu().numpy().copy()
-    state.__dict__["radiation_flux_by_group"] = flux_g.cpu().numpy().copy()
+    state.__dict__["radiation_energy_by_group"] = rad_g
+    state.__dict__["radiation_flux_by_group"] = flux_g
     state.time = state.time + dt
     state.previous_total_energy = total
     state.count += 1
@@ -254,7 +263,7 @@ def step(state, Ntarget, Nboundary, Nsource, Nmax, T_boundary, dt, mesh, energy_
         "boundary_emission": boundary_emission,
         "N_boundary": n_boundary,
         "boundary_loss": boundary_loss,
-        "boundary_loss_by_group": eng.escaped_group.cpu().numpy().copy(),
+        "boundary_loss_by_group": loss_by_group,
         "source_emission": source_emission,
         "energy_residual": residual,
         "Nmax_next": (min(Nmax + Nmax_growth, Nmax_final) if Nmax_final is not None else Nmax + Nmax_growth)

@@ -166,22 +166,14 @@ def _report_buffers(state, eng: Engine, n: int) -> dict:
             "esc": buf[o + G:o + 2 * G]}
 
 
-def _report_early(state, eng: Engine) -> tuple:
+def _report_early(state, eng: Engine) -> dict:
     """Gather the report's sections that are final before the comb (all but the post-comb
     energies) and copy them into this step's host buffer on the engine's side stream, after
-    the work the current stream holds (the material update), so both run beside the comb.
-    Returns (the side stream's event after the copies, the buffer's parts)."""
-    G, nc = eng.ng, eng.nc
+    the work the current stream holds (the material update), so both run beside the comb; the
+    engine's "report" event is recorded after the copies.  Returns the buffer's parts."""
     hb = _report_buffers(state, eng, eng.report_buffer().numel())
-    side = eng.side_stream()
-    side.wait_stream(torch.cuda.current_stream(eng.device))
-    with torch.cuda.stream(side):
-        eng.mg_report_fields(state._e, state._T, state._Tr, sections="early")
-        hb["pre"].copy_(eng.report_dev[:G * nc], non_blocking=True)
-        hb["all"][2 * G * nc:].copy_(eng.report_dev[2 * G * nc:], non_blocking=True)
-    done = torch.cuda.Event()
-    done.record(side)
-    return done, hb
+    eng.mg_report_to_host(state._e, state._T, state._Tr, hb["all"], sections="early", beside=True)
+    return hb
 
 
 def _law_buffers(state, eng: Engine, sigma: torch.Tensor) -> tuple:
@@ -325,21 +317,21 @@ def step(state, Ntarget, Nboundary, Nsource, Nmax, T_boundary, dt, edges1, edges
     # every reported field in the reference's layout in one device buffer (one kernel), then
     # one copy into a fresh pinned buffer that the host arrays view
     if early is None:
-        hb = _report_buffers(state, eng, eng.mg_report_fields(state._e, state._T, state._Tr))
-        copies = [(eng.report_dev, hb["all"])]
+        hb = _report_buffers(state, eng, eng.report_buffer().numel())
+        eng.mg_report_to_host(state._e, state._T, state._Tr, hb["all"])
     else:
-        hb = early[1]
-        eng.mg_report_fields(None, None, None, sections="post")
-        copies = [(eng.report_dev[G * nc:2 * G * nc], hb["post"])]
+        hb = early
+        eng.mg_report_to_host(None, None, None, hb["all"], sections="post")
+    eng.queue_summary()
+    if early is not None:
+        eng.event("report").synchronize()  # done long before the comb
     ms_src, ms_tr = eng.phase_times()  # waits for the tracking only (the comb still runs)
     try:
-        sm = eng.fetch(copies)
+        sm = eng.fetch()
     except _lib.ImcError as ex:
         if ex.status == 3:
             raise AssertionError("non-finite or non-positive material state") from ex
         raise
-    if early is not None:
-        early[0].synchronize()  # done long before the comb
     if not use_scalar_intensity_Tr:
         pre = eng.spare
         acc = torch.zeros(G * nc, dtype=torch.float64, device=eng.device)
