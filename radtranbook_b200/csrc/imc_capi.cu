@@ -453,7 +453,7 @@ imc_status transport_async(const imc_mesh* mesh, const imc_material* mat, const 
     if (cap_hit) return IMC_ERR_EVENT_CAP;
   } else {
     IMC_CUDA(imc_launch_track(ta, mesh->geometry,
-                              TrackLaunch{block, bps, sm_count(), smem_cells, smem_tally, wide_ok}, s));
+                              TrackLaunch{block, bps, sm_count(), smem_cells, smem_tally, wide_ok, n_upper}, s));
   }
   if (pe.ok) { IMC_CUDA(cudaEventRecord(pe.e[2], s)); pe.recorded = true; }
   IMC_CUDA(imc_launch_tally_finalize(ta, s));

@@ -62,6 +62,7 @@ constexpr size_t kSmemPerBlock = 226 * 1024;  // dynamic shared memory of a wide
 struct TrackLaunch {
   int block, blocks_per_sm, sms;
   bool smem_cells, smem_tally, wide_ok;
+  long long n_bound;  // the bank holds no more entries than this
 };
 cudaError_t imc_launch_track(const TrackArgs& a, int geom, const TrackLaunch& l, cudaStream_t s);
 // Event-by-event tracking (reserved bit 3 of imc_step_params): scratch bytes for a bank of

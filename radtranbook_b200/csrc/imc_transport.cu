@@ -248,10 +248,69 @@ __device__ __forceinline__ void add_event_counts(const TrackArgs& a, const unsig
 // event): the same ten launches 14.5 ms at 1, 13.2 at 4, 12.6 at 8, 12.6 at 12.
 constexpr int kRefillMin = 8;
 constexpr int kWideThreads = 1024;
-enum : int { T_GLOBAL = 0, T_SMALL, T_WIDE };
+enum : int { T_GLOBAL = 0, T_SMALL, T_WIDE, T_HASH };
+constexpr bool wide_block(int tally) { return tally == T_WIDE || tally == T_HASH; }
+
+// T_HASH, for meshes past T_WIDE: one wide block per SM keeps the sums of the (group, cell) entries
+// its histories touch in an open table in shared memory (deposition, and census energy for the comb).
+// An entry takes the first free of kHashProbes slots; one that finds none adds to global memory.
+// With T_GLOBAL the adds of every warp meet at the few entries where the radiation is, and the L2
+// slices that hold those serve one add after another, loads of other warps waiting behind them: a
+// ten-group crooked pipe (126 thousand entries, 2.1 M histories of 1.2 events) spent 255 us a launch
+// at 19 % of its issue slots, 56 MB of DRAM traffic.  So, an SM adds once per entry and launch:
+// 16 launches 3.12 -> 1.45 ms, 2 M particles a step 9.2 -> 3.1 ms; one group, 200 x 400 cells, 2 M
+// particles 21.6 -> 17.5 ms (20.6 with 4096 slots), 140 x 210 cells, 500 thousand 4.2 -> 3.2 ms.
+// It takes its start and end (164 KB cleared, then read) to earn: below a history or two per lane
+// T_GLOBAL's smaller blocks are as fast or faster (200 x 400 cells at 30 thousand particles a step
+// 0.92 against 1.04 ms, 100 thousand 1.65 against 1.70, 200 thousand 2.61 against 2.40).
+constexpr int kHashSlots = 8192, kHashProbes = 4;
+constexpr uint32_t kHashPerLane = 2;  // histories per lane from which T_HASH is taken
+struct HashTally {
+  unsigned long long* dep;
+  double* cen;
+  int* key;
+};
+__device__ __forceinline__ HashTally hash_tally(void* p) {
+  unsigned long long* d = static_cast<unsigned long long*>(p);
+  double* c = reinterpret_cast<double*>(d + kHashSlots);
+  return HashTally{d, c, reinterpret_cast<int*>(c + kHashSlots)};
+}
+__device__ __forceinline__ int hash_slot(const HashTally& t, int entry) {
+  const unsigned h = ((unsigned)entry * 2654435761u) >> 8;
+#pragma unroll 1
+  for (int p = 0; p < kHashProbes; ++p) {
+    const int q = (int)((h + (unsigned)p) & (unsigned)(kHashSlots - 1));
+    int k = *(volatile int*)(t.key + q);
+    if (k == entry) return q;
+    if (k == -1) {
+      k = atomicCAS(t.key + q, -1, entry);
+      if (k == -1 || k == entry) return q;
+    }
+  }
+  return -1;
+}
+// Census energy of the warp's lanes (all call it), grouped by entry first: the table's FP64 add is a
+// compare-and-swap loop, which lanes of one entry would take in turn.
+__device__ __forceinline__ void hash_census(const HashTally& t, bool flush, int entry, double v, double* global,
+                                            WarpStage* st) {
+  if (__ballot_sync(FULL, flush) == 0u) return;
+  const int lane = threadIdx.x & 31;
+  const unsigned peers = __match_any_sync(FULL, flush ? entry : -1 - lane);
+  st->a[lane] = v;
+  __syncwarp();
+  if (flush && (__ffs(peers) - 1) == lane) {
+    double sum = 0.0;
+    unsigned m = peers;
+    while (m) { const int l = __ffs(m) - 1; m &= m - 1; sum += st->a[l]; }
+    const int q = hash_slot(t, entry);
+    if (q >= 0) atomicAdd(t.cen + q, sum);
+    else atomicAdd(global + entry, sum);
+  }
+  __syncwarp();
+}
 
 template <int GEOM, bool SMEM_CELLS, bool MG, bool CF, int TALLY>
-__global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY == T_WIDE ? 1 : 4) k_track(TrackArgs a) {
+__global__ void __launch_bounds__(wide_block(TALLY) ? kWideThreads : 256, wide_block(TALLY) ? 1 : 4) k_track(TrackArgs a) {
   pdl_wait();     // the previous kernel of the stream has completed
   pdl_trigger();  // the next one may be scheduled
   const float dtk = a.dt_dev ? (float)*a.dt_dev : a.dt;  // graph replay: step length and Philox
@@ -278,6 +337,9 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
     for (int q = threadIdx.x; q < ncg; q += blockDim.x) CS[q] = a.sass[q];
   if (TD_S) for (int q = threadIdx.x; q < ncg; q += blockDim.x) TD[q] = 0ull;
   if (TS_S) for (int q = threadIdx.x; q < ncg; q += blockDim.x) TS[q] = 0.0;
+  const HashTally HT = hash_tally(TD);
+  if (TALLY == T_HASH)
+    for (int q = threadIdx.x; q < kHashSlots; q += blockDim.x) { HT.dep[q] = 0ull; HT.cen[q] = 0.0; HT.key[q] = -1; }
   if (threadIdx.x < B_N) blk_cnt[threadIdx.x] = 0u;
   if (threadIdx.x < 4) blk_esc[threadIdx.x] = 0ull;
   __syncthreads();
@@ -318,7 +380,9 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
       int cen_bin = 0;
       if (pend) { cen = history_retire<GEOM>(a, h, cen_bin); s_ev += h.ev; }
       if (a.ecen) {
-        warp_tally1(cen, cen_bin, (double)h.w, a.ecen, st);
+        // (the table's entries are (group, cell): a multigroup census summed by cell alone goes past it)
+        if (TALLY == T_HASH && (!MG || a.ecen_by_group)) hash_census(HT, cen, cen_bin, (double)h.w, a.ecen, st);
+        else warp_tally1(cen, cen_bin, (double)h.w, a.ecen, st);
         n_alive += cen ? 1u : 0u;
       }
       pend = false;
@@ -407,7 +471,14 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
     const double vs = (double)o.wd;
     if (TD_S && ud) smem_add_u64(TD + o.cell, ud);
     if (TS_S && o.wd != 0.f) atomicAdd(TS + o.cell, vs);
-    if (TALLY == T_GLOBAL) warp_tally_fx(ud != 0ull || o.wd != 0.f, o.cell, ud, vs, a.dep_fx, a.si, st);
+    if (TALLY == T_HASH) {
+      if (ud) {
+        const int q = hash_slot(HT, o.cell);
+        if (q >= 0) smem_add_u64(HT.dep + q, ud);
+        else atomicAdd(a.dep_fx + o.cell, ud);
+      }
+      warp_tally1(o.wd != 0.f, o.cell, vs, a.si, st);
+    } else if (TALLY == T_GLOBAL) warp_tally_fx(ud != 0ull || o.wd != 0.f, o.cell, ud, vs, a.dep_fx, a.si, st);
     else if (!TD_S) warp_tally_fx(ud != 0ull, o.cell, ud, 0.0, a.dep_fx, a.si, st);
     else if (!TS_S) warp_tally1(o.wd != 0.f, o.cell, vs, a.si, st);
   }
@@ -419,6 +490,13 @@ __global__ void __launch_bounds__(TALLY == T_WIDE ? kWideThreads : 256, TALLY ==
   }
   add_event_counts(a, blk_cnt, blk_esc, s_ev, s_cen, s_sc);
   // the block's tallies (every warp's last flush is behind the __syncthreads above)
+  if (TALLY == T_HASH)
+    for (int q = threadIdx.x; q < kHashSlots; q += blockDim.x) {
+      const int e = HT.key[q];
+      if (e < 0) continue;
+      if (HT.dep[q]) atomicAdd(a.dep_fx + e, HT.dep[q]);
+      if (HT.cen[q] != 0.0) atomicAdd(a.ecen + e, HT.cen[q]);
+    }
   if (TD_S) for (int q = threadIdx.x; q < ncg; q += blockDim.x) if (TD[q]) atomicAdd(a.dep_fx + q, TD[q]);
   if (TS_S) for (int q = threadIdx.x; q < ncg; q += blockDim.x) if (TS[q] != 0.0) atomicAdd(a.si + q, TS[q]);
 }
@@ -454,6 +532,12 @@ cudaError_t launch_geom(const TrackArgs& a, const TrackLaunch& l, cudaStream_t s
     if (sm && track_smem(a, wide, true, 1) <= kSmemPerBlock)
       return launch_sized(k_track<GEOM, true, MG, CF, T_WIDE>, a, wide, l.sms, track_smem(a, wide, true, 1), s);
     return launch_sized(k_track<GEOM, false, MG, CF, T_WIDE>, a, wide, l.sms, track_smem(a, wide, false, 1), s);
+  }
+  if constexpr (!CF) {
+    const size_t sh = track_smem(a, wide, false, 0) + 20 * (size_t)kHashSlots;
+    if (!st && l.wide_ok && block <= 256 && sh <= kSmemPerBlock &&
+        l.n_bound >= (long long)kHashPerLane * l.sms * wide)
+      return launch_sized(k_track<GEOM, false, MG, CF, T_HASH>, a, wide, l.sms, sh, s);
   }
   if (sm && st) return launch_sized(k_track<GEOM, true, MG, CF, T_SMALL>, a, block, grid, track_smem(a, block, true, 2), s);
   return sm ? launch_sized(k_track<GEOM, true, MG, CF, T_GLOBAL>, a, block, grid, track_smem(a, block, true, 0), s)
