@@ -85,19 +85,14 @@ __global__ void __launch_bounds__(256) k_comb_ecen(CombArgs a) {
 }
 
 // copies of one entry: floor(w / ew + xi), xi its comb uniform (word k % 4 of Philox block
-// (k / 4, 1, step, TAG_COMB), k the pre-comb index).  The quotient is formed in FP32 first, off
-// by at most 1e-6 of itself; only where that leaves the floor open is it divided in FP64.
+// (k / 4, 1, step, TAG_COMB), k the pre-comb index)
 __device__ __forceinline__ int comb_copies(const CombArgs& a, float wf, int bk, bool compact, uint32_t xw, int& b) {
   b = 0;
   if (!(wf > 0.f) || !bin_ok(a, bk)) return 0;
   b = bk;
   if (compact) return 1;
   const double ew = a.ew[b];
-  if (!(ew > 0.0)) return 0;
-  const float s = __fdividef(wf, (float)ew) + u01f(xw);
-  const float fl = floorf(s), fr = s - fl, open = 1e-6f * (s + 1.f);
-  if (s < 4e6f && fr > open && fr < 1.f - open) return (int)fl;  // false for an infinite or NaN quotient
-  return (int)floor((double)wf / ew + u01d(xw));
+  return ew > 0.0 ? comb_floor(wf, ew, xw) : 0;
 }
 
 // Copies per entry, per tile and per bin.  A block takes `per` consecutive tiles, its warps

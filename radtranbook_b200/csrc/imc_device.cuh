@@ -292,9 +292,8 @@ __device__ __forceinline__ void counts_init(BlockCounts<S>& t) {
   for (int i = threadIdx.x; i < S; i += blockDim.x) { t.key[i] = -1; t.val[i] = 0u; }
 }
 
-template <int S>
-__device__ __forceinline__ void counts_add(BlockCounts<S>& t, int bin, unsigned v,
-                                           unsigned long long* __restrict__ global) {
+template <int S, typename G>
+__device__ __forceinline__ void counts_add(BlockCounts<S>& t, int bin, unsigned v, G* __restrict__ global) {
   const unsigned h = ((unsigned)bin * 2654435761u) >> 8;
 #pragma unroll 1
   for (int p = 0; p < BINS_PROBES; ++p) {
@@ -302,13 +301,23 @@ __device__ __forceinline__ void counts_add(BlockCounts<S>& t, int bin, unsigned 
     const int old = atomicCAS(&t.key[s], -1, bin);
     if (old == -1 || old == bin) { atomicAdd(&t.val[s], v); return; }
   }
-  atomicAdd(global + bin, (unsigned long long)v);
+  atomicAdd(global + bin, (G)v);
 }
 
-template <int S>
-__device__ __forceinline__ void counts_flush(BlockCounts<S>& t, unsigned long long* __restrict__ global) {
+template <int S, typename G>
+__device__ __forceinline__ void counts_flush(BlockCounts<S>& t, G* __restrict__ global) {
   for (int i = threadIdx.x; i < S; i += blockDim.x)
-    if (t.key[i] >= 0) atomicAdd(global + t.key[i], (unsigned long long)t.val[i]);
+    if (t.key[i] >= 0) atomicAdd(global + t.key[i], (G)t.val[i]);
+}
+
+// Comb copies of an entry of weight wf in a bin of comb weight ew > 0: floor(w / ew + xi), xi the
+// uniform of the Philox word xw.  The quotient is formed in FP32 first, off by at most 1e-6 of itself;
+// only where that leaves the floor open is it divided in FP64.
+__device__ __forceinline__ int comb_floor(float wf, double ew, uint32_t xw) {
+  const float s = __fdividef(wf, (float)ew) + u01f(xw);
+  const float fl = floorf(s), fr = s - fl, open = 1e-6f * (s + 1.f);
+  if (s < 4e6f && fr > open && fr < 1.f - open) return (int)fl;  // false for an infinite or NaN quotient
+  return (int)floor((double)wf / ew + u01d(xw));
 }
 
 // ---- energy tallies in 64-bit fixed point ----
