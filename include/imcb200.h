@@ -407,6 +407,23 @@ IMC_API imc_status imc_fields_to_host(const imc_mesh* mesh, const double* const*
                                       void* done, void* stream);
 IMC_API imc_status imc_fields_from_host(const imc_mesh* mesh, const double* src, int32_t n, double* const* fields,
                                         void* stream);
+/* A device loop's step bookkeeping, in one launch at the step's end (everything on the device): the
+ * step summary into row k of hist_sum; with slot k = out_slot[k] < n_out, T and Tr (and by group Eg)
+ * into row slot of the snapshots; T and Tr (and by group Eg, group-major) of the fiducial cells into
+ * row k of the histories; then k + 1 to k, and the next step's dt, step counter and comb target from
+ * the schedules (left as they are behind the last of n_steps).  k_ticket: [0] k, [1] 0 between steps.
+ * Eg, snap_Eg and hist_Eg: multigroup only, else NULL. */
+typedef struct {
+  int64_t n_steps, n_out;
+  const double* dt_sched; const int32_t* step_sched; const int64_t* nmax_sched; const int64_t* out_slot;
+  double* dt; int32_t* step; int64_t* nmax; int64_t* k_ticket;
+  const imc_step_summary* summary; imc_step_summary* hist_sum;
+  const double* T; const double* Tr; const double* Eg;
+  double* snap_T; double* snap_Tr; double* snap_Eg;
+  const int64_t* fid; int64_t n_fid;
+  double* hist_T; double* hist_Tr; double* hist_Eg;
+} imc_loop_record;
+IMC_API imc_status imc_loop_record_async(const imc_mesh* mesh, const imc_loop_record* rec, void* stream);
 /* An asynchronous copy of bytes from src to dst (device or pinned host) and `done` (an event)
  * recorded after it. */
 IMC_API imc_status imc_copy_record(void* dst, const void* src, size_t bytes, void* done, void* stream);

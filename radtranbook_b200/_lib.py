@@ -120,6 +120,13 @@ class ImcStepSummary(ctypes.Structure):
     ]
 
 
+class ImcLoopRecord(ctypes.Structure):
+    _fields_ = [("n_steps", c_int64), ("n_out", c_int64)] + [(k, c_void_p) for k in (
+        "dt_sched", "step_sched", "nmax_sched", "out_slot", "dt", "step", "nmax", "k_ticket", "summary", "hist_sum",
+        "T", "Tr", "Eg", "snap_T", "snap_Tr", "snap_Eg", "fid")] + [("n_fid", c_int64)] + [
+        (k, c_void_p) for k in ("hist_T", "hist_Tr", "hist_Eg")]
+
+
 # name -> (restype, argtypes); every symbol declared in include/imcb200.h
 # batched 1-D slab problems
 (BL_TOTAL, BL_PREV, BL_INTERNAL, BL_RADIATION, BL_BOUNDARY, BL_ESCAPED, BL_EMISSION, BL_COMB_DISC, BL_CLOSURE,
@@ -181,6 +188,7 @@ SIGNATURES = {
     "imc_mg_report_to_host": (c_int, [POINTER(ImcMesh)] + [c_void_p] * 13),
     "imc_fields_to_host": (c_int, [POINTER(ImcMesh), c_void_p, c_int32, c_void_p, c_void_p, c_void_p]),
     "imc_fields_from_host": (c_int, [POINTER(ImcMesh), c_void_p, c_int32, c_void_p, c_void_p]),
+    "imc_loop_record_async": (c_int, [POINTER(ImcMesh), POINTER(ImcLoopRecord), c_void_p]),
     "imc_copy_record": (c_int, [c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "imc_bank_moments": (c_int, [POINTER(ImcMesh), POINTER(ImcBank), c_void_p, c_void_p, c_void_p]),
     "imc_bank_energy_by_bin": (c_int, [POINTER(ImcMesh), POINTER(ImcBank), c_void_p, c_int32, c_void_p,

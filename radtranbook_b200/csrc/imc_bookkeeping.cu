@@ -534,6 +534,54 @@ cudaError_t imc_launch_mg_report(const ReportArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// The bookkeeping of a step in a captured loop (imc_loop_record): bound by launches, nine indexed copies
+// of a few doubles each before (20 us of a 230 us step), one kernel now.  The last block to finish
+// moves k on: a ticket, no block waits.
+__global__ void __launch_bounds__(256) k_loop_record(imc_loop_record r, int nc, int ng) {
+  pdl_wait();     // the previous kernel of the stream has completed
+  pdl_trigger();  // the next one may be scheduled
+  const long long k = r.k_ticket[0];
+  if (k < 0 || k >= r.n_steps) return;  // block-uniform
+  const long long slot = r.out_slot[k];
+  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+  if (slot >= 0 && slot < r.n_out) {
+    for (size_t c = first; c < (size_t)nc; c += stride) {
+      r.snap_T[(size_t)slot * nc + c] = r.T[c];
+      r.snap_Tr[(size_t)slot * nc + c] = r.Tr[c];
+    }
+    const size_t ncg = (size_t)nc * ng;
+    if (r.Eg) for (size_t c = first; c < ncg; c += stride) r.snap_Eg[(size_t)slot * ncg + c] = r.Eg[c];
+  }
+  constexpr size_t kWords = sizeof(imc_step_summary) / 8;
+  static_assert(sizeof(imc_step_summary) % 8 == 0, "the summary is copied in 8-byte words");
+  if (first < kWords)
+    reinterpret_cast<long long*>(r.hist_sum + k)[first] = reinterpret_cast<const long long*>(r.summary)[first];
+  for (size_t f = first; f < (size_t)r.n_fid; f += stride) {
+    const size_t c = (size_t)r.fid[f];
+    r.hist_T[(size_t)k * r.n_fid + f] = r.T[c];
+    r.hist_Tr[(size_t)k * r.n_fid + f] = r.Tr[c];
+    if (r.Eg)
+      for (int g = 0; g < ng; ++g) r.hist_Eg[((size_t)k * ng + g) * r.n_fid + f] = r.Eg[(size_t)g * nc + c];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    const unsigned long long t = atomicAdd(reinterpret_cast<unsigned long long*>(r.k_ticket + 1), 1ull);
+    if (t == gridDim.x - 1ull) {
+      r.k_ticket[1] = 0;
+      r.k_ticket[0] = k + 1;
+      if (k + 1 < r.n_steps) { *r.dt = r.dt_sched[k + 1]; *r.step = r.step_sched[k + 1]; *r.nmax = r.nmax_sched[k + 1]; }
+    }
+  }
+}
+
+cudaError_t imc_launch_loop_record(const imc_loop_record& r, int nc, int ng, cudaStream_t s) {
+  ++g_imc_launches;
+  const unsigned blocks = (unsigned)std::min(64, std::max(1, (nc * (r.Eg ? ng : 1) + 1023) / 1024));
+  IMC_LAUNCH_PDL(k_loop_record, blocks, 256, 0, s, r, nc, ng);
+  return cudaGetLastError();
+}
+
 // Cell fields to or from the reference's order, the grid side contiguous across a warp (it may be
 // pinned host memory).  A step's e, T and Tr reach the host in one launch, where stacking,
 // transposing and copying them took eight calls and 86 us of the host.

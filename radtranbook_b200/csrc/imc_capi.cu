@@ -914,6 +914,18 @@ imc_status imc_fields_from_host(const imc_mesh* mesh, const double* src, int32_t
   return IMC_OK;
 }
 
+imc_status imc_loop_record_async(const imc_mesh* mesh, const imc_loop_record* rec, void* stream) {
+  imc_status st = check_mesh(mesh);
+  if (st != IMC_OK) return st;
+  if (!rec || !rec->dt_sched || !rec->step_sched || !rec->nmax_sched || !rec->out_slot || !rec->dt || !rec->step ||
+      !rec->nmax || !rec->k_ticket || !rec->summary || !rec->hist_sum || !rec->T || !rec->Tr || rec->n_steps < 1 ||
+      rec->n_out < 0 || (rec->n_out > 0 && (!rec->snap_T || !rec->snap_Tr || (rec->Eg && !rec->snap_Eg))) ||
+      rec->n_fid < 0 || (rec->n_fid > 0 && (!rec->fid || !rec->hist_T || !rec->hist_Tr || (rec->Eg && !rec->hist_Eg))))
+    return IMC_ERR_INVALID_ARG;
+  IMC_CUDA(imc_launch_loop_record(*rec, mesh->nx * mesh->ny, std::max(1, mesh->n_groups), (cudaStream_t)stream));
+  return IMC_OK;
+}
+
 imc_status imc_copy_record(void* dst, const void* src, size_t bytes, void* done, void* stream) {
   if (!dst || !src || !done) return IMC_ERR_INVALID_ARG;
   IMC_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, (cudaStream_t)stream));

@@ -215,6 +215,7 @@ struct ReportArgs {
   long long q0, q1;  // the entries of out written: [q0, q1), sections whose input is NULL skipped
 };
 cudaError_t imc_launch_mg_report(const ReportArgs& a, cudaStream_t s);
+cudaError_t imc_launch_loop_record(const imc_loop_record& r, int nc, int ng, cudaStream_t s);
 // up to four cell fields between the flat order i + nx j and (nx, ny) C order
 struct FieldsArgs { int nx, ny, n; double* flat[4]; double* grid; };
 cudaError_t imc_launch_fields(const FieldsArgs& a, bool to_grid, cudaStream_t s);

@@ -37,7 +37,7 @@ import torch
 
 from . import _lib
 from ._gray import _law, _same, face_temperatures
-from .engine import C_LIGHT
+from .engine import C_LIGHT, _ptr
 from .materials import GroupedOpacity, evaluate, evaluate_groups, is_device
 
 
@@ -137,6 +137,8 @@ class DeviceLoop:
             fid = [int(i) + nx * int(j) for i, j in fiducial_cells]
         else:
             fid = [int(i) for i in fiducial_cells]
+        if any(c < 0 or c >= eng.nc for c in fid):
+            raise ValueError("a fiducial cell lies outside the mesh")
         self.fid = torch.as_tensor(np.asarray(fid, dtype=np.int64), device=dev)
         self.cap_census = int(census_margin * self.nmax_top) + 2 * eng.nc * eng.ng + 4096
         self.step_dev = torch.zeros(1, dtype=torch.int32, device=dev)
@@ -145,17 +147,15 @@ class DeviceLoop:
         self.k_done = 0  # steps run so far (the Nmax schedule continues across run() calls)
         if self.mg:
             self.rad_last = torch.zeros(eng.ng * eng.nc, dtype=torch.float64, device=dev)
-        self.k_dev = torch.zeros(1, dtype=torch.int64, device=dev)
+        self.k_dev = torch.zeros(2, dtype=torch.int64, device=dev)  # the run's step index, the record's ticket
         self._cap = (0, -1)   # (steps, outputs) the history buffers hold
         self._graphs = {}     # (id of the bank holding the census, steps per graph) -> graph
 
     # ------------------------------------------------------------------ one captured step
     def _enqueue_step(self) -> None:
         st, eng, kw = self.state, self.eng, self.kw
-        # prologue: this step's dt and Philox step counter
-        torch.index_select(self.dt_sched, 0, self.k_dev, out=self.dt_dev)
-        torch.index_select(self.step_sched, 0, self.k_dev, out=self.step_dev)
-        torch.index_select(self.nmax_sched, 0, self.k_dev, out=self.nmax_dev)
+        # (this step's dt, Philox step counter and comb target were set by run(), or by the last
+        # step's record)
         like = st.grid(st._T)
         if self.law is not None:
             sigma, cvv = self.law_sigma, self.law_cv
@@ -173,9 +173,6 @@ class DeviceLoop:
             eng.material_update(st._e, st._Tr)
         if self.mg:
             self.rad_last.copy_(eng.si)
-            if self.fid.numel():
-                at_fid = eng.si.view(eng.ng, eng.nc).index_select(1, self.fid)
-                self.hist_Eg.index_copy_(0, self.k_dev, at_fid.view(1, -1))
         eng.comb_async(self.nmax_top, 0, st._e, per_group=self.mg, step_dev=self.step_dev,
                        out_capacity=self.cap_census, n_max_dev=self.nmax_dev)
         if self.conserve:
@@ -183,17 +180,16 @@ class DeviceLoop:
         if self.law is None:
             Tn = evaluate(self.inv_eos, st.grid(st._e), _no_host, like)
             st._T.copy_(st.flat(Tn))
-        # epilogue: summary, fiducial temperatures, output snapshots
-        self.hist_sum.index_copy_(0, self.k_dev, eng.summary_dev.view(1, -1))
-        if self.fid.numel():
-            self.hist_T.index_copy_(0, self.k_dev, st._T.index_select(0, self.fid).view(1, -1))
-            self.hist_Tr.index_copy_(0, self.k_dev, st._Tr.index_select(0, self.fid).view(1, -1))
-        slot = torch.index_select(self.out_slot, 0, self.k_dev)
-        self.snap_T.index_copy_(0, slot, st._T.view(1, -1))
-        self.snap_Tr.index_copy_(0, slot, st._Tr.view(1, -1))
-        if self.mg:
-            self.snap_Eg.index_copy_(0, slot, self.rad_last.view(1, -1))
-        self.k_dev.add_(1)
+        # epilogue: summary, fiducial histories, output snapshots, the next step's schedule entries
+        rec = _lib.ImcLoopRecord(
+            self._cap[0], self._cap[1], _ptr(self.dt_sched), _ptr(self.step_sched), _ptr(self.nmax_sched),
+            _ptr(self.out_slot), _ptr(self.dt_dev), _ptr(self.step_dev), _ptr(self.nmax_dev), _ptr(self.k_dev),
+            _ptr(eng.summary_dev), _ptr(self.hist_sum), _ptr(st._T), _ptr(st._Tr),
+            _ptr(self.rad_last) if self.mg else None, _ptr(self.snap_T), _ptr(self.snap_Tr),
+            _ptr(self.snap_Eg) if self.mg else None, _ptr(self.fid), self.fid.numel(), _ptr(self.hist_T),
+            _ptr(self.hist_Tr), _ptr(self.hist_Eg) if self.mg else None)
+        _lib.check("imc_loop_record_async", eng.lib.imc_loop_record_async(
+            ctypes.byref(eng.cmesh), ctypes.byref(rec), eng._stream()))
         # the comb wrote the next census into the spare bank: swap (sizes stay upper bounds)
         eng.spare.size = self.cap_census
         eng.bank, eng.spare = eng.spare, eng.bank
@@ -296,6 +292,9 @@ class DeviceLoop:
         g2 = self._graph(2) if n >= 2 else None
         g1 = self._graph(1) if n % 2 else None
         self.k_dev.zero_()
+        self.dt_dev.copy_(self.dt_sched[:1])
+        self.step_dev.copy_(self.step_sched[:1])
+        self.nmax_dev.copy_(self.nmax_sched[:1])
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record()
         for _ in range(n // 2):
