@@ -43,11 +43,11 @@ B_SEG_2D = 72  # bytes per 2-D gray segment: 36-byte record loaded + stored
 B_SEG_2D_MG = 80  # 2-D multigroup: the 36-byte record plus the group index, loaded + stored
 B_SEG_1D = 56  # 1-D gray: a 28-byte record loaded + stored
 # DRAM bytes and warp instructions of the tracking kernel per segment on this workload, from
-# one full-size launch under ncu (dram__bytes_read.sum + dram__bytes_write.sum = 402.25 MB,
-# smsp__inst_executed.sum = 1.520 G, for 67.18 M segments); the histories stay in registers
+# one full-size launch under ncu (dram__bytes_read.sum + dram__bytes_write.sum = 401.50 MB,
+# smsp__inst_executed.sum = 0.988 G, for 67.17 M segments); the histories stay in registers
 # across their events, and the kernel is bound by instruction issue.
-DRAM_B_PER_SEG_MEASURED = 402.252544e6 / 67176386
-WARP_INST_PER_SEG_MEASURED = 1520147524 / 67176386
+DRAM_B_PER_SEG_MEASURED = 401.502208e6 / 67172504
+WARP_INST_PER_SEG_MEASURED = 988366300 / 67172504
 ISSUE_SLOTS_PER_CYCLE = 148 * 4  # SMs x warp schedulers, one warp instruction each per cycle
 
 

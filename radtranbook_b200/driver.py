@@ -6,11 +6,12 @@ step, with no host synchronisation between steps.
 The drivers' dt schedule depends only on (dt_initial, growth factor, dt_max, output times), not
 on the solution, so it is computed on the host first (adaptive_schedule) and written to device
 memory.  A two-step graph is captured once (its two steps alternate the double-buffered bank):
-a prologue reads this step's dt and Philox step counter from the schedule into device
-scalars that every kernel reads at run time (imc_step_params.step_dev / dt_dev,
-imc_comb_async_dev), then the step itself (device material callables, sources, tracking,
-material update, comb), then an epilogue copies the step summary, the fiducial temperatures
-and (at output steps) the temperature fields into device history buffers.  The graph is
+every kernel reads its step's dt and Philox step counter from device scalars at run time
+(imc_step_params.step_dev / dt_dev, imc_comb_async_dev); the step itself (device material
+callables, sources, tracking, material update, comb) is followed by one record kernel
+(imc_loop_record_async): the step summary, the fiducial temperatures and (at output steps) the
+temperature fields go into device history buffers, the next step's dt, counter and comb target
+from the schedule into the scalars.  The graph is
 replayed n/2 times (a one-step graph finishes an odd count); one synchronisation at the end
 brings the histories back, and the FP64 energy ledger of every step is rebuilt from the
 stored summaries exactly as the eager step builds it.
