@@ -368,15 +368,19 @@ def gray_step(state: GrayState, *, Ntarget, Nboundary, Nsource, Nmax, T_boundary
         hp = state._hpin.numpy()
         Tn = np.asarray(inv_eos(hp[:n].reshape(shape)), dtype=np.float64)
         T_ref = hp[n:2 * n].reshape(shape)
-        np.copyto(T_ref, Tn)
+
+        def put(dst, values):  # a field in the reference's layout, or a scalar
+            np.copyto(dst.reshape(shape), np.broadcast_to(np.asarray(values, dtype=np.float64), shape))
+
+        put(T_ref, Tn)
         stage = _pinned(state, "up", 3 * n)
         up = stage.numpy()
-        np.copyto(up[:n].reshape(shape), Tn)
+        put(up[:n], Tn)
         dst = [state._T]
         if not is_device(sigma_a_func) and not is_device(cv):
             sig_n, cv_n = _device_field(state, "sigma", n), _device_field(state, "cv", n)
-            np.copyto(up[n:2 * n].reshape(shape), sigma_a_func(T_ref))
-            np.copyto(up[2 * n:].reshape(shape), cv(T_ref))
+            put(up[n:2 * n], sigma_a_func(T_ref))
+            put(up[2 * n:], cv(T_ref))
             dst += [sig_n, cv_n]
             state.__dict__["_host_next"] = ((sigma_a_func, cv), state.count + 1, sig_n, cv_n)
         eng.fields_from_host(stage, dst)

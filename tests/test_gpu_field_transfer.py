@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 import torch
 
+from radtranbook_b200 import imc2d, problems
 from radtranbook_b200.engine import C_LIGHT, Engine
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +55,24 @@ def test_bank_moments(cuda, n, nc, G):
         ref = np.bincount(b, v, nc * G).reshape(G, nc) * scale
         mag = np.bincount(b, np.abs(v), nc * G).reshape(G, nc) * scale
         assert np.all(np.abs(got[k] - ref) <= (n + 3) * 2.0 ** -53 * mag)
+
+
+def test_host_callables_may_return_anything_array_like(cuda):
+    """Object arrays, lists and scalars from host material callables give the float arrays' steps: the same
+    histories, temperatures to the order of the FP64 weight sum (1e-12 after three steps)."""
+    out = []
+    for wrap in (lambda x: x, lambda x: x.astype(object), lambda x: x.tolist()):
+        p = problems.crooked_pipe(nr=9, nz=20)
+        st = imc2d.init_simulation(2000, p["Tinit"], p["Tr_init"], p["edges1"], p["edges2"], p["eos_host"],
+                                   p["inv_eos_host"], geometry="rz")
+        sig = lambda T: wrap(np.asarray(p["sigma_host"](T)))  # noqa: E731, B023
+        inv = lambda e: wrap(np.asarray(p["inv_eos_host"](e)))  # noqa: E731, B023
+        cv = lambda T: wrap(np.broadcast_to(p["cv_host"](T), T.shape).copy())  # noqa: E731, B023
+        for _ in range(3):
+            st, info = imc2d.step(st, 1500, 1500, 0, 6000, p["T_boundary"], p["dt"], p["edges1"], p["edges2"], sig, inv,
+                                  cv, p["source"], reflect=p["reflect"], geometry="rz",
+                                  boundary_source_func=p["boundary_source_func"])
+        out.append((st.temperature.copy(), info["profiling"]["transport_events"]["total"]))
+    for T, ev in out[1:]:
+        assert ev == out[0][1]
+        np.testing.assert_allclose(T, out[0][0], rtol=1e-12)
