@@ -189,21 +189,22 @@ __global__ void __launch_bounds__(WIDE ? kAdjWide : 256, WIDE ? 1 : 4) k_adjoint
   }
 }
 
+template <auto Kernel>
+cudaError_t launch_replay(const AdjointArgs& a, int grid, int block, size_t sh, cudaStream_t s) {
+  const cudaError_t e = smem_opt_in<Kernel>(sh);
+  if (e != cudaSuccess) return e;
+  Kernel<<<grid, block, sh, s>>>(a);
+  return cudaGetLastError();
+}
+
 template <int GEOM>
 cudaError_t launch_adj(const AdjointArgs& a, int block, int bps, int sms, cudaStream_t s) {
   k_adjoint_tables<<<(a.t.nc + 255) / 256, 256, 0, s>>>(a);
   const size_t edges = sizeof(float2) * (a.t.nx + a.t.ny);
   const size_t wide_sh = edges + sizeof(double) * (size_t)a.t.nc;
-  const bool wide = block <= 256 && wide_sh <= kSmemPerBlock;
-  auto kernel = wide ? k_adjoint<GEOM, true> : k_adjoint<GEOM, false>;
-  const size_t sh = wide ? wide_sh : edges + (size_t)(block / 32) * sizeof(WarpStage);
-  if (sh > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    if (e != cudaSuccess) return e;
-  }
-  if (wide) kernel<<<sms, std::max(128, std::min(kAdjWide, block * bps)) & ~31, sh, s>>>(a);
-  else kernel<<<sms * bps, block, sh, s>>>(a);
-  return cudaGetLastError();
+  if (block <= 256 && wide_sh <= kSmemPerBlock)
+    return launch_replay<k_adjoint<GEOM, true>>(a, sms, std::max(128, std::min(kAdjWide, block * bps)) & ~31, wide_sh, s);
+  return launch_replay<k_adjoint<GEOM, false>>(a, sms * bps, block, edges + (size_t)(block / 32) * sizeof(WarpStage), s);
 }
 
 }  // namespace

@@ -20,6 +20,7 @@
 #include <cstring>
 #include "imc_batch.h"
 #include "imc_event.cuh"
+#include "imc_internal.h"
 #include "imc_sample.cuh"
 
 using namespace imcdev;
@@ -795,19 +796,15 @@ cudaError_t imc_batch_launch_track(const BatchArgs& a, int block, int grid, cuda
   ++g_imc_launches;
   if (a.form != 2 && a.max_cells > 0 && a.max_cells <= IMC_BATCH_SMEM_CELLS) {
     const size_t sh = units_smem(a.max_cells);
-    if (sh > 48 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(k_btrack_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-      if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = smem_opt_in<k_btrack_units>(sh);
+    if (e != cudaSuccess) return e;
     const long long blocks = std::max(1LL, (long long)grid * block / kUnitThreads);
     k_btrack_units<<<(unsigned)blocks, kUnitThreads, sh, s>>>(a);
     return cudaGetLastError();
   }
   const size_t sh = (size_t)(block / 32) * sizeof(WarpStage) + pref_bytes(a);
-  if (sh > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(k_btrack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = smem_opt_in<k_btrack>(sh);
+  if (e != cudaSuccess) return e;
   k_btrack<<<grid, block, sh, s>>>(a);
   return cudaGetLastError();
 }
@@ -821,13 +818,11 @@ cudaError_t imc_batch_launch_comb_ecen(const BatchArgs& a, cudaStream_t s) {
 cudaError_t imc_batch_launch_comb_copy(const BatchArgs& a, cudaStream_t s) {
   const int g = (int)std::min<long long>(std::max<long long>(a.max_tiles, 1), (long long)sm_count() * 8);
   const size_t sh = pref_bytes(a) + scatter_bytes();
-  if (sh > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(k_bcomb_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    if (e != cudaSuccess) return e;
-  }
+  cudaError_t e = smem_opt_in<k_bcomb_scatter>(sh);
+  if (e != cudaSuccess) return e;
   g_imc_launches += 4;
   k_bcomb_count<<<g, kCombThreads, pref_bytes(a), s>>>(a);
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_bcomb_scan<<<1, 1024, 0, s>>>(a);
   e = cudaGetLastError();

@@ -457,10 +457,8 @@ cudaError_t imc_launch_plan(const PlanArgs& a, cudaStream_t s) {
   IMC_LAUNCH_PDL(k_plan_cells, (std::max(a.nc, std::max(a.nx, a.ny) + 1) + 255) / 256, 256, 0, s, a);
   const size_t cnt = sizeof(int) * (size_t)a.nc;
   const bool smem_cnt = cnt <= 200 * 1024;
-  if (smem_cnt && cnt > 32 * 1024) {  // beside the kernel's own 8 KB
-    const cudaError_t e = cudaFuncSetAttribute(k_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cnt);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = smem_opt_in<k_plan>(smem_cnt ? cnt : 0);
+  if (e != cudaSuccess) return e;
   IMC_LAUNCH_PDL(k_plan, 2, NT, smem_cnt ? cnt : 0, s, a, smem_cnt ? 1 : 0);
   return cudaGetLastError();
 }
@@ -1061,24 +1059,22 @@ __global__ void __launch_bounds__(NT) k_ic_plan_mg(IcMgArgs a) {
 
 // Launch shape of the per-cell multigroup plan: as many cells a block as leave one
 // (cell, group edge) pair per thread (the edge integrals are the long part; at most 32 cells),
-// two doubles per pair and cell of shared memory; above 48 KB the kernel is opted in to more.
-template <typename K>
-cudaError_t launch_plan_cells(K kernel, const PlanMgArgs& a, cudaStream_t s) {
+// two doubles per pair and cell of shared memory.
+template <auto Kernel>
+cudaError_t launch_plan_cells(const PlanMgArgs& a, cudaStream_t s) {
   const long long E = (long long)a.ng + 1;
   const int cb = (int)std::max(1LL, std::min(32LL, 256LL / E));
   const size_t smem = (size_t)2 * cb * (E + 1) * sizeof(double);
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = smem_opt_in<Kernel>(smem);
+  if (e != cudaSuccess) return e;
   const int blocks = (a.nc + cb - 1) / cb;
-  IMC_LAUNCH_PDL(kernel, blocks, 256, smem, s, a, cb);
+  IMC_LAUNCH_PDL(Kernel, blocks, 256, smem, s, a, cb);
   return cudaSuccess;
 }
 
 cudaError_t imc_launch_plan_mg(const PlanMgArgs& a, cudaStream_t s) {
   g_imc_launches += 2;
-  const cudaError_t e = launch_plan_cells(k_plan_mg_cells<false>, a, s);
+  const cudaError_t e = launch_plan_cells<k_plan_mg_cells<false>>(a, s);
   if (e != cudaSuccess) return e;
   IMC_LAUNCH_PDL(k_plan_mg, 2, NT, 0, s, a);
   return cudaGetLastError();
@@ -1086,7 +1082,7 @@ cudaError_t imc_launch_plan_mg(const PlanMgArgs& a, cudaStream_t s) {
 
 cudaError_t imc_launch_plan_mg1d(const PlanMgArgs& a, cudaStream_t s) {
   g_imc_launches += 2;
-  const cudaError_t e = launch_plan_cells(k_plan_mg_cells<true>, a, s);
+  const cudaError_t e = launch_plan_cells<k_plan_mg_cells<true>>(a, s);
   if (e != cudaSuccess) return e;
   IMC_LAUNCH_PDL(k_plan_mg1d, 1, NT, 0, s, a);
   return cudaGetLastError();

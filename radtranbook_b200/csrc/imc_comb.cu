@@ -362,10 +362,8 @@ cudaError_t imc_launch_comb_count(const CombArgs& a, cudaStream_t s) {
   const size_t dense = sizeof(unsigned) * (size_t)a.nb;
   if (a.n_bound >= (1LL << 19) && dense <= 100 * 1024) {
     int per = (int)std::min<long long>(kCountMaxTiles, std::max<long long>(4, (ntiles + 295) / 296));
-    if (dense > 48 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(k_comb_count<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dense);
-      if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = smem_opt_in<k_comb_count<true>>(dense);
+    if (e != cudaSuccess) return e;
     IMC_LAUNCH_PDL(k_comb_count<true>, (unsigned)((ntiles + per - 1) / per), 512, dense, s, a, ntiles, per);
   } else {
     const int per = 1, threads = 32 * (TILE / WARP_ENTRIES);

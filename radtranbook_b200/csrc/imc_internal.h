@@ -5,10 +5,34 @@
 // upper bounds used to size grids, and every kernel reads its true element count from the
 // summary, so a whole step runs without a host round trip.
 #pragma once
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "../../include/imcb200.h"
+
+// Lets a launch of Kernel take `smem` bytes of dynamic shared memory.  The limit is the function's,
+// not the launch's, so it is raised once per device, to all that a block may have beside the
+// kernel's static bytes, and never set to one launch's size: two host threads on meshes of
+// different sizes would lower it between the other's two calls.  Launches that stay under 48 KB
+// with any of these kernels' static bytes (at most 9 KB) need no opt-in.
+constexpr size_t kSmemNoOptIn = 32 * 1024;
+template <auto Kernel>
+cudaError_t smem_opt_in(size_t smem) {
+  if (smem <= kSmemNoOptIn) return cudaSuccess;
+  static std::atomic<unsigned long long> done{0ull};  // devices it has been raised on
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  cudaFuncAttributes at{};
+  if ((e = cudaFuncGetAttributes(&at, Kernel)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
+}
 
 // ---------------------------------------------------------------------------------
 // Tracking

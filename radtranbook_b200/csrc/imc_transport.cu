@@ -509,13 +509,11 @@ inline size_t track_smem(const TrackArgs& a, int block, bool cells, int tallies)
   return sh + 8ull * tallies * a.nc * a.ng;
 }
 
-template <typename K>
-cudaError_t launch_sized(K kernel, const TrackArgs& a, int block, int grid, size_t sh, cudaStream_t s) {
-  if (sh > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    if (e != cudaSuccess) return e;
-  }
-  IMC_LAUNCH_PDL(kernel, grid, block, sh, s, a);
+template <auto Kernel>
+cudaError_t launch_sized(const TrackArgs& a, int block, int grid, size_t sh, cudaStream_t s) {
+  const cudaError_t e = smem_opt_in<Kernel>(sh);
+  if (e != cudaSuccess) return e;
+  IMC_LAUNCH_PDL(Kernel, grid, block, sh, s, a);
   return cudaGetLastError();
 }
 
@@ -530,18 +528,18 @@ cudaError_t launch_geom(const TrackArgs& a, const TrackLaunch& l, cudaStream_t s
   const int wide = std::max(128, std::min(kWideThreads, block * l.blocks_per_sm)) & ~31;
   if (!st && l.wide_ok && block <= 256 && track_smem(a, wide, false, 1) <= kSmemPerBlock) {
     if (sm && track_smem(a, wide, true, 1) <= kSmemPerBlock)
-      return launch_sized(k_track<GEOM, true, MG, CF, T_WIDE>, a, wide, l.sms, track_smem(a, wide, true, 1), s);
-    return launch_sized(k_track<GEOM, false, MG, CF, T_WIDE>, a, wide, l.sms, track_smem(a, wide, false, 1), s);
+      return launch_sized<k_track<GEOM, true, MG, CF, T_WIDE>>(a, wide, l.sms, track_smem(a, wide, true, 1), s);
+    return launch_sized<k_track<GEOM, false, MG, CF, T_WIDE>>(a, wide, l.sms, track_smem(a, wide, false, 1), s);
   }
   if constexpr (!CF) {
     const size_t sh = track_smem(a, wide, false, 0) + 20 * (size_t)kHashSlots;
     if (!st && l.wide_ok && block <= 256 && sh <= kSmemPerBlock &&
         l.n_bound >= (long long)kHashPerLane * l.sms * wide)
-      return launch_sized(k_track<GEOM, false, MG, CF, T_HASH>, a, wide, l.sms, sh, s);
+      return launch_sized<k_track<GEOM, false, MG, CF, T_HASH>>(a, wide, l.sms, sh, s);
   }
-  if (sm && st) return launch_sized(k_track<GEOM, true, MG, CF, T_SMALL>, a, block, grid, track_smem(a, block, true, 2), s);
-  return sm ? launch_sized(k_track<GEOM, true, MG, CF, T_GLOBAL>, a, block, grid, track_smem(a, block, true, 0), s)
-            : launch_sized(k_track<GEOM, false, MG, CF, T_GLOBAL>, a, block, grid, track_smem(a, block, false, 0), s);
+  if (sm && st) return launch_sized<k_track<GEOM, true, MG, CF, T_SMALL>>(a, block, grid, track_smem(a, block, true, 2), s);
+  return sm ? launch_sized<k_track<GEOM, true, MG, CF, T_GLOBAL>>(a, block, grid, track_smem(a, block, true, 0), s)
+            : launch_sized<k_track<GEOM, false, MG, CF, T_GLOBAL>>(a, block, grid, track_smem(a, block, false, 0), s);
 }
 
 // ---------------------------------------------------------------------------------
@@ -670,10 +668,8 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
 template <int GEOM, bool MG, bool CF>
 cudaError_t launch_event(const TrackArgs& a, const EventScratch& e, int cur, int block, int grid, cudaStream_t s) {
   const size_t sh = (block / 32) * sizeof(WarpStage) + sizeof(float2) * (a.nx + a.ny);
-  if (sh > 48 * 1024) {
-    cudaError_t err = cudaFuncSetAttribute(k_event<GEOM, MG, CF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    if (err != cudaSuccess) return err;
-  }
+  const cudaError_t err = smem_opt_in<k_event<GEOM, MG, CF>>(sh);
+  if (err != cudaSuccess) return err;
   k_event<GEOM, MG, CF><<<grid, block, sh, s>>>(a, e, cur);
   return cudaGetLastError();
 }
