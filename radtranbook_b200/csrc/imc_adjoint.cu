@@ -52,7 +52,8 @@ __global__ void k_adjoint_tables(AdjointArgs A) {
 // pass, are loaded kAdjRefillMin at a time.  Both passes of 4e6 histories on 128 x 128 cells:
 // 3.5 ms, against 6.4 ms with the global tally, the factors formed per visit (two FP64 divisions)
 // and a lane reloaded whenever it ends.
-template <int GEOM, bool WIDE>
+// EDGES: the edges are staged in shared memory (else, on a long mesh, read through L1).
+template <int GEOM, bool WIDE, bool EDGES>
 __global__ void __launch_bounds__(WIDE ? kAdjWide : 256, WIDE ? 1 : 4) k_adjoint(AdjointArgs A) {
   const TrackArgs& a = A.t;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -60,8 +61,10 @@ __global__ void __launch_bounds__(WIDE ? kAdjWide : 256, WIDE ? 1 : 4) k_adjoint
   float2* E1 = reinterpret_cast<float2*>(smem + (WIDE ? 0 : sizeof(WarpStage) * (blockDim.x >> 5)));
   float2* E2 = E1 + a.nx;
   double* G = reinterpret_cast<double*>(E2 + a.ny);  // WIDE: [nc]
-  for (int q = threadIdx.x; q < a.nx; q += blockDim.x) E1[q] = make_float2(a.e1[q], a.e1[q + 1]);
-  for (int q = threadIdx.x; q < a.ny; q += blockDim.x) E2[q] = make_float2(a.e2[q], a.e2[q + 1]);
+  if (EDGES) {
+    for (int q = threadIdx.x; q < a.nx; q += blockDim.x) E1[q] = make_float2(a.e1[q], a.e1[q + 1]);
+    for (int q = threadIdx.x; q < a.ny; q += blockDim.x) E2[q] = make_float2(a.e2[q], a.e2[q + 1]);
+  }
   if (WIDE) for (int q = threadIdx.x; q < a.nc; q += blockDim.x) G[q] = 0.0;
   __syncthreads();
 
@@ -132,7 +135,8 @@ __global__ void __launch_bounds__(WIDE ? kAdjWide : 256, WIDE ? 1 : 4) k_adjoint
       } else {
         const U4 r = draw_next(a.rk, key, rkx, ev);
         ++ev;
-        const Flight f = next_flight<GEOM, true>(E1[ci], E2[cj], ss, x, y, u, v, dcen, r);
+        const Flight f = next_flight<GEOM, true>(cell_edges<EDGES>(E1, a.e1, ci), cell_edges<EDGES>(E2, a.e2, cj), ss,
+                                                 x, y, u, v, dcen, r);
         const float wn = w * __expf(-sa * f.d);
         const double dd = (double)w - (double)wn;  // exact
         const double ac = __ldg(A.score + c);
@@ -200,11 +204,14 @@ cudaError_t launch_replay(const AdjointArgs& a, int grid, int block, size_t sh, 
 template <int GEOM>
 cudaError_t launch_adj(const AdjointArgs& a, int block, int bps, int sms, cudaStream_t s) {
   k_adjoint_tables<<<(a.t.nc + 255) / 256, 256, 0, s>>>(a);
-  const size_t edges = sizeof(float2) * (a.t.nx + a.t.ny);
+  const size_t edges = sizeof(float2) * ((size_t)a.t.nx + a.t.ny), stages = (size_t)(block / 32) * sizeof(WarpStage);
   const size_t wide_sh = edges + sizeof(double) * (size_t)a.t.nc;
   if (block <= 256 && wide_sh <= kSmemPerBlock)
-    return launch_replay<k_adjoint<GEOM, true>>(a, sms, std::max(128, std::min(kAdjWide, block * bps)) & ~31, wide_sh, s);
-  return launch_replay<k_adjoint<GEOM, false>>(a, sms * bps, block, edges + (size_t)(block / 32) * sizeof(WarpStage), s);
+    return launch_replay<k_adjoint<GEOM, true, true>>(a, sms, std::max(128, std::min(kAdjWide, block * bps)) & ~31,
+                                                      wide_sh, s);
+  if (edges + stages <= kSmemPerBlock)
+    return launch_replay<k_adjoint<GEOM, false, true>>(a, sms * bps, block, edges + stages, s);
+  return launch_replay<k_adjoint<GEOM, false, false>>(a, sms * bps, block, stages, s);
 }
 
 }  // namespace

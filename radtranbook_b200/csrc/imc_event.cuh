@@ -28,6 +28,13 @@ __device__ __forceinline__ float scatter_flight(float ss, float L, uint32_t x, f
   return BIGF;
 }
 
+// The (lower, upper) edges of cell i along one direction: from a shared-memory table of pairs, or from
+// the edges themselves through L1.
+template <bool STAGED>
+__device__ __forceinline__ float2 cell_edges(const float2* staged, const float* e, int i) {
+  return STAGED ? staged[i] : make_float2(__ldg(e + i), __ldg(e + i + 1));
+}
+
 struct Flight {
   float d;           // path length
   int evt;           // EV_*

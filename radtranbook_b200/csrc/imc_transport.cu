@@ -60,7 +60,8 @@ struct EvOut {
   bool finished;   // the history ended: history_retire stores its final state
 };
 
-template <int GEOM, bool SMEM_CELLS, bool MG, bool CF>
+// EDGES: E1, E2 hold the edges in shared memory (else they are read from the FP32 copies through L1)
+template <int GEOM, bool SMEM_CELLS, bool MG, bool CF, bool EDGES>
 __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut& o, const float2* E1,
                                               const float2* E2, const float2* CS, unsigned* blk_cnt,
                                               unsigned long long* blk_esc, unsigned long long* dep_t,
@@ -83,8 +84,9 @@ __device__ __forceinline__ void history_event(const TrackArgs& a, Hist& h, EvOut
     finished = true;
   } else {
     ++h.ev;
-    const Flight f = next_flight<GEOM, !MG2>(E1[h.ci], ONED ? make_float2(0.f, 0.f) : E2[h.cj], ss, x, y, u, v, h.dcen,
-                                             r);
+    const float2 e1 = cell_edges<EDGES>(E1, a.e1, h.ci);
+    const float2 e2 = ONED ? make_float2(0.f, 0.f) : cell_edges<EDGES>(E2, a.e2, h.cj);
+    const Flight f = next_flight<GEOM, !MG2>(e1, e2, ss, x, y, u, v, h.dcen, r);
     const float d = f.d;
     const int evt = f.evt, di = f.di, dj = f.dj;
     // implicit capture (the energy removed is counted at the flush, w_in - w)
@@ -248,7 +250,9 @@ __device__ __forceinline__ void add_event_counts(const TrackArgs& a, const unsig
 // event): the same ten launches 14.5 ms at 1, 13.2 at 4, 12.6 at 8, 12.6 at 12.
 constexpr int kRefillMin = 8;
 constexpr int kWideThreads = 1024;
-enum : int { T_GLOBAL = 0, T_SMALL, T_WIDE, T_HASH };
+//   T_LONG    as T_GLOBAL, on a mesh so long that its edges alone overfill a block's shared memory
+//             (8 bytes a cell: from 28 thousand cells in one direction): they stay in global memory
+enum : int { T_GLOBAL = 0, T_SMALL, T_WIDE, T_HASH, T_LONG };
 constexpr bool wide_block(int tally) { return tally == T_WIDE || tally == T_HASH; }
 
 // T_HASH, for meshes past T_WIDE: one wide block per SM keeps the sums of the (group, cell) entries
@@ -327,12 +331,15 @@ __global__ void __launch_bounds__(wide_block(TALLY) ? kWideThreads : 256, wide_b
   float2* E1 = reinterpret_cast<float2*>(stages + nwarps);  // (lower, upper) edge per index
   float2* E2 = E1 + a.nx;
   float2* CS = E2 + a.ny;
+  constexpr bool EDGES = TALLY != T_LONG;
   const int ncg = a.nc * a.ng;
   unsigned long long* TD = reinterpret_cast<unsigned long long*>(CS + (SMEM_CELLS ? ncg : 0));
   double* TS = reinterpret_cast<double*>(TD + (TD_S ? ncg : 0));
   unsigned long long* const dep_t = TD_S ? TD : a.dep_fx;
-  for (int q = threadIdx.x; q < a.nx; q += blockDim.x) E1[q] = make_float2(a.e1[q], a.e1[q + 1]);
-  for (int q = threadIdx.x; q < a.ny; q += blockDim.x) E2[q] = make_float2(a.e2[q], a.e2[q + 1]);
+  if (EDGES) {
+    for (int q = threadIdx.x; q < a.nx; q += blockDim.x) E1[q] = make_float2(a.e1[q], a.e1[q + 1]);
+    for (int q = threadIdx.x; q < a.ny; q += blockDim.x) E2[q] = make_float2(a.e2[q], a.e2[q + 1]);
+  }
   if (SMEM_CELLS)
     for (int q = threadIdx.x; q < ncg; q += blockDim.x) CS[q] = a.sass[q];
   if (TD_S) for (int q = threadIdx.x; q < ncg; q += blockDim.x) TD[q] = 0ull;
@@ -446,8 +453,9 @@ __global__ void __launch_bounds__(wide_block(TALLY) ? kWideThreads : 256, wide_b
       for (int rep = 0; rep < kEvents; ++rep) {
         EvOut o{0, false, 0.f, 0.0, false};
         if (has) {
-          history_event<GEOM, SMEM_CELLS, MG, CF>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t,
-                                                  draw_next(a.rk, h.key, rkx, h.ev), weight_floor, inv_q, s_cen, s_sc);
+          history_event<GEOM, SMEM_CELLS, MG, CF, true>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t,
+                                                        draw_next(a.rk, h.key, rkx, h.ev), weight_floor, inv_q, s_cen,
+                                                        s_sc);
           if (o.finished) { has = false; pend = true; }
         }
         __syncwarp();  // the warp together again: lanes left apart run the next event one by one
@@ -460,8 +468,9 @@ __global__ void __launch_bounds__(wide_block(TALLY) ? kWideThreads : 256, wide_b
     }
     EvOut o{0, false, 0.f, 0.0, false};
     if (has) {
-      history_event<GEOM, SMEM_CELLS, MG, CF>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t,
-                                              draw_next(a.rk, h.key, rkx, h.ev), weight_floor, inv_q, s_cen, s_sc);
+      history_event<GEOM, SMEM_CELLS, MG, CF, EDGES>(a, h, o, E1, E2, CS, blk_cnt, blk_esc, dep_t,
+                                                     draw_next(a.rk, h.key, rkx, h.ev), weight_floor, inv_q, s_cen,
+                                                     s_sc);
       if (o.finished) { has = false; pend = true; }
     }
     // ---------------- tallies ----------------
@@ -478,7 +487,7 @@ __global__ void __launch_bounds__(wide_block(TALLY) ? kWideThreads : 256, wide_b
         else atomicAdd(a.dep_fx + o.cell, ud);
       }
       warp_tally1(o.wd != 0.f, o.cell, vs, a.si, st);
-    } else if (TALLY == T_GLOBAL) warp_tally_fx(ud != 0ull || o.wd != 0.f, o.cell, ud, vs, a.dep_fx, a.si, st);
+    } else if (TALLY == T_GLOBAL || TALLY == T_LONG) warp_tally_fx(ud != 0ull || o.wd != 0.f, o.cell, ud, vs, a.dep_fx, a.si, st);
     else if (!TD_S) warp_tally_fx(ud != 0ull, o.cell, ud, 0.0, a.dep_fx, a.si, st);
     else if (!TS_S) warp_tally1(o.wd != 0.f, o.cell, vs, a.si, st);
   }
@@ -503,8 +512,9 @@ __global__ void __launch_bounds__(wide_block(TALLY) ? kWideThreads : 256, wide_b
 
 // dynamic shared memory of the tracking kernels: per-warp staging, edges, the cell table and
 // `tallies` 8-byte block tallies per (group, cell)
+inline size_t stage_smem(int block) { return (size_t)(block / 32) * sizeof(WarpStage); }
 inline size_t track_smem(const TrackArgs& a, int block, bool cells, int tallies) {
-  size_t sh = (block / 32) * sizeof(WarpStage) + sizeof(float2) * (a.nx + a.ny);
+  size_t sh = stage_smem(block) + sizeof(float2) * ((size_t)a.nx + a.ny);
   if (cells) sh += sizeof(float2) * a.nc * a.ng;
   return sh + 8ull * tallies * a.nc * a.ng;
 }
@@ -517,11 +527,17 @@ cudaError_t launch_sized(const TrackArgs& a, int block, int grid, size_t sh, cud
   return cudaGetLastError();
 }
 
-// T_SMALL is built only with the shared-memory cell table (small meshes)
+// T_SMALL is built only with the shared-memory cell table (small meshes).  Tallies or a table that were
+// asked for and fit by themselves, but not beside a long mesh's edges, are left in global memory.
 template <int GEOM, bool MG, bool CF = false>
 cudaError_t launch_geom(const TrackArgs& a, const TrackLaunch& l, cudaStream_t s) {
   const int block = l.block, grid = l.sms * l.blocks_per_sm;
-  const bool sm = l.smem_cells, st = l.smem_tally;
+  const size_t edges = track_smem(a, block, false, 0) - stage_smem(block);
+  auto fits = [&](bool cells, int tallies) { return track_smem(a, block, cells, tallies) <= kSmemPerBlock; };
+  auto asked = [&](bool cells, int tallies) {  // (what cannot fit without the edges fails at the launch)
+    return fits(cells, tallies) || track_smem(a, block, cells, tallies) - edges > kSmemPerBlock;
+  };
+  const bool sm = l.smem_cells, st = l.smem_tally && asked(true, 2);
   // One wide block per SM holding as many threads as the requested shape keeps resident there,
   // when its tally fits; the cell table beside it if that fits too (else it is read through L1,
   // which measured the same on the crooked pipe).
@@ -538,8 +554,11 @@ cudaError_t launch_geom(const TrackArgs& a, const TrackLaunch& l, cudaStream_t s
       return launch_sized<k_track<GEOM, false, MG, CF, T_HASH>>(a, wide, l.sms, sh, s);
   }
   if (sm && st) return launch_sized<k_track<GEOM, true, MG, CF, T_SMALL>>(a, block, grid, track_smem(a, block, true, 2), s);
-  return sm ? launch_sized<k_track<GEOM, true, MG, CF, T_GLOBAL>>(a, block, grid, track_smem(a, block, true, 0), s)
-            : launch_sized<k_track<GEOM, false, MG, CF, T_GLOBAL>>(a, block, grid, track_smem(a, block, false, 0), s);
+  if (sm && asked(true, 0))
+    return launch_sized<k_track<GEOM, true, MG, CF, T_GLOBAL>>(a, block, grid, track_smem(a, block, true, 0), s);
+  if (fits(false, 0))
+    return launch_sized<k_track<GEOM, false, MG, CF, T_GLOBAL>>(a, block, grid, track_smem(a, block, false, 0), s);
+  return launch_sized<k_track<GEOM, false, MG, CF, T_LONG>>(a, block, grid, stage_smem(block), s);
 }
 
 // ---------------------------------------------------------------------------------
@@ -581,7 +600,7 @@ __global__ void k_event_init(TrackArgs a, EventScratch e) {
   }
 }
 
-template <int GEOM, bool MG, bool CF>
+template <int GEOM, bool MG, bool CF, bool EDGES>
 __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int cur) {
   const uint32_t stepk = a.step_dev ? *a.step_dev : a.step;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -591,8 +610,10 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
   const int nwarps = blockDim.x >> 5;
   float2* E1 = reinterpret_cast<float2*>(stages + nwarps);
   float2* E2 = E1 + a.nx;
-  for (int q = threadIdx.x; q < a.nx; q += blockDim.x) E1[q] = make_float2(a.e1[q], a.e1[q + 1]);
-  for (int q = threadIdx.x; q < a.ny; q += blockDim.x) E2[q] = make_float2(a.e2[q], a.e2[q + 1]);
+  if (EDGES) {
+    for (int q = threadIdx.x; q < a.nx; q += blockDim.x) E1[q] = make_float2(a.e1[q], a.e1[q + 1]);
+    for (int q = threadIdx.x; q < a.ny; q += blockDim.x) E2[q] = make_float2(a.e2[q], a.e2[q + 1]);
+  }
   if (threadIdx.x < B_N) blk_cnt[threadIdx.x] = 0u;
   if (threadIdx.x < 4) blk_esc[threadIdx.x] = 0ull;
   __syncthreads();
@@ -639,8 +660,8 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
         h.tab = __ldg(a.sass + (MG ? c + a.nc * h.grp : c));
         h.key = draw_key(a.rk, a.id_base + pid, stepk, TAG_TRANSPORT);
         const uint32_t ev0 = h.ev;
-        history_event<GEOM, false, MG, CF>(a, h, o, E1, E2, nullptr, blk_cnt, blk_esc, a.dep_fx,
-                                           draw_next(a.rk, h.key, rkx, h.ev), weight_floor, inv_q, s_cen, s_sc);
+        history_event<GEOM, false, MG, CF, EDGES>(a, h, o, E1, E2, nullptr, blk_cnt, blk_esc, a.dep_fx,
+                                                  draw_next(a.rk, h.key, rkx, h.ev), weight_floor, inv_q, s_cen, s_sc);
         s_ev += h.ev - ev0;
         int bin;
         if (o.finished) history_retire<GEOM>(a, h, bin);
@@ -667,10 +688,14 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
 
 template <int GEOM, bool MG, bool CF>
 cudaError_t launch_event(const TrackArgs& a, const EventScratch& e, int cur, int block, int grid, cudaStream_t s) {
-  const size_t sh = (block / 32) * sizeof(WarpStage) + sizeof(float2) * (a.nx + a.ny);
-  const cudaError_t err = smem_opt_in<k_event<GEOM, MG, CF>>(sh);
+  const size_t sh = track_smem(a, block, false, 0);
+  if (sh > kSmemPerBlock) {
+    k_event<GEOM, MG, CF, false><<<grid, block, stage_smem(block), s>>>(a, e, cur);
+    return cudaGetLastError();
+  }
+  const cudaError_t err = smem_opt_in<k_event<GEOM, MG, CF, true>>(sh);
   if (err != cudaSuccess) return err;
-  k_event<GEOM, MG, CF><<<grid, block, sh, s>>>(a, e, cur);
+  k_event<GEOM, MG, CF, true><<<grid, block, sh, s>>>(a, e, cur);
   return cudaGetLastError();
 }
 
