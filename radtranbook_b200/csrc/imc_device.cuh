@@ -311,12 +311,16 @@ __device__ __forceinline__ void counts_flush(BlockCounts<S>& t, G* __restrict__ 
 }
 
 // Comb copies of an entry of weight wf in a bin of comb weight ew > 0: floor(w / ew + xi), xi the
-// uniform of the Philox word xw.  The quotient is formed in FP32 first, off by at most 1e-6 of itself;
-// only where that leaves the floor open is it divided in FP64.
+// uniform of the Philox word xw.  The quotient is formed in FP32 first; only where that leaves the
+// floor open is it divided in FP64.  With ew normal in FP32 and its reciprocal too, the FP32 sum is
+// off by at most 5e-7 (s + 1): ew's rounding and the sum's 2^-24 each, the quotient 2 ulp.  Outside
+// that range (an FP32 subnormal keeps few digits of ew; above 2^126 the quotient is 0) every copy is
+// divided in FP64.
 __device__ __forceinline__ int comb_floor(float wf, double ew, uint32_t xw) {
-  const float s = __fdividef(wf, (float)ew) + u01f(xw);
+  const float ef = (float)ew;
+  const float s = __fdividef(wf, ef) + u01f(xw);
   const float fl = floorf(s), fr = s - fl, open = 1e-6f * (s + 1.f);
-  if (s < 4e6f && fr > open && fr < 1.f - open) return (int)fl;  // false for an infinite or NaN quotient
+  if (ef > 2e-38f && ef < 8e37f && s < 4e6f && fr > open && fr < 1.f - open) return (int)fl;
   return (int)floor((double)wf / ew + u01d(xw));
 }
 
