@@ -7,6 +7,7 @@ material energy, combs the census, and the energy ledger is closed in FP64.
 """
 from __future__ import annotations
 
+import functools
 import time as _time
 import weakref
 
@@ -266,6 +267,25 @@ def face_temperatures(dim: int, geometry: str, T_boundary, time_now: float, e1: 
     return out
 
 
+def settled(step):
+    """A step whose exceptions leave nothing in flight: its kernels and copies fill pinned host
+    buffers through raw pointers, of which torch's allocator does not know, and an exception may be
+    the end of the state that keeps them."""
+
+    @functools.wraps(step)
+    def run(state, *args, **kwargs):
+        try:
+            return step(state, *args, **kwargs)
+        except BaseException:
+            eng = getattr(state, "_engine", None)
+            if eng is not None:
+                eng.settle()
+            raise
+
+    return run
+
+
+@settled
 def gray_step(state: GrayState, *, Ntarget, Nboundary, Nsource, Nmax, T_boundary, dt, sigma_a_func, inv_eos, cv,
               source, reflect, theta, use_scalar_intensity_Tr, conserve_comb_energy, T_emit_floor=0.0,
               rz_linear_source=True, max_events=0, boundary_source_func=None, geometry="slab",

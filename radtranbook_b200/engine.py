@@ -8,6 +8,7 @@ bank grows; the library guarantees nothing was modified in that case.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 from dataclasses import dataclass, field
 
@@ -549,6 +550,15 @@ class Engine:
             ev = self._events[name] = torch.cuda.Event()
             ev.record(torch.cuda.current_stream(self.device))
         return ev
+
+    def settle(self) -> None:
+        """Wait for all that the current and the side stream hold (an error of the device's own is
+        left to the next call)."""
+        side = self.__dict__.get("_side_stream")
+        with contextlib.suppress(RuntimeError):
+            torch.cuda.current_stream(self.device).synchronize()
+            if side is not None:
+                side.synchronize()
 
     def fields_to_host(self, fields, out: torch.Tensor, done: "torch.cuda.Event | None" = None) -> None:
         """Queue up to four cell fields (flat, device) into the pinned `out` in the reference's

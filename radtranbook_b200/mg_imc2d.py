@@ -24,7 +24,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._gray import GrayState, _host_copy, _law, _same, _staged, check_partition, face_temperatures
+from ._gray import GrayState, _host_copy, _law, _same, _staged, check_partition, face_temperatures, settled
 from .partition import local_count, sum_scalars, sum_tensors, summary_totals, world_of
 from .engine import A_RAD, C_LIGHT, Engine
 from .materials import evaluate, evaluate_groups
@@ -209,6 +209,7 @@ def _boundary_energy_estimate(geometry, e1, e2, Tb, dt, bsf) -> float:
     return E
 
 
+@settled
 def step(state, Ntarget, Nboundary, Nsource, Nmax, T_boundary, dt, edges1, edges2, energy_edges, sigma_a_funcs,
          inv_eos, cv, source, reflect=(False, False, False, False), theta=1.0, use_scalar_intensity_Tr=True,
          conserve_comb_energy=False, geometry="xy", max_events_per_particle=1_000_000, boundary_source_func=None,
