@@ -194,33 +194,33 @@ __global__ void __launch_bounds__(WIDE ? kAdjWide : 256, WIDE ? 1 : 4) k_adjoint
 }
 
 template <auto Kernel>
-cudaError_t launch_replay(const AdjointArgs& a, int grid, int block, size_t sh, cudaStream_t s) {
+cudaError_t launch_replay(const AdjointArgs& a, int block, int bps, size_t sh, cudaStream_t s) {
   const cudaError_t e = smem_opt_in<Kernel>(sh);
   if (e != cudaSuccess) return e;
-  Kernel<<<grid, block, sh, s>>>(a);
+  Kernel<<<a.t.sms * resident_blocks<Kernel>(bps, block, sh), block, sh, s>>>(a);
   return cudaGetLastError();
 }
 
 template <int GEOM>
-cudaError_t launch_adj(const AdjointArgs& a, int block, int bps, int sms, cudaStream_t s) {
+cudaError_t launch_adj(const AdjointArgs& a, int block, int bps, cudaStream_t s) {
   k_adjoint_tables<<<(a.t.nc + 255) / 256, 256, 0, s>>>(a);
   const size_t edges = sizeof(float2) * ((size_t)a.t.nx + a.t.ny), stages = (size_t)(block / 32) * sizeof(WarpStage);
   const size_t wide_sh = edges + sizeof(double) * (size_t)a.t.nc;
   if (block <= 256 && wide_sh <= kSmemPerBlock)
-    return launch_replay<k_adjoint<GEOM, true, true>>(a, sms, std::max(128, std::min(kAdjWide, block * bps)) & ~31,
+    return launch_replay<k_adjoint<GEOM, true, true>>(a, std::max(128, std::min(kAdjWide, block * bps)) & ~31, 1,
                                                       wide_sh, s);
   if (edges + stages <= kSmemPerBlock)
-    return launch_replay<k_adjoint<GEOM, false, true>>(a, sms * bps, block, edges + stages, s);
-  return launch_replay<k_adjoint<GEOM, false, false>>(a, sms * bps, block, stages, s);
+    return launch_replay<k_adjoint<GEOM, false, true>>(a, block, bps, edges + stages, s);
+  return launch_replay<k_adjoint<GEOM, false, false>>(a, block, bps, stages, s);
 }
 
 }  // namespace
 
-cudaError_t imc_launch_adjoint(const AdjointArgs& a, int geom, int block, int bps, int sms, cudaStream_t s) {
+cudaError_t imc_launch_adjoint(const AdjointArgs& a, int geom, int block, int bps, cudaStream_t s) {
   g_imc_launches += 2;
   switch (geom) {
-    case G_XY: return launch_adj<G_XY>(a, block, bps, sms, s);
-    case G_RZ: return launch_adj<G_RZ>(a, block, bps, sms, s);
+    case G_XY: return launch_adj<G_XY>(a, block, bps, s);
+    case G_RZ: return launch_adj<G_RZ>(a, block, bps, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -442,7 +442,7 @@ imc_status transport_async(const imc_mesh* mesh, const imc_material* mat, const 
     A.t = ta; A.sa64 = tal->sigma_a; A.ss64 = tal->sigma_s; A.sig64 = mat->sigma;
     A.score = ws_ptr<double>(workspace, L.ecen);  // no comb follows, and the sources are made
     A.chain = ws_ptr<double2>(workspace, L.tilt);
-    IMC_CUDA(imc_launch_adjoint(A, mesh->geometry, block, bps, sm_count(), s));
+    IMC_CUDA(imc_launch_adjoint(A, mesh->geometry, block, bps, s));
     if (pe.ok) { IMC_CUDA(cudaEventRecord(pe.e[2], s)); pe.recorded = true; }
     return IMC_OK;
   }

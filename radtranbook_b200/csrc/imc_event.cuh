@@ -157,7 +157,9 @@ __device__ __forceinline__ Flight next_flight(float2 e1, float2 e2, float ss, fl
 // scheduler.  (With every run a ticket, the warps that came first held the work of a small bank
 // while other schedulers had none: one of 592 executed 6.5 times the average of a 4k slab step's
 // instructions.  The twenty launches of a 20k crooked-pipe run 0.67 -> 0.52 ms, of a 4k slab run
-// 5.5 -> 4.0.)  Later runs are guided tickets: a share of what is left, at most `chunk`, at least 32, so
+// 5.5 -> 4.0.)  So the grid has no more blocks than are resident (resident_blocks): dealt to twice as many,
+// half the runs of a 40k slab wave waited for the other half (256 x 8 threads an SM: 7.97 ms, now 4.48).
+// Later runs are guided tickets: a share of what is left, at most `chunk`, at least 32, so
 // early ones are long contiguous (coherent) runs and the drain is finely balanced.
 struct Runs { uint32_t next, end; };  // the warp's current run
 

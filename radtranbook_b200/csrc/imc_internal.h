@@ -34,6 +34,18 @@ cudaError_t smem_opt_in(size_t smem) {
   return e;
 }
 
+// At most `asked` blocks per SM: what an SM holds of Kernel at this launch shape.  A persistent grid deals
+// every block a share of the work at once, so blocks beyond those would keep theirs waiting.  (A
+// kernel bound to 64 registers is known to fit 1024 threads, where its shared memory does too.)
+template <auto Kernel>
+int resident_blocks(int asked, int block, size_t smem) {
+  if (asked <= 1 || (asked * block <= 1024 && (size_t)asked * (smem + 2048) <= 227 * 1024)) return asked;
+  int most = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most, Kernel, block, smem) != cudaSuccess)
+    (void)cudaGetLastError();  // a shape that cannot run: the launch says so
+  return most > 0 && most < asked ? most : asked;
+}
+
 // ---------------------------------------------------------------------------------
 // Tracking
 // ---------------------------------------------------------------------------------
@@ -113,7 +125,7 @@ struct AdjointArgs {
   double* score;          // [c] cot / V: score per unit of deposited energy
   double2* chain;         // [c] (f^2, (1 - f^2) / sigma_s): the chain rule's factors
 };
-cudaError_t imc_launch_adjoint(const AdjointArgs& a, int geom, int block, int blocks_per_sm, int sms, cudaStream_t s);
+cudaError_t imc_launch_adjoint(const AdjointArgs& a, int geom, int block, int blocks_per_sm, cudaStream_t s);
 
 // ---------------------------------------------------------------------------------
 // Workspace layout (byte offsets into the caller's workspace, 256-aligned pieces)

@@ -520,10 +520,10 @@ inline size_t track_smem(const TrackArgs& a, int block, bool cells, int tallies)
 }
 
 template <auto Kernel>
-cudaError_t launch_sized(const TrackArgs& a, int block, int grid, size_t sh, cudaStream_t s) {
+cudaError_t launch_sized(const TrackArgs& a, int block, int bps, size_t sh, cudaStream_t s) {
   const cudaError_t e = smem_opt_in<Kernel>(sh);
   if (e != cudaSuccess) return e;
-  IMC_LAUNCH_PDL(Kernel, grid, block, sh, s, a);
+  IMC_LAUNCH_PDL(Kernel, a.sms * resident_blocks<Kernel>(bps, block, sh), block, sh, s, a);
   return cudaGetLastError();
 }
 
@@ -531,7 +531,7 @@ cudaError_t launch_sized(const TrackArgs& a, int block, int grid, size_t sh, cud
 // asked for and fit by themselves, but not beside a long mesh's edges, are left in global memory.
 template <int GEOM, bool MG, bool CF = false>
 cudaError_t launch_geom(const TrackArgs& a, const TrackLaunch& l, cudaStream_t s) {
-  const int block = l.block, grid = l.sms * l.blocks_per_sm;
+  const int block = l.block;
   const size_t edges = track_smem(a, block, false, 0) - stage_smem(block);
   auto fits = [&](bool cells, int tallies) { return track_smem(a, block, cells, tallies) <= kSmemPerBlock; };
   auto asked = [&](bool cells, int tallies) {  // (what cannot fit without the edges fails at the launch)
@@ -544,21 +544,21 @@ cudaError_t launch_geom(const TrackArgs& a, const TrackLaunch& l, cudaStream_t s
   const int wide = std::max(128, std::min(kWideThreads, block * l.blocks_per_sm)) & ~31;
   if (!st && l.wide_ok && block <= 256 && track_smem(a, wide, false, 1) <= kSmemPerBlock) {
     if (sm && track_smem(a, wide, true, 1) <= kSmemPerBlock)
-      return launch_sized<k_track<GEOM, true, MG, CF, T_WIDE>>(a, wide, l.sms, track_smem(a, wide, true, 1), s);
-    return launch_sized<k_track<GEOM, false, MG, CF, T_WIDE>>(a, wide, l.sms, track_smem(a, wide, false, 1), s);
+      return launch_sized<k_track<GEOM, true, MG, CF, T_WIDE>>(a, wide, 1, track_smem(a, wide, true, 1), s);
+    return launch_sized<k_track<GEOM, false, MG, CF, T_WIDE>>(a, wide, 1, track_smem(a, wide, false, 1), s);
   }
   if constexpr (!CF) {
     const size_t sh = track_smem(a, wide, false, 0) + 20 * (size_t)kHashSlots;
     if (!st && l.wide_ok && block <= 256 && sh <= kSmemPerBlock &&
         l.n_bound >= (long long)kHashPerLane * l.sms * wide)
-      return launch_sized<k_track<GEOM, false, MG, CF, T_HASH>>(a, wide, l.sms, sh, s);
+      return launch_sized<k_track<GEOM, false, MG, CF, T_HASH>>(a, wide, 1, sh, s);
   }
-  if (sm && st) return launch_sized<k_track<GEOM, true, MG, CF, T_SMALL>>(a, block, grid, track_smem(a, block, true, 2), s);
+  if (sm && st) return launch_sized<k_track<GEOM, true, MG, CF, T_SMALL>>(a, block, l.blocks_per_sm, track_smem(a, block, true, 2), s);
   if (sm && asked(true, 0))
-    return launch_sized<k_track<GEOM, true, MG, CF, T_GLOBAL>>(a, block, grid, track_smem(a, block, true, 0), s);
+    return launch_sized<k_track<GEOM, true, MG, CF, T_GLOBAL>>(a, block, l.blocks_per_sm, track_smem(a, block, true, 0), s);
   if (fits(false, 0))
-    return launch_sized<k_track<GEOM, false, MG, CF, T_GLOBAL>>(a, block, grid, track_smem(a, block, false, 0), s);
-  return launch_sized<k_track<GEOM, false, MG, CF, T_LONG>>(a, block, grid, stage_smem(block), s);
+    return launch_sized<k_track<GEOM, false, MG, CF, T_GLOBAL>>(a, block, l.blocks_per_sm, track_smem(a, block, false, 0), s);
+  return launch_sized<k_track<GEOM, false, MG, CF, T_LONG>>(a, block, l.blocks_per_sm, stage_smem(block), s);
 }
 
 // ---------------------------------------------------------------------------------
