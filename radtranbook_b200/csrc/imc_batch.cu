@@ -842,6 +842,7 @@ namespace {
     cudaError_t e__ = (call);                       \
     if (e__ != cudaSuccess) {                       \
       imc_note_cuda_error((int)e__);                \
+      (void)cudaGetLastError();                     \
       return IMC_ERR_CUDA;                          \
     }                                               \
   } while (0)

@@ -25,11 +25,13 @@ thread_local int g_last_cuda = 0;
 
 inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
+// (an error is reported once: left in the runtime, the next call's launch checks would find it again)
 #define IMC_CUDA(call)                              \
   do {                                              \
     cudaError_t e__ = (call);                       \
     if (e__ != cudaSuccess) {                       \
       g_last_cuda = (int)e__;                       \
+      (void)cudaGetLastError();                     \
       return IMC_ERR_CUDA;                          \
     }                                               \
   } while (0)
