@@ -96,8 +96,8 @@ __global__ void k_bmaterial_fleck(BatchArgs a, int update) {
 // Per-instance source plan: emission counts/weights/offsets, linear-T slopes, boundary
 // faces, this step's bank layout inside the instance's slot range.  Also clears the
 // instance's tallies and accumulators for the step.
-__global__ void __launch_bounds__(NT) k_bplan(BatchArgs a, int smem_cnt) {
-  extern __shared__ int cnt_sh[];  // smem_cnt: the counts while they are scanned
+__global__ void __launch_bounds__(NT) k_bplan(BatchArgs a, int smem_cells) {
+  extern __shared__ int cnt_sh[];  // [smem_cells] the counts while they are scanned, where the instance's fit
   __shared__ double red[NT];
   __shared__ long long sh[32];
   const int k = blockIdx.x, t = threadIdx.x;
@@ -108,8 +108,8 @@ __global__ void __launch_bounds__(NT) k_bplan(BatchArgs a, int smem_cnt) {
     a.dep_fx[cb + c] = 0ull; a.si[cb + c] = 0.0; a.ecen[cb + c] = 0.0; a.ncopy[cb + c] = 0.0;
   }
   double e_emit;
-  const long long n_emit = plan_volume(a.emit_E + cb, a.n_target[k], nc, 1, nc, smem_cnt ? cnt_sh : nullptr, a.emit_n + cb,
-                                       a.emit_off + cb + k, a.emit_w + cb, a.emitted + cb, red, sh, &e_emit);
+  const long long n_emit = plan_volume(a.emit_E + cb, a.n_target[k], nc, 1, nc, nc <= smem_cells ? cnt_sh : nullptr,
+                                       a.emit_n + cb, a.emit_off + cb + k, a.emit_w + cb, a.emitted + cb, red, sh, &e_emit);
   // centred slopes of T, zeroed when an edge value goes negative (IMC/IMC1D.py:254-262)
   for (int i = t; i < nc; i += NT) {
     double s = 0.0;
@@ -282,8 +282,9 @@ cudaError_t imc_batch_launch_material_fleck(const BatchArgs& a, int update, cuda
 }
 cudaError_t imc_batch_launch_plan(const BatchArgs& a, cudaStream_t s) {
   ++g_imc_launches;
-  const bool smem_cnt = a.max_cells > 0 && a.max_cells <= 8192;
-  k_bplan<<<a.K, NT, smem_cnt ? sizeof(int) * (size_t)a.max_cells : 0, s>>>(a, smem_cnt ? 1 : 0);
+  // 32 KB at most; max_cells is the caller's word, so the kernel compares each instance with it
+  const int smem_cells = a.max_cells > 0 && a.max_cells <= 8192 ? a.max_cells : 0;
+  k_bplan<<<a.K, NT, sizeof(int) * (size_t)smem_cells, s>>>(a, smem_cells);
   return cudaGetLastError();
 }
 cudaError_t imc_batch_launch_ic_plan(const BatchArgs& a, const double* tr, cudaStream_t s) {
