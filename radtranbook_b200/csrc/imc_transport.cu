@@ -250,8 +250,10 @@ __device__ __forceinline__ void add_event_counts(const TrackArgs& a, const unsig
 // event): the same ten launches 14.5 ms at 1, 13.2 at 4, 12.6 at 8, 12.6 at 12.
 constexpr int kRefillMin = 8;
 constexpr int kWideThreads = 1024;
-//   T_LONG    as T_GLOBAL, on a mesh so long that its edges alone overfill a block's shared memory
-//             (8 bytes a cell: from 28 thousand cells in one direction): they stay in global memory
+//   T_LONG    as T_GLOBAL, on a mesh so long that its edges (8 bytes a cell) in shared memory would leave
+//             fewer blocks resident (edges_pay): they are read through L1.  Slabs of 14, 20 and 28 thousand
+//             cells, three steps of a million particles: 23.2, 23.5 and 23.8 ms with the edges staged in
+//             the one block that then fits an SM, 9.6, 9.7 and 9.8 so
 enum : int { T_GLOBAL = 0, T_SMALL, T_WIDE, T_HASH, T_LONG };
 constexpr bool wide_block(int tally) { return tally == T_WIDE || tally == T_HASH; }
 
@@ -527,6 +529,10 @@ cudaError_t launch_sized(const TrackArgs& a, int block, int bps, size_t sh, cuda
   return cudaGetLastError();
 }
 
+// Whether edges in shared memory, `sh` bytes a block with the rest, leave room for `want` blocks an SM
+// (228 KB, a block's own share 1 KB and its static bytes).
+inline bool edges_pay(size_t sh, int want) { return (size_t)std::max(1, want) * (sh + 1280) <= 228 * 1024; }
+
 // T_SMALL is built only with the shared-memory cell table (small meshes).  Tallies or a table that were
 // asked for and fit by themselves, but not beside a long mesh's edges, are left in global memory.
 template <int GEOM, bool MG, bool CF = false>
@@ -556,7 +562,7 @@ cudaError_t launch_geom(const TrackArgs& a, const TrackLaunch& l, cudaStream_t s
   if (sm && st) return launch_sized<k_track<GEOM, true, MG, CF, T_SMALL>>(a, block, l.blocks_per_sm, track_smem(a, block, true, 2), s);
   if (sm && asked(true, 0))
     return launch_sized<k_track<GEOM, true, MG, CF, T_GLOBAL>>(a, block, l.blocks_per_sm, track_smem(a, block, true, 0), s);
-  if (fits(false, 0))
+  if (edges_pay(track_smem(a, block, false, 0), std::min(l.blocks_per_sm, 1024 / block)))
     return launch_sized<k_track<GEOM, false, MG, CF, T_GLOBAL>>(a, block, l.blocks_per_sm, track_smem(a, block, false, 0), s);
   return launch_sized<k_track<GEOM, false, MG, CF, T_LONG>>(a, block, l.blocks_per_sm, stage_smem(block), s);
 }
@@ -600,20 +606,15 @@ __global__ void k_event_init(TrackArgs a, EventScratch e) {
   }
 }
 
-template <int GEOM, bool MG, bool CF, bool EDGES>
+// (The edges are read through L1: staged in shared memory by every launch they took from 2 % longer, at
+// a hundred cells, to 3.4 times as long, at 27 thousand, where they leave one block an SM.)
+template <int GEOM, bool MG, bool CF>
 __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int cur) {
   const uint32_t stepk = a.step_dev ? *a.step_dev : a.step;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ unsigned blk_cnt[B_N];
   __shared__ unsigned long long blk_esc[4];
   WarpStage* stages = reinterpret_cast<WarpStage*>(smem);
-  const int nwarps = blockDim.x >> 5;
-  float2* E1 = reinterpret_cast<float2*>(stages + nwarps);
-  float2* E2 = E1 + a.nx;
-  if (EDGES) {
-    for (int q = threadIdx.x; q < a.nx; q += blockDim.x) E1[q] = make_float2(a.e1[q], a.e1[q + 1]);
-    for (int q = threadIdx.x; q < a.ny; q += blockDim.x) E2[q] = make_float2(a.e2[q], a.e2[q + 1]);
-  }
   if (threadIdx.x < B_N) blk_cnt[threadIdx.x] = 0u;
   if (threadIdx.x < 4) blk_esc[threadIdx.x] = 0ull;
   __syncthreads();
@@ -660,7 +661,7 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
         h.tab = __ldg(a.sass + (MG ? c + a.nc * h.grp : c));
         h.key = draw_key(a.rk, a.id_base + pid, stepk, TAG_TRANSPORT);
         const uint32_t ev0 = h.ev;
-        history_event<GEOM, false, MG, CF, EDGES>(a, h, o, E1, E2, nullptr, blk_cnt, blk_esc, a.dep_fx,
+        history_event<GEOM, false, MG, CF, false>(a, h, o, nullptr, nullptr, nullptr, blk_cnt, blk_esc, a.dep_fx,
                                                   draw_next(a.rk, h.key, rkx, h.ev), weight_floor, inv_q, s_cen, s_sc);
         s_ev += h.ev - ev0;
         int bin;
@@ -688,14 +689,7 @@ __global__ void __launch_bounds__(256) k_event(TrackArgs a, EventScratch e, int 
 
 template <int GEOM, bool MG, bool CF>
 cudaError_t launch_event(const TrackArgs& a, const EventScratch& e, int cur, int block, int grid, cudaStream_t s) {
-  const size_t sh = track_smem(a, block, false, 0);
-  if (sh > kSmemPerBlock) {
-    k_event<GEOM, MG, CF, false><<<grid, block, stage_smem(block), s>>>(a, e, cur);
-    return cudaGetLastError();
-  }
-  const cudaError_t err = smem_opt_in<k_event<GEOM, MG, CF, true>>(sh);
-  if (err != cudaSuccess) return err;
-  k_event<GEOM, MG, CF, true><<<grid, block, sh, s>>>(a, e, cur);
+  k_event<GEOM, MG, CF><<<grid, block, stage_smem(block), s>>>(a, e, cur);
   return cudaGetLastError();
 }
 

@@ -1,7 +1,7 @@
-"""Meshes long in one direction, whose edges alone overfill a block's shared memory: tracking, the
-event-by-event form and the adjoint read them through L1.  Sizes on both sides of the shared-memory
-tables (28,400 cells beside a block's other arrays) and past what one float per edge would fit in
-(57,000); edges are multiples of 2^-12, exact in FP32.
+"""Meshes long in one direction, whose edges would leave few blocks an SM or overfill a block's shared
+memory: tracking, the event-by-event form and the adjoint read them through L1.  Sizes around the last
+mesh that has a block tally (13,400 cells) and past what pairs (28,400) and single floats (57,000) of
+edges would fit in; edges are multiples of 2^-12, exact in FP32.
 
 Tracking against the event-by-event form (histories and tallies as in its own test: counts and census
 entry by entry, deposition and escapes 1e-12) and against the oracle (FP32 against FP64 tracking, as
@@ -45,7 +45,7 @@ def _run(geometry, n, cuda, launch=None):
 
 
 @pytest.mark.parametrize("geometry", ["slab", "spherical"])
-@pytest.mark.parametrize("n", [28_000, 29_000, 40_000, 60_000])
+@pytest.mark.parametrize("n", [14_000, 28_000, 29_000, 40_000, 60_000])
 def test_long_1d_mesh(cuda, geometry, n):
     gpu = _run(geometry, n, cuda)
     event_form._same(gpu, _run(geometry, n, cuda, {"event_based": 1}))
@@ -84,3 +84,21 @@ def test_adjoint_on_a_long_mesh(cuda, n):
                 setup.reflect, max_events=setup.max_events, sources_only=True)
     ref = o.adjoint_vjp(Tc, sigma, cvc, 0, setup.dt, 1.0, setup.reflect, cot, max_events=setup.max_events)
     assert np.abs(g - ref).sum() <= 2e-3 * np.abs(ref).sum()
+
+
+def test_no_cliff_where_the_block_tally_ends(cuda):
+    """14,000 cells against 13,000, the last thousand with a block tally: the step took 2.7 times as long
+    with the edges in the shared memory of the one block that then fits an SM; 1.2 through L1."""
+    def best(n):
+        e1, e2, vol, T, sig, cv, face = _case("slab", n)
+        eng = Engine("slab", e1, e2, vol, seed=SEED)
+        dev = lambda a: None if a is None else torch.as_tensor(a, device=cuda)  # noqa: E731
+        t = []
+        for _ in range(4):  # the first one warms up
+            eng.init_census(dev(T), 300_000)
+            r = eng.transport(dev(T), dev(sig), dev(cv), None, 2, 1e-3, 1.0, 0, 0, 0, [None] * 4, (False,) * 4)
+            t.append(r.report.ms_transport)
+        return min(t)
+
+    short, long = best(13_000), best(14_000)
+    assert long <= 1.8 * short, (long, short)
