@@ -7,7 +7,6 @@ material energy, combs the census, and the energy ledger is closed in FP64.
 """
 from __future__ import annotations
 
-import functools
 import time as _time
 import weakref
 
@@ -267,25 +266,6 @@ def face_temperatures(dim: int, geometry: str, T_boundary, time_now: float, e1: 
     return out
 
 
-def settled(step):
-    """A step whose exceptions leave nothing in flight: its kernels and copies fill pinned host
-    buffers through raw pointers, of which torch's allocator does not know, and an exception may be
-    the end of the state that keeps them."""
-
-    @functools.wraps(step)
-    def run(state, *args, **kwargs):
-        try:
-            return step(state, *args, **kwargs)
-        except BaseException:
-            eng = getattr(state, "_engine", None)
-            if eng is not None:
-                eng.settle()
-            raise
-
-    return run
-
-
-@settled
 def gray_step(state: GrayState, *, Ntarget, Nboundary, Nsource, Nmax, T_boundary, dt, sigma_a_func, inv_eos, cv,
               source, reflect, theta, use_scalar_intensity_Tr, conserve_comb_energy, T_emit_floor=0.0,
               rz_linear_source=True, max_events=0, boundary_source_func=None, geometry="slab",
@@ -365,59 +345,63 @@ def gray_step(state: GrayState, *, Ntarget, Nboundary, Nsource, Nmax, T_boundary
     # law: they go to the host before the comb.  A host inv_eos then evaluates T from that e
     # while the comb runs.
     host_inv = law is None and not conserve_comb_energy and not is_device(inv_eos)
-    early = law is not None or host_inv
-    if early:
-        state.report(eng.event("fields") if host_inv else None)
-    eng.comb_async(Nmax, state.count, state._e)
-    if conserve_comb_energy:
-        sum_tensors(dist, [eng.disc])
-        state._e.add_(eng.disc[: eng.nc] / eng.vol)
-    if law is None and like is None:
-        like = state.grid(state._T)
-    if law is not None:
-        pass  # T = e / cv came with the material update
-    elif host_inv:
-        # the report holds e, (the old) T and Tr in the reference's layout: T = inv_eos(e)
-        # replaces the T slot (the host mirror this step returns), and goes up to the device, with
-        # the next step's opacity and heat capacity at this T when both are host callables (the
-        # next step takes them if it passes the same callables and nothing has set T since): one
-        # launch behind the comb, ahead of the summary that the step waits for
-        eng.event("fields").synchronize()
-        n = eng.nc
-        shape = (n,) if state._dim == 1 else tuple(state._shape)
-        hp = state._hpin.numpy()
-        Tn = np.asarray(inv_eos(hp[:n].reshape(shape)), dtype=np.float64)
-        T_ref = hp[n:2 * n].reshape(shape)
-
-        def put(dst, values):  # a field in the reference's layout, or a scalar
-            np.copyto(dst.reshape(shape), np.broadcast_to(np.asarray(values, dtype=np.float64), shape))
-
-        put(T_ref, Tn)
-        stage = _pinned(state, "up", 3 * n)
-        up = stage.numpy()
-        put(up[:n], Tn)
-        dst = [state._T]
-        if not is_device(sigma_a_func) and not is_device(cv):
-            sig_n, cv_n = _device_field(state, "sigma", n), _device_field(state, "cv", n)
-            put(up[n:2 * n], sigma_a_func(T_ref))
-            put(up[2 * n:], cv(T_ref))
-            dst += [sig_n, cv_n]
-            state.__dict__["_host_next"] = ((sigma_a_func, cv), state.count + 1, sig_n, cv_n)
-        eng.fields_from_host(stage, dst)
-        _lib.TRANSFER["h2d"] += 8 * n * len(dst)
-    else:
-        Tn = evaluate(inv_eos, state.grid(state._e), lambda: _host_copy(state.grid(state._e)), like)
-        state._T.copy_(state.flat(Tn))
-    if not early:
-        state.report()
-    eng.queue_summary()
-    # the phase times wait for the tracking only: read while the comb still runs on the device
-    ms_src, ms_tr = eng.phase_times()
     try:
-        sm = eng.fetch()
-    except _lib.ImcError as ex:
-        if ex.status == 3:
-            raise AssertionError("Fleck factor out of bounds / non-positive temperature in material state") from ex
+        early = law is not None or host_inv
+        if early:
+            state.report(eng.event("fields") if host_inv else None)
+        eng.comb_async(Nmax, state.count, state._e)
+        if conserve_comb_energy:
+            sum_tensors(dist, [eng.disc])
+            state._e.add_(eng.disc[: eng.nc] / eng.vol)
+        if law is None and like is None:
+            like = state.grid(state._T)
+        if law is not None:
+            pass  # T = e / cv came with the material update
+        elif host_inv:
+            # the report holds e, (the old) T and Tr in the reference's layout: T = inv_eos(e)
+            # replaces the T slot (the host mirror this step returns), and goes up to the device, with
+            # the next step's opacity and heat capacity at this T when both are host callables (the
+            # next step takes them if it passes the same callables and nothing has set T since): one
+            # launch behind the comb, ahead of the summary that the step waits for
+            eng.event("fields").synchronize()
+            n = eng.nc
+            shape = (n,) if state._dim == 1 else tuple(state._shape)
+            hp = state._hpin.numpy()
+            Tn = np.asarray(inv_eos(hp[:n].reshape(shape)), dtype=np.float64)
+            T_ref = hp[n:2 * n].reshape(shape)
+
+            def put(dst, values):  # a field in the reference's layout, or a scalar
+                np.copyto(dst.reshape(shape), np.broadcast_to(np.asarray(values, dtype=np.float64), shape))
+
+            put(T_ref, Tn)
+            stage = _pinned(state, "up", 3 * n)
+            up = stage.numpy()
+            put(up[:n], Tn)
+            dst = [state._T]
+            if not is_device(sigma_a_func) and not is_device(cv):
+                sig_n, cv_n = _device_field(state, "sigma", n), _device_field(state, "cv", n)
+                put(up[n:2 * n], sigma_a_func(T_ref))
+                put(up[2 * n:], cv(T_ref))
+                dst += [sig_n, cv_n]
+                state.__dict__["_host_next"] = ((sigma_a_func, cv), state.count + 1, sig_n, cv_n)
+            eng.fields_from_host(stage, dst)
+            _lib.TRANSFER["h2d"] += 8 * n * len(dst)
+        else:
+            Tn = evaluate(inv_eos, state.grid(state._e), lambda: _host_copy(state.grid(state._e)), like)
+            state._T.copy_(state.flat(Tn))
+        if not early:
+            state.report()
+        eng.queue_summary()
+        # the phase times wait for the tracking only: read while the comb still runs on the device
+        ms_src, ms_tr = eng.phase_times()
+        try:
+            sm = eng.fetch()
+        except _lib.ImcError as ex:
+            if ex.status == 3:
+                raise AssertionError("Fleck factor out of bounds / non-positive temperature in material state") from ex
+            raise
+    except BaseException:
+        eng.settle()  # the report's kernels fill a pinned buffer that torch's allocator thinks idle
         raise
     t_post = _time.perf_counter()
     pre_comb = eng.spare  # the tracked (pre-comb) bank after the swap

@@ -26,7 +26,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._gray import GrayState, _host_copy, _pinned, _staged, check_partition, face_temperatures, settled
+from ._gray import GrayState, _host_copy, _pinned, _staged, check_partition, face_temperatures
 from .engine import A_RAD, C_LIGHT, Engine
 from .materials import evaluate, evaluate_groups
 from .mg_imc2d import planck_fractions
@@ -135,7 +135,6 @@ def _budget(state, sig_h, cv_h, T_inner, T_outer, source, energy_edges, dt, thet
     return part(E_in), part(E_out), part(E_src), part(E_emit)
 
 
-@settled
 def step(state, Ntarget, Nboundary, Nsource, Nmax, T_boundary, dt, mesh, energy_edges, sigma_a_funcs, inv_eos, cv,
          source, reflect=(False, False), theta=1.0, use_scalar_intensity_Tr=True, conserve_comb_energy=True,
          max_events_per_particle=1_000_000, T_emit_floor=0.0, particle_budget_fmin=0.0, Nmax_growth=0,
@@ -196,14 +195,18 @@ def step(state, Ntarget, Nboundary, Nsource, Nmax, T_boundary, dt, mesh, energy_
     hm = _pinned(state, "moments", (2 * I + 1) * G)
     hm[:2 * G * I].copy_(moments.reshape(-1), non_blocking=True)
     hm[2 * G * I:].copy_(eng.escaped_group, non_blocking=True)
-    state.report()
-    eng.queue_summary()
-    ms_src, ms_tr = eng.phase_times()  # waits for the tracking only (the comb still runs)
     try:
+        state.report()
+        eng.queue_summary()
+        ms_src, ms_tr = eng.phase_times()  # waits for the tracking only (the comb still runs)
         sm = eng.fetch()
     except _lib.ImcError as ex:
+        eng.settle()
         if ex.status == 3:
             raise AssertionError("non-finite or non-positive material state") from ex
+        raise
+    except BaseException:
+        eng.settle()  # the report's kernel fills a pinned buffer that torch's allocator thinks idle
         raise
     if not use_scalar_intensity_Tr:
         pre = eng.spare  # the tracked bank before the comb

@@ -24,7 +24,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._gray import GrayState, _host_copy, _law, _same, _staged, check_partition, face_temperatures, settled
+from ._gray import GrayState, _host_copy, _law, _same, _staged, check_partition, face_temperatures
 from .partition import local_count, sum_scalars, sum_tensors, summary_totals, world_of
 from .engine import A_RAD, C_LIGHT, Engine
 from .materials import evaluate, evaluate_groups
@@ -209,7 +209,6 @@ def _boundary_energy_estimate(geometry, e1, e2, Tb, dt, bsf) -> float:
     return E
 
 
-@settled
 def step(state, Ntarget, Nboundary, Nsource, Nmax, T_boundary, dt, edges1, edges2, energy_edges, sigma_a_funcs,
          inv_eos, cv, source, reflect=(False, False, False, False), theta=1.0, use_scalar_intensity_Tr=True,
          conserve_comb_energy=False, geometry="xy", max_events_per_particle=1_000_000, boundary_source_func=None,
@@ -295,43 +294,47 @@ def step(state, Ntarget, Nboundary, Nsource, Nmax, T_boundary, dt, edges1, edges
     else:
         state.__dict__.pop("_law_next", None)
         eng.material_update(state._e, state._Tr)
-    # with the device law (and no comb discrepancy booked into e) every reported field but the
-    # post-comb energies is final now: gathered and copied to the host beside the comb
-    early = _report_early(state, eng) if law is not None and not conserve_comb_energy else None
-    # the comb is queued next (the host prepares the by-group fields while it runs); it also
-    # writes the energy after it per (group, cell) bin: the post-comb radiation energy by
-    # group without a pass over the new census
-    eng.comb_async(nmax_l, state.count, state._e, per_group=True, write_after=True)
-    nx, ny = state._shape
-
-    def to_grid3(x):  # device (G, nc) in flat cell order -> (G, nx, ny) C order, flattened
-        return x.reshape(G, ny, nx).transpose(1, 2).reshape(-1)
-
-    sum_tensors(dist, [eng.comb_after])
-    if conserve_comb_energy:
-        sum_tensors(dist, [eng.disc])
-        state._e.add_(eng.disc.view(G, nc).sum(0) / eng.vol)
-    if law is None:
-        Tn = evaluate(inv_eos, state.grid(state._e), lambda: _host_copy(state.grid(state._e)), like,
-                      **_staged(state, "T_new", nc))
-        state._T.copy_(state.flat(Tn))
-    # every reported field in the reference's layout in one device buffer (one kernel), then
-    # one copy into a fresh pinned buffer that the host arrays view
-    if early is None:
-        hb = _report_buffers(state, eng, eng.report_buffer().numel())
-        eng.mg_report_to_host(state._e, state._T, state._Tr, hb["all"])
-    else:
-        hb = early
-        eng.mg_report_to_host(None, None, None, hb["all"], sections="post")
-    eng.queue_summary()
-    if early is not None:
-        eng.event("report").synchronize()  # done long before the comb
-    ms_src, ms_tr = eng.phase_times()  # waits for the tracking only (the comb still runs)
     try:
-        sm = eng.fetch()
-    except _lib.ImcError as ex:
-        if ex.status == 3:
-            raise AssertionError("non-finite or non-positive material state") from ex
+        # with the device law (and no comb discrepancy booked into e) every reported field but the
+        # post-comb energies is final now: gathered and copied to the host beside the comb
+        early = _report_early(state, eng) if law is not None and not conserve_comb_energy else None
+        # the comb is queued next (the host prepares the by-group fields while it runs); it also
+        # writes the energy after it per (group, cell) bin: the post-comb radiation energy by
+        # group without a pass over the new census
+        eng.comb_async(nmax_l, state.count, state._e, per_group=True, write_after=True)
+        nx, ny = state._shape
+
+        def to_grid3(x):  # device (G, nc) in flat cell order -> (G, nx, ny) C order, flattened
+            return x.reshape(G, ny, nx).transpose(1, 2).reshape(-1)
+
+        sum_tensors(dist, [eng.comb_after])
+        if conserve_comb_energy:
+            sum_tensors(dist, [eng.disc])
+            state._e.add_(eng.disc.view(G, nc).sum(0) / eng.vol)
+        if law is None:
+            Tn = evaluate(inv_eos, state.grid(state._e), lambda: _host_copy(state.grid(state._e)), like,
+                          **_staged(state, "T_new", nc))
+            state._T.copy_(state.flat(Tn))
+        # every reported field in the reference's layout in one device buffer (one kernel), then
+        # one copy into a fresh pinned buffer that the host arrays view
+        if early is None:
+            hb = _report_buffers(state, eng, eng.report_buffer().numel())
+            eng.mg_report_to_host(state._e, state._T, state._Tr, hb["all"])
+        else:
+            hb = early
+            eng.mg_report_to_host(None, None, None, hb["all"], sections="post")
+        eng.queue_summary()
+        if early is not None:
+            eng.event("report").synchronize()  # done long before the comb
+        ms_src, ms_tr = eng.phase_times()  # waits for the tracking only (the comb still runs)
+        try:
+            sm = eng.fetch()
+        except _lib.ImcError as ex:
+            if ex.status == 3:
+                raise AssertionError("non-finite or non-positive material state") from ex
+            raise
+    except BaseException:
+        eng.settle()  # the report's kernels fill a pinned buffer that torch's allocator thinks idle
         raise
     if not use_scalar_intensity_Tr:
         pre = eng.spare
