@@ -224,6 +224,22 @@ __device__ __forceinline__ void warp_tally1(bool flush, int key, double va, doub
   __syncwarp();
 }
 
+// An add per flushing lane into a block's shared tally, the lanes of the cell `hot` (warp-uniform) as one:
+// an FP64 shared-memory add is a compare-and-swap loop, which lanes of one cell take in turn.  Every
+// lane of the warp calls it (converged).
+__device__ __forceinline__ void smem_tally_hot(bool flush, int cell, double v, double* t, int hot) {
+  const bool mine = flush && cell == hot;
+  if (__popc(__ballot_sync(FULL, mine)) >= 4) {
+    double s = mine ? v : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(t + hot, s);
+    if (flush && !mine) atomicAdd(t + cell, v);
+  } else if (flush) {
+    atomicAdd(t + cell, v);
+  }
+}
+
 // ---- block-aggregated per-bin sums ----
 // The census of a step piles up in a few cells (the hottest radiation), so even after
 // per-warp aggregation thousands of FP64 atomics land on each of those addresses and
