@@ -486,6 +486,7 @@ imc_status comb_async(const imc_mesh* mesh, const imc_bank* in, imc_bank* out, i
   ca.n_live = ws_ptr<unsigned long long>(workspace, L.comb_mode + 8);
   ca.ticket = ws_ptr<unsigned long long>(workspace, L.comb_mode + 16);
   ca.d_n_in = &sum->n_bank; ca.n_bound = in->size; ca.out_capacity = out->capacity;
+  ca.n_max = n_max < 0 ? -n_max : n_max;
   ca.w = in->weight; ca.cell = in->cell; ca.group = in->group;
   ca.p1 = in->pos1; ca.p2 = two_d ? in->pos2 : nullptr; ca.d1 = in->dir1; ca.d2 = two_d ? in->dir2 : nullptr;
   ca.ecen = ws_ptr<double>(workspace, L.ecen); ca.ew = ws_ptr<double>(workspace, L.ew);

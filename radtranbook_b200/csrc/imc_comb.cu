@@ -225,19 +225,21 @@ __host__ __device__ inline size_t scatter_smem(bool two_d, bool grp) {
 // 16-byte loads (one thread per four entries), each thread notes its entries' output positions, and
 // one thread per output copy then copies its entry's fields from shared memory, so the global loads
 // and the stores of a warp are both contiguous.  A tile with more than SCAT_MAP copies finds the
-// entries of the others by a binary search of the scanned counts.  The remaining blocks take 256
+// entries of the others by a binary search of the scanned counts, and one with more than four times that
+// those of all.  `split` blocks share a tile, each staging it and writing a stretch of its copies, where
+// a small bank makes many copies an entry (scatter_split).  The remaining blocks take 256
 // bins each: disc and the energy after the comb.  Against tiles of 4096 entries, a search for
 // every copy, the copy weight gathered per copy and a launch of its own for the bins: 28 -> 13 us
 // for 91 thousand entries, 29 -> 20 us for 1.7 M; 8.7 M take the same 88 us (0.40 GB moved, at two
 // thirds of the rate of a copy).
-__global__ void __launch_bounds__(SCAT_T) k_comb_scatter(CombArgs a, long long ntiles) {
+__global__ void __launch_bounds__(SCAT_T) k_comb_scatter(CombArgs a, long long ntiles, int split) {
   pdl_wait();     // the previous kernel of the stream has completed
   pdl_trigger();  // the next one may be scheduled
   extern __shared__ __align__(16) int sm_tile[];
   __shared__ int sh[SCAT_T / 32];
   const bool compact = *a.mode != 0;
-  if ((long long)blockIdx.x >= ntiles) {
-    const long long b = ((long long)blockIdx.x - ntiles) * blockDim.x + threadIdx.x;
+  if ((long long)blockIdx.x >= ntiles * split) {
+    const long long b = ((long long)blockIdx.x - ntiles * split) * blockDim.x + threadIdx.x;
     double after = 0.0;
     if (b < a.nb) {
       // compact only: every live entry kept with its weight, nothing is lost
@@ -259,7 +261,8 @@ __global__ void __launch_bounds__(SCAT_T) k_comb_scatter(CombArgs a, long long n
   float* sD2 = sP2 + TILE;                            // 2-D only
   int* sG = reinterpret_cast<int*>(two_d ? sD2 + TILE : sP2);  // with a group array only
   unsigned short* entry = reinterpret_cast<unsigned short*>(sm_tile + TILE * (1 + scatter_fields(two_d, grp)));
-  const long long tile0 = (long long)blockIdx.x * TILE;
+  const long long tile = split > 1 ? blockIdx.x / split : blockIdx.x;
+  const long long tile0 = tile * TILE;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const long long n_in = min((long long)*a.d_n_in, (long long)a.n_bound);
   const int q0 = 4 * threadIdx.x;
@@ -315,22 +318,28 @@ __global__ void __launch_bounds__(SCAT_T) k_comb_scatter(CombArgs a, long long n
   for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(FULL, x, o); if (lane >= o) x += y; }
   if (lane == 31) sh[wid] = x;
   __syncthreads();
-  int run = x - s4;
-  for (int q = 0; q < wid; ++q) run += sh[q];
+  int run = x - s4, total = 0;
+  for (int q = 0; q < SCAT_T / 32; ++q) { if (q < wid) run += sh[q]; total += sh[q]; }
+  const int mapped = total <= 4 * SCAT_MAP ? SCAT_MAP : 0;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    for (int o = run; o < run + c[j] && o < SCAT_MAP; ++o) entry[o] = (unsigned short)(q0 + j);
+    for (int o = run; o < run + c[j] && o < mapped; ++o) entry[o] = (unsigned short)(q0 + j);
     run += c[j];
     incl[q0 + j] = run;
   }
   __syncthreads();
-  const int total = incl[TILE - 1];
-  const long long out0 = a.blk[blockIdx.x];
-  for (int o = threadIdx.x; o < total; o += blockDim.x) {
+  int first = 0, last = total;
+  if (split > 1) {
+    const int share = (total / split / SCAT_T + 1) * SCAT_T, part = (int)(blockIdx.x - tile * split);
+    first = min(total, part * share);
+    last = min(total, first + share);
+  }
+  const long long out0 = a.blk[tile];
+  for (int o = first + threadIdx.x; o < last; o += blockDim.x) {
     const long long dst = out0 + o;
     if (dst >= a.out_capacity) break;  // overflow: flagged by the scan, caller regrows
     int e;
-    if (o < SCAT_MAP) {
+    if (o < mapped) {
       e = entry[o];
     } else {
       int lo = 0, hi = TILE - 1;  // the entry j with incl[j-1] <= o < incl[j]
@@ -373,11 +382,20 @@ cudaError_t imc_launch_comb_count(const CombArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// Blocks a tile: one per SCAT_MAP copies that the target asks of each, as long as they all fit the chip
+// (four blocks an SM).
+static int scatter_split(long long n_max, long long ntiles) {
+  const long long copies = n_max / std::max(1LL, ntiles);
+  return (int)std::max(1LL, std::min((copies + SCAT_MAP - 1) / SCAT_MAP, 4LL * 148 / std::max(1LL, ntiles)));
+}
+
 cudaError_t imc_launch_comb_scatter(const CombArgs& a, cudaStream_t s) {
   const long long ntiles = (a.n_bound + TILE - 1) / TILE;
   ++g_imc_launches;
+  const int split = scatter_split(a.n_max, ntiles);
   const size_t smem = scatter_smem(a.p2 != nullptr, a.group != nullptr);
   static_assert(sizeof(int) * TILE * 8 + 2 * SCAT_MAP <= 48 * 1024, "no opt-in for the largest layout");
-  IMC_LAUNCH_PDL(k_comb_scatter, (unsigned)(ntiles + (a.nb + SCAT_T - 1) / SCAT_T), SCAT_T, smem, s, a, ntiles);
+  IMC_LAUNCH_PDL(k_comb_scatter, (unsigned)(ntiles * split + (a.nb + SCAT_T - 1) / SCAT_T), SCAT_T, smem, s, a, ntiles,
+                 split);
   return cudaGetLastError();
 }

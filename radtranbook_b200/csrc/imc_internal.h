@@ -325,6 +325,7 @@ struct CombArgs {
   const int64_t* d_n_in;       // entries to comb (device)
   long long n_bound;           // host upper bound of *d_n_in (grid sizing)
   long long out_capacity;
+  long long n_max;             // host bound of the comb target (the scatter's split of a tile's copies)
   const float* w; const int* cell; const int* group;
   const float* p1; const float* p2; const float* d1; const float* d2;
   double* ecen; double* ew; unsigned long long* ncopy; int* cnt; long long* blk;  // ncopy: copies per bin
