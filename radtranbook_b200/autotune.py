@@ -1,11 +1,13 @@
 """Launch-shape autotuner for the tracking kernel.
 
-The tracking kernel is a persistent grid whose warps claim `chunk` histories per atomic
-ticket and refill finished lanes at every event boundary.  Its speed depends on:
+The tracking kernel is a persistent grid whose warps claim runs of at most `chunk` histories.
+Its speed depends on:
   block_size     threads per block (64..256; the kernel is compiled for <= 256)
-  blocks_per_sm  resident blocks requested per SM (grid = blocks_per_sm x SMs)
-  chunk          histories claimed per warp ticket (refill cadence / bank tile)
-  smem_cells     stage the per-cell (sigma_a, sigma_s) table in shared memory
+  blocks_per_sm  blocks asked for per SM (those an SM holds are launched); meshes past the small
+                 block tally run one wide block per SM, of block_size x blocks_per_sm threads (at
+                 most 1024), so shapes with the same product are the same launch there
+  chunk          histories claimed per warp ticket, at most
+  smem_cells     stage the per-cell (sigma_a, sigma_s) table in shared memory, where it fits
 The tuner replays the engine's last transport on a snapshot of the census bank for every
 candidate (the Philox streams make each trial the identical work), times the tracking
 phase with CUDA events, restores the census and installs the fastest shape.

@@ -26,7 +26,7 @@ struct BatchArgs {
   int* cell_inst;        // [n_cells] instance of a cell
   float* ef;             // [n_cells + K] FP32 edges
   double* vol;           // [n_cells] dx
-  float2* sass;          // [n_cells] (sigma_a, sigma_s) FP32
+  float2* sass;          // [n_cells] (Fleck absorption or 0, scatter slot: scatter_entry), FP32
   double2* cellf;        // [n_cells] (1/V, 1/(sigma_a V dt) or -1/(V dt))
   double* emit_E;        // [n_cells]
   long long* emit_n;     // [n_cells]

@@ -6,16 +6,16 @@
 //   xy/rz  IMC/IMC2D.py:711-935 (events), 938-1107 (history loop)
 //   multigroup  MG_IMC/MG_IMC2D.py:580-989 (xy, rz), MG_IMC/MG_IMC1D.py:276-461 (sphere)
 //
-// Execution model: a persistent grid (blocks_per_sm x SMs).  Each warp claims a chunk of
-// bank indices with one atomic ticket and keeps 32 histories in registers.  Every loop
-// iteration advances every live lane by one event (distance to face / effective scatter /
-// census, implicit capture w *= exp(-sigma_a s)); at each event boundary, lanes whose
-// history ended are refilled from the warp's chunk, so warps do not carry dead lanes until
-// the bank drains (the in-warp form of bank compaction between events).  Particle state is
-// FP32; energy removed from a history is accounted as the exact FP64 difference of its
-// FP32 weights, accumulated in registers while the history stays in one cell and flushed
-// through warp-aggregated FP64 reductions when it leaves.  Random numbers: Philox keyed by
-// the run seed, counter (id_base + bank index, event number, step, TAG_TRANSPORT).
+// Execution model: a persistent grid of the blocks that are resident.  Each warp keeps 32
+// histories in registers, from a run of bank indices: its first one is dealt to it, later ones
+// are guided atomic tickets (imc_event.cuh, Runs).  An event advances every live lane (distance
+// to face / effective scatter / census, implicit capture w *= exp(-sigma_a s)); lanes whose
+// history ended wait until kRefillMin of the warp are idle, then are stored and refilled
+// together, so warps do not carry dead lanes until the bank drains (the in-warp form of bank
+// compaction between events).  Particle state is FP32; energy removed from a history is
+// accounted as the exact FP64 difference of its FP32 weights while it stays in one cell, and
+// flushed in fixed point when it leaves, into one of the tallies below.  Random numbers: Philox
+// keyed by the run seed, counter (id_base + bank index, event number, step, TAG_TRANSPORT).
 #include <algorithm>
 
 #include "imc_event.cuh"
@@ -247,7 +247,10 @@ __device__ __forceinline__ void add_event_counts(const TrackArgs& a, const unsig
 // Ended histories wait until kRefillMin lanes of the warp are idle; then their final states and
 // census sums are stored and the lanes refilled in one go, so this part runs once per kRefillMin
 // endings instead of whenever any lane ends (at about 8 segments per history, nearly every
-// event): the same ten launches 14.5 ms at 1, 13.2 at 4, 12.6 at 8, 12.6 at 12.
+// event): the same ten launches 14.5 ms at 1, 13.2 at 4, 12.6 at 8, 12.6 at 12; with the flights as
+// they are now 11.9, 10.8, 10.2 (and 10.3 at 16).  Eight launches of a multigroup slab, a million
+// particles each: 5.9, 5.5, 5.4 (5.8 at 16); four of a sphere, a million each: 9.0, 8.9, 9.3 (10.4);
+// slabs of 4 thousand to 4 million, banks of 20 thousand and larger meshes: within 1 % from 1 to 16.
 constexpr int kRefillMin = 8;
 constexpr int kWideThreads = 1024;
 //   T_LONG    as T_GLOBAL, on a mesh so long that its edges (8 bytes a cell) in shared memory would leave
@@ -358,8 +361,10 @@ __global__ void __launch_bounds__(wide_block(TALLY) ? kWideThreads : 256, wide_b
   WarpStage* st = stages + (threadIdx.x >> 5);
   const uint32_t n = (uint32_t)*a.n_dev;
 
-  // T_SMALL: events between two looks at the idle lanes (long histories; 1 in the checked build,
-  // which looks at every history before every event)
+  // T_SMALL: events between two looks at the idle lanes (1 in the checked build, which looks at every
+  // history before every event).  Tracking with 1, these, and twice as many: twenty steps of a 4k slab
+  // 4.08, 3.90, 3.84 ms, 40k 6.77, 6.59, 6.53, three of a 4M slab (short histories) 1.34, 1.43, 1.65;
+  // eight of a 1M multigroup slab 5.70, 5.42, 5.28; five of a 1M 40 x 40 mesh 1.76, 1.68, 1.71.
 #ifdef IMC_CHECKED
   constexpr int kEvents = 1;
 #else
