@@ -302,6 +302,7 @@ __device__ __forceinline__ void census_wsum(const SourceJobs& j, int blk, int nb
   for (long long k = t0; k < n; k += stride) s += (double)j.census_w[k];
   for (int v = 0; v < j.n_vol; ++v) {
     const FillArgs& a = j.vol[v];
+    if (*a.d_n <= 0) continue;  // no plan was made (a fixed source of zeros): its tables hold anything
     for (long long o = t0; o < a.nbins; o += stride) {
       const long long cnt = a.off[o + 1] - a.off[o];
       if (cnt <= 0) continue;
